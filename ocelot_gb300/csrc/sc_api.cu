@@ -109,8 +109,8 @@ Layout make_layout(const Plan& p, int64_t n) {
     L.tw_x = take(cs * p.Mx);
     L.tw_y = take(cs * p.My);
     L.tw_z = take(cs * p.Mz);
-    L.part_frame = take(8 * 3 * (size_t)p.part_blocks);
-    L.part_ext = take(8 * 11 * (size_t)p.part_blocks);
+    L.part_frame = take(8 * PART_FRAME_DOUBLES * (size_t)p.part_blocks);
+    L.part_ext = take(8 * PART_EXT_DOUBLES * (size_t)p.part_blocks);
     // n-independent regions first: the Green's-function cache keeps its
     // offset when the same workspace serves kicks of different n
     L.qgrid = take(rs * ncell);
@@ -619,7 +619,7 @@ int sc_kick(sc_plan* plan, void* ws_v, size_t ws_bytes, double* rp, int64_t ld, 
     const int passes = sort_passes(p.key_bits);
     cudaStream_t side = plan->side;
     mark(plan, 0, s);
-    SC_CUDA(launch_frame(p, L, ws, kp, rp, s), "frame");
+    SC_CUDA(launch_frame(p, L, ws, kp, rp, q, s), "frame");
     mark(plan, 1, s);
     SC_CUDA(launch_extent(p, L, ws, kp, rp, q, s), "extent");
     mark(plan, 2, s);
@@ -937,7 +937,6 @@ int sc_batch_set(sc_batch* b, const sc_beam* beams, int nbeams, void* stream) {
         B.kp = make_params(p, m.n, m.ld, m.energy_gev, m.zstep, m.mesh_scale, m.mesh_shift);
         B.L = make_layout(p, m.n);
         const bool rp_ok = ((uintptr_t)m.rparticles % 16 == 0) && (m.ld % 2 == 0);
-        B.vec_rp = rp_ok;
         B.vec_rpq = rp_ok && ((uintptr_t)m.q % 16 == 0);
         size_t fs[3], gs[3];
         batch_fft_tiling(B, fs);

@@ -53,6 +53,7 @@ struct ScState {
     float phi_scalef;            // (float)(phi_norm / phi_denom): the FP32 form's potential scale
     // Green's-function cache: spacing of the spectrum held in the workspace
     double igf_h[3];
+    double qmom[5];              // charge x lab position (3), charge, |charge|: the frame pass's sums
     // FP32 copies of the per-kick constants, written once by the finalizes
     float Tf[3][3];
     float g0f, ig0f, kxyf, kzf;
@@ -177,6 +178,9 @@ struct Layout {
     size_t total;
 };
 
+// doubles per block of the frame's and the extent's partial results (sc_particles.cu)
+constexpr int PART_FRAME_DOUBLES = 8, PART_EXT_DOUBLES = 18;
+
 struct Plan {
     int nx, ny, nz, prec;
     bool sorted_deposit;  // FP64 always; FP32 with SC_FP32_SORTED_DEPOSIT
@@ -208,7 +212,7 @@ cudaError_t launch_init_workspace(const Plan& p, const Layout& L, char* ws, cuda
 
 // per-particle stages (sc_particles.cu)
 cudaError_t launch_frame(const Plan& p, const Layout& L, char* ws, const KickParams& kp,
-                         const double* rp, cudaStream_t s);
+                         const double* rp, const double* q, cudaStream_t s);
 cudaError_t launch_extent(const Plan& p, const Layout& L, char* ws, const KickParams& kp,
                           const double* rp, const double* q, cudaStream_t s);
 // rp: the particles (exact recomputation of near-face keys in the FP32 form), or nullptr
@@ -313,7 +317,7 @@ struct BatchBeam {
     KickParams kp;
     Layout L;
     Plan p;
-    int vec_rp, vec_rpq;              // 16-byte row accesses allowed: rparticles / rparticles and q
+    int vec_rpq;                      // 16-byte accesses of rparticles and q allowed
     int has_tm;                       // a transport map to apply before the kick (sc_tmap_batched)
     double tm[42];                    // R (row-major), then B
     int fft_nc, fft_tky, fft_tkx;     // convolution tiling

@@ -205,7 +205,10 @@ __device__ __forceinline__ void block_minmax_f(float (&v)[NV], float (&sm)[SZ]) 
     __syncthreads();
 }
 
-constexpr int PART_EXT = 11;
+constexpr int PART_EXT = 11;                 // doubles per block: the el_field entry's extent
+constexpr int FRAME_PART = PART_FRAME_DOUBLES;  // doubles per block: sums of the frame pass
+constexpr int EXT_PART = PART_EXT_DOUBLES;      // doubles per block: extent partials (ExtPart)
+static_assert(PART_EXT <= EXT_PART, "one region holds either");
 
 // ---------------------------------------------------------------------------
 // FP64 transforms in the reference's operation order
@@ -484,29 +487,32 @@ __device__ __forceinline__ void st_rows(double* __restrict__ row, int64_t i, boo
 // few particles after it (the end of the beam) are read directly.
 // ---------------------------------------------------------------------------
 constexpr int PT_TILE = 2 * PT;
-constexpr int FR_STAGES = 4;  // tile buffers of the frame kernel (12 KB each)
-constexpr int EX_STAGES = 2;  // tile buffers of the extent kernel (28 KB each)
+constexpr int FR_STAGES = 2;  // tile buffers of the frame kernel (28 KB each)
+constexpr int EX_TILE = 4 * PT;  // particles per tile of the extent kernel (four per thread, FP32 rows)
+constexpr int EX_STAGES = 3;  // its tile buffers (12 KB each)
 
-struct BlockTiles {
+template <int TILE>
+struct BlockTilesOf {
     int64_t n, first, stride, mine;
-    __device__ BlockTiles(int64_t n_, VBlk vb) : n(n_), first(vb.x), stride(vb.nx) {
-        const int64_t nt = (n + PT_TILE - 1) / PT_TILE;
+    __device__ BlockTilesOf(int64_t n_, VBlk vb) : n(n_), first(vb.x), stride(vb.nx) {
+        const int64_t nt = (n + TILE - 1) / TILE;
         mine = first < nt ? (nt - 1 - first) / stride + 1 : 0;
     }
-    __device__ int64_t start(int64_t t) const { return (first + t * stride) * PT_TILE; }
+    __device__ int64_t start(int64_t t) const { return (first + t * stride) * TILE; }
     __device__ int count(int64_t t) const {
         const int64_t c = n - start(t);
-        return (int)(c < PT_TILE ? c : PT_TILE);
+        return (int)(c < TILE ? c : TILE);
     }
 };
+using BlockTiles = BlockTilesOf<PT_TILE>;
 
 // Runs body(t, stage) for each of the block's tiles once its rows have
 // landed in tile buffer `stage`; issue(t, stage, bar) (thread 0) starts the
 // loads of local tile t.  Every thread of the block must call it; body must
 // not synchronise the block.  Returns false if a wait gave up after `limit`
 // tries, after waiting (with the full limit) for the loads still in flight.
-template <int STAGES, typename Issue, typename Body>
-__device__ __forceinline__ bool stream_tiles(const BlockTiles& T, uint64_t* bar, unsigned limit, Issue&& issue,
+template <int STAGES, typename Tiles, typename Issue, typename Body>
+__device__ __forceinline__ bool stream_tiles(const Tiles& T, uint64_t* bar, unsigned limit, Issue&& issue,
                                              Body&& body) {
     const bool lead = threadIdx.x == 0;
     if (lead) {
@@ -539,9 +545,10 @@ __device__ __forceinline__ bool stream_tiles(const BlockTiles& T, uint64_t* bar,
 }
 
 // shared memory of the streamed kernels: the tile buffers, then the barriers
-constexpr size_t FR_SMEM = (size_t)FR_STAGES * 3 * PT_TILE * sizeof(double) + FR_STAGES * sizeof(uint64_t);
-constexpr size_t EX_SMEM = (size_t)EX_STAGES * 7 * PT_TILE * sizeof(double) + EX_STAGES * sizeof(uint64_t);
-static_assert(3 * (EX_SMEM + 1024 + 5 * 1024) <= 228 * 1024, "three extent blocks must fit an SM");
+constexpr size_t FR_SMEM = (size_t)FR_STAGES * 7 * PT_TILE * sizeof(double) + FR_STAGES * sizeof(uint64_t);
+constexpr size_t EX_BUF = (size_t)EX_STAGES * 3 * EX_TILE * sizeof(float);
+constexpr size_t EX_SMEM = EX_BUF + EX_STAGES * sizeof(uint64_t);
+static_assert(3 * (FR_SMEM + 1024 + 5 * 1024) <= 228 * 1024, "three frame blocks must fit an SM");
 
 // ---------------------------------------------------------------------------
 // last-block reductions: every block writes its partials, the last block to
@@ -647,11 +654,14 @@ __device__ void frame_finalize(const double* part, int nblk, const KickParams& k
 }
 
 
-// FP32 form: per-block momentum sums as double-float pairs (hi[3], lo[3]),
-// reduced on the FP32 pipes
+// FP32 form: a block's sums of the frame pass as double-float pairs: the
+// momenta (0..2), charge times lab position (3..5), charge (6), |charge| (7).
+// The finalize of the frame reduces the momenta on the FP32 pipes; the charge
+// moments wait for the extent pass (extent_body), off the frame's chain.
 struct FramePart32 {
-    float hi[3], lo[3];
+    float hi[8], lo[8];
 };
+static_assert(sizeof(FramePart32) == FRAME_PART * sizeof(double), "a block's slot of frame partials");
 __device__ void frame_finalize32(const FramePart32* part, int nblk, const KickParams& kp, ScState* st) {
     __shared__ float sm[3 * 64];
     float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
@@ -790,36 +800,6 @@ __device__ void mesh_finalize(const double* part, int nblk, const KickParams& kp
     mesh_finish(mn, mx, qs, kp, st, gamma_override, lab_sums);
 }
 
-// FP32 form: per-block extremes as ord64 keys (integer min/max) and the
-// charge moments of the lab positions as double-float pairs
-struct ExtPart32 {
-    unsigned long long mn[3], mx[3];
-    float hi[5], lo[5];
-};
-static_assert(sizeof(ExtPart32) <= PART_EXT * sizeof(double), "ExtPart32 must fit a block's partial slot");
-__device__ void mesh_finalize32(const ExtPart32* part, int nblk, const KickParams& kp, ScState* st) {
-    __shared__ unsigned long long smu[3 * 32];
-    __shared__ float smf[5 * 64];
-    unsigned long long mn[3] = {~0ull, ~0ull, ~0ull}, mx[3] = {0ull, 0ull, 0ull};
-    float hi[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, lo[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
-        for (int k = 0; k < 3; ++k) {
-            const unsigned long long a = __ldcg(&part[b].mn[k]), c = __ldcg(&part[b].mx[k]);
-            mn[k] = a < mn[k] ? a : mn[k];
-            mx[k] = c > mx[k] ? c : mx[k];
-        }
-        for (int k = 0; k < 5; ++k) df_add(hi[k], lo[k], __ldcg(&part[b].hi[k]), __ldcg(&part[b].lo[k]));
-    }
-    block_minmax_u64<3, false>(mn, smu);
-    block_minmax_u64<3, true>(mx, smu);
-    block_sum_df<5>(hi, lo, smf);
-    const double dmn[3] = {unord64(mn[0]), unord64(mn[1]), unord64(mn[2])};
-    const double dmx[3] = {unord64(mx[0]), unord64(mx[1]), unord64(mx[2])};
-    double qs[5];
-    for (int k = 0; k < 5; ++k) qs[k] = (double)hi[k] + (double)lo[k];
-    mesh_finish(dmn, dmx, qs, kp, st, -1.0, true);
-}
-
 // ---------------------------------------------------------------------------
 // frame: sum of momenta (+ FP64: lab coordinates stored for later stages)
 // ---------------------------------------------------------------------------
@@ -889,124 +869,147 @@ __device__ __forceinline__ void st_rowf(float* __restrict__ row, int64_t i, bool
     else row[i] = a;
 }
 
-// qzero != nullptr (batched kicks): the beam's blocks also clear its
-// fixed-point charge grid of nzero cells for the deposit of this kick
+// FP32 frame pass: one read of the particles gives the momentum sums of the
+// mean-velocity frame and, because neither needs that frame, the lab positions
+// (stored in FP32, 12 bytes a particle, for the extent and keys passes) and
+// their charge moments.  The extent pass used to read all seven rows again for
+// them: frame + extent 19 + 52 us per 2M particles with the rows read twice.
+struct FrameSums32 {
+    float p[3] = {0.f, 0.f, 0.f};              // momenta
+    float m[5] = {0.f, 0.f, 0.f, 0.f, 0.f};    // charge x lab position, charge, |charge|
+    // f: the six coordinates and the charge rounded to FP32; returns the lab position
+    __device__ __forceinline__ void add(const float (&f)[7], const KickParams& kp, float (&l)[3]) {
+        float px, py, pz, E;
+        mom32(f[1], f[3], f[5], kp, px, py, pz, E);
+        p[0] += px;
+        p[1] += py;
+        p[2] += pz;
+        lab32(f[0], f[2], f[4], px, py, pz, E, kp, l);
+        const float qi = f[6];
+        for (int j = 0; j < 3; ++j) m[j] = fmaf(qi, l[j], m[j]);
+        m[3] += qi;
+        m[4] += fabsf(qi);
+    }
+    // the block's sums into its slot; the last block forms the frame
+    __device__ __forceinline__ void out(FramePart32* part, const KickParams& kp, ScState* st, VBlk vb) {
+        __shared__ float sm[8 * 64];
+        const float v[8] = {p[0], p[1], p[2], m[0], m[1], m[2], m[3], m[4]};
+        float hi[8], lo[8];
+        block_sum_f2<8>(v, hi, lo, sm);
+        if (threadIdx.x == 0)
+            for (int k = 0; k < 8; ++k) {
+                part[vb.x].hi[k] = hi[k];
+                part[vb.x].lo[k] = lo[k];
+            }
+        if (arrive_last(&st->done_frame, vb.nx)) frame_finalize32(part, vb.nx, kp, st);
+    }
+};
+
+// qzero != nullptr: the beam's blocks also clear its fixed-point charge grid
+// of nzero cells for the deposit of this kick
 template <bool VEC>
-__device__ __forceinline__ void frame32_body(const double* __restrict__ rp, const KickParams& kp,
-                                             double* __restrict__ part, ScState* st,
-                                             unsigned long long* __restrict__ qzero, int64_t nzero, VBlk vb) {
-    __shared__ float smf[3 * 64];
+__device__ __forceinline__ void frame32_body(const double* __restrict__ rp, const double* __restrict__ q,
+                                             const KickParams& kp, float* __restrict__ X, double* __restrict__ part,
+                                             ScState* st, unsigned long long* __restrict__ qzero, int64_t nzero,
+                                             VBlk vb) {
     if (qzero)
         for (int64_t i = vb.x * (int64_t)blockDim.x + threadIdx.x; i < nzero; i += (int64_t)vb.nx * blockDim.x)
             qzero[i] = 0ull;
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-    const int64_t n = kp.n, ld = kp.ld;
+    FrameSums32 S;
+    const int64_t n = kp.n, ld = kp.ld, nX = kp.nX;
     PAIR_LOOP_BEGIN(n)
-    double xq[2], yq[2], d[2];
-    ld_row(rp + ld, i0_, pair_, xq[0], xq[1]);
-    ld_row(rp + 3 * ld, i0_, pair_, yq[0], yq[1]);
-    ld_row(rp + 5 * ld, i0_, pair_, d[0], d[1]);
-    for (int w = 0; w < W_; ++w) {
-        float px, py, pz, E;
-        mom32(d2f(xq[w]), d2f(yq[w]), d2f(d[w]), kp, px, py, pz, E);
-        a0 += px;
-        a1 += py;
-        a2 += pz;
+    float f[2][7], l[2][3];
+    for (int k = 0; k < 7; ++k) {
+        double a, b;
+        ld_row(k < 6 ? rp + k * ld : q, i0_, pair_, a, b);
+        f[0][k] = d2f(a);
+        f[1][k] = d2f(b);
     }
+    for (int w = 0; w < W_; ++w) S.add(f[w], kp, l[w]);
+    for (int j = 0; j < 3; ++j) st_rowf(X + j * nX, i0_, pair_, l[0][j], l[1][j]);
     PAIR_LOOP_END
-    const float a[3] = {a0, a1, a2};
-    float hi[3], lo[3];
-    block_sum_f2<3>(a, hi, lo, smf);
-    FramePart32* fp = reinterpret_cast<FramePart32*>(part);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 3; ++k) {
-            fp[vb.x].hi[k] = hi[k];
-            fp[vb.x].lo[k] = lo[k];
-        }
-    if (arrive_last(&st->done_frame, vb.nx)) frame_finalize32(fp, vb.nx, kp, st);
+    S.out(reinterpret_cast<FramePart32*>(part), kp, st, vb);
 }
 
-// qzero != nullptr: also zeroes the nzero cells of the fixed-point charge
-// grid for this kick's deposit
 template <bool VEC>
-__global__ void __launch_bounds__(PT, 4) k_frame32(const double* __restrict__ rp, KickParams kp,
-                                                   double* __restrict__ part, ScState* st,
-                                                   unsigned long long* __restrict__ qzero, int64_t nzero) {
+__global__ void __launch_bounds__(PT, 3) k_frame32(const double* __restrict__ rp, const double* __restrict__ q,
+                                                   KickParams kp, float* __restrict__ X, double* __restrict__ part,
+                                                   ScState* st, unsigned long long* __restrict__ qzero,
+                                                   int64_t nzero) {
     pdl_wait();
-    frame32_body<VEC>(rp, kp, part, st, qzero, nzero, hw_vblk());
+    frame32_body<VEC>(rp, q, kp, X, part, st, qzero, nzero, hw_vblk());
 }
 
-// frame32_body with the rows x', y', delta streamed through shared memory
-// (rows 16-byte aligned, even stride)
-__device__ __forceinline__ void frame32_tma_body(const double* __restrict__ rp, const KickParams& kp,
+// frame32_body with the six rows and the charges streamed through shared
+// memory (rows and q 16-byte aligned, even stride)
+__device__ __forceinline__ void frame32_tma_body(const double* __restrict__ rp, const double* __restrict__ q,
+                                                 const KickParams& kp, float* __restrict__ X,
                                                  double* __restrict__ part, ScState* st,
                                                  unsigned long long* __restrict__ qzero, int64_t nzero, VBlk vb) {
     extern __shared__ __align__(128) unsigned char smraw[];
-    __shared__ float smf[3 * 64];
-    double* buf = reinterpret_cast<double*>(smraw);  // [FR_STAGES][3][PT_TILE]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(buf + FR_STAGES * 3 * PT_TILE);
+    double* buf = reinterpret_cast<double*>(smraw);  // [FR_STAGES][7][PT_TILE]
+    uint64_t* bar = reinterpret_cast<uint64_t*>(buf + FR_STAGES * 7 * PT_TILE);
     if (qzero)
         for (int64_t i = vb.x * (int64_t)blockDim.x + threadIdx.x; i < nzero; i += (int64_t)vb.nx * blockDim.x)
             qzero[i] = 0ull;
-    const int64_t n = kp.n, ld = kp.ld;
-    const BlockTiles T(n, vb);
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-    auto addf = [&](float xq, float yq, float d) {
-        float px, py, pz, E;
-        mom32(xq, yq, d, kp, px, py, pz, E);
-        a0 += px;
-        a1 += py;
-        a2 += pz;
-    };
-    auto add = [&](double xq, double yq, double d) { addf(d2f(xq), d2f(yq), d2f(d)); };
+    const int64_t n = kp.n, ld = kp.ld, nX = kp.nX;
+    const BlockTiles Tl(n, vb);
+    FrameSums32 S;
     auto issue = [&](int64_t t, int s, uint64_t* b) {
-        const int64_t i0 = T.start(t);
-        const unsigned bytes = (unsigned)(T.count(t) & ~1) * 8u;
-        mbar_arrive_expect_tx(b, 3u * bytes);
-        if (bytes)
-            for (int r = 0; r < 3; ++r) bulk_load(buf + (s * 3 + r) * PT_TILE, rp + (2 * r + 1) * ld + i0, bytes, b);
+        const int64_t i0 = Tl.start(t);
+        const unsigned bytes = (unsigned)(Tl.count(t) & ~1) * 8u;
+        mbar_arrive_expect_tx(b, 7u * bytes);
+        if (bytes) {
+            for (int k = 0; k < 6; ++k) bulk_load(buf + (s * 7 + k) * PT_TILE, rp + k * ld + i0, bytes, b);
+            bulk_load(buf + (s * 7 + 6) * PT_TILE, q + i0, bytes, b);
+        }
     };
     auto body = [&](int64_t t, int s) {
-        const int cnt = T.count(t), staged = cnt & ~1, j = 2 * threadIdx.x;
-        const double* B = buf + s * 3 * PT_TILE;
+        const int cnt = Tl.count(t), staged = cnt & ~1, j = 2 * threadIdx.x;
+        const int64_t i0 = Tl.start(t);
+        const double* B = buf + s * 7 * PT_TILE;
         if (j + 1 < staged) {
-            const double2 x = *reinterpret_cast<const double2*>(B + j);
-            const double2 y = *reinterpret_cast<const double2*>(B + PT_TILE + j);
-            const double2 d = *reinterpret_cast<const double2*>(B + 2 * PT_TILE + j);
-            unsigned rg = 0u;  // one range check for both particles (d2f_nr)
-            const float f[6] = {d2f_nr(x.x, rg), d2f_nr(y.x, rg), d2f_nr(d.x, rg),
-                                d2f_nr(x.y, rg), d2f_nr(y.y, rg), d2f_nr(d.y, rg)};
-            if (d2f_range_ok(rg)) {
-                addf(f[0], f[1], f[2]);
-                addf(f[3], f[4], f[5]);
-            } else {
-                add(x.x, y.x, d.x);
-                add(x.y, y.y, d.y);
+            double r0[7], r1[7];
+            for (int k = 0; k < 7; ++k) {
+                const double2 v = *reinterpret_cast<const double2*>(B + k * PT_TILE + j);
+                r0[k] = v.x;
+                r1[k] = v.y;
             }
+            float f0[7], f1[7];
+            unsigned rg = 0u;  // one range check for both particles (d2f_nr)
+            for (int k = 0; k < 7; ++k) {
+                f0[k] = d2f_nr(r0[k], rg);
+                f1[k] = d2f_nr(r1[k], rg);
+            }
+            if (!d2f_range_ok(rg))
+                for (int k = 0; k < 7; ++k) {
+                    f0[k] = d2f_edge(r0[k]);
+                    f1[k] = d2f_edge(r1[k]);
+                }
+            float l0[3], l1[3];
+            S.add(f0, kp, l0);
+            S.add(f1, kp, l1);
+            for (int k = 0; k < 3; ++k) *reinterpret_cast<float2*>(X + k * nX + i0 + j) = make_float2(l0[k], l1[k]);
         } else if (j < cnt) {
-            const int64_t i = T.start(t) + j;
-            add(rp[ld + i], rp[3 * ld + i], rp[5 * ld + i]);
+            const int64_t i = i0 + j;
+            float f[7], l[3];
+            for (int k = 0; k < 6; ++k) f[k] = d2f(rp[k * ld + i]);
+            f[6] = d2f(q[i]);
+            S.add(f, kp, l);
+            for (int k = 0; k < 3; ++k) X[k * nX + i] = l[k];
         }
     };
-    if (!stream_tiles<FR_STAGES>(T, bar, kp.wait_limit[0], issue, body) && threadIdx.x == 0)
+    if (!stream_tiles<FR_STAGES>(Tl, bar, kp.wait_limit[0], issue, body) && threadIdx.x == 0)
         atomicExch(&st->frame_timeout, 1);
-    const float a[3] = {a0, a1, a2};
-    float hi[3], lo[3];
-    block_sum_f2<3>(a, hi, lo, smf);
-    FramePart32* fp = reinterpret_cast<FramePart32*>(part);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 3; ++k) {
-            fp[vb.x].hi[k] = hi[k];
-            fp[vb.x].lo[k] = lo[k];
-        }
-    if (arrive_last(&st->done_frame, vb.nx)) frame_finalize32(fp, vb.nx, kp, st);
+    S.out(reinterpret_cast<FramePart32*>(part), kp, st, vb);
 }
 
-__global__ void __launch_bounds__(PT, 4) k_frame32_tma(const double* __restrict__ rp, KickParams kp,
+__global__ void __launch_bounds__(PT, 3) k_frame32_tma(const double* __restrict__ rp, const double* __restrict__ q,
+                                                       KickParams kp, float* __restrict__ X,
                                                        double* __restrict__ part, ScState* st,
                                                        unsigned long long* __restrict__ qzero, int64_t nzero) {
     pdl_wait();
-    frame32_tma_body(rp, kp, part, st, qzero, nzero, hw_vblk());
+    frame32_tma_body(rp, q, kp, X, part, st, qzero, nzero, hw_vblk());
 }
 
 // ---------------------------------------------------------------------------
@@ -1113,310 +1116,258 @@ __device__ __forceinline__ void xyz_fine32(const double* __restrict__ rp, int64_
 }
 
 
-// FP32 extent.  Pass 1 computes the rotated positions in FP32, stores them and
-// reduces FP32 extremes and charge moments.  Pass 2 re-walks the block's
-// particles and evaluates in FP64 (xyz_fine) every particle whose
-// FP32 coordinate lies within a rounding margin of the block's FP32 extreme:
-// the FP64 extreme of the block is among them, so the mesh step equals the
-// FP64 form's.
-template <bool VEC>
-__device__ __forceinline__ void extent32_body(const double* __restrict__ rp, const double* __restrict__ q,
-                                              const KickParams& kp, float* __restrict__ X, double* __restrict__ part,
-                                              ScState* st, VBlk vb) {
-    __shared__ float smq[5 * 64];
-    __shared__ float smf[3 * 32];
-    __shared__ float bmin[3], bmax[3];
-    __shared__ unsigned long long emin[3], emax[3];
-    float mnf[3] = {INFINITY, INFINITY, INFINITY}, mxf[3] = {-INFINITY, -INFINITY, -INFINITY};
-    float qsf[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-    const int64_t n = kp.n, ld = kp.ld, nX = kp.nX;
-    const bool ok = st->status == SC_OK;
-    float T[3][3];
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) T[i][j] = st->Tf[i][j];
-    const float g0 = st->g0f;
-    if (ok) {
-        PAIR_LOOP_BEGIN(n)
-        float r[6][2], qq[2];
-        for (int k = 0; k < 6; ++k) {
-            double a, b;
-            ld_row(rp + k * ld, i0_, pair_, a, b);
-            r[k][0] = d2f(a);
-            r[k][1] = d2f(b);
-        }
-        {
-            double a, b;
-            ld_row(q, i0_, pair_, a, b);
-            qq[0] = d2f(a);
-            qq[1] = d2f(b);
-        }
-        float v[3][2];
-        for (int w = 0; w < W_; ++w) {
-            float px, py, pz, E;
-            mom32(r[1][w], r[3][w], r[5][w], kp, px, py, pz, E);
-            float lw[3], vw[3];
-            lab32(r[0][w], r[2][w], r[4][w], px, py, pz, E, kp, lw);
-            rot32(lw, T, g0, vw);
-            for (int j = 0; j < 3; ++j) v[j][w] = vw[j];
-            const float qi = qq[w];
-            for (int j = 0; j < 3; ++j) {  // charge moments of the lab positions
-                mnf[j] = fminf(mnf[j], v[j][w]);
-                mxf[j] = fmaxf(mxf[j], v[j][w]);
-                qsf[j] = fmaf(qi, lw[j], qsf[j]);
-            }
-            qsf[3] += qi;
-            qsf[4] += fabsf(qi);
-        }
-        for (int j = 0; j < 3; ++j) st_rowf(X + j * nX, i0_, pair_, v[j][0], v[j][1]);
-        PAIR_LOOP_END
+// order-preserving map of a float onto int (its own inverse)
+__device__ __forceinline__ int ord32(int i) { return i ^ ((i >> 31) & 0x7fffffff); }
+// block minima and maxima of three floats; every thread receives them
+__device__ __forceinline__ void block_extremes(float (&mn)[3], float (&mx)[3], int (&sm)[6 * 32]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int v[6];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        v[c] = __reduce_min_sync(FULL, ord32(__float_as_int(mn[c])));
+        v[3 + c] = __reduce_max_sync(FULL, ord32(__float_as_int(mx[c])));
     }
-    // float extremes reduce exactly in float; the sums in double
-    block_minmax_f<3, false>(mnf, smf);
-    block_minmax_f<3, true>(mxf, smf);
-    float qhi[5], qlo[5];
-    block_sum_f2<5>(qsf, qhi, qlo, smq);
-    if (threadIdx.x == 0)
-        for (int j = 0; j < 3; ++j) {
-            bmin[j] = mnf[j];
-            bmax[j] = mxf[j];
-            emin[j] = ord64(INFINITY);
-            emax[j] = ord64(-INFINITY);
-        }
+    if (lane == 0)
+#pragma unroll
+        for (int c = 0; c < 6; ++c) sm[c * 32 + warp] = v[c];
     __syncthreads();
-    float tol[3];
-    for (int j = 0; j < 3; ++j)  // 2^-18 of the coordinate scale: 64x the FP32 rounding bound of v
-        tol[j] = ldexpf(fmaxf(fabsf(bmin[j]), fabsf(bmax[j])) + (bmax[j] - bmin[j]), -18);
-    if (ok) {
-        double Td[3][3];
-        for (int a = 0; a < 3; ++a)
-            for (int b = 0; b < 3; ++b) Td[a][b] = st->T[a][b];
-        const double g0d = st->gamma0;
-        // the same particles as pass 1 (same pair mapping), so the block's FP32
-        // extremes bound them
-        PAIR_LOOP_BEGIN(n)
-        for (int w = 0; w < W_; ++w) {
-            const int64_t i = i0_ + w;
-            bool cand = false;
-            for (int j = 0; j < 3; ++j) {
-                const float v = X[j * nX + i];
-                cand |= (v <= bmin[j] + tol[j]) || (v >= bmax[j] - tol[j]);
-            }
-            if (cand) {
-                double v[3];
-                xyz_fine(rp, ld, i, kp, Td, g0d, v);
-                for (int j = 0; j < 3; ++j) {
-                    if (X[j * nX + i] <= bmin[j] + tol[j]) atomicMin(&emin[j], ord64(v[j]));
-                    if (X[j * nX + i] >= bmax[j] - tol[j]) atomicMax(&emax[j], ord64(v[j]));
-                }
-            }
-        }
-        PAIR_LOOP_END
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const int lo = lane < nw ? sm[c * 32 + lane] : 0x7fffffff;
+        const int hi = lane < nw ? sm[(3 + c) * 32 + lane] : (int)0x80000000;
+        mn[c] = __int_as_float(ord32(__reduce_min_sync(FULL, lo)));
+        mx[c] = __int_as_float(ord32(__reduce_max_sync(FULL, hi)));
     }
     __syncthreads();
-    ExtPart32* ep = reinterpret_cast<ExtPart32*>(part);
-    if (threadIdx.x == 0 && SC_IDX_OK(st, 12, vb.x, kp.n > 0 ? vb.nx : 0)) {
-        for (int k = 0; k < 3; ++k) {
-            ep[vb.x].mn[k] = emin[k];
-            ep[vb.x].mx[k] = emax[k];
-        }
-        for (int k = 0; k < 5; ++k) {
-            ep[vb.x].hi[k] = qhi[k];
-            ep[vb.x].lo[k] = qlo[k];
-        }
+}
+// Margin of an FP32 rotated coordinate around an extreme of axis j: 2^-18 of
+// the axis's scale (64x the FP32 rounding of a coordinate) plus 2^-20 of the
+// lab position's length, from which the rotation of a tilted beam may cancel.
+// 1e-36 keeps the margin positive where the scale underflows.
+__device__ __forceinline__ void extent_margin(const float (&mn)[3], const float (&mx)[3], float g0, float ig0,
+                                              float (&tol)[3]) {
+    float M[3];
+    for (int j = 0; j < 3; ++j) M[j] = fmaxf(fabsf(mn[j]), fabsf(mx[j]));
+    const float len = M[0] + M[1] + M[2] * ig0;
+    for (int j = 0; j < 3; ++j)
+        tol[j] = ldexpf(M[j] + (mx[j] - mn[j]), -18) + ldexpf(j == 2 ? len * g0 : len, -20) + 1e-36f;
+}
+// the extremes a coordinate triple may be (bits 0..2 min x, y, z; 3..5 max);
+// written so that a NaN counts as a candidate
+__device__ __forceinline__ unsigned extent_sides(const float (&v)[3], const float (&mn)[3], const float (&mx)[3],
+                                                 const float (&tol)[3]) {
+    unsigned sd = 0u;
+    for (int j = 0; j < 3; ++j) {
+        if (!(v[j] > mn[j] + tol[j])) sd |= 1u << j;
+        if (!(v[j] < mx[j] - tol[j])) sd |= 8u << j;
     }
-    if (arrive_last(&st->done_extent, vb.nx)) mesh_finalize32(ep, vb.nx, kp, st);
+    return sd;
 }
 
-template <bool VEC>
-__global__ void __launch_bounds__(PT, 4) k_extent32(const double* __restrict__ rp, const double* __restrict__ q,
-                                                    KickParams kp, float* __restrict__ X, double* __restrict__ part,
-                                                    ScState* st) {
-    pdl_wait();
-    extent32_body<VEC>(rp, q, kp, X, part, st, hw_vblk());
-}
+__device__ __forceinline__ float f4(const float4& v, int w) { return w == 0 ? v.x : w == 1 ? v.y : w == 2 ? v.z : v.w; }
 
-constexpr int EX_SCAN = 4;  // tiles whose coordinates a pass-2 thread loads before checking them
+// A block's part of the extent: its FP32 extremes and the particles within the
+// margin of them (up to EX_CAND, else the block has evaluated its own: emn,
+// emx as ord64 keys).
+constexpr int EX_CAND = 16;
+struct ExtPart {
+    float mn[3], mx[3];
+    int count, exact;
+    unsigned long long emn[3], emx[3];
+    uint32_t cand[EX_CAND];
+};
+static_assert(sizeof(ExtPart) == EXT_PART * sizeof(double), "a block's slot of extent partials");
+constexpr int EX_BLOCKS = (int)(EX_BUF / (EX_CAND * sizeof(uint32_t)));  // blocks whose lists fit the tile buffers
 
-// extent32_body with the six rows and the charges streamed through shared
-// memory (rows and q 16-byte aligned, even stride).  Pass 2 is walked only
-// by the threads whose own FP32 extreme lies within the margin of the
-// block's: a particle of any other thread is farther from the block's
-// extreme than that thread's extreme, so the candidates are the same.  Each
-// such thread loads the coordinates of EX_SCAN tiles before it checks them,
-// one round trip per EX_SCAN tiles instead of one per tile.
-__device__ __forceinline__ void extent32_tma_body(const double* __restrict__ rp, const double* __restrict__ q,
-                                                  const KickParams& kp, float* __restrict__ X,
-                                                  double* __restrict__ part, ScState* st, VBlk vb) {
+// Extent of the rotated positions.  The FP32 positions (rot32 of the lab
+// positions the frame pass stored, 12 bytes a particle) give each block's
+// extremes; the mesh step must equal the FP64 form's, so the particles within
+// the FP32 margin of an extreme are evaluated with the FP64 form's operations
+// (xyz_fine).  On this GPU's narrow FP64 pipe one such evaluation is several
+// microseconds of dependent arithmetic, and every block evaluating its own
+// half a dozen candidates took about 20 us whatever N: so a block only lists
+// them, and the last block evaluates, one per thread, those that are still
+// candidates for the extremes of all blocks.  A block with more than EX_CAND
+// (many particles sharing an extreme coordinate) evaluates its own, so that
+// the last block's share stays bounded.  2M / 64^3, frame + extent: 71 -> 58 us.
+// Block 0 reduces the charge moments of the frame pass meanwhile (F64: FP64
+// sums, else double-float pairs).  nX rows of X; all waits bounded.
+template <bool F64>
+__device__ __forceinline__ void extent_body(const double* __restrict__ rp, const float* __restrict__ X,
+                                            const double* __restrict__ fpart, const KickParams& kp,
+                                            ExtPart* __restrict__ ep, ScState* st, VBlk vb) {
     extern __shared__ __align__(128) unsigned char smraw[];
-    __shared__ float smq[5 * 64];
-    __shared__ float smf[3 * 32];
-    __shared__ float bmin[3], bmax[3];
+    __shared__ double smq[5 * 32];
+    __shared__ int smi[6 * 32];
     __shared__ unsigned long long emin[3], emax[3];
-    double* buf = reinterpret_cast<double*>(smraw);  // [EX_STAGES][7][PT_TILE]
-    uint64_t* bar = reinterpret_cast<uint64_t*>(buf + EX_STAGES * 7 * PT_TILE);
-    float mnf[3] = {INFINITY, INFINITY, INFINITY}, mxf[3] = {-INFINITY, -INFINITY, -INFINITY};
-    float qsf[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+    __shared__ uint32_t s_cand[EX_CAND];
+    __shared__ int s_n;
+    float* buf = reinterpret_cast<float*>(smraw);  // [EX_STAGES][3][EX_TILE]
+    uint64_t* bar = reinterpret_cast<uint64_t*>(smraw + EX_BUF);
     const int64_t n = kp.n, ld = kp.ld, nX = kp.nX;
+    if (threadIdx.x < 3) {
+        emin[threadIdx.x] = ord64(INFINITY);
+        emax[threadIdx.x] = ord64(-INFINITY);
+    }
+    if (threadIdx.x == 0) s_n = 0;
     const bool ok = !__syncthreads_or(st->status != SC_OK);
+    if (vb.x == 0 && ok) {
+        static_assert(sizeof(smq) == 5 * 64 * sizeof(float), "the scratch of either sum");
+        float(&smf)[5 * 64] = reinterpret_cast<float(&)[5 * 64]>(smq);
+        float hi[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, lo[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
+        const FramePart32* fp = reinterpret_cast<const FramePart32*>(fpart);
+        for (int b = threadIdx.x; b < vb.nx; b += blockDim.x)
+            for (int k = 0; k < 5; ++k) df_add(hi[k], lo[k], fp[b].hi[3 + k], fp[b].lo[3 + k]);
+        block_sum_df<5>(hi, lo, smf);
+        if (threadIdx.x == 0)
+            for (int k = 0; k < 5; ++k) st->qmom[k] = (double)hi[k] + (double)lo[k];
+    }
     float T[3][3];
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j) T[i][j] = st->Tf[i][j];
-    const float g0 = st->g0f;
-    const BlockTiles Tl(ok ? n : 0, vb);
-    // one particle: rotated position, extremes and charge moments; returns v
-    // f: the six coordinates and the charge rounded to FP32
-    auto one = [&](const float (&f)[7], float (&v)[3]) {
-        float px, py, pz, E;
-        mom32(f[1], f[3], f[5], kp, px, py, pz, E);
-        float l[3];
-        lab32(f[0], f[2], f[4], px, py, pz, E, kp, l);
+    const float g0 = st->g0f, ig0 = st->ig0f;
+    const BlockTilesOf<EX_TILE> Tl(ok ? n : 0, vb);
+    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+    auto rot = [&](int64_t i, float (&v)[3]) {
+        const float l[3] = {X[i], X[nX + i], X[2 * nX + i]};
         rot32(l, T, g0, v);
-        const float qi = f[6];
-        for (int j = 0; j < 3; ++j) {  // charge moments of the lab positions
-            mnf[j] = fminf(mnf[j], v[j]);
-            mxf[j] = fmaxf(mxf[j], v[j]);
-            qsf[j] = fmaf(qi, l[j], qsf[j]);
-        }
-        qsf[3] += qi;
-        qsf[4] += fabsf(qi);
     };
     auto issue = [&](int64_t t, int s, uint64_t* b) {
         const int64_t i0 = Tl.start(t);
-        const unsigned bytes = (unsigned)(Tl.count(t) & ~1) * 8u;
-        mbar_arrive_expect_tx(b, 7u * bytes);
-        if (bytes) {
-            for (int k = 0; k < 6; ++k) bulk_load(buf + (s * 7 + k) * PT_TILE, rp + k * ld + i0, bytes, b);
-            bulk_load(buf + (s * 7 + 6) * PT_TILE, q + i0, bytes, b);
-        }
+        // whole 16-byte groups: a row of X has room for n rounded up to 4
+        const unsigned bytes = (unsigned)((Tl.count(t) + 3) & ~3) * 4u;
+        mbar_arrive_expect_tx(b, 3u * bytes);
+        for (int k = 0; k < 3; ++k) bulk_load(buf + (s * 3 + k) * EX_TILE, X + k * nX + i0, bytes, b);
     };
     auto body = [&](int64_t t, int s) {
-        const int cnt = Tl.count(t), staged = cnt & ~1, j = 2 * threadIdx.x;
-        const int64_t i0 = Tl.start(t);
-        const double* B = buf + s * 7 * PT_TILE;
-        if (j + 1 < staged) {
-            double r0[6], r1[6];
-            for (int k = 0; k < 6; ++k) {
-                const double2 v = *reinterpret_cast<const double2*>(B + k * PT_TILE + j);
-                r0[k] = v.x;
-                r1[k] = v.y;
-            }
-            const double2 qq = *reinterpret_cast<const double2*>(B + 6 * PT_TILE + j);
-            float f0[7], f1[7];
-            unsigned rg = 0u;  // one range check for both particles (d2f_nr)
-            for (int k = 0; k < 6; ++k) {
-                f0[k] = d2f_nr(r0[k], rg);
-                f1[k] = d2f_nr(r1[k], rg);
-            }
-            f0[6] = d2f_nr(qq.x, rg);
-            f1[6] = d2f_nr(qq.y, rg);
-            if (!d2f_range_ok(rg)) {
-                for (int k = 0; k < 6; ++k) {
-                    f0[k] = d2f_edge(r0[k]);
-                    f1[k] = d2f_edge(r1[k]);
-                }
-                f0[6] = d2f_edge(qq.x);
-                f1[6] = d2f_edge(qq.y);
-            }
-            float v0[3], v1[3];
-            one(f0, v0);
-            one(f1, v1);
-            for (int k = 0; k < 3; ++k) *reinterpret_cast<float2*>(X + k * nX + i0 + j) = make_float2(v0[k], v1[k]);
-        } else if (j < cnt) {
-            const int64_t i = i0 + j;
-            float f[7];
-            for (int k = 0; k < 6; ++k) f[k] = d2f(rp[k * ld + i]);
-            f[6] = d2f(q[i]);
+        const int cnt = Tl.count(t), j = 4 * threadIdx.x;
+        const float* B = buf + s * 3 * EX_TILE;
+        float4 r[3];
+        for (int k = 0; k < 3; ++k) r[k] = *reinterpret_cast<const float4*>(B + k * EX_TILE + j);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            if (j + w >= cnt) break;
+            const float l[3] = {f4(r[0], w), f4(r[1], w), f4(r[2], w)};
             float v[3];
-            one(f, v);
-            for (int k = 0; k < 3; ++k) X[k * nX + i] = v[k];
+            rot32(l, T, g0, v);
+            for (int c = 0; c < 3; ++c) {
+                mn[c] = fminf(mn[c], v[c]);
+                mx[c] = fmaxf(mx[c], v[c]);
+            }
         }
     };
     const bool streamed = stream_tiles<EX_STAGES>(Tl, bar, kp.wait_limit[1], issue, body);
     if (!streamed && threadIdx.x == 0) atomicCAS(&st->status, SC_OK, SC_ERR_TIMEOUT);
-    const float my_mn[3] = {mnf[0], mnf[1], mnf[2]}, my_mx[3] = {mxf[0], mxf[1], mxf[2]};
-    // float extremes reduce exactly in float; the sums in double
-    block_minmax_f<3, false>(mnf, smf);
-    block_minmax_f<3, true>(mxf, smf);
-    float qhi[5], qlo[5];
-    block_sum_f2<5>(qsf, qhi, qlo, smq);
-    if (threadIdx.x == 0)
-        for (int j = 0; j < 3; ++j) {
-            bmin[j] = mnf[j];
-            bmax[j] = mxf[j];
-            emin[j] = ord64(INFINITY);
-            emax[j] = ord64(-INFINITY);
-        }
-    __syncthreads();
+    // the block's extremes, and the particles near them: only a thread whose
+    // own extreme is within the margin can hold one
+    const float my_mn[3] = {mn[0], mn[1], mn[2]}, my_mx[3] = {mx[0], mx[1], mx[2]};
+    block_extremes(mn, mx, smi);
     float tol[3];
+    extent_margin(mn, mx, g0, ig0, tol);
     bool mine = false;
-    for (int j = 0; j < 3; ++j) {  // 2^-18 of the coordinate scale: 64x the FP32 rounding bound of v
-        tol[j] = ldexpf(fmaxf(fabsf(bmin[j]), fabsf(bmax[j])) + (bmax[j] - bmin[j]), -18);
-        mine |= (my_mn[j] <= bmin[j] + tol[j]) || (my_mx[j] >= bmax[j] - tol[j]);
-    }
-    if (ok && streamed && mine) {
-        double Td[3][3];
-        for (int a = 0; a < 3; ++a)
-            for (int b = 0; b < 3; ++b) Td[a][b] = st->T[a][b];
-        const double g0d = st->gamma0;
-        for (int64_t t0 = 0; t0 < Tl.mine; t0 += EX_SCAN) {
-            float xv[EX_SCAN][2][3];
-#pragma unroll
-            for (int u = 0; u < EX_SCAN; ++u)
-#pragma unroll
-                for (int w = 0; w < 2; ++w) {
-                    const int64_t t = t0 + u;
-                    const int jj = 2 * threadIdx.x + w;
-                    const bool valid = t < Tl.mine && jj < Tl.count(t);
-                    const int64_t i = valid ? Tl.start(t) + jj : 0;
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) xv[u][w][j] = valid ? X[j * nX + i] : NAN;
-                }
-            // the extremes each particle may be: 6 bits per particle (min x, y, z; max x, y, z)
-            unsigned long long sides = 0;
-#pragma unroll
-            for (int u = 0; u < EX_SCAN; ++u)
-#pragma unroll
-                for (int w = 0; w < 2; ++w)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) {  // NaN (no particle) is no candidate
-                        const int b = 6 * (2 * u + w);
-                        if (xv[u][w][j] <= bmin[j] + tol[j]) sides |= 1ull << (b + j);
-                        if (xv[u][w][j] >= bmax[j] - tol[j]) sides |= 8ull << (b + j);
-                    }
-            while (sides) {
-                const int p = (__ffsll((long long)sides) - 1) / 6;  // first candidate: particle p of the chunk
-                const unsigned sd = (unsigned)(sides >> (6 * p)) & 63u;
-                sides &= ~(63ull << (6 * p));
-                const int64_t i = Tl.start(t0 + p / 2) + 2 * threadIdx.x + (p & 1);
-                double v[3];
-                xyz_fine(rp, ld, i, kp, Td, g0d, v);
-                for (int j = 0; j < 3; ++j) {
-                    if (sd & (1u << j)) atomicMin(&emin[j], ord64(v[j]));
-                    if (sd & (8u << j)) atomicMax(&emax[j], ord64(v[j]));
-                }
+    for (int j = 0; j < 3; ++j) mine |= !(my_mn[j] > mn[j] + tol[j]) || !(my_mx[j] < mx[j] - tol[j]);
+    mine = mine && streamed;
+    auto scan = [&](auto&& f) {  // f(particle, sides) for this thread's candidates
+        for (int64_t t = 0; t < Tl.mine; ++t)
+            for (int w = 0; w < 4; ++w) {
+                const int j = 4 * threadIdx.x + w;
+                if (j >= Tl.count(t)) break;
+                const int64_t i = Tl.start(t) + j;
+                float v[3];
+                rot(i, v);
+                const unsigned sd = extent_sides(v, mn, mx, tol);
+                if (sd) f(i, sd);
             }
+    };
+    auto exact = [&](int64_t i, unsigned sd) {
+        double v[3];
+        xyz_fine(rp, ld, i, kp, st->T, st->gamma0, v);
+        for (int j = 0; j < 3; ++j) {
+            if (sd & (1u << j)) atomicMin(&emin[j], ord64(v[j]));
+            if (sd & (8u << j)) atomicMax(&emax[j], ord64(v[j]));
         }
+    };
+    if (mine)
+        scan([&](int64_t i, unsigned) {
+            const int k = atomicAdd(&s_n, 1);
+            if (k < EX_CAND) s_cand[k] = (uint32_t)i;  // n < 2^31
+        });
+    __syncthreads();
+    const int found = s_n;
+    if (found > EX_CAND) {
+        if (mine) scan(exact);
+        __syncthreads();
+    }
+    ExtPart& mypart = ep[vb.x];
+    if (threadIdx.x < EX_CAND) mypart.cand[threadIdx.x] = s_cand[threadIdx.x];
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 3; ++k) {
+            mypart.mn[k] = mn[k];
+            mypart.mx[k] = mx[k];
+            mypart.emn[k] = emin[k];
+            mypart.emx[k] = emax[k];
+        }
+        mypart.count = found > EX_CAND ? 0 : found;
+        mypart.exact = found > EX_CAND;
+    }
+    if (!arrive_last(&st->done_extent, vb.nx)) return;
+    // last block: the extremes of all blocks, their candidates in the tile buffers
+    uint32_t* list = reinterpret_cast<uint32_t*>(smraw);
+    if (threadIdx.x < 3) {
+        emin[threadIdx.x] = ord64(INFINITY);
+        emax[threadIdx.x] = ord64(-INFINITY);
+    }
+    if (threadIdx.x == 0) s_n = 0;
+    for (int j = 0; j < 3; ++j) {
+        mn[j] = INFINITY;
+        mx[j] = -INFINITY;
+    }
+    for (int b = threadIdx.x; b < vb.nx; b += blockDim.x)
+        for (int j = 0; j < 3; ++j) {
+            mn[j] = fminf(mn[j], __ldcg(&ep[b].mn[j]));
+            mx[j] = fmaxf(mx[j], __ldcg(&ep[b].mx[j]));
+        }
+    block_extremes(mn, mx, smi);
+    extent_margin(mn, mx, g0, ig0, tol);
+    for (int b = threadIdx.x; b < vb.nx; b += blockDim.x) {
+        bool near = false;
+        for (int j = 0; j < 3; ++j)
+            near |= !(__ldcg(&ep[b].mn[j]) > mn[j] + tol[j]) || !(__ldcg(&ep[b].mx[j]) < mx[j] - tol[j]);
+        if (!near) continue;
+        if (__ldcg(&ep[b].exact))
+            for (int j = 0; j < 3; ++j) {
+                atomicMin(&emin[j], __ldcg(&ep[b].emn[j]));
+                atomicMax(&emax[j], __ldcg(&ep[b].emx[j]));
+            }
+        const int c = __ldcg(&ep[b].count);
+        const int at = c ? atomicAdd(&s_n, c) : 0;
+        for (int e = 0; e < c && at + e < EX_BLOCKS * EX_CAND; ++e) list[at + e] = __ldcg(&ep[b].cand[e]);
     }
     __syncthreads();
-    ExtPart32* ep = reinterpret_cast<ExtPart32*>(part);
-    if (threadIdx.x == 0 && SC_IDX_OK(st, 12, vb.x, kp.n > 0 ? vb.nx : 0)) {
-        for (int k = 0; k < 3; ++k) {
-            ep[vb.x].mn[k] = emin[k];
-            ep[vb.x].mx[k] = emax[k];
-        }
-        for (int k = 0; k < 5; ++k) {
-            ep[vb.x].hi[k] = qhi[k];
-            ep[vb.x].lo[k] = qlo[k];
-        }
+    const int nl = s_n < EX_BLOCKS * EX_CAND ? s_n : EX_BLOCKS * EX_CAND;
+    for (int e = threadIdx.x; e < nl; e += blockDim.x) {
+        const int64_t i = list[e];
+        float v[3];
+        rot(i, v);
+        const unsigned sd = extent_sides(v, mn, mx, tol);
+        if (sd) exact(i, sd);
     }
-    if (arrive_last(&st->done_extent, vb.nx)) mesh_finalize32(ep, vb.nx, kp, st);
+    __syncthreads();
+    double dmn[3], dmx[3], qs[5];
+    for (int j = 0; j < 3; ++j) {
+        dmn[j] = unord64(emin[j]);
+        dmx[j] = unord64(emax[j]);
+    }
+    for (int k = 0; k < 5; ++k) qs[k] = __ldcg(&st->qmom[k]);
+    mesh_finish(dmn, dmx, qs, kp, st, -1.0, true);
 }
 
-__global__ void __launch_bounds__(PT, 3) k_extent32_tma(const double* __restrict__ rp, const double* __restrict__ q,
-                                                        KickParams kp, float* __restrict__ X,
-                                                        double* __restrict__ part, ScState* st) {
+template <bool F64>
+__global__ void __launch_bounds__(PT, 3) k_extent(const double* __restrict__ rp, const float* __restrict__ X,
+                                                  const double* __restrict__ fpart, KickParams kp,
+                                                  ExtPart* __restrict__ ep, ScState* st) {
     pdl_wait();
-    extent32_tma_body(rp, q, kp, X, part, st, hw_vblk());
+    extent_body<F64>(rp, X, fpart, kp, ep, st, hw_vblk());
 }
 
 // el_field entry: X given as [n][3] rotated positions; z scaled by gamma in place
@@ -1616,6 +1567,8 @@ constexpr int KEYS_FINE = 1024;
 // its cell with a 64-bit integer atomic.  Integer addition is exact and
 // associative, so the charge grid does not depend on the order of the
 // atomics: deterministic, the same alone and in a batch.
+// rp != nullptr (the kick): X holds lab positions, rotated here as the extent
+// pass rotates them.
 template <bool VEC>
 __device__ __forceinline__ void keys32_body(float* __restrict__ X, uint32_t* __restrict__ keys,
                                             const double* __restrict__ rp, const double* __restrict__ q,
@@ -1625,7 +1578,9 @@ __device__ __forceinline__ void keys32_body(float* __restrict__ X, uint32_t* __r
     // loop, one per thread (KEYS_FINE of them per block; more go inline)
     __shared__ uint32_t s_fine[KEYS_FINE];
     __shared__ int s_nfine;
+    __shared__ __align__(16) float s_T[3][4];  // the rotation, read once per round: it holds no registers meanwhile
     if (threadIdx.x == 0) s_nfine = 0;
+    if (threadIdx.x < 9) s_T[threadIdx.x / 3][threadIdx.x % 3] = st->Tf[threadIdx.x / 3][threadIdx.x % 3];
     if (__syncthreads_or(st->status != SC_OK)) return;  // the same decision in every thread of the block
     const int64_t n = kp.n, ld = kp.ld, nX = kp.nX;
     float of[3], is[3];
@@ -1657,6 +1612,26 @@ __device__ __forceinline__ void keys32_body(float* __restrict__ X, uint32_t* __r
                 for (int j = 0; j < 3; ++j) ld_rowf(X + j * nX, i0_, pair_, vg[u][j][0], vg[u][j][1]);
                 if (qfix) ld_row(q, i0_, pair_, qg[u][0], qg[u][1]);
             }
+        }
+        if (rp) {
+            float T[3][3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                float pad;
+                asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];"
+                             : "=f"(T[i][0]), "=f"(T[i][1]), "=f"(T[i][2]), "=f"(pad)
+                             : "r"(smem_u32(s_T[i])));
+            }
+#pragma unroll
+            for (int u = 0; u < KG; ++u)
+#pragma unroll
+                for (int w = 0; w < 2; ++w) {
+                    const float l[3] = {vg[u][0][w], vg[u][1][w], vg[u][2][w]};
+                    float r[3];
+                    rot32(l, T, g0, r);
+#pragma unroll
+                    for (int j = 0; j < 3; ++j) vg[u][j][w] = r[j];
+                }
         }
 #pragma unroll
         for (int u = 0; u < KG; ++u) {
@@ -1713,11 +1688,8 @@ __device__ __forceinline__ void keys32_body(float* __restrict__ X, uint32_t* __r
             slow &= slow - 1;
             const int64_t p_ = pg_ + (bit >> 1) * pstride_;
             const int64_t i = (VEC && p_ < npair_ ? 2 * p_ : (VEC ? n - 1 : p_)) + (bit & 1);
-            double T[3][3];
-            for (int a = 0; a < 3; ++a)
-                for (int b = 0; b < 3; ++b) T[a][b] = st->T[a][b];
             double xv[3], e[3];
-            xyz_fine32(rp, ld, i, kp, T, st->gamma0, xv);
+            xyz_fine32(rp, ld, i, kp, st->T, st->gamma0, xv);
             for (int j = 0; j < 3; ++j)  // the FP64 form's grid coordinate (k_keys64)
                 e[j] = __dsub_rn(div_checked(xv[j], st->steps[j], st->isteps[j]), st->xoff[j]);
             uint32_t key = 0u;
@@ -2383,18 +2355,19 @@ __global__ void __launch_bounds__(PT) k_gather_xyz(const R* __restrict__ X, cons
 // ---------------------------------------------------------------------------
 // batched particle stages: one launch over every beam of a batch
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(PT, 4) kb_frame32(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(PT, 3) kb_frame32(const BatchBeam* __restrict__ beams,
                                                     const int* __restrict__ start, int nb) {
     pdl_wait();
     const int b = batch_beam(start, nb);
     const BatchBeam& B = beams[b];
     const VBlk vb = batch_vblk(start, b, B.gx[BS_PART], 1);
     ScState* st = reinterpret_cast<ScState*>(B.ws + B.L.state);
+    float* X = reinterpret_cast<float*>(B.ws + B.L.X);
     double* part = reinterpret_cast<double*>(B.ws + B.L.part_frame);
     unsigned long long* qz = reinterpret_cast<unsigned long long*>(B.ws + B.L.qfix);
     const int64_t nc = (int64_t)B.p.nx * B.p.ny * B.p.nz;
-    if (B.vec_rp) frame32_tma_body(B.rp, B.kp, part, st, qz, nc, vb);
-    else frame32_body<false>(B.rp, B.kp, part, st, qz, nc, vb);
+    if (B.vec_rpq) frame32_tma_body(B.rp, B.q, B.kp, X, part, st, qz, nc, vb);
+    else frame32_body<false>(B.rp, B.q, B.kp, X, part, st, qz, nc, vb);
 }
 
 __global__ void __launch_bounds__(PT, 3) kb_extent32(const BatchBeam* __restrict__ beams,
@@ -2404,10 +2377,9 @@ __global__ void __launch_bounds__(PT, 3) kb_extent32(const BatchBeam* __restrict
     const BatchBeam& B = beams[b];
     const VBlk vb = batch_vblk(start, b, B.gx[BS_PART], 1);
     ScState* st = reinterpret_cast<ScState*>(B.ws + B.L.state);
-    float* X = reinterpret_cast<float*>(B.ws + B.L.X);
-    double* part = reinterpret_cast<double*>(B.ws + B.L.part_ext);
-    if (B.vec_rpq) extent32_tma_body(B.rp, B.q, B.kp, X, part, st, vb);
-    else extent32_body<false>(B.rp, B.q, B.kp, X, part, st, vb);
+    extent_body<false>(B.rp, reinterpret_cast<const float*>(B.ws + B.L.X),
+                       reinterpret_cast<const double*>(B.ws + B.L.part_frame), B.kp,
+                       reinterpret_cast<ExtPart*>(B.ws + B.L.part_ext), st, vb);
 }
 
 __global__ void __launch_bounds__(PT, 4) kb_keys32(const BatchBeam* __restrict__ beams,
@@ -2521,7 +2493,7 @@ cudaError_t prepare_particle_kernels() {
     }
     if ((e = set_smem(k_frame32_tma, FR_SMEM))) return e;
     if ((e = set_smem(kb_frame32, FR_SMEM))) return e;
-    if ((e = set_smem(k_extent32_tma, EX_SMEM))) return e;
+    if ((e = set_smem(k_extent<false>, EX_SMEM))) return e;
     return set_smem(kb_extent32, EX_SMEM);
 }
 
@@ -2535,7 +2507,8 @@ static bool vec_ok(const double* rp, int64_t ld, const double* q) {
 // the next one in flight)
 static int particle_blocks(const Plan& p, int64_t n) {
     int64_t b = (n + PT_TILE - 1) / PT_TILE;
-    const int64_t cap = 3 * (int64_t)p.sm_count;
+    int64_t cap = 3 * (int64_t)p.sm_count;
+    if (cap > EX_BLOCKS) cap = EX_BLOCKS;  // the extent's last block lists every block's candidates
     if (b > cap) b = cap;
     return (int)(b > 0 ? b : 1);
 }
@@ -2543,7 +2516,7 @@ static int particle_blocks(const Plan& p, int64_t n) {
 int batch_particle_blocks(const Plan& p, int64_t n) { return particle_blocks(p, n); }
 
 cudaError_t launch_frame(const Plan& p, const Layout& L, char* ws, const KickParams& kp, const double* rp,
-                         cudaStream_t s) {
+                         const double* q, cudaStream_t s) {
     ScState* st = reinterpret_cast<ScState*>(ws + L.state);
     double* part = reinterpret_cast<double*>(ws + L.part_frame);
     const int nb = particle_blocks(p, kp.n);
@@ -2554,8 +2527,9 @@ cudaError_t launch_frame(const Plan& p, const Layout& L, char* ws, const KickPar
         // kernel follows the extent kernel without a memset between them
         unsigned long long* qz = p.sorted_deposit ? nullptr : reinterpret_cast<unsigned long long*>(ws + L.qfix);
         const int64_t nz = qz ? (int64_t)p.nx * p.ny * p.nz : 0;
-        vec_ok(rp, kp.ld, nullptr) ? launch(k_frame32_tma, nb, PT, FR_SMEM, s, rp, kp, part, st, qz, nz)
-                                   : launch(k_frame32<false>, nb, PT, 0, s, rp, kp, part, st, qz, nz);
+        float* X = reinterpret_cast<float*>(ws + L.X);
+        vec_ok(rp, kp.ld, q) ? launch(k_frame32_tma, nb, PT, FR_SMEM, s, rp, q, kp, X, part, st, qz, nz)
+                             : launch(k_frame32<false>, nb, PT, 0, s, rp, q, kp, X, part, st, qz, nz);
     }
     return cudaGetLastError();
 }
@@ -2569,9 +2543,8 @@ cudaError_t launch_extent(const Plan& p, const Layout& L, char* ws, const KickPa
         launch(k_extent64, nb, PT, 0, s, reinterpret_cast<const double*>(ws + L.xp), q, kp,
                                      reinterpret_cast<double*>(ws + L.X), part, st);
     else
-        vec_ok(rp, kp.ld, q)
-            ? launch(k_extent32_tma, nb, PT, EX_SMEM, s, rp, q, kp, reinterpret_cast<float*>(ws + L.X), part, st)
-            : launch(k_extent32<false>, nb, PT, 0, s, rp, q, kp, reinterpret_cast<float*>(ws + L.X), part, st);
+        launch(k_extent<false>, nb, PT, EX_SMEM, s, rp, reinterpret_cast<const float*>(ws + L.X),
+               reinterpret_cast<const double*>(ws + L.part_frame), kp, reinterpret_cast<ExtPart*>(part), st);
     return cudaGetLastError();
 }
 
