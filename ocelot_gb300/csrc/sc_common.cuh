@@ -458,6 +458,8 @@ __device__ __forceinline__ void bulk_wait_read() {
 }
 // every bulk group has completed
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+// starts bringing the line of p into L2
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // Per-thread asynchronous copies global -> shared (cp.async): 8 bytes, both
 // addresses 8-byte aligned; src_bytes 0 fills the 8 bytes with zeros.  A
 // thread's copies form groups (commit) and wait_group<N> waits until at most

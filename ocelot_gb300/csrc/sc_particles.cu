@@ -566,51 +566,56 @@ __device__ __forceinline__ bool arrive_last(unsigned int* counter, int nblk) {
     return last;
 }
 
-// mean momentum -> basis T, gamma0, beta0 (sc.py:224-239, 243-248); called by
-// the last block of a frame kernel with all per-block momentum sums in part
-// Mean-velocity frame from the momentum sums (valid in thread 0); called by
-// every thread of the last block.  The FP64 operations are the serial
+// mean momentum -> basis T, gamma0, beta0 (sc.py:224-239, 243-248) from the
+// momentum sums acc (shared memory); called by every thread of the last block
+// of a frame kernel, after a barrier.  The FP64 operations are the serial
 // ones of sc.py:224-239, 243-248, spread over lanes: lane k of warp 0 takes
 // component k of each basis vector and warp 1 the gamma0 chain, so the
 // dependent FP64 divisions and square roots (very slow on this GPU's FP64
-// pipe) form three short chains instead of one long one.  Each value goes
+// pipe) form three short chains instead of one long one; warp 2 keeps the
+// status words, whose loads the chains do not wait for.  Each value goes
 // through exactly the serial sequence of operations.
-__device__ void frame_finish(const double (&acc)[3], const KickParams& kp, ScState* st) {
-    __shared__ double s_acc[3];
-    __shared__ double s_gamma0;
-    __shared__ int s_bad1;
-    if (threadIdx.x == 0) {
-        st->done_frame = 0;
-        st->kick_next = 0;  // the tile counter of this kick's gather + kick
-        // the previous kick's outcome, kept before this kick resets the status
-        if (st->status != SC_OK && st->first_error == SC_OK) st->first_error = st->status;
-        for (int k = 0; k < 3; ++k) s_acc[k] = acc[k];
-    }
-    __syncthreads();
+__device__ __forceinline__ void frame_finish(const double* acc, const KickParams& kp, ScState* st) {
+    __shared__ int s_bad1, s_timeout;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, k = lane < 3 ? lane : 0;
-    if (warp > 1) return;
+    if (warp > 2) return;
+    if (warp == 2) {
+        if (lane == 0) {
+            const int prev = st->status, first = st->first_error, timeout = st->frame_timeout;
+            st->done_frame = 0;
+            st->kick_next = 0;  // the tile counter of this kick's gather + kick
+            // the previous kick's outcome, kept before this kick resets the status
+            if (prev != SC_OK && first == SC_OK) st->first_error = prev;
+            if (timeout) st->frame_timeout = 0;
+            s_timeout = timeout;
+        }
+        asm volatile("bar.sync 1, 96;" ::: "memory");
+        return;
+    }
     const double nn = (double)kp.n;
-    double t3k = __ddiv_rn(s_acc[k], nn);
+    double t3k = __ddiv_rn(acc[k], nn);
     double t3[3] = {__shfl_sync(FULL, t3k, 0), __shfl_sync(FULL, t3k, 1), __shfl_sync(FULL, t3k, 2)};
     const double Pav = __dsqrt_rn(__fma_rn(t3[2], t3[2], __fma_rn(t3[1], t3[1], __dmul_rn(t3[0], t3[0]))));
     if (warp == 1) {
+        const double pm = __ddiv_rn(Pav, kp.m_e_eV);
+        const double gamma0 = __dsqrt_rn(__dadd_rn(__dmul_rn(pm, pm), 1.0));
+        // lane 0: 1 / gamma0^2 (beta0), lane 1: 1 / gamma0 -- one division for both
+        const double rec = __drcp_rn(lane == 0 ? __dmul_rn(gamma0, gamma0) : gamma0);
+        const double beta0 = __dsqrt_rn(__dsub_rn(1.0, rec));
+        if (lane == 1) st->ig0f = (float)rec;
         if (lane == 0) {
-            const double pm = __ddiv_rn(Pav, kp.m_e_eV);
-            const double gamma0 = __dsqrt_rn(__dadd_rn(__dmul_rn(pm, pm), 1.0));
-            const double beta0 = __dsqrt_rn(__dsub_rn(1.0, __drcp_rn(__dmul_rn(gamma0, gamma0))));
+            const double kxy = __dmul_rn(kp.cdT, __dsub_rn(1.0, __dmul_rn(beta0, beta0)));
             st->Pav = Pav;
             st->gamma0 = gamma0;
             st->beta0 = beta0;
-            st->kxy = __dmul_rn(kp.cdT, __dsub_rn(1.0, __dmul_rn(beta0, beta0)));
+            st->kxy = kxy;
             st->kz = kp.cdT;
             st->g0f = (float)gamma0;
-            st->ig0f = (float)(1.0 / gamma0);
-            st->kxyf = (float)st->kxy;
+            st->kxyf = (float)kxy;
             st->kzf = (float)kp.cdT;
-            s_gamma0 = gamma0;
             s_bad1 = !(Pav > 0.0) || !isfinite(Pav) || !isfinite(gamma0);
         }
-        asm volatile("bar.sync 1, 64;" ::: "memory");
+        asm volatile("bar.sync 1, 96;" ::: "memory");
         return;
     }
     t3k = __ddiv_rn(t3k, Pav);
@@ -632,60 +637,81 @@ __device__ void frame_finish(const double (&acc)[3], const KickParams& kp, ScSta
         st->Tf[lane][1] = (float)t2[lane];
         st->Tf[lane][2] = (float)t3[lane];
     }
-    asm volatile("bar.sync 1, 64;" ::: "memory");
+    asm volatile("bar.sync 1, 96;" ::: "memory");
     if (lane == 0) {
         int status = SC_OK;
-        if (s_bad1 || !isfinite(s_gamma0) || !isfinite(t1[0]) || !isfinite(t2[1])) status = SC_ERR_NONFINITE;
-        if (st->frame_timeout) {
-            status = SC_ERR_TIMEOUT;
-            st->frame_timeout = 0;
-        }
+        if (s_bad1 || !isfinite(t1[0]) || !isfinite(t2[1])) status = SC_ERR_NONFINITE;
+        if (s_timeout) status = SC_ERR_TIMEOUT;
         st->status = status;
     }
 }
 
 __device__ void frame_finalize(const double* part, int nblk, const KickParams& kp, ScState* st) {
     __shared__ double sm[3 * 32];
+    __shared__ double s_acc[3];
     double acc[3] = {0.0, 0.0, 0.0};
     for (int b = threadIdx.x; b < nblk; b += blockDim.x)
         for (int k = 0; k < 3; ++k) acc[k] += __ldcg(part + b * 3 + k);
     block_sum<3>(acc, sm);
-    frame_finish(acc, kp, st);
+    if (threadIdx.x == 0)
+        for (int k = 0; k < 3; ++k) s_acc[k] = acc[k];
+    __syncthreads();
+    frame_finish(s_acc, kp, st);
 }
 
 
 // FP32 form: a block's sums of the frame pass as double-float pairs: the
 // momenta (0..2), charge times lab position (3..5), charge (6), |charge| (7).
-// The finalize of the frame reduces the momenta on the FP32 pipes; the charge
-// moments wait for the extent pass (extent_body), off the frame's chain.
+// The last block reduces them on the FP32 pipes, one quantity per warp (a
+// block-wide tree over three of them, then the charge moments in the extent
+// pass, took 2.4 + 2.5 us at 10k particles; all eight this way 0.9 us).
 struct FramePart32 {
     float hi[8], lo[8];
 };
 static_assert(sizeof(FramePart32) == FRAME_PART * sizeof(double), "a block's slot of frame partials");
+static_assert(PT == 8 * 32, "one warp per quantity");
 __device__ void frame_finalize32(const FramePart32* part, int nblk, const KickParams& kp, ScState* st) {
-    __shared__ float sm[3 * 64];
-    float hi[3] = {0.f, 0.f, 0.f}, lo[3] = {0.f, 0.f, 0.f};
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-        for (int k = 0; k < 3; ++k) df_add(hi[k], lo[k], __ldcg(&part[b].hi[k]), __ldcg(&part[b].lo[k]));
-    block_sum_df<3>(hi, lo, sm);
-    const double acc[3] = {(double)hi[0] + (double)lo[0], (double)hi[1] + (double)lo[1],
-                           (double)hi[2] + (double)lo[2]};
-    frame_finish(acc, kp, st);
+    __shared__ double s_acc[3];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float hi = 0.f, lo = 0.f;
+#pragma unroll 4
+    for (int b = lane; b < nblk; b += 32) df_add(hi, lo, __ldcg(&part[b].hi[w]), __ldcg(&part[b].lo[w]));
+    for (int o = 16; o; o >>= 1) df_add(hi, lo, __shfl_down_sync(FULL, hi, o), __shfl_down_sync(FULL, lo, o));
+    if (lane == 0) (w < 3 ? s_acc[w] : st->qmom[w - 3]) = (double)hi + (double)lo;
+    __syncthreads();
+    frame_finish(s_acc, kp, st);
 }
+
+// what mesh_finish needs of the state, loaded ahead of it (a load in its chain
+// is a round trip to L2)
+struct MeshPre {
+    int status;
+    double T[3], gamma0;  // column lane % 3 of T
+    double igf_h;         // component lane % 3 of the Green cache's spacing
+    __device__ __forceinline__ void load(const ScState* st, bool lab_sums) {
+        const int a = (threadIdx.x & 31) % 3;
+        status = __ldcg(&st->status);
+        igf_h = __ldcg(&st->igf_h[a]);
+        if (lab_sums) {
+            for (int i = 0; i < 3; ++i) T[i] = st->T[i][a];
+            gamma0 = st->gamma0;
+        }
+    }
+};
 
 // steps, X_off, potential scale, Green cache check (sc.py:172-186, 167)
 // part layout per block (PART_EXT doubles): min[3], max[3], sum q*x[3], sum q, sum |q|
-// lab_sums: the sums q*x are of lab positions (the FP32 extent); they are
+// lab_sums: the sums q*x are of lab positions (the kick's frame pass); they are
 // rotated into the beam frame and scaled by gamma0 here (a linear map, so
 // the same charge-weighted mean)
-// Mesh step, offset and derived constants from the extremes and charge
-// moments (valid in thread 0); called by every thread of the last block.
-// Lane k of warp 0 takes axis k with the serial FP64 operations of
-// sc.py:172-186, so the divisions of the three axes run side by side.
-__device__ void mesh_finish(const double (&mn)[3], const double (&mx)[3], const double (&qs)[5], const KickParams& kp,
-                            ScState* st, double gamma_override, bool lab_sums) {
-    __shared__ double s_mn[3], s_mx[3], s_qs[5];
-    if (threadIdx.x == 0) {
+// Mesh step, offset and derived constants from the extremes mn, mx and charge
+// moments qs; the first warp of the last block, all lanes.  Lane k takes
+// axis k with the serial FP64 operations of sc.py:172-186, so the divisions
+// of the three axes run side by side.
+__device__ __forceinline__ void mesh_finish(const double* mn, const double* mx, const double* qs, const MeshPre& pre,
+                                            const KickParams& kp, ScState* st, double gamma_override, bool lab_sums) {
+    const int lane = threadIdx.x, k = lane < 3 ? lane : 0;
+    if (lane == 0) {
         st->done_extent = 0;
         if (gamma_override > 0.0) {
             st->gamma0 = gamma_override;
@@ -693,25 +719,9 @@ __device__ void mesh_finish(const double (&mn)[3], const double (&mx)[3], const 
             st->ig0f = (float)(1.0 / gamma_override);
             st->status = SC_OK;
         }
-        for (int k = 0; k < 3; ++k) {
-            s_mn[k] = mn[k];
-            s_mx[k] = mx[k];
-        }
-        for (int k = 0; k < 5; ++k) s_qs[k] = qs[k];
     }
-    __syncthreads();
-    if (threadIdx.x >= 32) return;
-    if (st->status != SC_OK) return;
-    const int lane = threadIdx.x, k = lane < 3 ? lane : 0;
-    double q3[3] = {s_qs[0], s_qs[1], s_qs[2]};
-    if (lab_sums) {
-        double r[3];
-        for (int j = 0; j < 3; ++j) r[j] = fma(q3[2], st->T[2][j], fma(q3[1], st->T[1][j], q3[0] * st->T[0][j]));
-        r[2] *= st->gamma0;
-        for (int j = 0; j < 3; ++j) q3[j] = r[j];
-    }
-    const double qsum = s_qs[3];
-    const int nm[3] = {kp.nx, kp.ny, kp.nz};
+    if (!(gamma_override > 0.0) && pre.status != SC_OK) return;
+    const double qsum = qs[3];
     // Every lane takes axis a = lane % 3 of the step; then group g = lane / 3
     // (0..4; lanes 15..31 repeat group 3) divides by it: g = 0 X_min,
     // g = 1 the charge-weighted mean (then / sum q), g = 2 1/step, g = 3 the
@@ -721,12 +731,18 @@ __device__ void mesh_finish(const double (&mn)[3], const double (&mx)[3], const 
     // divisions instead of seven; each value is the same operation sequence
     // as the serial form.
     const int a = lane % 3, g = lane < 15 ? lane / 3 : 3;
-    double XX = __dsub_rn(s_mx[a], s_mn[a]);
+    const int nma = a == 0 ? kp.nx : a == 1 ? kp.ny : kp.nz, nmk = k == 0 ? kp.nx : k == 1 ? kp.ny : kp.nz;
+    double q3 = qs[a];
+    if (lab_sums) {
+        q3 = fma(qs[2], pre.T[2], fma(qs[1], pre.T[1], qs[0] * pre.T[0]));
+        if (a == 2) q3 *= pre.gamma0;
+    }
+    double XX = __dsub_rn(mx[a], mn[a]);
     if (!isnan(kp.mesh_scale)) XX = __dmul_rn(XX, kp.mesh_scale);
-    const double stepa = __ddiv_rn(XX, (double)(nm[a] - 3));
+    const double stepa = __ddiv_rn(XX, (double)(nma - 3));
     const double steps[3] = {__shfl_sync(FULL, stepa, 0), __shfl_sync(FULL, stepa, 1), __shfl_sync(FULL, stepa, 2)};
     const double hm = fmax(steps[0], fmax(steps[1], steps[2]));
-    const double num = g == 0 ? s_mn[a] : g == 1 ? q3[a] : g == 2 ? 1.0 : __dmul_rn(5.0, hm);
+    const double num = g == 0 ? mn[a] : g == 1 ? q3 : g == 2 ? 1.0 : __dmul_rn(5.0, hm);
     const double r1 = __ddiv_rn(num, stepa);
     const double pden = __dmul_rn(__dmul_rn(__dmul_rn(kp.four_pi_eps0, steps[0]), steps[1]), steps[2]);
     const double n2 = g == 4 ? kp.phi_norm : r1, d2 = g == 4 ? pden : qsum;
@@ -745,18 +761,20 @@ __device__ void mesh_finish(const double (&mn)[3], const double (&mx)[3], const 
         if (lane == 0) st->status = SC_ERR_DEGENERATE;
         return;
     }
+    const bool same = __all_sync(FULL, lane >= 3 || stepk == pre.igf_h);  // lane k < 3: axis k
     // near box of the hybrid Green's function along axis k (igf_box_of)
-    int bk = v >= (double)nm[k] ? nm[k] : (int)ceil(v) + 1;
-    if (bk > nm[k]) bk = nm[k];
+    int bk = v >= (double)nmk ? nmk : (int)ceil(v) + 1;
+    if (bk > nmk) bk = nmk;
     if (lane < 3) {
         st->steps[k] = stepk;
+        st->igf_h[k] = stepk;
         st->xoff[k] = xoffk;
         st->isteps[k] = istepk;
         st->stepsf[k] = (float)stepk;
         st->istepsf[k] = (float)istepk;
         st->xofff[k] = (float)xoffk;
         st->igf_box[k] = bk;
-        if (k < 2) st->igf_tbox[k] = igf_tbox_of(steps, k, nm[k]);
+        if (k < 2) st->igf_tbox[k] = igf_tbox_of(steps, k, nmk);
         if (k == 2) st->igf_line = igf_line_of(steps);
     }
     if (lane == 1) st->phi_norm = kp.phi_norm;
@@ -764,7 +782,7 @@ __device__ void mesh_finish(const double (&mn)[3], const double (&mx)[3], const 
         // fixed-point unit of the exact deposit: sum |q| * 2^S < 2^62, so no
         // cell (nor the total) can overflow a signed 64-bit accumulator
         int e2;
-        frexp(s_qs[4], &e2);
+        frexp(qs[4], &e2);
         const int S = 62 - e2;
         st->qfix_shift = S;
         st->qfix_scale = ldexp(1.0, S);
@@ -773,9 +791,7 @@ __device__ void mesh_finish(const double (&mn)[3], const double (&mx)[3], const 
     if (lane == 0) {
         st->phi_denom = pden;
         st->phi_scalef = (float)scale;
-        const bool same = steps[0] == st->igf_h[0] && steps[1] == st->igf_h[1] && steps[2] == st->igf_h[2];
         st->igf_rebuild = same ? 0 : 1;
-        for (int j = 0; j < 3; ++j) st->igf_h[j] = steps[j];
     }
 }
 
@@ -797,7 +813,19 @@ __device__ void mesh_finalize(const double* part, int nblk, const KickParams& kp
     block_minmax<3, false>(mn, sm);
     block_minmax<3, true>(mx, sm);
     block_sum<5>(qs, sm);
-    mesh_finish(mn, mx, qs, kp, st, gamma_override, lab_sums);
+    __shared__ double s_fin[11];  // the extremes and sums, for the first warp
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < 3; ++k) {
+            s_fin[k] = mn[k];
+            s_fin[3 + k] = mx[k];
+        }
+        for (int k = 0; k < 5; ++k) s_fin[6 + k] = qs[k];
+    }
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    MeshPre pre;
+    pre.load(st, lab_sums);
+    mesh_finish(s_fin, s_fin + 3, s_fin + 6, pre, kp, st, gamma_override, lab_sums);
 }
 
 // ---------------------------------------------------------------------------
@@ -1177,7 +1205,8 @@ struct ExtPart {
     uint32_t cand[EX_CAND];
 };
 static_assert(sizeof(ExtPart) == EXT_PART * sizeof(double), "a block's slot of extent partials");
-constexpr int EX_BLOCKS = (int)(EX_BUF / (EX_CAND * sizeof(uint32_t)));  // blocks whose lists fit the tile buffers
+constexpr int EX_BLOCKS = 2 * PT;  // blocks of an extent at most (two per thread of the last one)
+static_assert(EX_BLOCKS * sizeof(uint32_t) <= EX_BUF, "the last block lists blocks in the tile buffers");
 
 // Extent of the rotated positions.  The FP32 positions (rot32 of the lab
 // positions the frame pass stored, 12 bytes a particle) give each block's
@@ -1190,14 +1219,9 @@ constexpr int EX_BLOCKS = (int)(EX_BUF / (EX_CAND * sizeof(uint32_t)));  // bloc
 // candidates for the extremes of all blocks.  A block with more than EX_CAND
 // (many particles sharing an extreme coordinate) evaluates its own, so that
 // the last block's share stays bounded.  2M / 64^3, frame + extent: 71 -> 58 us.
-// Block 0 reduces the charge moments of the frame pass meanwhile (F64: FP64
-// sums, else double-float pairs).  nX rows of X; all waits bounded.
-template <bool F64>
 __device__ __forceinline__ void extent_body(const double* __restrict__ rp, const float* __restrict__ X,
-                                            const double* __restrict__ fpart, const KickParams& kp,
-                                            ExtPart* __restrict__ ep, ScState* st, VBlk vb) {
+                                            const KickParams& kp, ExtPart* __restrict__ ep, ScState* st, VBlk vb) {
     extern __shared__ __align__(128) unsigned char smraw[];
-    __shared__ double smq[5 * 32];
     __shared__ int smi[6 * 32];
     __shared__ unsigned long long emin[3], emax[3];
     __shared__ uint32_t s_cand[EX_CAND];
@@ -1211,17 +1235,6 @@ __device__ __forceinline__ void extent_body(const double* __restrict__ rp, const
     }
     if (threadIdx.x == 0) s_n = 0;
     const bool ok = !__syncthreads_or(st->status != SC_OK);
-    if (vb.x == 0 && ok) {
-        static_assert(sizeof(smq) == 5 * 64 * sizeof(float), "the scratch of either sum");
-        float(&smf)[5 * 64] = reinterpret_cast<float(&)[5 * 64]>(smq);
-        float hi[5] = {0.f, 0.f, 0.f, 0.f, 0.f}, lo[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
-        const FramePart32* fp = reinterpret_cast<const FramePart32*>(fpart);
-        for (int b = threadIdx.x; b < vb.nx; b += blockDim.x)
-            for (int k = 0; k < 5; ++k) df_add(hi[k], lo[k], fp[b].hi[3 + k], fp[b].lo[3 + k]);
-        block_sum_df<5>(hi, lo, smf);
-        if (threadIdx.x == 0)
-            for (int k = 0; k < 5; ++k) st->qmom[k] = (double)hi[k] + (double)lo[k];
-    }
     float T[3][3];
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j) T[i][j] = st->Tf[i][j];
@@ -1291,6 +1304,7 @@ __device__ __forceinline__ void extent_body(const double* __restrict__ rp, const
         scan([&](int64_t i, unsigned) {
             const int k = atomicAdd(&s_n, 1);
             if (k < EX_CAND) s_cand[k] = (uint32_t)i;  // n < 2^31
+            for (int r = 0; r < 6; ++r) prefetch_l2(rp + r * ld + i);  // the last block may evaluate it
         });
     __syncthreads();
     const int found = s_n;
@@ -1311,63 +1325,82 @@ __device__ __forceinline__ void extent_body(const double* __restrict__ rp, const
         mypart.exact = found > EX_CAND;
     }
     if (!arrive_last(&st->done_extent, vb.nx)) return;
-    // last block: the extremes of all blocks, their candidates in the tile buffers
+    // last block: the extremes of all blocks; the blocks near them are listed
+    // in the tile buffers, and thread t takes candidate t % EX_CAND of listed
+    // block t / EX_CAND: three round trips to L2 (the blocks' extremes, the
+    // candidates, their coordinates) before the FP64 evaluation
     uint32_t* list = reinterpret_cast<uint32_t*>(smraw);
+    MeshPre pre;
+    pre.load(st, true);
+    __shared__ double s_fin[11];
+    if (threadIdx.x >= 32 && threadIdx.x < 37) s_fin[threadIdx.x - 26] = __ldcg(&st->qmom[threadIdx.x - 32]);
     if (threadIdx.x < 3) {
         emin[threadIdx.x] = ord64(INFINITY);
         emax[threadIdx.x] = ord64(-INFINITY);
     }
     if (threadIdx.x == 0) s_n = 0;
+    constexpr int NB = (EX_BLOCKS + PT - 1) / PT;  // blocks per thread
+    float bmn[NB][3], bmx[NB][3];
+    int bex[NB];
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+        const int b = threadIdx.x + u * PT;
+        bex[u] = 0;
+        for (int j = 0; j < 3; ++j) {
+            bmn[u][j] = b < vb.nx ? __ldcg(&ep[b].mn[j]) : INFINITY;
+            bmx[u][j] = b < vb.nx ? __ldcg(&ep[b].mx[j]) : -INFINITY;
+        }
+        if (b < vb.nx) bex[u] = __ldcg(&ep[b].exact);
+    }
     for (int j = 0; j < 3; ++j) {
         mn[j] = INFINITY;
         mx[j] = -INFINITY;
-    }
-    for (int b = threadIdx.x; b < vb.nx; b += blockDim.x)
-        for (int j = 0; j < 3; ++j) {
-            mn[j] = fminf(mn[j], __ldcg(&ep[b].mn[j]));
-            mx[j] = fmaxf(mx[j], __ldcg(&ep[b].mx[j]));
+#pragma unroll
+        for (int u = 0; u < NB; ++u) {
+            mn[j] = fminf(mn[j], bmn[u][j]);
+            mx[j] = fmaxf(mx[j], bmx[u][j]);
         }
+    }
     block_extremes(mn, mx, smi);
     extent_margin(mn, mx, g0, ig0, tol);
-    for (int b = threadIdx.x; b < vb.nx; b += blockDim.x) {
+#pragma unroll
+    for (int u = 0; u < NB; ++u) {
+        const int b = threadIdx.x + u * PT;
         bool near = false;
-        for (int j = 0; j < 3; ++j)
-            near |= !(__ldcg(&ep[b].mn[j]) > mn[j] + tol[j]) || !(__ldcg(&ep[b].mx[j]) < mx[j] - tol[j]);
-        if (!near) continue;
-        if (__ldcg(&ep[b].exact))
+        for (int j = 0; j < 3; ++j) near |= !(bmn[u][j] > mn[j] + tol[j]) || !(bmx[u][j] < mx[j] - tol[j]);
+        if (b >= vb.nx || !near) continue;
+        if (bex[u])
             for (int j = 0; j < 3; ++j) {
                 atomicMin(&emin[j], __ldcg(&ep[b].emn[j]));
                 atomicMax(&emax[j], __ldcg(&ep[b].emx[j]));
             }
-        const int c = __ldcg(&ep[b].count);
-        const int at = c ? atomicAdd(&s_n, c) : 0;
-        for (int e = 0; e < c && at + e < EX_BLOCKS * EX_CAND; ++e) list[at + e] = __ldcg(&ep[b].cand[e]);
+        else list[atomicAdd(&s_n, 1)] = (uint32_t)b;
     }
     __syncthreads();
-    const int nl = s_n < EX_BLOCKS * EX_CAND ? s_n : EX_BLOCKS * EX_CAND;
-    for (int e = threadIdx.x; e < nl; e += blockDim.x) {
-        const int64_t i = list[e];
+    const int nl = s_n * EX_CAND;
+    for (int t = threadIdx.x; t < nl; t += PT) {
+        const ExtPart& P = ep[list[t / EX_CAND]];
+        const int e = t % EX_CAND, count = __ldcg(&P.count);
+        const int64_t i = e < EX_CAND && __ldcg(&P.cand[e]) < n ? __ldcg(&P.cand[e]) : 0;
         float v[3];
         rot(i, v);
-        const unsigned sd = extent_sides(v, mn, mx, tol);
+        const unsigned sd = e < count ? extent_sides(v, mn, mx, tol) : 0u;
         if (sd) exact(i, sd);
     }
     __syncthreads();
-    double dmn[3], dmx[3], qs[5];
-    for (int j = 0; j < 3; ++j) {
-        dmn[j] = unord64(emin[j]);
-        dmx[j] = unord64(emax[j]);
+    if (threadIdx.x >= 32) return;
+    if (threadIdx.x < 3) {
+        s_fin[threadIdx.x] = unord64(emin[threadIdx.x]);
+        s_fin[3 + threadIdx.x] = unord64(emax[threadIdx.x]);
     }
-    for (int k = 0; k < 5; ++k) qs[k] = __ldcg(&st->qmom[k]);
-    mesh_finish(dmn, dmx, qs, kp, st, -1.0, true);
+    __syncwarp();
+    mesh_finish(s_fin, s_fin + 3, s_fin + 6, pre, kp, st, -1.0, true);
 }
 
-template <bool F64>
 __global__ void __launch_bounds__(PT, 3) k_extent(const double* __restrict__ rp, const float* __restrict__ X,
-                                                  const double* __restrict__ fpart, KickParams kp,
-                                                  ExtPart* __restrict__ ep, ScState* st) {
+                                                  KickParams kp, ExtPart* __restrict__ ep, ScState* st) {
     pdl_wait();
-    extent_body<F64>(rp, X, fpart, kp, ep, st, hw_vblk());
+    extent_body(rp, X, kp, ep, st, hw_vblk());
 }
 
 // el_field entry: X given as [n][3] rotated positions; z scaled by gamma in place
@@ -2377,9 +2410,8 @@ __global__ void __launch_bounds__(PT, 3) kb_extent32(const BatchBeam* __restrict
     const BatchBeam& B = beams[b];
     const VBlk vb = batch_vblk(start, b, B.gx[BS_PART], 1);
     ScState* st = reinterpret_cast<ScState*>(B.ws + B.L.state);
-    extent_body<false>(B.rp, reinterpret_cast<const float*>(B.ws + B.L.X),
-                       reinterpret_cast<const double*>(B.ws + B.L.part_frame), B.kp,
-                       reinterpret_cast<ExtPart*>(B.ws + B.L.part_ext), st, vb);
+    extent_body(B.rp, reinterpret_cast<const float*>(B.ws + B.L.X), B.kp,
+                reinterpret_cast<ExtPart*>(B.ws + B.L.part_ext), st, vb);
 }
 
 __global__ void __launch_bounds__(PT, 4) kb_keys32(const BatchBeam* __restrict__ beams,
@@ -2493,7 +2525,7 @@ cudaError_t prepare_particle_kernels() {
     }
     if ((e = set_smem(k_frame32_tma, FR_SMEM))) return e;
     if ((e = set_smem(kb_frame32, FR_SMEM))) return e;
-    if ((e = set_smem(k_extent<false>, EX_SMEM))) return e;
+    if ((e = set_smem(k_extent, EX_SMEM))) return e;
     return set_smem(kb_extent32, EX_SMEM);
 }
 
@@ -2508,7 +2540,7 @@ static bool vec_ok(const double* rp, int64_t ld, const double* q) {
 static int particle_blocks(const Plan& p, int64_t n) {
     int64_t b = (n + PT_TILE - 1) / PT_TILE;
     int64_t cap = 3 * (int64_t)p.sm_count;
-    if (cap > EX_BLOCKS) cap = EX_BLOCKS;  // the extent's last block lists every block's candidates
+    if (cap > EX_BLOCKS) cap = EX_BLOCKS;
     if (b > cap) b = cap;
     return (int)(b > 0 ? b : 1);
 }
@@ -2543,8 +2575,8 @@ cudaError_t launch_extent(const Plan& p, const Layout& L, char* ws, const KickPa
         launch(k_extent64, nb, PT, 0, s, reinterpret_cast<const double*>(ws + L.xp), q, kp,
                                      reinterpret_cast<double*>(ws + L.X), part, st);
     else
-        launch(k_extent<false>, nb, PT, EX_SMEM, s, rp, reinterpret_cast<const float*>(ws + L.X),
-               reinterpret_cast<const double*>(ws + L.part_frame), kp, reinterpret_cast<ExtPart*>(part), st);
+        launch(k_extent, nb, PT, EX_SMEM, s, rp, reinterpret_cast<const float*>(ws + L.X), kp,
+               reinterpret_cast<ExtPart*>(part), st);
     return cudaGetLastError();
 }
 
