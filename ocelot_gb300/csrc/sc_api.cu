@@ -135,7 +135,6 @@ Layout make_layout(const Plan& p, int64_t n) {
     L.dt_z = take(p.spectral ? cs * p.Mz : 0);
     L.W2 = take(p.spectral ? cs * (size_t)p.nx * p.My * Kz : 0);
     L.W3 = take(p.spectral ? cs * (size_t)p.nx * p.My * Kz : 0);
-    L.xp = take(p.prec == SC_FP64 ? 8 * 6 * (size_t)n : 0);
     L.X = take(rs * 3 * (size_t)((n + 3) / 4 * 4));
     L.keys = take(4 * (size_t)n);
     // the radix sort's buffers: only the sorted deposit uses them
@@ -621,7 +620,7 @@ int sc_kick(sc_plan* plan, void* ws_v, size_t ws_bytes, double* rp, int64_t ld, 
     mark(plan, 0, s);
     SC_CUDA(launch_frame(p, L, ws, kp, rp, q, s), "frame");
     mark(plan, 1, s);
-    SC_CUDA(launch_extent(p, L, ws, kp, rp, q, s), "extent");
+    SC_CUDA(launch_extent(p, L, ws, kp, rp, s), "extent");
     mark(plan, 2, s);
     // fork: the FP64 Green's-function table and its spectrum (they need only
     // the mesh step) run on the side stream while the deposit runs here

@@ -53,6 +53,9 @@ struct ScState {
     float phi_scalef;            // (float)(phi_norm / phi_denom): the FP32 form's potential scale
     // Green's-function cache: spacing of the spectrum held in the workspace
     double igf_h[3];
+    // the FP64 kick: lab position -> grid coordinate (rotation, gamma0, 1/steps)
+    // and field -> lab kick in units of pref (rotation, kick factors)
+    double Tg[3][3], Tk[3][3];
     double qmom[5];              // charge x lab position (3), charge, |charge|: the frame pass's sums
     // FP32 copies of the per-kick constants, written once by the finalizes
     float Tf[3][3];
@@ -80,7 +83,7 @@ struct ScState {
     int first_error;             // first non-OK status of any kick since sc_workspace_init
     long long check_index;       // ... and the offending index (checked builds)
 };
-static_assert(sizeof(ScState) <= 512, "the state must fit the 512 bytes the static IGF scratch reserves");
+static_assert(sizeof(ScState) <= 1024, "the state must fit the 1024 bytes the static IGF scratch reserves");
 constexpr int WS_MAGIC = 0x5c6b0e11;
 
 // Near box of the hybrid Green's function: along each axis the cells with
@@ -161,8 +164,7 @@ int choose_fft_length(int n);  // smallest supported length >= 2n-1, 0 if none
 struct Layout {
     size_t state, tw_x, tw_y, tw_z;              // twiddles (Cx<R>[M])
     size_t part_frame, part_ext;                 // per-block partial sums (double)
-    size_t xp;                                   // FP64: 6 x n lab coordinates
-    size_t X;                                    // 3 x n grid coordinates (R)
+    size_t X;                                    // 3 x n: lab positions (FP32) of a kick, grid coordinates (R) of el_field
     size_t keys, sort_keys, sort_perm, sort_q, sort_tmp_k, sort_tmp_v, sort_hist, sort_tot;
     size_t qgrid, phi, ex, ey, ez;               // [nx][ny][nz] (R)
     size_t exq, eyq, ezq;                        // FP32 form: [nx][ny][nz] gather octs (8 floats, 32-byte aligned)
@@ -214,7 +216,7 @@ cudaError_t launch_init_workspace(const Plan& p, const Layout& L, char* ws, cuda
 cudaError_t launch_frame(const Plan& p, const Layout& L, char* ws, const KickParams& kp,
                          const double* rp, const double* q, cudaStream_t s);
 cudaError_t launch_extent(const Plan& p, const Layout& L, char* ws, const KickParams& kp,
-                          const double* rp, const double* q, cudaStream_t s);
+                          const double* rp, cudaStream_t s);
 // rp: the particles (exact recomputation of near-face keys in the FP32 form), or nullptr
 // FP32 form without the sorted deposit: also accumulates q into the
 // fixed-point grid (the deposit), zeroed first unless qfix_zeroed (the

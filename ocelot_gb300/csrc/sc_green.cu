@@ -687,7 +687,7 @@ cudaError_t launch_batch_green(const BatchBeam* beams, const int* sz, const int*
 // a zeroed stand-in for the workspace state that the kernels are handed.
 // ---------------------------------------------------------------------------
 constexpr long long kStaticMaxCorners = SC_SYM_KERNEL_STATIC_MAX_CORNERS;
-constexpr long long kScratchState = 64;  // doubles (512 bytes >= sizeof(ScState))
+constexpr long long kScratchState = 128;  // doubles (1024 bytes >= sizeof(ScState))
 static __device__ __align__(256) double g_igf_scratch[kScratchState + kStaticMaxCorners];
 
 namespace {

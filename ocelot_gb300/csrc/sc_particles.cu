@@ -10,9 +10,13 @@
 //           the lab-frame kick (sc.py:244-250) and the transform back to MAD
 //           (coord_transform.py:16-54), written into rparticles
 //
-// Two forms.  FP64 performs the reference's floating-point operations in the
-// reference's order (explicit _rn intrinsics, so nothing is contracted into
-// FMAs except where numpy's BLAS itself uses FMAs: the 3x3 rotations).  FP32
+// Two forms.  FP64 decides everything discrete -- the mesh step and offset,
+// the NGP cells, which samples lie outside the mesh -- with the reference's
+// floating-point operations in the reference's order (explicit _rn intrinsics,
+// so nothing is contracted into FMAs except where numpy's BLAS itself uses
+// FMAs: the 3x3 rotations), and computes the rest in FP64 with fewer
+// operations (kick64_one), because this GPU issues an FP64 instruction about
+// 1/64 as often as an FP32 one.  FP32
 // computes every per-particle quantity in FP32 and writes the kick as small
 // increments, each derived in closed form so that it carries no cancellation,
 // added to the FP64 coordinates:
@@ -123,35 +127,6 @@ __device__ __forceinline__ void block_sum_f2(const float (&v)[NV], float (&hi)[N
     block_sum_df<NV>(hi, lo, sm);
 }
 
-// block minimum or maximum of order-preserving 64-bit keys (ord64 of
-// doubles) on the integer pipes; thread 0 receives the result
-template <int NV, bool MAX, int SZ>
-__device__ __forceinline__ void block_minmax_u64(unsigned long long (&v)[NV], unsigned long long (&sm)[SZ]) {
-    static_assert(SZ >= NV * 32, "block_minmax_u64: shared scratch too small");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int c = 0; c < NV; ++c)
-        for (int o = 16; o; o >>= 1) {
-            const unsigned long long w = __shfl_down_sync(FULL, v[c], o);
-            v[c] = MAX ? (w > v[c] ? w : v[c]) : (w < v[c] ? w : v[c]);
-        }
-    if (lane == 0)
-#pragma unroll
-        for (int c = 0; c < NV; ++c) sm[c * 32 + warp] = v[c];
-    __syncthreads();
-    if (warp == 0) {
-#pragma unroll
-        for (int c = 0; c < NV; ++c) {
-            v[c] = lane < nw ? sm[c * 32 + lane] : (MAX ? 0ull : ~0ull);
-            for (int o = 16; o; o >>= 1) {
-                const unsigned long long w = __shfl_down_sync(FULL, v[c], o);
-                v[c] = MAX ? (w > v[c] ? w : v[c]) : (w < v[c] ? w : v[c]);
-            }
-        }
-    }
-    __syncthreads();
-}
-
 template <int NV, bool MAX, int SZ>
 __device__ __forceinline__ void block_minmax(double (&v)[NV], double (&sm)[SZ]) {
     static_assert(SZ >= NV * 32, "block_minmax: shared scratch too small");
@@ -175,32 +150,6 @@ __device__ __forceinline__ void block_minmax(double (&v)[NV], double (&sm)[SZ]) 
                 v[c] = MAX ? fmax(v[c], w) : fmin(v[c], w);
             }
         }
-    }
-    __syncthreads();
-}
-
-template <int NV, bool MAX, int SZ>
-__device__ __forceinline__ void block_minmax_f(float (&v)[NV], float (&sm)[SZ]) {
-    static_assert(SZ >= NV * 32, "block_minmax_f: shared scratch too small");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-#pragma unroll
-    for (int c = 0; c < NV; ++c)
-        for (int o = 16; o; o >>= 1) {
-            const float w = __shfl_xor_sync(FULL, v[c], o);
-            v[c] = MAX ? fmaxf(v[c], w) : fminf(v[c], w);
-        }
-    if (lane == 0)
-#pragma unroll
-        for (int c = 0; c < NV; ++c) sm[c * 32 + warp] = v[c];
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < NV; ++c) {
-        float r = lane < nw ? sm[c * 32 + lane] : (MAX ? -INFINITY : INFINITY);
-        for (int o = 16; o; o >>= 1) {
-            const float w = __shfl_xor_sync(FULL, r, o);
-            r = MAX ? fmaxf(r, w) : fminf(r, w);
-        }
-        v[c] = r;  // every thread holds the block result
     }
     __syncthreads();
 }
@@ -266,24 +215,6 @@ __device__ __forceinline__ void mad_to_cart64(const double r[6], const KickParam
     xp[3] = __dmul_rn(__dmul_rn(__dmul_rn(u0, gamma), beta), kp.m_e_eV);
     xp[4] = __dmul_rn(__dmul_rn(__dmul_rn(u1, gamma), beta), kp.m_e_eV);
     xp[5] = __dmul_rn(__dmul_rn(__dmul_rn(u2, gamma), beta), kp.m_e_eV);
-}
-
-// xp_2_xxstg_mad (coord_transform.py:16-54); pos = lab x,y,z, p = new momenta
-__device__ __forceinline__ void cart_to_mad64(const double pos[3], const double p[3], const KickParams& kp,
-                                              double r[6]) {
-    const double s = __dadd_rn(__dadd_rn(__dmul_rn(p[0], p[0]), __dmul_rn(p[1], p[1])), __dmul_rn(p[2], p[2]));
-    const double gamma = __dsqrt_rn(__dadd_rn(1.0, div_rb(s, kp.m2, kp.r_m2)));
-    const double beta = __dsqrt_rn(__dsub_rn(1.0, __drcp_rn(__dmul_rn(gamma, gamma))));
-    const double p0 = __dsqrt_rn(s);
-    const double rp0 = __drcp_rn(p0);
-    const double u0 = div_rb(p[0], p0, rp0), u1 = div_rb(p[1], p0, rp0), u2 = div_rb(p[2], p0, rp0);
-    const double cdt = __ddiv_rn(-pos[2], __dmul_rn(beta, u2));
-    r[0] = __dadd_rn(pos[0], __dmul_rn(__dmul_rn(beta, u0), cdt));
-    r[2] = __dadd_rn(pos[1], __dmul_rn(__dmul_rn(beta, u1), cdt));
-    r[5] = div_rb(__dsub_rn(div_rb(gamma, kp.gamref, kp.r_gamref), 1.0), kp.betaref, kp.r_betaref);
-    r[4] = cdt;
-    r[1] = div_rb(p[0], kp.pref, kp.r_pref);
-    r[3] = div_rb(p[1], kp.pref, kp.r_pref);
 }
 
 // numpy's [N,3]@[3,3] row product: fma(a2,b2, fma(a1,b1, a0*b0))
@@ -646,20 +577,6 @@ __device__ __forceinline__ void frame_finish(const double* acc, const KickParams
     }
 }
 
-__device__ void frame_finalize(const double* part, int nblk, const KickParams& kp, ScState* st) {
-    __shared__ double sm[3 * 32];
-    __shared__ double s_acc[3];
-    double acc[3] = {0.0, 0.0, 0.0};
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-        for (int k = 0; k < 3; ++k) acc[k] += __ldcg(part + b * 3 + k);
-    block_sum<3>(acc, sm);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 3; ++k) s_acc[k] = acc[k];
-    __syncthreads();
-    frame_finish(s_acc, kp, st);
-}
-
-
 // FP32 form: a block's sums of the frame pass as double-float pairs: the
 // momenta (0..2), charge times lab position (3..5), charge (6), |charge| (7).
 // The last block reduces them on the FP32 pipes, one quantity per warp (a
@@ -699,6 +616,19 @@ struct MeshPre {
     }
 };
 
+// The FP64 form's: the momenta in units of the reference momentum.
+__device__ void frame_finalize64(const double* part, int nblk, const KickParams& kp, ScState* st) {
+    __shared__ double s_acc[3];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double v = 0.0;
+#pragma unroll 4
+    for (int b = lane; b < nblk; b += 32) v += __ldcg(part + b * FRAME_PART + w);
+    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(FULL, v, o);
+    if (lane == 0) (w < 3 ? s_acc[w] : st->qmom[w - 3]) = w < 3 ? v * kp.pref : v;
+    __syncthreads();
+    frame_finish(s_acc, kp, st);
+}
+
 // steps, X_off, potential scale, Green cache check (sc.py:172-186, 167)
 // part layout per block (PART_EXT doubles): min[3], max[3], sum q*x[3], sum q, sum |q|
 // lab_sums: the sums q*x are of lab positions (the kick's frame pass); they are
@@ -709,7 +639,8 @@ struct MeshPre {
 // axis k with the serial FP64 operations of sc.py:172-186, so the divisions
 // of the three axes run side by side.
 __device__ __forceinline__ void mesh_finish(const double* mn, const double* mx, const double* qs, const MeshPre& pre,
-                                            const KickParams& kp, ScState* st, double gamma_override, bool lab_sums) {
+                                            const KickParams& kp, ScState* st, double gamma_override, bool lab_sums,
+                                            bool kick64 = false) {
     const int lane = threadIdx.x, k = lane < 3 ? lane : 0;
     if (lane == 0) {
         st->done_extent = 0;
@@ -788,6 +719,17 @@ __device__ __forceinline__ void mesh_finish(const double* mn, const double* mx, 
         st->qfix_scale = ldexp(1.0, S);
         st->qfix_inv = (float)ldexp(1.0, -S);
     }
+    if (kick64) {  // kick64_one's two matrices, entry (lane / 3, lane % 3) in lane 0..8
+        const int i = lane / 3 % 3;
+        const double t = i == 0 ? pre.T[0] : i == 1 ? pre.T[1] : pre.T[2];
+        const double ist = __shfl_sync(FULL, r1, 6 + a);
+        const double tg = (a == 2 ? t * pre.gamma0 : t) * ist;
+        const double tk = t * ((a == 2 ? st->kz : st->kxy * pre.gamma0) * kp.r_pref);
+        if (lane < 9) {
+            st->Tg[i][a] = tg;
+            st->Tk[i][a] = tk;
+        }
+    }
     if (lane == 0) {
         st->phi_denom = pden;
         st->phi_scalef = (float)scale;
@@ -795,8 +737,8 @@ __device__ __forceinline__ void mesh_finish(const double* mn, const double* mx, 
     }
 }
 
-__device__ void mesh_finalize(const double* part, int nblk, const KickParams& kp, ScState* st, double gamma_override,
-                              bool lab_sums = false) {
+__device__ void mesh_finalize(const double* part, int nblk, const KickParams& kp, ScState* st,
+                              double gamma_override) {
     __shared__ double sm[5 * 32];
     double mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
     double qs[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
@@ -824,34 +766,97 @@ __device__ void mesh_finalize(const double* part, int nblk, const KickParams& kp
     __syncthreads();
     if (threadIdx.x >= 32) return;
     MeshPre pre;
-    pre.load(st, lab_sums);
-    mesh_finish(s_fin, s_fin + 3, s_fin + 6, pre, kp, st, gamma_override, lab_sums);
+    pre.load(st, false);
+    mesh_finish(s_fin, s_fin + 3, s_fin + 6, pre, kp, st, gamma_override, false);
 }
 
 // ---------------------------------------------------------------------------
-// frame: sum of momenta (+ FP64: lab coordinates stored for later stages)
+// frame: momentum sums, lab positions (FP32) and their charge moments
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(PT) k_frame64(const double* __restrict__ rp, KickParams kp,
-                                                double* __restrict__ xp, double* __restrict__ part, ScState* st) {
+// FP64 1/x and sqrt(x) for positive x well inside the exponent range: the
+// hardware's approximation and two Newton-Raphson steps (the square root by
+// Goldschmidt's iteration with a final residual correction).  Within an ulp or
+// so of the exact value, not always correctly rounded; five and eight FP64
+// instructions instead of the dozen of the IEEE forms with their range checks.
+__device__ __forceinline__ double rcp64(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    y = fma(y, fma(-x, y, 1.0), y);
+    return fma(y, fma(-x, y, 1.0), y);
+}
+// one Newton-Raphson step: ~2^-44 relative, for a factor of a small increment
+__device__ __forceinline__ double rcp64_once(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return fma(y, fma(-x, y, 1.0), y);
+}
+__device__ __forceinline__ double sqrt64(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    double g = x * y, h = 0.5 * y;
+    const double r = fma(-g, h, 0.5);
+    g = fma(g, r, g);
+    h = fma(h, r, h);
+    return fma(fma(-g, g, x), h, g);
+}
+
+// One particle of the FP64 form in units of the reference momentum pref (and
+// pref c for the energy).  With x', y' the transverse momenta and delta =
+// (E - E_ref) / (pref c),
+//   e = 1/beta_ref + delta,  |p|^2 = e^2 - (m c / pref)^2 = 1 + delta (delta + 2/beta_ref),
+//   pz = sqrt(|p|^2 - x'^2 - y'^2),  lab position (x, y, 0) - tau p / e
+// -- xxstg_2_xp_mad (coord_transform.py:57-96) with its normalisations
+// cancelled: 20 FP64 instructions instead of 95.
+struct Mad64 {
+    double pz, e, s;  // s = tau / e
+    double l[3];      // lab position
+};
+__device__ __forceinline__ Mad64 mad64(double x, double xq, double y, double yq, double tau, double d,
+                                       const KickParams& kp) {
+    Mad64 m;
+    m.e = kp.r_betaref + d;
+    m.pz = sqrt64(fma(-xq, xq, fma(-yq, yq, fma(d, d + 2.0 * kp.r_betaref, 1.0))));
+    m.s = tau * rcp64(m.e);
+    m.l[0] = fma(-xq, m.s, x);
+    m.l[1] = fma(-yq, m.s, y);
+    m.l[2] = -(m.pz * m.s);
+    return m;
+}
+
+// bound by the FP64 pipe, 28 instructions per particle (it read the rows and
+// stored six FP64 lab coordinates with 98 before: 2M particles 344 -> 114 us)
+__global__ void __launch_bounds__(PT) k_frame64(const double* __restrict__ rp, const double* __restrict__ q,
+                                                KickParams kp, float* __restrict__ X, double* __restrict__ part,
+                                                ScState* st) {
     pdl_wait();
-    __shared__ double sm[3 * 32];
-    double acc[3] = {0.0, 0.0, 0.0};
-    const int64_t n = kp.n, ld = kp.ld;
+    __shared__ double sm[8][PT];
+    double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    const int64_t n = kp.n, ld = kp.ld, nX = kp.nX;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double r[6], c[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) r[k] = rp[k * ld + i];
-        mad_to_cart64(r, kp, c);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) xp[k * n + i] = c[k];
-        acc[0] += c[3];
-        acc[1] += c[4];
-        acc[2] += c[5];
+        const double xq = rp[ld + i], yq = rp[3 * ld + i], qi = q[i];
+        const Mad64 m = mad64(rp[i], xq, rp[2 * ld + i], yq, rp[4 * ld + i], rp[5 * ld + i], kp);
+        a[0] += xq;
+        a[1] += yq;
+        a[2] += m.pz;
+        for (int j = 0; j < 3; ++j) {
+            a[3 + j] = fma(qi, m.l[j], a[3 + j]);
+            X[j * nX + i] = d2f(m.l[j]);
+        }
+        a[6] += qi;
+        a[7] += fabs(qi);
     }
-    block_sum<3>(acc, sm);
-    if (threadIdx.x == 0)
-        for (int k = 0; k < 3; ++k) part[blockIdx.x * 3 + k] = acc[k];
-    if (arrive_last(&st->done_frame, gridDim.x)) frame_finalize(part, gridDim.x, kp, st);
+    // the block's sums, one quantity per warp: 13 FP64 additions per warp (a
+    // shuffle tree in every warp over all eight would be 40)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sm[k][threadIdx.x] = a[k];
+    __syncthreads();
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double v = 0.0;
+#pragma unroll
+    for (int u = 0; u < PT / 32; ++u) v += sm[w][lane + 32 * u];
+    for (int o = 16; o; o >>= 1) v += __shfl_down_sync(FULL, v, o);
+    if (lane == 0) part[blockIdx.x * FRAME_PART + w] = v;
+    if (arrive_last(&st->done_frame, gridDim.x)) frame_finalize64(part, gridDim.x, kp, st);
 }
 
 // Pair-wise particle loop of the FP32 kernels: with VEC each thread takes two
@@ -1060,38 +1065,6 @@ __device__ __forceinline__ void extent_block_out(double (&mn)[3], double (&mx)[3
     }
 }
 
-__global__ void __launch_bounds__(PT) k_extent64(const double* __restrict__ xp, const double* __restrict__ q,
-                                                 KickParams kp, double* __restrict__ X, double* __restrict__ part,
-                                                 ScState* st) {
-    pdl_wait();
-    __shared__ double sm[5 * 32];
-    double mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-    double qs[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-    const int64_t n = kp.n;
-    const bool ok = st->status == SC_OK;
-    double T[3][3];
-    for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) T[i][j] = st->T[i][j];
-    const double g0 = st->gamma0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; ok && i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double a0 = xp[i], a1 = xp[n + i], a2 = xp[2 * n + i];
-        double v[3];
-        for (int j = 0; j < 3; ++j) v[j] = dot3_blas(a0, a1, a2, T[0][j], T[1][j], T[2][j]);
-        v[2] = __dmul_rn(v[2], g0);
-        const double qi = q[i];
-        for (int j = 0; j < 3; ++j) {
-            X[j * kp.nX + i] = v[j];
-            mn[j] = fmin(mn[j], v[j]);
-            mx[j] = fmax(mx[j], v[j]);
-            qs[j] += qi * v[j];
-        }
-        qs[3] += qi;
-        qs[4] += fabs(qi);
-    }
-    extent_block_out(mn, mx, qs, sm, part, blockIdx.x);
-    if (arrive_last(&st->done_extent, gridDim.x)) mesh_finalize(part, gridDim.x, kp, st, -1.0);
-}
-
 // Rotated position (z scaled by gamma0) of particle i with the FP64 form's
 // operations, for the few particles whose FP32 position is too close to a
 // cell face or to the extent to decide.  (Forming only the lab position's
@@ -1102,8 +1075,8 @@ __global__ void __launch_bounds__(PT) k_extent64(const double* __restrict__ xp, 
 // so the keys agree except for a particle within ~1e-14 cells of a face.
 __device__ __forceinline__ void xyz_fine(const double* __restrict__ rp, int64_t ld, int64_t i, const KickParams& kp,
                                          const double (&T)[3][3], double g0, double v[3]) {
-    // the FP64 form's operations: xxstg_2_xp_mad, the BLAS-order rotation
-    // and the gamma0 product (k_frame64, k_extent64)
+    // the reference's operations: xxstg_2_xp_mad, the BLAS-order rotation
+    // and the gamma0 product (sc.py:218-233)
     double r[6], xp[6];
     for (int k = 0; k < 6; ++k) r[k] = rp[k * ld + i];
     mad_to_cart64(r, kp, xp);
@@ -1220,7 +1193,8 @@ static_assert(EX_BLOCKS * sizeof(uint32_t) <= EX_BUF, "the last block lists bloc
 // (many particles sharing an extreme coordinate) evaluates its own, so that
 // the last block's share stays bounded.  2M / 64^3, frame + extent: 71 -> 58 us.
 __device__ __forceinline__ void extent_body(const double* __restrict__ rp, const float* __restrict__ X,
-                                            const KickParams& kp, ExtPart* __restrict__ ep, ScState* st, VBlk vb) {
+                                            const KickParams& kp, ExtPart* __restrict__ ep, ScState* st, VBlk vb,
+                                            bool kick64 = false) {
     extern __shared__ __align__(128) unsigned char smraw[];
     __shared__ int smi[6 * 32];
     __shared__ unsigned long long emin[3], emax[3];
@@ -1394,13 +1368,13 @@ __device__ __forceinline__ void extent_body(const double* __restrict__ rp, const
         s_fin[3 + threadIdx.x] = unord64(emax[threadIdx.x]);
     }
     __syncwarp();
-    mesh_finish(s_fin, s_fin + 3, s_fin + 6, pre, kp, st, -1.0, true);
+    mesh_finish(s_fin, s_fin + 3, s_fin + 6, pre, kp, st, -1.0, true, kick64);
 }
 
 __global__ void __launch_bounds__(PT, 3) k_extent(const double* __restrict__ rp, const float* __restrict__ X,
-                                                  KickParams kp, ExtPart* __restrict__ ep, ScState* st) {
+                                                  KickParams kp, ExtPart* __restrict__ ep, ScState* st, int kick64) {
     pdl_wait();
-    extent_body(rp, X, kp, ep, st, hw_vblk());
+    extent_body(rp, X, kp, ep, st, hw_vblk(), kick64 != 0);
 }
 
 // el_field entry: X given as [n][3] rotated positions; z scaled by gamma in place
@@ -1467,15 +1441,8 @@ __device__ __forceinline__ bool key_of(double fx, double fy, double fz, const Ki
     return in;
 }
 
-// FP64: whether 0 <= c <= hi (c = -0.0 included, NaN excluded) and floor(c)
-// for such c, both on the bit pattern: the order of non-negative doubles is
-// the order of their bits, and the integer part is the significand shifted
-// by the exponent.  Equal to the double compares and floor(), without the
-// FP64 pipe, which this GPU issues at a fraction of its integer rate.
-__device__ __forceinline__ bool in_range64(double c, double hi) {
-    const long long b = __double_as_longlong(c);
-    return (b >= 0 || b == (long long)0x8000000000000000ull) && b <= __double_as_longlong(hi);
-}
+// floor(c) of a non-negative double from its bit pattern (the significand
+// shifted by the exponent): no FP64 instruction
 __device__ __forceinline__ int floor_nonneg64(double c) {  // 0 <= c < 2^31
     const long long b = __double_as_longlong(c);
     const int e = (int)((b >> 52) & 0x7ff) - 1023;
@@ -1602,7 +1569,8 @@ constexpr int KEYS_FINE = 1024;
 // atomics: deterministic, the same alone and in a batch.
 // rp != nullptr (the kick): X holds lab positions, rotated here as the extent
 // pass rotates them.
-template <bool VEC>
+// EXACT (the FP64 form): the particles beyond the list take the exact key too.
+template <bool VEC, bool EXACT = false>
 __device__ __forceinline__ void keys32_body(float* __restrict__ X, uint32_t* __restrict__ keys,
                                             const double* __restrict__ rp, const double* __restrict__ q,
                                             unsigned long long* __restrict__ qfix, const KickParams& kp, ScState* st,
@@ -1721,6 +1689,13 @@ __device__ __forceinline__ void keys32_body(float* __restrict__ X, uint32_t* __r
             slow &= slow - 1;
             const int64_t p_ = pg_ + (bit >> 1) * pstride_;
             const int64_t i = (VEC && p_ < npair_ ? 2 * p_ : (VEC ? n - 1 : p_)) + (bit & 1);
+            if constexpr (EXACT) {
+                uint32_t key = 0u;
+                float gf[3];
+                bad |= !key_fine(rp, ld, i, kp, st, key, gf);
+                keys[i] = key;
+                continue;
+            }
             double xv[3], e[3];
             xyz_fine32(rp, ld, i, kp, st->T, st->gamma0, xv);
             for (int j = 0; j < 3; ++j)  // the FP64 form's grid coordinate (k_keys64)
@@ -1749,61 +1724,71 @@ __device__ __forceinline__ void keys32_body(float* __restrict__ X, uint32_t* __r
     if (bad) atomicCAS(&st->status, SC_OK, SC_ERR_NONFINITE);
 }
 
-template <bool VEC>
+template <bool VEC, bool EXACT = false>
 __global__ void __launch_bounds__(PT, 4) k_keys32(float* __restrict__ X, uint32_t* __restrict__ keys,
                                                   const double* __restrict__ rp, const double* __restrict__ q,
                                                   unsigned long long* __restrict__ qfix, KickParams kp, ScState* st) {
     pdl_wait();
-    keys32_body<VEC>(X, keys, rp, q, qfix, kp, st, hw_vblk());
+    keys32_body<VEC, EXACT>(X, keys, rp, q, qfix, kp, st, hw_vblk());
 }
 
 // ---------------------------------------------------------------------------
 // trilinear gather, scipy.ndimage.map_coordinates(order=1, mode='constant')
 // semantics: a sample outside [0, n-1] in any axis is 0
 // ---------------------------------------------------------------------------
-template <typename R>
-__device__ __forceinline__ R trilerp(const R* __restrict__ F, int nx, int ny, int nz, R c0, R c1, R c2) {
-    int i, j, k;
-    if constexpr (sizeof(R) == 8) {
-        if (!in_range64(c0, nx - 1) || !in_range64(c1, ny - 1) || !in_range64(c2, nz - 1)) return 0;
-        i = floor_nonneg64(c0);
-        j = floor_nonneg64(c1);
-        k = floor_nonneg64(c2);
-    } else {
-        if (!(c0 >= 0) || !(c1 >= 0) || !(c2 >= 0) || c0 > nx - 1 || c1 > ny - 1 || c2 > nz - 1) return 0;
-        i = (int)floor(c0);
-        j = (int)floor(c1);
-        k = (int)floor(c2);
-    }
-    if (i > nx - 2) i = nx - 2;
-    if (j > ny - 2) j = ny - 2;
-    if (k > nz - 2) k = nz - 2;
-    const R tx = c0 - i, ty = c1 - j, tz = c2 - k;
-    const R wx[2] = {1 - tx, tx}, wy[2] = {1 - ty, ty}, wz[2] = {1 - tz, tz};
-    const R* b = F + ((size_t)i * ny + j) * nz + k;
-    R acc = 0;
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-        for (int bb = 0; bb < 2; ++bb)
-#pragma unroll
-            for (int cc = 0; cc < 2; ++cc) {
-                const R f = b[((size_t)a * ny + bb) * nz + cc];
-                if (sizeof(R) == 8)
-                    acc = (R)__dadd_rn((double)acc, __dmul_rn(__dmul_rn(__dmul_rn((double)f, (double)wx[a]), (double)wy[bb]), (double)wz[cc]));
-                else
-                    acc += f * wx[a] * wy[bb] * wz[cc];
-            }
-    return acc;
+// FP64: cell and weight of a grid coordinate X along one axis of length n,
+// plain (a) and at the half-cell-staggered coordinate X + 0.5 (b), each clamped
+// into the mesh with whether the sample is valid.  floor(X) and the range tests
+// work on integers and the staggered pair follows from the plain one: two FP64
+// instructions per axis.
+struct Axis64 {
+    int ia, ib;
+    double ta, tb;
+    bool oka, okb;
+};
+__device__ __forceinline__ bool zero64(double v) { return (__double_as_longlong(v) << 1) == 0; }
+__device__ __forceinline__ Axis64 axis64(double X, int n) {
+    Axis64 A;
+    const int hi = __double2hiint(X);
+    const bool neg = hi < 0;
+    // |X| >= 2^20, infinities and NaN: outside every mesh
+    const bool far = (hi & 0x7fffffff) >= 0x41300000;
+    int i = far ? -2 : (neg ? -1 : floor_nonneg64(X));
+    if (neg && (hi & 0x7fffffff) > 0x3ff00000) i = -2;  // below -1 (to the high word): no sample either way
+    if (neg && zero64(X)) i = 0;  // -0
+    const double t = far ? 0.0 : X - f2d_exact((float)i);
+    const bool half = __double2hiint(t) >= 0x3fe00000;  // t >= 0.5 (t in [0, 1])
+    A.ta = t;
+    A.tb = t + (half ? -0.5 : 0.5);
+    A.ia = i;
+    A.ib = i + (half ? 1 : 0);
+    A.oka = A.ia >= 0 && (A.ia < n - 1 || (A.ia == n - 1 && zero64(A.ta)));
+    A.okb = A.ib >= 0 && (A.ib < n - 1 || (A.ib == n - 1 && zero64(A.tb)));
+    if (A.ia >= n - 1) A.ia = n - 2, A.ta = 1.0;
+    if (A.ib >= n - 1) A.ib = n - 2, A.tb = 1.0;
+    A.ia = A.ia < 0 ? 0 : A.ia;
+    A.ib = A.ib < 0 ? 0 : A.ib;
+    return A;
 }
-
-template <typename R>
-__device__ __forceinline__ void gather3(const R* ex, const R* ey, const R* ez, int nx, int ny, int nz, R X0, R X1,
-                                        R X2, R& e0, R& e1, R& e2) {
-    const R h = (R)0.5;
-    e0 = trilerp<R>(ex, nx, ny, nz, X0, X1 + h, X2 + h);
-    e1 = trilerp<R>(ey, nx, ny, nz, X0 + h, X1, X2 + h);
-    e2 = trilerp<R>(ez, nx, ny, nz, X0 + h, X1 + h, X2);
+__device__ __forceinline__ double lerp64(double a, double b, double t) { return fma(t, b - a, a); }
+__device__ __forceinline__ double sample64(const double* __restrict__ F, int i, int j, int k, double tx, double ty,
+                                           double tz, int ny, int nz, bool ok) {
+    const double* b = F + ((size_t)i * ny + j) * nz + k;
+    const size_t sx = (size_t)ny * nz;
+    const double y0 = lerp64(lerp64(b[0], b[1], tz), lerp64(b[nz], b[nz + 1], tz), ty);
+    const double y1 = lerp64(lerp64(b[sx], b[sx + 1], tz), lerp64(b[sx + nz], b[sx + nz + 1], tz), ty);
+    const double v = lerp64(y0, y1, tx);
+    return ok ? v : 0.0;
+}
+// the three staggered components at grid coordinates X: 48 FP64 instructions
+// (the eight-corner sums with their weights were 96)
+__device__ __forceinline__ void gather64(const double* __restrict__ ex, const double* __restrict__ ey,
+                                         const double* __restrict__ ez, int nx, int ny, int nz, const double (&X)[3],
+                                         double (&e)[3]) {
+    const Axis64 x = axis64(X[0], nx), y = axis64(X[1], ny), z = axis64(X[2], nz);
+    e[0] = sample64(ex, x.ia, y.ib, z.ib, x.ta, y.tb, z.tb, ny, nz, x.oka && y.okb && z.okb);
+    e[1] = sample64(ey, x.ib, y.ia, z.ib, x.tb, y.ta, z.tb, ny, nz, x.okb && y.oka && z.okb);
+    e[2] = sample64(ez, x.ib, y.ib, z.ia, x.tb, y.tb, z.ta, ny, nz, x.okb && y.okb && z.oka);
 }
 
 // trilinear sample from the FP32 gather octs (one 32-byte load)
@@ -1834,43 +1819,83 @@ __device__ __forceinline__ void gather3o(const float* ox, const float* oy, const
     e2 = trilerp_o(oz, nx, ny, nz, X0 + 0.5f, X1 + 0.5f, X2);
 }
 
+// Grid coordinates of particle i with the reference's operations (k_keys64's),
+// for the particles within rounding of the edge of the sampled range.
+__device__ __noinline__ void grid64_exact(const double* rp, int64_t ld, int64_t i, const KickParams* kp,
+                                          const ScState* st, double* X) {
+    double v[3];
+    xyz_fine(rp, ld, i, *kp, st->T, st->gamma0, v);
+    for (int j = 0; j < 3; ++j) X[j] = __dsub_rn(div_checked(v[j], st->steps[j], st->isteps[j]), st->xoff[j]);
+}
+// whether X lies within 1e-6 (1e-4 at the far end) of an edge of the plain or
+// staggered sampled range, where rounding decides between a sample and zero
+__device__ __forceinline__ bool near_edge64(double X, int n) {
+    const float x = d2f_kick(X), top = (float)(n - 1);
+    return fabsf(x) < 1e-6f || fabsf(x + 0.5f) < 1e-6f || fabsf(x - top) < 1e-4f || fabsf(x - (top - 0.5f)) < 1e-4f;
+}
+
+// Gather + kick of the FP64 form.  Bound by the FP64 pipe: 118 instructions per
+// particle, from rparticles alone, in units of the reference momentum (mad64):
+//   p' = p + Tk e   (Tk: the frame's rotation with the kick's factors, so the
+//                    rotation into the frame and back is done once, on e)
+//   e' = sqrt(|p'|^2 + (m c / pref)^2),  w = -z_lab / pz'
+//   tau' = w e',  x = x_lab + x' w,  delta' = delta + (|p'|^2 - |p|^2) / (e + e')
+// -- sc.py:218-250 and xp_2_xxstg_mad (coord_transform.py:16-54) with the
+// normalisations cancelled; the reference's operations took 226 and read 84
+// bytes a particle of stored coordinates (2M / 64^3: 885 -> 469 us).  (delta as
+// an increment: e' - 1/beta_ref, ten instructions less, carries the rounding
+// of e' ~ 1 into delta ~ 1e-3.)  The grid
+// coordinates are lab position x Tg - X_off (Tg: rotation, gamma0 and steps in
+// one matrix).
 // rec != nullptr (the record-field mode): the field samples before the gamma0
-// factor go to rec[i], rec[nX + i], rec[2 nX + i] (rec may be X itself: each
-// thread writes only the entries it has read)
-__global__ void __launch_bounds__(PT) k_kick64(double* __restrict__ rp, const double* __restrict__ xp,
-                                               const double* X, const double* __restrict__ ex,
+// factor go to rec[i], rec[nX + i], rec[2 nX + i]
+__global__ void __launch_bounds__(PT, 2) k_kick64(double* __restrict__ rp, const double* __restrict__ ex,
                                                const double* __restrict__ ey, const double* __restrict__ ez,
-                                               KickParams kp, const ScState* st, double* rec) {
+                                               const __grid_constant__ KickParams kp, const ScState* st,
+                                               double* __restrict__ rec) {
     pdl_wait();
     if (st->status) return;
     const int64_t n = kp.n, ld = kp.ld;
-    double T[3][3];
+    double Tg[3][3], Tk[3][3];
     for (int i = 0; i < 3; ++i)
-        for (int j = 0; j < 3; ++j) T[i][j] = st->T[i][j];
-    const double g0 = st->gamma0, kxy = st->kxy, kz = st->kz;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double e0, e1, e2;
-        gather3<double>(ex, ey, ez, kp.nx, kp.ny, kp.nz, X[i], X[kp.nX + i], X[2 * kp.nX + i], e0, e1, e2);
-        if (rec) {
-            rec[i] = e0;
-            rec[kp.nX + i] = e1;
-            rec[2 * kp.nX + i] = e2;
+        for (int j = 0; j < 3; ++j) {
+            Tg[i][j] = st->Tg[i][j];
+            Tk[i][j] = st->Tk[i][j];
         }
-        e0 = __dmul_rn(e0, g0);
-        e1 = __dmul_rn(e1, g0);
-        const double p0 = xp[3 * n + i], p1 = xp[4 * n + i], p2 = xp[5 * n + i];
-        double pr[3];
-        for (int j = 0; j < 3; ++j) pr[j] = dot3_blas(p0, p1, p2, T[0][j], T[1][j], T[2][j]);
-        pr[0] = __dadd_rn(pr[0], __dmul_rn(kxy, e0));
-        pr[1] = __dadd_rn(pr[1], __dmul_rn(kxy, e1));
-        pr[2] = __dadd_rn(pr[2], __dmul_rn(kz, e2));
-        double pn[3];
-        for (int k = 0; k < 3; ++k) pn[k] = dot3_blas(pr[0], pr[1], pr[2], T[k][0], T[k][1], T[k][2]);
-        const double pos[3] = {xp[i], xp[n + i], xp[2 * n + i]};
-        double r[6];
-        cart_to_mad64(pos, pn, kp, r);
-#pragma unroll
-        for (int k = 0; k < 6; ++k) rp[k * ld + i] = r[k];
+    const double o0 = st->xoff[0], o1 = st->xoff[1], o2 = st->xoff[2];
+    const double mu2 = kp.r_grbr * kp.r_grbr;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double xq = rp[ld + i], yq = rp[3 * ld + i];
+        const Mad64 m = mad64(rp[i], xq, rp[2 * ld + i], yq, rp[4 * ld + i], rp[5 * ld + i], kp);
+        double X[3] = {fma(m.l[2], Tg[2][0], fma(m.l[1], Tg[1][0], fma(m.l[0], Tg[0][0], -o0))),
+                       fma(m.l[2], Tg[2][1], fma(m.l[1], Tg[1][1], fma(m.l[0], Tg[0][1], -o1))),
+                       fma(m.l[2], Tg[2][2], fma(m.l[1], Tg[1][2], fma(m.l[0], Tg[0][2], -o2)))};
+        if (near_edge64(X[0], kp.nx) || near_edge64(X[1], kp.ny) || near_edge64(X[2], kp.nz)) {
+            double Xe[3];
+            grid64_exact(rp, ld, i, &kp, st, Xe);
+            for (int j = 0; j < 3; ++j) X[j] = Xe[j];
+        }
+        double e[3];
+        gather64(ex, ey, ez, kp.nx, kp.ny, kp.nz, X, e);
+        if (rec) {
+            rec[i] = e[0];
+            rec[kp.nX + i] = e[1];
+            rec[2 * kp.nX + i] = e[2];
+        }
+        const double dx = fma(Tk[0][2], e[2], fma(Tk[0][1], e[1], Tk[0][0] * e[0]));
+        const double dy = fma(Tk[1][2], e[2], fma(Tk[1][1], e[1], Tk[1][0] * e[0]));
+        const double dz = fma(Tk[2][2], e[2], fma(Tk[2][1], e[1], Tk[2][0] * e[0]));
+        const double px = xq + dx, py = yq + dy, pz = m.pz + dz;
+        const double en = sqrt64(fma(px, px, fma(py, py, fma(pz, pz, mu2))));
+        const double dp2 = fma(dx, xq + px, fma(dy, yq + py, dz * (m.pz + pz)));  // |p'|^2 - |p|^2
+        const double w = -m.l[2] * rcp64(pz);
+        const double d = rp[5 * ld + i];
+        rp[i] = fma(px, w, m.l[0]);
+        rp[ld + i] = px;
+        rp[2 * ld + i] = fma(py, w, m.l[1]);
+        rp[3 * ld + i] = py;
+        rp[4 * ld + i] = w * en;
+        rp[5 * ld + i] = fma(dp2, rcp64_once(m.e + en), d);
     }
 }
 
@@ -2371,17 +2396,20 @@ __global__ void __launch_bounds__(PT) k_gather_xyz(const R* __restrict__ X, cons
     const int64_t n = kp.n, nX = kp.nX;
     const double g0 = st->gamma0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        R e0, e1, e2;
-        if (sizeof(R) == 4)
-            gather3o(reinterpret_cast<const float*>(ex), reinterpret_cast<const float*>(ey),
-                     reinterpret_cast<const float*>(ez), kp.nx, kp.ny, kp.nz, (float)X[i], (float)X[nX + i],
-                     (float)X[2 * nX + i], *reinterpret_cast<float*>(&e0), *reinterpret_cast<float*>(&e1),
-                     *reinterpret_cast<float*>(&e2));
-        else
-            gather3<R>(ex, ey, ez, kp.nx, kp.ny, kp.nz, X[i], X[nX + i], X[2 * nX + i], e0, e1, e2);
-        out[3 * i] = __dmul_rn((double)e0, g0);
-        out[3 * i + 1] = __dmul_rn((double)e1, g0);
-        out[3 * i + 2] = (double)e2;
+        if constexpr (sizeof(R) == 8) {
+            const double c[3] = {X[i], X[nX + i], X[2 * nX + i]};
+            double e[3];
+            gather64(ex, ey, ez, kp.nx, kp.ny, kp.nz, c, e);
+            out[3 * i] = __dmul_rn(e[0], g0);
+            out[3 * i + 1] = __dmul_rn(e[1], g0);
+            out[3 * i + 2] = e[2];
+        } else {
+            float e0, e1, e2;
+            gather3o(ex, ey, ez, kp.nx, kp.ny, kp.nz, X[i], X[nX + i], X[2 * nX + i], e0, e1, e2);
+            out[3 * i] = __dmul_rn((double)e0, g0);
+            out[3 * i + 1] = __dmul_rn((double)e1, g0);
+            out[3 * i + 2] = (double)e2;
+        }
     }
 }
 
@@ -2553,7 +2581,7 @@ cudaError_t launch_frame(const Plan& p, const Layout& L, char* ws, const KickPar
     double* part = reinterpret_cast<double*>(ws + L.part_frame);
     const int nb = particle_blocks(p, kp.n);
     if (p.prec == SC_FP64)
-        launch(k_frame64, nb, PT, 0, s, rp, kp, reinterpret_cast<double*>(ws + L.xp), part, st);
+        launch(k_frame64, nb, PT, 0, s, rp, q, kp, reinterpret_cast<float*>(ws + L.X), part, st);
     else {
         // the exact deposit's fixed-point grid is zeroed here, so the keys
         // kernel follows the extent kernel without a memset between them
@@ -2567,16 +2595,10 @@ cudaError_t launch_frame(const Plan& p, const Layout& L, char* ws, const KickPar
 }
 
 cudaError_t launch_extent(const Plan& p, const Layout& L, char* ws, const KickParams& kp, const double* rp,
-                          const double* q, cudaStream_t s) {
-    ScState* st = reinterpret_cast<ScState*>(ws + L.state);
-    double* part = reinterpret_cast<double*>(ws + L.part_ext);
-    const int nb = particle_blocks(p, kp.n);
-    if (p.prec == SC_FP64)
-        launch(k_extent64, nb, PT, 0, s, reinterpret_cast<const double*>(ws + L.xp), q, kp,
-                                     reinterpret_cast<double*>(ws + L.X), part, st);
-    else
-        launch(k_extent, nb, PT, EX_SMEM, s, rp, reinterpret_cast<const float*>(ws + L.X), kp,
-               reinterpret_cast<ExtPart*>(part), st);
+                          cudaStream_t s) {
+    launch(k_extent, particle_blocks(p, kp.n), PT, EX_SMEM, s, rp, reinterpret_cast<const float*>(ws + L.X), kp,
+           reinterpret_cast<ExtPart*>(ws + L.part_ext), reinterpret_cast<ScState*>(ws + L.state),
+           p.prec == SC_FP64 ? 1 : 0);
     return cudaGetLastError();
 }
 
@@ -2604,7 +2626,10 @@ cudaError_t launch_keys(const Plan& p, const Layout& L, char* ws, const KickPara
     ScState* st = reinterpret_cast<ScState*>(ws + L.state);
     const int nb = particle_blocks(p, kp.n);
     uint32_t* keys = reinterpret_cast<uint32_t*>(ws + L.keys);
-    if (p.prec == SC_FP64)
+    if (p.prec == SC_FP64 && rp)
+        launch(k_keys32<true, true>, nb, PT, 0, s, reinterpret_cast<float*>(ws + L.X), keys, rp, (const double*)nullptr,
+               (unsigned long long*)nullptr, kp, st);
+    else if (p.prec == SC_FP64)
         launch(k_keys64, nb, PT, 0, s, reinterpret_cast<double*>(ws + L.X), keys, kp, st);
     else
     {
@@ -2629,10 +2654,9 @@ cudaError_t launch_gather_kick(const Plan& p, const Layout& L, char* ws, const K
     const ScState* st = reinterpret_cast<const ScState*>(ws + L.state);
     const int nb = particle_blocks(p, kp.n);
     if (p.prec == SC_FP64)
-        launch(k_kick64, nb, PT, 0, s, rp, reinterpret_cast<const double*>(ws + L.xp),
-                                   reinterpret_cast<const double*>(ws + L.X), reinterpret_cast<const double*>(ws + L.ex),
-                                   reinterpret_cast<const double*>(ws + L.ey), reinterpret_cast<const double*>(ws + L.ez),
-                                   kp, st, p.record_field ? reinterpret_cast<double*>(ws + L.X) : nullptr);
+        launch(k_kick64, nb, PT, 0, s, rp, reinterpret_cast<const double*>(ws + L.ex),
+               reinterpret_cast<const double*>(ws + L.ey), reinterpret_cast<const double*>(ws + L.ez), kp, st,
+               p.record_field ? reinterpret_cast<double*>(ws + L.X) : nullptr);
     else
     {
         const float* ox = reinterpret_cast<const float*>(ws + L.exq);
