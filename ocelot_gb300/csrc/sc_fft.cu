@@ -24,6 +24,10 @@
 namespace ocsc {
 
 constexpr int FFT_THREADS = 256;
+// FP64: two blocks per SM at least (128 registers), so that one block's loads
+// overlap the other's arithmetic
+template <typename R>
+constexpr int FFT_MINB = sizeof(R) == 8 ? 2 : 0;  // 0: no bound
 
 // complex lines (two real lines each) per block of the z passes: up to 8,
 // so that a 64^3 mesh gives 256 blocks
@@ -152,7 +156,7 @@ __device__ __forceinline__ void zfwd_body(R* __restrict__ q, const long long* __
     const int y0 = vb.x * 2 * NC;
     stage_charge_lines<R>(q, qfix, a, lz, x, y0, NC, ny, nz, Mz, st, (long long)vb.ny * ny * nz, 21);
     __syncthreads();
-    Cx<R>* res = fft_lines<R, false>(a, b, lz, NC, rz, tw);
+    Cx<R>* res = fft_lines<R, false, true>(a, b, lz, NC, rz, tw);
     for (DivWalk w(threadIdx.x, blockDim.x, Kz); w.q < NC; w.next()) {
         const int c = w.q, k = w.r;
         const int ya = y0 + 2 * c, yb = ya + 1;
@@ -166,7 +170,7 @@ __device__ __forceinline__ void zfwd_body(R* __restrict__ q, const long long* __
 }
 
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS) k_zfwd(R* __restrict__ q, const long long* __restrict__ qfix,
+__global__ void __launch_bounds__(FFT_THREADS, FFT_MINB<R>) k_zfwd(R* __restrict__ q, const long long* __restrict__ qfix,
                                                       Cx<R>* __restrict__ W, int ny, int nz, int My, int Kz,
                                                       RadixPlan rz, const Cx<R>* __restrict__ twg, int NC,
                                                       const ScState* st) {
@@ -218,13 +222,13 @@ __device__ __forceinline__ void ypass_body(Cx<R>* __restrict__ W, int nx, int ny
         }
     }
     __syncthreads();
-    Cx<R>* res = fft_lines<R, INV>(a, b, ls, TK, ry, tw);
+    Cx<R>* res = fft_lines<R, INV, true>(a, b, ls, TK, ry, tw);
     const int nout = INV ? ny : My;
     if (live)
         for (int y = cm.r0; y < nout; y += cm.rs) W[base + (size_t)y * Kz] = res[cm.kk * ls + y];
     if (W3) {
         __syncthreads();  // a and b are free
-        Cx<R>* res3 = fft_lines<R, INV>(c, a, ls, TK, ry, tw);
+        Cx<R>* res3 = fft_lines<R, INV, true>(c, a, ls, TK, ry, tw);
         if (live)
             for (int y = cm.r0; y < nout; y += cm.rs) W3[base + (size_t)y * Kz] = res3[cm.kk * ls + y];
     }
@@ -233,7 +237,7 @@ __device__ __forceinline__ void ypass_body(Cx<R>* __restrict__ W, int nx, int ny
 // blockIdx.y = 0: W (and, with spectral fields, W x D(ky) into W3);
 // blockIdx.y = 1 (inverse, spectral fields): the x-differenced grid W2 in place
 template <typename R, bool INV>
-__global__ void __launch_bounds__(FFT_THREADS) k_ypass(Cx<R>* __restrict__ W, int nx, int ny, int My, int Kz,
+__global__ void __launch_bounds__(FFT_THREADS, FFT_MINB<R>) k_ypass(Cx<R>* __restrict__ W, int nx, int ny, int My, int Kz,
                                                        RadixPlan ry, const Cx<R>* __restrict__ twg,
                                                        int TK, const ScState* st, Spec<R> sp) {
     pdl_wait();
@@ -282,7 +286,7 @@ __device__ __forceinline__ void xconv_body(Cx<R>* __restrict__ W, const R* __res
             if (x0 + u * cm.rs < Mx) la[x0 + u * cm.rs] = v[u];
     }
     __syncthreads();
-    Cx<R>* res = fft_lines<R, false>(a, b, ls, TK, rx, tw);
+    Cx<R>* res = fft_lines<R, false, true>(a, b, ls, TK, rx, tw);
     Cx<R>* lr = res + cm.kk * ls;
     Cx<R>* lc = c + cm.kk * ls;
     for (int x0 = cm.r0; x0 < Mx; x0 += U * cm.rs) {
@@ -309,19 +313,19 @@ __device__ __forceinline__ void xconv_body(Cx<R>* __restrict__ W, const R* __res
         }
     }
     __syncthreads();
-    Cx<R>* res2 = fft_lines<R, true>(res, res == a ? b : a, ls, TK, rx, tw);
+    Cx<R>* res2 = fft_lines<R, true, true>(res, res == a ? b : a, ls, TK, rx, tw);
     if (live)
         for (int x = cm.r0; x < nx; x += cm.rs) W[(size_t)x * ncol + col] = res2[cm.kk * ls + x];
     if (W2) {
         __syncthreads();  // a and b are free
-        Cx<R>* res3 = fft_lines<R, true>(c, a, ls, TK, rx, tw);
+        Cx<R>* res3 = fft_lines<R, true, true>(c, a, ls, TK, rx, tw);
         if (live)
             for (int x = cm.r0; x < nx; x += cm.rs) W2[(size_t)x * ncol + col] = res3[cm.kk * ls + x];
     }
 }
 
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS) k_xconv(Cx<R>* __restrict__ W, const R* __restrict__ G,
+__global__ void __launch_bounds__(FFT_THREADS, FFT_MINB<R>) k_xconv(Cx<R>* __restrict__ W, const R* __restrict__ G,
                                                        int nx, int My, int Kz, int Ky, RadixPlan rx,
                                                        const Cx<R>* __restrict__ twg, int TK, const ScState* st,
                                                        Spec<R> sp) {
@@ -391,7 +395,7 @@ __device__ __forceinline__ void zinv_body(const Cx<R>* __restrict__ W, R* __rest
         }
     }
     __syncthreads();
-    Cx<R>* res = fft_lines<R, true>(a, b, lz, NC, rz, tw);
+    Cx<R>* res = fft_lines<R, true, true>(a, b, lz, NC, rz, tw);
     const double norm = st->phi_norm, denom = st->phi_denom;
     const R fscale = (R)st->phi_scalef * mul;  // (float)(norm / denom), computed once by the mesh finalize
     for (DivWalk w(threadIdx.x, blockDim.x, nz); w.q < NC; w.next()) {
@@ -414,7 +418,7 @@ __device__ __forceinline__ void zinv_body(const Cx<R>* __restrict__ W, R* __rest
 
 // blockIdx.z: the output (0 the potential; with spectral fields 1 Ex, 2 Ey, 3 Ez)
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS) k_zinv(const Cx<R>* __restrict__ W, R* __restrict__ phi,
+__global__ void __launch_bounds__(FFT_THREADS, FFT_MINB<R>) k_zinv(const Cx<R>* __restrict__ W, R* __restrict__ phi,
                                                       int ny, int nz, int My, int Kz, RadixPlan rz,
                                                       const Cx<R>* __restrict__ twg, int NC,
                                                       const ScState* st, Spec<R> sp) {
@@ -548,7 +552,9 @@ __global__ void k_field_octs_spectral(const float* __restrict__ ex, const float*
 // lines use the second buffer (forward) or whichever buffer the y result
 // does not occupy (inverse).
 // ---------------------------------------------------------------------------
-constexpr int PLANE_THREADS = 1024;
+// FP64: 512, for the 128 registers of the two-step transforms
+template <typename R>
+constexpr int PLANE_THREADS = sizeof(R) == 8 ? 512 : 1024;
 
 template <typename R>
 static size_t plane_smem(const Plan& p) {
@@ -580,7 +586,7 @@ __device__ __forceinline__ void zy_fwd_body(R* __restrict__ q, const long long* 
     // F1: two charge rows per complex line (as k_zfwd)
     stage_charge_lines<R>(q, qfix, A1, lz, x, 0, ncz, ny, nz, Mz, st, (long long)nx * ny * nz, 25);
     __syncthreads();
-    const Cx<R>* res1 = fft_lines<R, false>(A1, B1, lz, ncz, rz, twz);
+    const Cx<R>* res1 = fft_lines<R, false, true>(A1, B1, lz, ncz, rz, twz);
     // unpack the two real lines into the y lines (column kz, row y); rows
     // ny..My-1 are the zero padding of F2
     for (DivWalk w(threadIdx.x, blockDim.x, Kz); w.q < ncz; w.next()) {
@@ -594,13 +600,13 @@ __device__ __forceinline__ void zy_fwd_body(R* __restrict__ q, const long long* 
     }
     for (DivWalk w(threadIdx.x, blockDim.x, Kz); w.q < My - ny; w.next()) A2[w.r * ly + ny + w.q] = cx<R>(0, 0);
     __syncthreads();
-    const Cx<R>* res2 = fft_lines<R, false>(A2, B2, ly, Kz, ry, twy);
+    const Cx<R>* res2 = fft_lines<R, false, true>(A2, B2, ly, Kz, ry, twy);
     Cx<R>* Wx = W + (size_t)x * My * Kz;  // the plane: row ky, column k at ky * Kz + k
     for (DivWalk w(threadIdx.x, blockDim.x, Kz); w.q < My; w.next()) Wx[w.q * Kz + w.r] = res2[w.r * ly + w.q];
 }
 
 template <typename R>
-__global__ void __launch_bounds__(PLANE_THREADS) k_zy_fwd(R* __restrict__ q, const long long* __restrict__ qfix,
+__global__ void __launch_bounds__(PLANE_THREADS<R>) k_zy_fwd(R* __restrict__ q, const long long* __restrict__ qfix,
                                                           Cx<R>* __restrict__ W, int ny, int nz, int My, int Kz,
                                                           RadixPlan rz, RadixPlan ry, const Cx<R>* __restrict__ twz,
                                                           const Cx<R>* __restrict__ twy, const ScState* st) {
@@ -647,7 +653,7 @@ __device__ __forceinline__ void yz_inv_body(const Cx<R>* __restrict__ W, R* __re
     }
     __syncthreads();
     // B2: inverse y; only rows y < ny are used
-    const Cx<R>* res2 = fft_lines<R, true>(A2, B2, ly, Kz, ry, twy);
+    const Cx<R>* res2 = fft_lines<R, true, true>(A2, B2, ly, Kz, ry, twy);
     Cx<R>* A1 = res2 == B2 ? A2 : B2;
     Cx<R>* B1 = A1 + ncz * lz;
     // B1: two output rows per complex line, Hermitian-extended (as k_zinv)
@@ -665,7 +671,7 @@ __device__ __forceinline__ void yz_inv_body(const Cx<R>* __restrict__ W, R* __re
         A1[c * lz + k] = lo ? cx<R>(A.x - B.y, A.y + B.x) : cx<R>(A.x + B.y, B.x - A.y);
     }
     __syncthreads();
-    const Cx<R>* res = fft_lines<R, true>(A1, B1, lz, ncz, rz, twz);
+    const Cx<R>* res = fft_lines<R, true, true>(A1, B1, lz, ncz, rz, twz);
     const double norm = st->phi_norm, denom = st->phi_denom;
     const R fscale = (R)st->phi_scalef * mul;  // (float)(norm / denom), computed once by the mesh finalize
     for (DivWalk w(threadIdx.x, blockDim.x, nz); w.q < ncz; w.next()) {
@@ -688,7 +694,7 @@ __device__ __forceinline__ void yz_inv_body(const Cx<R>* __restrict__ W, R* __re
 
 // blockIdx.y: the output (0 the potential; with spectral fields 1 Ex, 2 Ey, 3 Ez)
 template <typename R>
-__global__ void __launch_bounds__(PLANE_THREADS) k_yz_inv(const Cx<R>* __restrict__ W, R* __restrict__ phi, int ny,
+__global__ void __launch_bounds__(PLANE_THREADS<R>) k_yz_inv(const Cx<R>* __restrict__ W, R* __restrict__ phi, int ny,
                                                           int nz, int My, int Kz, RadixPlan rz, RadixPlan ry,
                                                           const Cx<R>* __restrict__ twz,
                                                           const Cx<R>* __restrict__ twy, const ScState* st,
@@ -772,7 +778,7 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
     const size_t smp = plane_smem<R>(p);
     if (plane_fwd && part != CONV_REST) {
         if ((e = set_smem(k_zy_fwd<R>, smp))) return e;
-        launch(k_zy_fwd<R>, p.nx, PLANE_THREADS, smp, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, p.ry, twz, twy, st);
+        launch(k_zy_fwd<R>, p.nx, PLANE_THREADS<R>, smp, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, p.ry, twz, twy, st);
     } else if (part != CONV_REST) {
         if ((e = set_smem(k_zfwd<R>, smz))) return e;
         launch(k_zfwd<R>, gz, FFT_THREADS, smz, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st);
@@ -787,7 +793,7 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
     const int nout = sp.W2 ? 4 - sp.f0 : 1;  // [the potential,] Ex, Ey, Ez
     if (plane_inv) {
         if ((e = set_smem(k_yz_inv<R>, smp))) return e;
-        launch(k_yz_inv<R>, dim3(p.nx, nout), PLANE_THREADS, smp, s, W, phi, p.ny, p.nz, p.My, Kz, p.rz, p.ry, twz, twy,
+        launch(k_yz_inv<R>, dim3(p.nx, nout), PLANE_THREADS<R>, smp, s, W, phi, p.ny, p.nz, p.My, Kz, p.rz, p.ry, twz, twy,
                st, sp);
         return cudaGetLastError();
     }
