@@ -23,11 +23,14 @@
 
 namespace ocsc {
 
-constexpr int FFT_THREADS = 256;
-// FP64: two blocks per SM at least (128 registers), so that one block's loads
-// overlap the other's arithmetic
+// FP64: blocks of 128 threads over half the columns (strided_cols), four or
+// more per SM (128 registers): the x pass of a 63^3 mesh is 1040 blocks, 6.8 per
+// SM, instead of 520, 3.4 (two resident: the second round half empty), and one
+// block's loads overlap the others' arithmetic
 template <typename R>
-constexpr int FFT_MINB = sizeof(R) == 8 ? 2 : 0;  // 0: no bound
+constexpr int FFT_THREADS = sizeof(R) == 8 ? 128 : 256;
+template <typename R>
+constexpr int FFT_MINB = sizeof(R) == 8 ? 4 : 0;  // 0: no bound
 
 // complex lines (two real lines each) per block of the z passes: up to 8,
 // so that a 64^3 mesh gives 256 blocks
@@ -39,7 +42,8 @@ static inline int z_lines_per_block(int Mz) {
 // of 16 columns would not fit in shared memory (FP64 at M = 512)
 template <typename R>
 static inline int strided_cols(int M, int nbuf = 2) {
-    int tk = 16;
+    // FP64: as many as give the block's 128 threads a work item each (Q per line, two_step_q64)
+    int tk = sizeof(R) == 8 && M > 64 ? 8 : 16;
     while (tk > 2 && sizeof(Cx<R>) * (size_t)(M + nbuf * tk * fft_ls(M)) > 200 * 1024) tk /= 2;
     return tk;
 }
@@ -79,6 +83,30 @@ struct Spec {
 template <typename R>
 __device__ __forceinline__ Cx<R> cmul(Cx<R> a, Cx<R> b) {
     return cx<R>(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+
+// Unpacking two real lines from one complex transform halves their sums; in
+// FP64 that factor rides on the potential's scale instead (out_scale64; a power
+// of two, so the same bits), four FP64 instructions per spectrum entry fewer.
+template <typename R>
+__device__ __forceinline__ constexpr R unpack_half() { return sizeof(R) == 8 ? (R)1 : (R)0.5; }
+template <typename R>
+__device__ __forceinline__ Cx<R> scaled(R re, R im, R h) {
+    if constexpr (sizeof(R) == 8) return cx<R>(re, im);
+    else return cx<R>(re * h, im * h);
+}
+// FP64 output: v / M / (4 pi eps0 hx hy hz) (sc.py:164-167); the division by
+// its reciprocal with one correction (correctly rounded up to the last bit's
+// ties), three instructions instead of the IEEE form's dozen
+struct OutScale64 {
+    double norm, denom, rdenom;
+    __device__ __forceinline__ double operator()(double v) const {
+        const double a = v * norm, q = a * rdenom;
+        return fma(fma(-q, denom, a), rdenom, q);
+    }
+};
+__device__ __forceinline__ OutScale64 out_scale64(const ScState* st) {
+    return OutScale64{0.5 * st->phi_norm, st->phi_denom, __drcp_rn(st->phi_denom)};
 }
 
 // Stage the charge of NC complex z lines into the line buffer a (line c at
@@ -162,15 +190,15 @@ __device__ __forceinline__ void zfwd_body(R* __restrict__ q, const long long* __
         const int ya = y0 + 2 * c, yb = ya + 1;
         const Cx<R> Z = res[c * lz + k];
         const Cx<R> Zm = res[c * lz + (k == 0 ? 0 : Mz - k)];
-        const R h = (R)0.5;
+        const R h = unpack_half<R>();
         if (!SC_IDX_OK(st, 24, ((long long)x * My + (yb < ny ? yb : ya)) * Kz + k, (long long)vb.ny * My * Kz)) continue;
-        if (ya < ny) W[((size_t)x * My + ya) * Kz + k] = cx<R>((Z.x + Zm.x) * h, (Z.y - Zm.y) * h);
-        if (yb < ny) W[((size_t)x * My + yb) * Kz + k] = cx<R>((Z.y + Zm.y) * h, (Zm.x - Z.x) * h);
+        if (ya < ny) W[((size_t)x * My + ya) * Kz + k] = scaled<R>(Z.x + Zm.x, Z.y - Zm.y, h);
+        if (yb < ny) W[((size_t)x * My + yb) * Kz + k] = scaled<R>(Z.y + Zm.y, Zm.x - Z.x, h);
     }
 }
 
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS, FFT_MINB<R>) k_zfwd(R* __restrict__ q, const long long* __restrict__ qfix,
+__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB<R>) k_zfwd(R* __restrict__ q, const long long* __restrict__ qfix,
                                                       Cx<R>* __restrict__ W, int ny, int nz, int My, int Kz,
                                                       RadixPlan rz, const Cx<R>* __restrict__ twg, int NC,
                                                       const ScState* st) {
@@ -237,7 +265,7 @@ __device__ __forceinline__ void ypass_body(Cx<R>* __restrict__ W, int nx, int ny
 // blockIdx.y = 0: W (and, with spectral fields, W x D(ky) into W3);
 // blockIdx.y = 1 (inverse, spectral fields): the x-differenced grid W2 in place
 template <typename R, bool INV>
-__global__ void __launch_bounds__(FFT_THREADS, FFT_MINB<R>) k_ypass(Cx<R>* __restrict__ W, int nx, int ny, int My, int Kz,
+__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB<R>) k_ypass(Cx<R>* __restrict__ W, int nx, int ny, int My, int Kz,
                                                        RadixPlan ry, const Cx<R>* __restrict__ twg,
                                                        int TK, const ScState* st, Spec<R> sp) {
     pdl_wait();
@@ -325,7 +353,7 @@ __device__ __forceinline__ void xconv_body(Cx<R>* __restrict__ W, const R* __res
 }
 
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS, FFT_MINB<R>) k_xconv(Cx<R>* __restrict__ W, const R* __restrict__ G,
+__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB<R>) k_xconv(Cx<R>* __restrict__ W, const R* __restrict__ G,
                                                        int nx, int My, int Kz, int Ky, RadixPlan rx,
                                                        const Cx<R>* __restrict__ twg, int TK, const ScState* st,
                                                        Spec<R> sp) {
@@ -396,16 +424,16 @@ __device__ __forceinline__ void zinv_body(const Cx<R>* __restrict__ W, R* __rest
     }
     __syncthreads();
     Cx<R>* res = fft_lines<R, true, true>(a, b, lz, NC, rz, tw);
-    const double norm = st->phi_norm, denom = st->phi_denom;
+    OutScale64 out64 = {};
+    if constexpr (sizeof(R) == 8) out64 = out_scale64(st);
     const R fscale = (R)st->phi_scalef * mul;  // (float)(norm / denom), computed once by the mesh finalize
     for (DivWalk w(threadIdx.x, blockDim.x, nz); w.q < NC; w.next()) {
         const int c = w.q, z = w.r;
         const int ya = y0 + 2 * c, yb = ya + 1;
         const Cx<R> v = res[c * lz + z];
-        if (sizeof(R) == 8) {
-            // out/(4*pi*eps0*hx*hy*hz) after the 1/M normalisation of ifftn (sc.py:164-167)
-            if (ya < ny) phi[((size_t)x * ny + ya) * nz + z] = (R)(((double)v.x * norm) / denom);
-            if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = (R)(((double)v.y * norm) / denom);
+        if constexpr (sizeof(R) == 8) {
+            if (ya < ny) phi[((size_t)x * ny + ya) * nz + z] = out64(v.x);
+            if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = out64(v.y);
         } else {
             const bool zx = zero_axis == 0 && x == nx - 1, zz = zero_axis == 2 && z == nz - 1;
             const bool za = zx || zz || (zero_axis == 1 && ya == ny - 1);
@@ -418,7 +446,7 @@ __device__ __forceinline__ void zinv_body(const Cx<R>* __restrict__ W, R* __rest
 
 // blockIdx.z: the output (0 the potential; with spectral fields 1 Ex, 2 Ey, 3 Ez)
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS, FFT_MINB<R>) k_zinv(const Cx<R>* __restrict__ W, R* __restrict__ phi,
+__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB<R>) k_zinv(const Cx<R>* __restrict__ W, R* __restrict__ phi,
                                                       int ny, int nz, int My, int Kz, RadixPlan rz,
                                                       const Cx<R>* __restrict__ twg, int NC,
                                                       const ScState* st, Spec<R> sp) {
@@ -432,25 +460,27 @@ __global__ void __launch_bounds__(FFT_THREADS, FFT_MINB<R>) k_zinv(const Cx<R>* 
     zinv_body<R>(src, out, ny, nz, My, Kz, rz, twg, NC, st, hw_vblk(), dz, mul, f - 1, (int)gridDim.y);
 }
 
-// Ex,Ey,Ez = forward differences / h, zero on the last plane (sc.py:195-200).
-// One block per (x, y) line of cells, one thread per z: no index division.
-template <typename R>
-__global__ void k_field_grids(const R* __restrict__ phi, R* __restrict__ ex, R* __restrict__ ey,
-                              R* __restrict__ ez, int nx, int ny, int nz, const ScState* st) {
+// FP64 form: Ex,Ey,Ez = forward differences / h, zero on the last plane
+// (sc.py:195-200); the quotient from the reciprocal 1/h with one correction
+// (the IEEE division's result up to its last bit).  One block per (x, y) line
+// of cells, one thread per z: no index division.
+__global__ void k_field_grids(const double* __restrict__ phi, double* __restrict__ ex, double* __restrict__ ey,
+                              double* __restrict__ ez, int nx, int ny, int nz, const ScState* st) {
     pdl_wait();
     if (st->status) return;
     const int j = blockIdx.x, i = blockIdx.y;
     const double hx = st->steps[0], hy = st->steps[1], hz = st->steps[2];
+    const double rx = st->isteps[0], ry = st->isteps[1], rz = st->isteps[2];
+    auto over = [](double a, double h, double r) {
+        const double q = a * r;
+        return fma(fma(-q, h, a), r, q);
+    };
     for (int k = threadIdx.x; k < nz; k += blockDim.x) {
         const int c = (i * ny + j) * nz + k;
-        const R p = phi[c];
-        R vx = 0, vy = 0, vz = 0;
-        if (i < nx - 1) vx = (R)(((double)p - (double)phi[c + ny * nz]) / hx);
-        if (j < ny - 1) vy = (R)(((double)p - (double)phi[c + nz]) / hy);
-        if (k < nz - 1) vz = (R)(((double)p - (double)phi[c + 1]) / hz);
-        ex[c] = vx;
-        ey[c] = vy;
-        ez[c] = vz;
+        const double p = phi[c];
+        ex[c] = i < nx - 1 ? over(p - phi[c + ny * nz], hx, rx) : 0.0;
+        ey[c] = j < ny - 1 ? over(p - phi[c + nz], hy, ry) : 0.0;
+        ez[c] = k < nz - 1 ? over(p - phi[c + 1], hz, rz) : 0.0;
     }
 }
 
@@ -594,9 +624,9 @@ __device__ __forceinline__ void zy_fwd_body(R* __restrict__ q, const long long* 
         const int ya = 2 * c, yb = ya + 1;
         const Cx<R> Z = res1[c * lz + k];
         const Cx<R> Zm = res1[c * lz + (k == 0 ? 0 : Mz - k)];
-        const R h = (R)0.5;
-        A2[k * ly + ya] = cx<R>((Z.x + Zm.x) * h, (Z.y - Zm.y) * h);
-        if (yb < ny) A2[k * ly + yb] = cx<R>((Z.y + Zm.y) * h, (Zm.x - Z.x) * h);
+        const R h = unpack_half<R>();
+        A2[k * ly + ya] = scaled<R>(Z.x + Zm.x, Z.y - Zm.y, h);
+        if (yb < ny) A2[k * ly + yb] = scaled<R>(Z.y + Zm.y, Zm.x - Z.x, h);
     }
     for (DivWalk w(threadIdx.x, blockDim.x, Kz); w.q < My - ny; w.next()) A2[w.r * ly + ny + w.q] = cx<R>(0, 0);
     __syncthreads();
@@ -672,16 +702,16 @@ __device__ __forceinline__ void yz_inv_body(const Cx<R>* __restrict__ W, R* __re
     }
     __syncthreads();
     const Cx<R>* res = fft_lines<R, true, true>(A1, B1, lz, ncz, rz, twz);
-    const double norm = st->phi_norm, denom = st->phi_denom;
+    OutScale64 out64 = {};
+    if constexpr (sizeof(R) == 8) out64 = out_scale64(st);
     const R fscale = (R)st->phi_scalef * mul;  // (float)(norm / denom), computed once by the mesh finalize
     for (DivWalk w(threadIdx.x, blockDim.x, nz); w.q < ncz; w.next()) {
         const int c = w.q, z = w.r;
         const int ya = 2 * c, yb = ya + 1;
         const Cx<R> v = res[c * lz + z];
-        if (sizeof(R) == 8) {
-            // out/(4*pi*eps0*hx*hy*hz) after the 1/M normalisation of ifftn (sc.py:164-167)
-            phi[((size_t)x * ny + ya) * nz + z] = (R)(((double)v.x * norm) / denom);
-            if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = (R)(((double)v.y * norm) / denom);
+        if constexpr (sizeof(R) == 8) {
+            phi[((size_t)x * ny + ya) * nz + z] = out64(v.x);
+            if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = out64(v.y);
         } else {
             const bool zx = zero_axis == 0 && x == nx - 1, zz = zero_axis == 2 && z == nz - 1;
             const bool za = zx || zz || (zero_axis == 1 && ya == ny - 1);
@@ -781,15 +811,15 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
         launch(k_zy_fwd<R>, p.nx, PLANE_THREADS<R>, smp, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, p.ry, twz, twy, st);
     } else if (part != CONV_REST) {
         if ((e = set_smem(k_zfwd<R>, smz))) return e;
-        launch(k_zfwd<R>, gz, FFT_THREADS, smz, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st);
+        launch(k_zfwd<R>, gz, FFT_THREADS<R>, smz, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st);
         if ((e = set_smem(k_ypass<R, false>, smy))) return e;
-        launch(k_ypass<R, false>, gy, FFT_THREADS, smy, s, W, p.nx, p.ny, p.My, Kz, p.ry, twy, tky, st, Spec<R>{});
+        launch(k_ypass<R, false>, gy, FFT_THREADS<R>, smy, s, W, p.nx, p.ny, p.My, Kz, p.ry, twy, tky, st, Spec<R>{});
     }
     if (part == CONV_FORWARD) return cudaGetLastError();
     const size_t smx = sizeof(Cx<R>) * (size_t)(p.Mx + nbuf * tkx * fft_ls(p.Mx));
     dim3 gx((p.My * Kz + tkx - 1) / tkx);  // the x pass's columns (ky, kz)
     if ((e = set_smem(k_xconv<R>, smx))) return e;
-    launch(k_xconv<R>, gx, FFT_THREADS, smx, s, W, G, p.nx, p.My, Kz, Ky, p.rx, twx, tkx, st, sp);
+    launch(k_xconv<R>, gx, FFT_THREADS<R>, smx, s, W, G, p.nx, p.My, Kz, Ky, p.rx, twx, tkx, st, sp);
     const int nout = sp.W2 ? 4 - sp.f0 : 1;  // [the potential,] Ex, Ey, Ez
     if (plane_inv) {
         if ((e = set_smem(k_yz_inv<R>, smp))) return e;
@@ -798,9 +828,9 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
         return cudaGetLastError();
     }
     if ((e = set_smem(k_ypass<R, true>, smyi))) return e;
-    launch(k_ypass<R, true>, gyi, FFT_THREADS, smyi, s, W, p.nx, p.ny, p.My, Kz, p.ry, twy, tkyi, st, sp);
+    launch(k_ypass<R, true>, gyi, FFT_THREADS<R>, smyi, s, W, p.nx, p.ny, p.My, Kz, p.ry, twy, tkyi, st, sp);
     if ((e = set_smem(k_zinv<R>, smz))) return e;
-    launch(k_zinv<R>, dim3(gz.x, gz.y, nout), FFT_THREADS, smz, s, W, phi, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st, sp);
+    launch(k_zinv<R>, dim3(gz.x, gz.y, nout), FFT_THREADS<R>, smz, s, W, phi, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st, sp);
     return cudaGetLastError();
 }
 
@@ -854,9 +884,9 @@ static cudaError_t field_t(const Plan& p, const Layout& L, char* ws, cudaStream_
                                          reinterpret_cast<float*>(ws + L.eyq), reinterpret_cast<float*>(ws + L.ezq),
                                          p.nx, p.ny, p.nz, st);
     else
-        launch(k_field_grids<R>, grid, bt, 0, s, reinterpret_cast<const R*>(ws + L.phi), reinterpret_cast<R*>(ws + L.ex),
-                                             reinterpret_cast<R*>(ws + L.ey), reinterpret_cast<R*>(ws + L.ez),
-                                             p.nx, p.ny, p.nz, st);
+        launch(k_field_grids, grid, bt, 0, s, reinterpret_cast<const double*>(ws + L.phi),
+               reinterpret_cast<double*>(ws + L.ex), reinterpret_cast<double*>(ws + L.ey),
+               reinterpret_cast<double*>(ws + L.ez), p.nx, p.ny, p.nz, st);
     return cudaGetLastError();
 }
 
@@ -877,7 +907,7 @@ cudaError_t launch_field_grids(const Plan& p, const Layout& L, char* ws, cudaStr
     const Plan& p = B.p;                                                        \
     const ScState* st = reinterpret_cast<const ScState*>(ws + L.state);
 
-__global__ void __launch_bounds__(FFT_THREADS) kb_zfwd(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(FFT_THREADS<float>) kb_zfwd(const BatchBeam* __restrict__ beams,
                                                        const int* __restrict__ start, int nb) {
     pdl_wait();
     BATCH_BEAM(BS_FFT_Z)
@@ -887,7 +917,7 @@ __global__ void __launch_bounds__(FFT_THREADS) kb_zfwd(const BatchBeam* __restri
 }
 
 // forward y pass
-__global__ void __launch_bounds__(FFT_THREADS) kb_yfwd(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(FFT_THREADS<float>) kb_yfwd(const BatchBeam* __restrict__ beams,
                                                        const int* __restrict__ start, int nb) {
     pdl_wait();
     BATCH_BEAM(BS_FFT_Y)
@@ -897,7 +927,7 @@ __global__ void __launch_bounds__(FFT_THREADS) kb_yfwd(const BatchBeam* __restri
 
 // inverse y pass: block row 0 takes W (and, with spectral fields, W x D(ky)
 // into W3), row 1 the x-differenced W2 (as k_ypass's blockIdx.y)
-__global__ void __launch_bounds__(FFT_THREADS) kb_yinv(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(FFT_THREADS<float>) kb_yinv(const BatchBeam* __restrict__ beams,
                                                        const int* __restrict__ start, int nb) {
     pdl_wait();
     BATCH_BEAM(BS_FFT_YI)
@@ -910,7 +940,7 @@ __global__ void __launch_bounds__(FFT_THREADS) kb_yinv(const BatchBeam* __restri
         ypass_body<float, true>(sp.W2, p.nx, p.ny, p.My, p.Mz / 2 + 1, p.ry, tw, B.fft_tky, st, vb);
 }
 
-__global__ void __launch_bounds__(FFT_THREADS) kb_xconv(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(FFT_THREADS<float>) kb_xconv(const BatchBeam* __restrict__ beams,
                                                         const int* __restrict__ start, int nb) {
     pdl_wait();
     BATCH_BEAM(BS_FFT_X)
@@ -922,7 +952,7 @@ __global__ void __launch_bounds__(FFT_THREADS) kb_xconv(const BatchBeam* __restr
 
 // inverse z pass: block group f writes output f (the potential; with spectral
 // fields also Ex, Ey, Ez), as k_zinv's blockIdx.z
-__global__ void __launch_bounds__(FFT_THREADS) kb_zinv(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(FFT_THREADS<float>) kb_zinv(const BatchBeam* __restrict__ beams,
                                                        const int* __restrict__ start, int nb) {
     pdl_wait();
     BATCH_BEAM(BS_FFT_ZI)
@@ -1004,13 +1034,13 @@ cudaError_t launch_batch_convolve(const BatchBeam* beams, const int* sz, const i
                                   cudaStream_t s, int part) {
     if (nb <= 0) return cudaSuccess;
     if (part != CONV_REST) {
-        launch(kb_zfwd, blocks[0], FFT_THREADS, smem[0], s, beams, sz, nb);
-        launch(kb_yfwd, blocks[1], FFT_THREADS, smem[1], s, beams, sy, nb);
+        launch(kb_zfwd, blocks[0], FFT_THREADS<float>, smem[0], s, beams, sz, nb);
+        launch(kb_yfwd, blocks[1], FFT_THREADS<float>, smem[1], s, beams, sy, nb);
     }
     if (part == CONV_FORWARD) return cudaGetLastError();
-    launch(kb_xconv, blocks[2], FFT_THREADS, smem[2], s, beams, sx, nb);
-    launch(kb_yinv, blocks[3], FFT_THREADS, smem[1], s, beams, syi, nb);
-    launch(kb_zinv, blocks[4], FFT_THREADS, smem[0], s, beams, szi, nb);
+    launch(kb_xconv, blocks[2], FFT_THREADS<float>, smem[2], s, beams, sx, nb);
+    launch(kb_yinv, blocks[3], FFT_THREADS<float>, smem[1], s, beams, syi, nb);
+    launch(kb_zinv, blocks[4], FFT_THREADS<float>, smem[0], s, beams, szi, nb);
     return cudaGetLastError();
 }
 
