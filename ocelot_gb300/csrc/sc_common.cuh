@@ -400,10 +400,21 @@ inline cudaError_t set_smem(K kernel, size_t bytes) {
     if (bytes <= 48 * 1024) return cudaSuccess;
     return smem_opt_in(reinterpret_cast<const void*>(kernel), bytes);
 }
+// Asks for an SM's whole shared memory beside this kernel.  A kernel that uses
+// little of it otherwise runs on an SM split in favour of L1, and a kernel of
+// the other stream that needs more shared memory than that split leaves waits
+// until the SM has drained: the radix scatter (18 KB a block) beside the Green's
+// function corners, for as long as those run.
+template <typename K>
+inline cudaError_t prefer_shared(K kernel) {
+    return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributePreferredSharedMemoryCarveout,
+                                cudaSharedmemCarveoutMaxShared);
+}
 // opts every kernel of a plan in (called when the plan is created)
 cudaError_t prepare_fft_kernels(const Plan& p);
 cudaError_t prepare_green_kernels(const Plan& p);
 cudaError_t prepare_particle_kernels();
+cudaError_t prepare_sort_kernels();
 
 // ---------------------------------------------------------------------------
 // bulk (TMA) copies between global and shared memory.  Loads complete on an

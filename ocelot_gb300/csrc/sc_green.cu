@@ -158,6 +158,7 @@ __device__ __forceinline__ void igf_corners_body(double* __restrict__ ig, R* __r
     // 32-bit index arithmetic: a mesh has fewer than 2^31 corners
     const unsigned total = (unsigned)cx1 * cy1 * cz1;
     const long long all = (long long)(nx + 1) * (ny + 1) * (nz + 1);
+    (void)all;  // read by the index checks of checked builds
     if (!a.hybrid) {
         for (unsigned c = vb.x * blockDim.x + threadIdx.x; c < total; c += vb.nx * blockDim.x) {
             double x, y, z;
@@ -471,16 +472,21 @@ cudaError_t launch_igf(const Plan& p, const Layout& L, char* ws, cudaStream_t s)
     a.hybrid = p.exact_igf ? 0 : 1;
     double* ig = reinterpret_cast<double*>(ws + L.igf_ig);
     const size_t nc = (size_t)(p.nx + 1) * (p.ny + 1) * (p.nz + 1);
-    // one block per SM: eight warps keep an SM's FP64 pipe busy, and the
-    // registers left over hold the blocks of the concurrent particle kernels
-    size_t gb = (nc + 255) / 256;
-    if (gb > (size_t)p.sm_count) gb = (size_t)p.sm_count;
+    // eight warps per SM keep its FP64 pipe busy, and the registers left over
+    // hold the blocks of the concurrent particle kernels.  The exact table (every
+    // corner in FP64, one thread each) in blocks of 64 threads, four per SM: a
+    // single block of 256 per SM doubled the time whenever two met on one SM
+    // (200k / 63^3: 122 to 240 us)
+    const int threads = p.exact_igf ? IGF_THREADS / 4 : IGF_THREADS;
+    size_t gb = (nc + threads - 1) / threads;
+    const size_t cap = (size_t)p.sm_count * (IGF_THREADS / threads);
+    if (gb > cap) gb = cap;
     const size_t nk = (size_t)p.nx * p.ny * p.nz;
     if (p.prec == SC_FP64)
-        launch(k_igf_corners<double>, (int)gb, IGF_THREADS, 0, s, ig, reinterpret_cast<double*>(ws + L.igf_k1), p.nx,
+        launch(k_igf_corners<double>, (int)gb, threads, 0, s, ig, reinterpret_cast<double*>(ws + L.igf_k1), p.nx,
                p.ny, p.nz, a, st);
     else
-        launch(k_igf_corners<float>, (int)gb, IGF_THREADS, 0, s, ig, reinterpret_cast<float*>(ws + L.igf_k1), p.nx,
+        launch(k_igf_corners<float>, (int)gb, threads, 0, s, ig, reinterpret_cast<float*>(ws + L.igf_k1), p.nx,
                p.ny, p.nz, a, st);
     if (p.prec == SC_FP64)
         launch(k_igf_diff<double>, grid_for(nk, p.sm_count), 256, 0, s, ig, reinterpret_cast<double*>(ws + L.igf_k1), p.nx,
@@ -538,6 +544,8 @@ static cudaError_t prepare_green_t(const Plan& p) {
     const int tky = green_cols<R>(p.My), tkx = green_cols<R>(p.Mx);
     const size_t smy = sizeof(Cx<R>) * (size_t)(p.My + 2 * tky * fft_ls(p.My));
     const size_t smx = sizeof(Cx<R>) * (size_t)(p.Mx + 2 * tkx * fft_ls(p.Mx));
+    if ((e = prefer_shared(k_igf_corners<R>))) return e;
+    if ((e = prefer_shared(k_igf_diff<R>))) return e;
     if ((e = set_smem(k_green_z<R>, smz))) return e;
     return set_smem(k_green_strided<R>, smx > smy ? smx : smy);
 }

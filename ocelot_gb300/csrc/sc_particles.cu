@@ -2554,6 +2554,9 @@ cudaError_t prepare_particle_kernels() {
     if ((e = set_smem(k_frame32_tma, FR_SMEM))) return e;
     if ((e = set_smem(kb_frame32, FR_SMEM))) return e;
     if ((e = set_smem(k_extent, EX_SMEM))) return e;
+    if ((e = prefer_shared(k_keys32<true, false>))) return e;
+    if ((e = prefer_shared(k_keys32<false, false>))) return e;
+    if ((e = prefer_shared(k_keys32<true, true>))) return e;
     return set_smem(kb_extent32, EX_SMEM);
 }
 

@@ -150,6 +150,13 @@ int sort_blocks(int64_t n) {
     return (int)((n + t - 1) / t);
 }
 
+cudaError_t prepare_sort_kernels() {
+    cudaError_t e;
+    if ((e = prefer_shared(k_rhist))) return e;
+    if ((e = prefer_shared(k_rrowscan))) return e;
+    return prefer_shared(k_rscatter);
+}
+
 int sort_passes(int key_bits) { return key_bits <= 0 ? 1 : (key_bits + RMAXBITS - 1) / RMAXBITS; }
 
 size_t sort_scratch_bytes(int64_t n, int key_bits) {
