@@ -24,8 +24,12 @@
 
 #include "sc_common.cuh"
 #include "sc_fft_dev.cuh"
+#include "sc_igf_fn.cuh"
 
 namespace ocsc {
+
+__device__ const LogEntry kLogTable[IGF_NLOG] = {SC_IGF_LOG_TABLE};
+__device__ const AtanEntry kAtanTable[IGF_NATAN] = {SC_IGF_ATAN_TABLE};
 
 struct IgfArgs {
     double hx, hy, hz;
@@ -130,13 +134,22 @@ __device__ __forceinline__ void igf_corner_xyz(unsigned c, int cy1, int cz1, dou
     z = __dsub_rn(__dmul_rn(hz, (double)k), __dmul_rn(hz, 0.5));
 }
 
+// Whether the corners may take igf::point_: steps well inside the exponent range
+// and not so unequal that x + r of a corner just below the axis vanishes
+__device__ __forceinline__ bool igf_regular(double hx, double hy, double hz) {
+    const double lo = fmin(hx, fmin(hy, hz)), hi = fmax(hx, fmax(hy, hz));
+    return lo > 1e-50 && hi < 1e50 && hi < lo * 0x1p20;
+}
+
 constexpr int IGF_THREADS = 256;
 constexpr int IGF_SPLIT = IGF_THREADS / 6;  // corners per block per round in the split form
 
 // IG on the corners of the near box (the whole octant when not hybrid),
 // stored with the box's corner strides.
 // The whole octant (the exact table): one thread per corner, bound by the
-// FP64 pipe.  The near box of the hybrid table has a few hundred corners, so
+// FP64 pipe -- igf::point_, about 130 FP64 instructions where igf_point with
+// CUDA's functions has 226 (63^3 beside the other stream: 173 -> 118 us); igf_point stays
+// for steps that point_ does not cover.  The near box of the hybrid table has a few hundred corners, so
 // the time is the latency of one igf_point -- on this GPU's narrow FP64 pipe
 // some 20 us of dependent arithmetic through three arctangents and three
 // logarithms.  There each corner's six terms go to six threads (the
@@ -160,6 +173,26 @@ __device__ __forceinline__ void igf_corners_body(double* __restrict__ ig, R* __r
     const long long all = (long long)(nx + 1) * (ny + 1) * (nz + 1);
     (void)all;  // read by the index checks of checked builds
     if (!a.hybrid) {
+        __shared__ LogEntry lt[IGF_NLOG];
+        __shared__ AtanEntry at[IGF_NATAN];
+        const bool fast = igf_regular(hx, hy, hz);
+        if (fast) {
+            for (int i = threadIdx.x; i < IGF_NLOG; i += blockDim.x) lt[i] = kLogTable[i];
+            for (int i = threadIdx.x; i < IGF_NATAN; i += blockDim.x) at[i] = kAtanTable[i];
+            __syncthreads();
+            const double bx = __dmul_rn(hx, 0.5), by = __dmul_rn(hy, 0.5), bz = __dmul_rn(hz, 0.5);
+            for (unsigned c = vb.x * blockDim.x + threadIdx.x; c < total; c += vb.nx * blockDim.x) {
+                const unsigned t = c / (unsigned)cz1;
+                const int k = (int)(c - t * (unsigned)cz1);
+                const int i = (int)(t / (unsigned)cy1), j = (int)(t - (unsigned)i * cy1);
+                const double x = __dsub_rn(__dmul_rn(hx, igf::widen((float)i)), bx);
+                const double y = __dsub_rn(__dmul_rn(hy, igf::widen((float)j)), by);
+                const double z = __dsub_rn(__dmul_rn(hz, igf::widen((float)k)), bz);
+                if (!SC_IDX_OK(st, 31, c, all)) continue;
+                ig[c] = igf::point_(x, y, z, lt, at);
+            }
+            return;
+        }
         for (unsigned c = vb.x * blockDim.x + threadIdx.x; c < total; c += vb.nx * blockDim.x) {
             double x, y, z;
             igf_corner_xyz(c, cy1, cz1, hx, hy, hz, x, y, z);
