@@ -78,6 +78,7 @@ struct ScState {
     unsigned int done_frame;     // blocks finished, for the last-block reductions
     unsigned int done_extent;
     unsigned int kick_next;      // tiles claimed by the gather + kick (reset by the frame finalize)
+    unsigned int igf_next;       // corners of the exact IGF table claimed (reset with the mesh)
     int frame_timeout;           // a frame block's bulk-copy wait gave up (the finalize reports it)
     int check_code;              // checked builds: first failed index check (kernel code)
     int first_error;             // first non-OK status of any kick since sc_workspace_init

@@ -181,7 +181,21 @@ __device__ __forceinline__ void igf_corners_body(double* __restrict__ ig, R* __r
             for (int i = threadIdx.x; i < IGF_NATAN; i += blockDim.x) at[i] = kAtanTable[i];
             __syncthreads();
             const double bx = __dmul_rn(hx, 0.5), by = __dmul_rn(hy, 0.5), bz = __dmul_rn(hz, 0.5);
-            for (unsigned c = vb.x * blockDim.x + threadIdx.x; c < total; c += vb.nx * blockDim.x) {
+            // A kick's table is claimed 32 corners per warp from a counter in
+            // the state (reset with the mesh): the blocks start while the
+            // deposit's hold some SMs, and a fixed share per block left the SMs
+            // that took several of them running long after the others
+            // (200k / 63^3: 118 -> 80 us)
+            const bool claim = a.use_state != 0;
+            const unsigned lane = threadIdx.x & 31u;
+            auto next = [&](unsigned c) -> unsigned {
+                if (!claim) return c + vb.nx * blockDim.x;
+                unsigned f = 0u;
+                if (lane == 0u) f = atomicAdd(&const_cast<ScState*>(st)->igf_next, 32u);
+                return __shfl_sync(0xffffffffu, f, 0) + lane;
+            };
+            for (unsigned c = claim ? next(0u) : vb.x * blockDim.x + threadIdx.x; c - lane < total; c = next(c)) {
+                if (c >= total) continue;
                 const unsigned t = c / (unsigned)cz1;
                 const int k = (int)(c - t * (unsigned)cz1);
                 const int i = (int)(t / (unsigned)cy1), j = (int)(t - (unsigned)i * cy1);

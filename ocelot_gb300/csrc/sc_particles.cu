@@ -734,6 +734,7 @@ __device__ __forceinline__ void mesh_finish(const double* mn, const double* mx, 
         st->phi_denom = pden;
         st->phi_scalef = (float)scale;
         st->igf_rebuild = same ? 0 : 1;
+        st->igf_next = 0;
     }
 }
 
@@ -1427,6 +1428,7 @@ __global__ void k_set_mesh(ScState* st, double hx, double hy, double hz, KickPar
     st->igf_tbox[1] = igf_tbox_of(h, 1, kp.ny);
     const bool same = hx == st->igf_h[0] && hy == st->igf_h[1] && hz == st->igf_h[2];
     st->igf_rebuild = same ? 0 : 1;
+    st->igf_next = 0;
     st->igf_h[0] = hx;
     st->igf_h[1] = hy;
     st->igf_h[2] = hz;
@@ -1849,7 +1851,8 @@ __device__ __forceinline__ bool near_edge64(double X, int n) {
 // one matrix).
 // rec != nullptr (the record-field mode): the field samples before the gamma0
 // factor go to rec[i], rec[nX + i], rec[2 nX + i]
-__global__ void __launch_bounds__(PT, 2) k_kick64(double* __restrict__ rp, const double* __restrict__ ex,
+constexpr int KICK64_THREADS = 128;
+__global__ void __launch_bounds__(KICK64_THREADS, 4) k_kick64(double* __restrict__ rp, const double* __restrict__ ex,
                                                const double* __restrict__ ey, const double* __restrict__ ez,
                                                const __grid_constant__ KickParams kp, const ScState* st,
                                                double* __restrict__ rec) {
@@ -2657,7 +2660,8 @@ cudaError_t launch_gather_kick(const Plan& p, const Layout& L, char* ws, const K
     const ScState* st = reinterpret_cast<const ScState*>(ws + L.state);
     const int nb = particle_blocks(p, kp.n);
     if (p.prec == SC_FP64)
-        launch(k_kick64, nb, PT, 0, s, rp, reinterpret_cast<const double*>(ws + L.ex),
+        launch(k_kick64, (int)((kp.n + KICK64_THREADS - 1) / KICK64_THREADS), KICK64_THREADS, 0, s, rp,
+               reinterpret_cast<const double*>(ws + L.ex),
                reinterpret_cast<const double*>(ws + L.ey), reinterpret_cast<const double*>(ws + L.ez), kp, st,
                p.record_field ? reinterpret_cast<double*>(ws + L.X) : nullptr);
     else
