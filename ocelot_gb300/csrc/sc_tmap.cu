@@ -467,6 +467,7 @@ __global__ void __launch_bounds__(MOM_THREADS) k_moments(const double* __restric
     double acc[MOM_K];
 #pragma unroll
     for (int k = 0; k < MOM_K; ++k) acc[k] = 0.0;
+    unsigned count = 0;  // particles taken (an FP64 addition less each)
     double v0[6];
     mom_prime(rp, ld, 0, v0);
     double tlo = -INFINITY, thi = INFINITY;
@@ -488,7 +489,7 @@ __global__ void __launch_bounds__(MOM_THREADS) k_moments(const double* __restric
         double d[6];
 #pragma unroll
         for (int k = 0; k < 6; ++k) d[k] = __dsub_rn(v[k], v0[k]);
-        acc[0] += 1.0;
+        ++count;
 #pragma unroll
         for (int k = 0; k < 6; ++k) acc[1 + k] += d[k];
         // xx, xpx, pxpx, yy, ypy, pypy, tautau, xy, pxpy, xpy, ypx, pp (d: x, y, px, py, tau, p)
@@ -499,60 +500,79 @@ __global__ void __launch_bounds__(MOM_THREADS) k_moments(const double* __restric
         acc[15] = __fma_rn(d[2], d[3], acc[15]);  acc[16] = __fma_rn(d[0], d[3], acc[16]);
         acc[17] = __fma_rn(d[1], d[2], acc[17]);  acc[18] = __fma_rn(d[5], d[5], acc[18]);
     }
+    if (pass == 1) acc[0] = (double)count;
+    // The block's sums, quantities dealt to warps through shared memory: 13
+    // FP64 additions per quantity and block, where a shuffle tree in every warp
+    // takes 40; then the last block's the same way, one warp per quantity over
+    // the blocks, and its divisions side by side in the lanes.  (One thread per
+    // quantity over 304 blocks and 18 divisions in a row took 17 us alone.)
     const int nk = pass == 0 ? 2 : MOM_K;
-    __shared__ double s_red[MOM_THREADS / 32][MOM_K];
-    __shared__ double s_sum[MOM_K];
+    constexpr int GRP = 5, NW = MOM_THREADS / 32;  // quantities in shared memory at a time
+    __shared__ double s_red[GRP][MOM_THREADS];
+    __shared__ double s_sum[MOM_K], s_m1[6];
     __shared__ bool s_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < MOM_K; ++k) {
-        if (k >= nk) break;
-        double v = acc[k];
+    for (int k0 = 0; k0 < MOM_K; k0 += GRP) {
+        if (k0 >= nk) break;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if (lane == 0) s_red[warp][k] = v;
+        for (int k = 0; k < GRP; ++k)
+            if (k0 + k < MOM_K) s_red[k][threadIdx.x] = acc[k0 + k];
+        __syncthreads();
+        if (warp < GRP && k0 + warp < nk) {
+            double v = 0.0;
+#pragma unroll
+            for (int u = 0; u < NW; ++u) v += s_red[warp][lane + 32 * u];
+            for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+            if (lane == 0) partial[(size_t)blockIdx.x * MOM_K + k0 + warp] = v;
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    if (threadIdx.x < nk) {
-        double v = 0.0;
-        for (int w = 0; w < MOM_THREADS / 32; ++w) v += s_red[w][threadIdx.x];
-        partial[(size_t)blockIdx.x * MOM_K + threadIdx.x] = v;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    if (threadIdx.x < nk) {
+    for (int k = warp; k < nk; k += NW) {
         double v = 0.0;
-        for (unsigned b = 0; b < gridDim.x; ++b) v += __ldcg(partial + (size_t)b * MOM_K + threadIdx.x);
-        s_sum[threadIdx.x] = v;
+#pragma unroll 4
+        for (unsigned b = lane; b < gridDim.x; b += 32) v += __ldcg(partial + (size_t)b * MOM_K + k);
+        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+        if (lane == 0) s_sum[k] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        if (pass == 0) {
+    if (warp != 0) return;
+    if (pass == 0) {
+        if (lane == 0) {
             const double m1 = s_sum[0] / (double)n;
             o[1] = __dadd_rn(v0[4], m1);
             o[2] = sqrt(fmax(__fma_rn(-m1, m1, s_sum[1] / (double)n), 0.0));
-        } else {
-            const double cnt = s_sum[0];
-            o[0] = cnt;
-            double m1[6];
-            for (int k = 0; k < 6; ++k) {
-                m1[k] = s_sum[1 + k] / cnt;
-                o[3 + k] = __dadd_rn(v0[k], m1[k]);
-            }
-            const int a[12] = {0, 0, 2, 1, 1, 3, 4, 0, 2, 0, 1, 5};
-            const int b[12] = {0, 2, 2, 1, 3, 3, 4, 1, 3, 3, 2, 5};
-            for (int k = 0; k < 12; ++k) {
-                double c = __fma_rn(-m1[a[k]], m1[b[k]], s_sum[7 + k] / cnt);
-                if (a[k] == b[k]) c = fmax(c, 0.0);   // a variance: not below 0 by rounding
-                o[9 + k] = cnt == 1.0 ? 0.0 : c;      // one particle: no spread, exactly
-            }
         }
-        *ticket = 0u;
+    } else {
+        const double cnt = s_sum[0];
+        const double mean = s_sum[lane < MOM_K ? lane : 0] / cnt;  // lane 1 + k: first moment k, 7 + k: product k
+        if (lane >= 1 && lane < 7) {
+            s_m1[lane - 1] = mean;
+            double r = v0[0];  // v0[lane - 1] without a register array indexed at run time
+#pragma unroll
+            for (int k = 1; k < 6; ++k)
+                if (lane == 1 + k) r = v0[k];
+            o[2 + lane] = __dadd_rn(r, mean);
+        }
+        __syncwarp();
+        if (lane == 0) o[0] = cnt;
+        if (lane >= 7 && lane < MOM_K) {
+            // xx, xpx, pxpx, yy, ypy, pypy, tautau, xy, pxpy, xpy, ypx, pp: the factors' indices, four bits each
+            const int k = lane - 7;
+            const int a = (int)((0x510204311200ull >> (4 * k)) & 15u), b = (int)((0x523314331220ull >> (4 * k)) & 15u);
+            double c = __fma_rn(-s_m1[a], s_m1[b], mean);
+            if (a == b) c = fmax(c, 0.0);      // a variance: not below 0 by rounding
+            o[9 + k] = cnt == 1.0 ? 0.0 : c;   // one particle: no spread, exactly
+        }
     }
+    if (lane == 0) *ticket = 0u;
 }
 
 cudaError_t launch_moments(const double* rp, int64_t ld, int64_t n, const int* counter, int nslots, int use_bounds,
