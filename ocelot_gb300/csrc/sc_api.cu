@@ -178,7 +178,7 @@ __global__ void k_init_ws(ScState* st, Cx<R>* tx, int Mx, Cx<R>* ty, int My, Cx<
     // past its M - R0 hold w_M^i, unused)
     double s, c;
     auto entry = [&](int M) {
-        const int m = (uses_two_step<R>(M) || i >= M - next_radix(M)) ? i : stage_tw_exponent(M, i);
+        const int m = (uses_two_step(M) || i >= M - next_radix(M)) ? i : stage_tw_exponent(M, i);
         sincospi(2.0 * m / M, &s, &c);
         return cx<R>((R)c, (R)-s);
     };

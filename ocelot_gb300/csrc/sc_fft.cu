@@ -20,6 +20,7 @@
 // HBM/L2 between passes; each pass stages whole lines in shared memory.
 #include "sc_common.cuh"
 #include "sc_fft_dev.cuh"
+#include "sc_fft_stream.cuh"
 
 namespace ocsc {
 
@@ -29,8 +30,7 @@ namespace ocsc {
 // block's loads overlap the others' arithmetic
 template <typename R>
 constexpr int FFT_THREADS = sizeof(R) == 8 ? 128 : 256;
-template <typename R>
-constexpr int FFT_MINB = sizeof(R) == 8 ? 4 : 0;  // 0: no bound
+constexpr int FFT_MINB = 4;
 
 // complex lines (two real lines each) per block of the z passes: up to 8,
 // so that a 64^3 mesh gives 256 blocks
@@ -42,10 +42,38 @@ static inline int z_lines_per_block(int Mz) {
 // of 16 columns would not fit in shared memory (FP64 at M = 512)
 template <typename R>
 static inline int strided_cols(int M, int nbuf = 2) {
-    // FP64: as many as give the block's 128 threads a work item each (Q per line, two_step_q64)
+    // FP64: as many as give the block's 128 threads a work item each (Q per line, two_step_q)
     int tk = sizeof(R) == 8 && M > 64 ? 8 : 16;
     while (tk > 2 && sizeof(Cx<R>) * (size_t)(M + nbuf * tk * fft_ls(M)) > 200 * 1024) tk /= 2;
     return tk;
+}
+// dynamic shared memory of the separate passes over lines of length M: the
+// streamed form's twiddles, difference factors, tables and lines
+// (sc_fft_stream.cuh), else twiddles and whole line buffers
+template <typename R>
+static inline size_t smem_zf(int M, int NC) {
+    return sizeof(Cx<R>) * (streamed<R>(M) ? M + NC * (size_t)(stream_la(M) + stream_lb<R>(M))
+                                                : M + 2 * NC * (size_t)fft_ls(M));
+}
+template <typename R>
+static inline size_t smem_zi(int M, int NC) {
+    return sizeof(Cx<R>) * (M + 2 * NC * (size_t)fft_ls(M));
+}
+template <typename R>
+static inline size_t smem_yf(int M, int TK) {
+    return sizeof(Cx<R>) * (streamed<R>(M) ? M + TK * (size_t)stream_lb<R>(M) : M + 2 * TK * (size_t)fft_ls(M));
+}
+template <typename R>
+static inline size_t smem_yi(int M, int TK, bool w3) {
+    return sizeof(Cx<R>) * (streamed<R>(M) ? (w3 ? 2 : 1) * (M + TK * (size_t)stream_lb<R>(M))
+                                                : M + (w3 ? 3 : 2) * TK * (size_t)fft_ls(M));
+}
+template <typename R>
+static inline size_t smem_x(int M, int TK, bool w2) {
+    return sizeof(Cx<R>) * (streamed<R>(M)
+                                ? (w2 ? 2 : 1) * M + TK * (size_t)(stream_la(M) +
+                                                                   (w2 && stream_dual_x(M) ? 2 : 1) * stream_lb<R>(M))
+                                : M + (w2 ? 3 : 2) * TK * (size_t)fft_ls(M));
 }
 // the plan's columns per block (SC_PARAM_FFT_COLS_X / _Y; 0: strided_cols),
 // never more than fit.  The columns are independent lines, so the grouping
@@ -167,24 +195,51 @@ __device__ __forceinline__ void stage_charge_lines(R* __restrict__ q, const long
 
 // qfix != nullptr: the charge arrives as the 64-bit fixed-point grid of the
 // FP32 form's exact deposit; it is scaled to R here and also stored in q
-// (the charge grid an inspection reads back)
-template <typename R>
+// (the charge grid an inspection reads back).
+//
+// STREAM: what the body's lines take -- ST_NO staged passes (any length), ST_ANY
+// by the length at run time (the batched kernels), a length the streamed pass
+// of that length.  The separate FP32 passes have a kernel per streamed length, with
+// as many threads as the length has items for 16 columns: a 64-point pass in blocks
+// of 256 leaves half of them idle in each step (32^3: z 5.4 -> 3.6 us, y 5.8 -> 2.5,
+// x 9.0 -> 3.9), and a shared kernel takes the registers of its longest line
+enum { ST_NO = 0, ST_ANY = -1 };
+template <typename R, int STREAM, typename F>
+__device__ __forceinline__ bool stream_pass(int L, F&& f) {
+    if constexpr (STREAM > 0) {
+        f(IntC<STREAM>{});
+        return true;
+    } else if constexpr (STREAM == ST_ANY) {
+        return with_stream<R>(L, f);
+    } else {
+        return false;
+    }
+}
+
+template <typename R, int STREAM>
 __device__ __forceinline__ void zfwd_body(R* __restrict__ q, const long long* __restrict__ qfix,
                                           Cx<R>* __restrict__ W, int ny, int nz, int My, int Kz,
                                           const RadixPlan& rz, const Cx<R>* __restrict__ twg, int NC,
                                           const ScState* st, VBlk vb) {
     extern __shared__ __align__(16) unsigned char smraw[];
     if (st->status) return;
-    const int Mz = rz.L, lz = fft_ls(Mz);
-    Cx<R>* tw = reinterpret_cast<Cx<R>*>(smraw);
-    Cx<R>* a = tw + Mz;
-    Cx<R>* b = a + NC * lz;
-    load_twiddles<R>(tw, twg, Mz);
+    const int Mz = rz.L;
     const int x = vb.y;
     const int y0 = vb.x * 2 * NC;
-    stage_charge_lines<R>(q, qfix, a, lz, x, y0, NC, ny, nz, Mz, st, (long long)vb.ny * ny * nz, 21);
-    __syncthreads();
-    Cx<R>* res = fft_lines<R, false, true>(a, b, lz, NC, rz, tw);
+    Cx<R>* res = nullptr;
+    int lz = stream_la(Mz);
+    if (!stream_pass<R, STREAM>(Mz, [&](auto L) {
+            res = zfwd_stream<R, decltype(L)::value>(q, qfix, x, y0, ny, nz, twg, NC, st, (long long)vb.ny * ny * nz);
+        })) {
+        lz = fft_ls(Mz);
+        Cx<R>* tw = reinterpret_cast<Cx<R>*>(smraw);
+        Cx<R>* a = tw + Mz;
+        Cx<R>* b = a + NC * lz;
+        load_twiddles<R>(tw, twg, Mz);
+        stage_charge_lines<R>(q, qfix, a, lz, x, y0, NC, ny, nz, Mz, st, (long long)vb.ny * ny * nz, 21);
+        __syncthreads();
+        res = fft_lines<R, false, true>(a, b, lz, NC, rz, tw);
+    }
     for (DivWalk w(threadIdx.x, blockDim.x, Kz); w.q < NC; w.next()) {
         const int c = w.q, k = w.r;
         const int ya = y0 + 2 * c, yb = ya + 1;
@@ -198,12 +253,20 @@ __device__ __forceinline__ void zfwd_body(R* __restrict__ q, const long long* __
 }
 
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB<R>) k_zfwd(R* __restrict__ q, const long long* __restrict__ qfix,
+__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB) k_zfwd(R* __restrict__ q, const long long* __restrict__ qfix,
                                                       Cx<R>* __restrict__ W, int ny, int nz, int My, int Kz,
                                                       RadixPlan rz, const Cx<R>* __restrict__ twg, int NC,
                                                       const ScState* st) {
     pdl_wait();
-    zfwd_body<R>(q, qfix, W, ny, nz, My, Kz, rz, twg, NC, st, hw_vblk());
+    zfwd_body<R, ST_NO>(q, qfix, W, ny, nz, My, Kz, rz, twg, NC, st, hw_vblk());
+}
+template <int L>
+__global__ void __launch_bounds__(128, 8) k_zfwd_s(float* __restrict__ q, const long long* __restrict__ qfix,
+                                                   Cx<float>* __restrict__ W, int ny, int nz, int My, int Kz,
+                                                   RadixPlan rz, const Cx<float>* __restrict__ twg, int NC,
+                                                   const ScState* st) {
+    pdl_wait();
+    zfwd_body<float, L>(q, qfix, W, ny, nz, My, Kz, rz, twg, NC, st, hw_vblk());
 }
 
 // strided pass along y: forward (rows < ny in, all My out) or inverse (all in, rows < ny out),
@@ -211,12 +274,16 @@ __global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB<R>) k_zfwd(R* __restr
 // x * Kz + kz; block vb.x takes TK consecutive ones (a block may straddle two
 // x planes).  W3 != nullptr (inverse, spectral fields): the block also
 // transforms its columns of W multiplied by D(ky) into W3 (a third line buffer)
-template <typename R, bool INV>
+template <typename R, bool INV, int STREAM>
 __device__ __forceinline__ void ypass_body(Cx<R>* __restrict__ W, int nx, int ny, int My, int Kz, const RadixPlan& ry,
                                            const Cx<R>* __restrict__ twg, int TK, const ScState* st, VBlk vb,
                                            Cx<R>* __restrict__ W3 = nullptr, const Cx<R>* __restrict__ dy = nullptr) {
     extern __shared__ __align__(16) unsigned char smraw[];
     if (st->status) return;
+    if (stream_pass<R, STREAM>(My, [&](auto L) {
+            ypass_stream<R, INV, decltype(L)::value>(W, nx, ny, Kz, twg, TK, vb, W3, dy);
+        }))
+        return;
     const int ls = fft_ls(My);
     Cx<R>* tw = reinterpret_cast<Cx<R>*>(smraw);
     Cx<R>* a = tw + My;
@@ -265,12 +332,21 @@ __device__ __forceinline__ void ypass_body(Cx<R>* __restrict__ W, int nx, int ny
 // blockIdx.y = 0: W (and, with spectral fields, W x D(ky) into W3);
 // blockIdx.y = 1 (inverse, spectral fields): the x-differenced grid W2 in place
 template <typename R, bool INV>
-__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB<R>) k_ypass(Cx<R>* __restrict__ W, int nx, int ny, int My, int Kz,
+__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB) k_ypass(Cx<R>* __restrict__ W, int nx, int ny, int My, int Kz,
                                                        RadixPlan ry, const Cx<R>* __restrict__ twg,
                                                        int TK, const ScState* st, Spec<R> sp) {
     pdl_wait();
-    if (blockIdx.y == 0) ypass_body<R, INV>(W, nx, ny, My, Kz, ry, twg, TK, st, hw_vblk(), sp.W3, sp.dy);
-    else ypass_body<R, INV>(sp.W2, nx, ny, My, Kz, ry, twg, TK, st, hw_vblk());
+    if (blockIdx.y == 0) ypass_body<R, INV, ST_NO>(W, nx, ny, My, Kz, ry, twg, TK, st, hw_vblk(), sp.W3, sp.dy);
+    else ypass_body<R, INV, ST_NO>(sp.W2, nx, ny, My, Kz, ry, twg, TK, st, hw_vblk());
+}
+template <bool INV, int L>
+__global__ void __launch_bounds__(stream_threads(L), stream_minb(L))
+    k_ypass_s(Cx<float>* __restrict__ W, int nx, int ny, int My, int Kz, RadixPlan ry,
+              const Cx<float>* __restrict__ twg, int TK, const ScState* st, Spec<float> sp) {
+    pdl_wait();
+    if (blockIdx.y == 0)
+        ypass_body<float, INV, L>(W, nx, ny, My, Kz, ry, twg, TK, st, hw_vblk(), INV ? sp.W3 : nullptr, sp.dy);
+    else ypass_body<float, INV, L>(sp.W2, nx, ny, My, Kz, ry, twg, TK, st, hw_vblk());
 }
 
 // x pass: forward FFT of the nx non-zero planes, Green multiply, inverse FFT, keep x < nx.
@@ -278,7 +354,7 @@ __global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB<R>) k_ypass(Cx<R>* __
 // element x of a column at x * My * Kz + column); block vb.x takes TK
 // consecutive ones.  W2 != nullptr (spectral fields): the product times D(kx)
 // goes through its own inverse transform (a third line buffer) into W2
-template <typename R>
+template <typename R, int STREAM>
 __device__ __forceinline__ void xconv_body(Cx<R>* __restrict__ W, const R* __restrict__ G, int nx, int My, int Kz,
                                            int Ky, const RadixPlan& rx, const Cx<R>* __restrict__ twg, int TK,
                                            const ScState* st, VBlk vb, Cx<R>* __restrict__ W2 = nullptr,
@@ -286,6 +362,10 @@ __device__ __forceinline__ void xconv_body(Cx<R>* __restrict__ W, const R* __res
     extern __shared__ __align__(16) unsigned char smraw[];
     if (st->status) return;
     const int Mx = rx.L;
+    if (stream_pass<R, STREAM>(Mx, [&](auto L) {
+            xconv_stream<R, decltype(L)::value>(W, G, nx, My, Kz, Ky, twg, TK, st, vb, W2, dx);
+        }))
+        return;
     const int ls = fft_ls(Mx);
     Cx<R>* tw = reinterpret_cast<Cx<R>*>(smraw);
     Cx<R>* a = tw + Mx;
@@ -353,12 +433,19 @@ __device__ __forceinline__ void xconv_body(Cx<R>* __restrict__ W, const R* __res
 }
 
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB<R>) k_xconv(Cx<R>* __restrict__ W, const R* __restrict__ G,
+__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB) k_xconv(Cx<R>* __restrict__ W, const R* __restrict__ G,
                                                        int nx, int My, int Kz, int Ky, RadixPlan rx,
                                                        const Cx<R>* __restrict__ twg, int TK, const ScState* st,
                                                        Spec<R> sp) {
     pdl_wait();
-    xconv_body<R>(W, G, nx, My, Kz, Ky, rx, twg, TK, st, hw_vblk(), sp.W2, sp.dx);
+    xconv_body<R, ST_NO>(W, G, nx, My, Kz, Ky, rx, twg, TK, st, hw_vblk(), sp.W2, sp.dx);
+}
+template <int L>
+__global__ void __launch_bounds__(stream_threads(L), stream_minb(L))
+    k_xconv_s(Cx<float>* __restrict__ W, const float* __restrict__ G, int nx, int My, int Kz, int Ky, RadixPlan rx,
+              const Cx<float>* __restrict__ twg, int TK, const ScState* st, Spec<float> sp) {
+    pdl_wait();
+    xconv_body<float, L>(W, G, nx, My, Kz, Ky, rx, twg, TK, st, hw_vblk(), sp.W2, sp.dx);
 }
 
 // Field outputs of the inverse passes (spectral fields, FP32): the grid a
@@ -387,13 +474,30 @@ __device__ __forceinline__ void zinv_body(const Cx<R>* __restrict__ W, R* __rest
                                           R mul = (R)1, int zero_axis = -1, int nx = 0) {
     extern __shared__ __align__(16) unsigned char smraw[];
     if (st->status) return;
+    const int x = vb.y;
+    const int y0 = vb.x * 2 * NC;
+    OutScale64 out64 = {};
+    if constexpr (sizeof(R) == 8) out64 = out_scale64(st);
+    const R fscale = (R)st->phi_scalef * mul;  // (float)(norm / denom), computed once by the mesh finalize
+    auto put = [&](int c, int z, Cx<R> v) {
+        if (z >= nz) return;
+        const int ya = y0 + 2 * c, yb = ya + 1;
+        if constexpr (sizeof(R) == 8) {
+            if (ya < ny) phi[((size_t)x * ny + ya) * nz + z] = out64(v.x);
+            if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = out64(v.y);
+        } else {
+            const bool zx = zero_axis == 0 && x == nx - 1, zz = zero_axis == 2 && z == nz - 1;
+            const bool za = zx || zz || (zero_axis == 1 && ya == ny - 1);
+            const bool zb = zx || zz || (zero_axis == 1 && yb == ny - 1);
+            if (ya < ny) phi[((size_t)x * ny + ya) * nz + z] = za ? (R)0 : v.x * fscale;
+            if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = zb ? (R)0 : v.y * fscale;
+        }
+    };
     const int Mz = rz.L, lz = fft_ls(Mz);
     Cx<R>* tw = reinterpret_cast<Cx<R>*>(smraw);
     Cx<R>* a = tw + Mz;
     Cx<R>* b = a + NC * lz;
     load_twiddles<R>(tw, twg, Mz);
-    const int x = vb.y;
-    const int y0 = vb.x * 2 * NC;
     constexpr int U = 4;  // elements per thread per round, their loads issued together
     for (DivWalk w(threadIdx.x, blockDim.x, Mz); w.q < NC;) {
         int cs[U], ks[U];
@@ -424,29 +528,12 @@ __device__ __forceinline__ void zinv_body(const Cx<R>* __restrict__ W, R* __rest
     }
     __syncthreads();
     Cx<R>* res = fft_lines<R, true, true>(a, b, lz, NC, rz, tw);
-    OutScale64 out64 = {};
-    if constexpr (sizeof(R) == 8) out64 = out_scale64(st);
-    const R fscale = (R)st->phi_scalef * mul;  // (float)(norm / denom), computed once by the mesh finalize
-    for (DivWalk w(threadIdx.x, blockDim.x, nz); w.q < NC; w.next()) {
-        const int c = w.q, z = w.r;
-        const int ya = y0 + 2 * c, yb = ya + 1;
-        const Cx<R> v = res[c * lz + z];
-        if constexpr (sizeof(R) == 8) {
-            if (ya < ny) phi[((size_t)x * ny + ya) * nz + z] = out64(v.x);
-            if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = out64(v.y);
-        } else {
-            const bool zx = zero_axis == 0 && x == nx - 1, zz = zero_axis == 2 && z == nz - 1;
-            const bool za = zx || zz || (zero_axis == 1 && ya == ny - 1);
-            const bool zb = zx || zz || (zero_axis == 1 && yb == ny - 1);
-            if (ya < ny) phi[((size_t)x * ny + ya) * nz + z] = za ? (R)0 : v.x * fscale;
-            if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = zb ? (R)0 : v.y * fscale;
-        }
-    }
+    for (DivWalk w(threadIdx.x, blockDim.x, nz); w.q < NC; w.next()) put(w.q, w.r, res[w.q * lz + w.r]);
 }
 
 // blockIdx.z: the output (0 the potential; with spectral fields 1 Ex, 2 Ey, 3 Ez)
 template <typename R>
-__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB<R>) k_zinv(const Cx<R>* __restrict__ W, R* __restrict__ phi,
+__global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB) k_zinv(const Cx<R>* __restrict__ W, R* __restrict__ phi,
                                                       int ny, int nz, int My, int Kz, RadixPlan rz,
                                                       const Cx<R>* __restrict__ twg, int NC,
                                                       const ScState* st, Spec<R> sp) {
@@ -779,6 +866,59 @@ __host__ __device__ __forceinline__ Spec<R> spec_of(const Plan& p, const Layout&
     return sp;
 }
 
+// f(IntC<L>) on the host for a streamed length (with_stream's list)
+template <typename F>
+static cudaError_t stream_host(int L, F&& f) {
+    switch (L) {
+        case 64: return f(IntC<64>{});
+        case 96: return f(IntC<96>{});
+        case 128: return f(IntC<128>{});
+        case 192: return f(IntC<192>{});
+        case 256: return f(IntC<256>{});
+        default: return cudaErrorInvalidValue;
+    }
+}
+// launches of the separate passes: the streamed kernel of the length, or the staged one
+template <typename R, typename... A>
+static cudaError_t launch_zfwd(int M, dim3 g, size_t sm, cudaStream_t s, A... a) {
+    cudaError_t e;
+    if constexpr (sizeof(R) == 4)
+        if (streamed<R>(M))
+            return stream_host(M, [&](auto L) -> cudaError_t {
+                auto* k = k_zfwd_s<decltype(L)::value>;
+                if ((e = set_smem(k, sm))) return e;
+                return launch(k, g, 128, sm, s, a...);
+            });
+    if ((e = set_smem(k_zfwd<R>, sm))) return e;
+    return launch(k_zfwd<R>, g, FFT_THREADS<R>, sm, s, a...);
+}
+template <typename R, bool INV, typename... A>
+static cudaError_t launch_ypass(int M, dim3 g, size_t sm, cudaStream_t s, A... a) {
+    cudaError_t e;
+    if constexpr (sizeof(R) == 4)
+        if (streamed<R>(M))
+            return stream_host(M, [&](auto L) -> cudaError_t {
+                constexpr int LL = decltype(L)::value;
+                if ((e = set_smem(k_ypass_s<INV, LL>, sm))) return e;
+                return launch(k_ypass_s<INV, LL>, g, stream_threads(LL), sm, s, a...);
+            });
+    if ((e = set_smem(k_ypass<R, INV>, sm))) return e;
+    return launch(k_ypass<R, INV>, g, FFT_THREADS<R>, sm, s, a...);
+}
+template <typename R, typename... A>
+static cudaError_t launch_xconv(int M, dim3 g, size_t sm, cudaStream_t s, A... a) {
+    cudaError_t e;
+    if constexpr (sizeof(R) == 4)
+        if (streamed<R>(M))
+            return stream_host(M, [&](auto L) -> cudaError_t {
+                constexpr int LL = decltype(L)::value;
+                if ((e = set_smem(k_xconv_s<LL>, sm))) return e;
+                return launch(k_xconv_s<LL>, g, stream_threads(LL), sm, s, a...);
+            });
+    if ((e = set_smem(k_xconv<R>, sm))) return e;
+    return launch(k_xconv<R>, g, FFT_THREADS<R>, sm, s, a...);
+}
+
 template <typename R>
 static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid, R* phi, const long long* qfix,
                               cudaStream_t s, int part, bool fields, bool want_phi) {
@@ -793,12 +933,11 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
     const Cx<R>* twz = reinterpret_cast<const Cx<R>*>(ws + L.tw_z);
     cudaError_t e;
     const int NC = z_lines_per_block(p.Mz);
-    const size_t smz = sizeof(Cx<R>) * (size_t)(p.Mz + 2 * NC * fft_ls(p.Mz));
+    const size_t smz = smem_zf<R>(p.Mz, NC), smzi = smem_zi<R>(p.Mz, NC);
     dim3 gz((p.ny + 2 * NC - 1) / (2 * NC), p.nx);
     const int tky = pass_cols<R>(p.fft_cols_y, p.My), tkx = pass_cols<R>(p.fft_cols_x, p.Mx, nbuf);
     const int tkyi = pass_cols<R>(p.fft_cols_y, p.My, nbuf);  // the y inverse
-    const size_t smy = sizeof(Cx<R>) * (size_t)(p.My + 2 * tky * fft_ls(p.My));
-    const size_t smyi = sizeof(Cx<R>) * (size_t)(p.My + nbuf * tkyi * fft_ls(p.My));
+    const size_t smy = smem_yf<R>(p.My, tky), smyi = smem_yi<R>(p.My, tkyi, sp.W2 != nullptr);
     const int ycols = p.nx * Kz;  // the y passes' columns (x, kz)
     dim3 gy((ycols + tky - 1) / tky);
     dim3 gyi((ycols + tkyi - 1) / tkyi, sp.W2 ? 2 : 1);
@@ -810,16 +949,14 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
         if ((e = set_smem(k_zy_fwd<R>, smp))) return e;
         launch(k_zy_fwd<R>, p.nx, PLANE_THREADS<R>, smp, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, p.ry, twz, twy, st);
     } else if (part != CONV_REST) {
-        if ((e = set_smem(k_zfwd<R>, smz))) return e;
-        launch(k_zfwd<R>, gz, FFT_THREADS<R>, smz, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st);
-        if ((e = set_smem(k_ypass<R, false>, smy))) return e;
-        launch(k_ypass<R, false>, gy, FFT_THREADS<R>, smy, s, W, p.nx, p.ny, p.My, Kz, p.ry, twy, tky, st, Spec<R>{});
+        if ((e = launch_zfwd<R>(p.Mz, gz, smz, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st))) return e;
+        if ((e = launch_ypass<R, false>(p.My, gy, smy, s, W, p.nx, p.ny, p.My, Kz, p.ry, twy, tky, st, Spec<R>{})))
+            return e;
     }
     if (part == CONV_FORWARD) return cudaGetLastError();
-    const size_t smx = sizeof(Cx<R>) * (size_t)(p.Mx + nbuf * tkx * fft_ls(p.Mx));
+    const size_t smx = smem_x<R>(p.Mx, tkx, sp.W2 != nullptr);
     dim3 gx((p.My * Kz + tkx - 1) / tkx);  // the x pass's columns (ky, kz)
-    if ((e = set_smem(k_xconv<R>, smx))) return e;
-    launch(k_xconv<R>, gx, FFT_THREADS<R>, smx, s, W, G, p.nx, p.My, Kz, Ky, p.rx, twx, tkx, st, sp);
+    if ((e = launch_xconv<R>(p.Mx, gx, smx, s, W, G, p.nx, p.My, Kz, Ky, p.rx, twx, tkx, st, sp))) return e;
     const int nout = sp.W2 ? 4 - sp.f0 : 1;  // [the potential,] Ex, Ey, Ez
     if (plane_inv) {
         if ((e = set_smem(k_yz_inv<R>, smp))) return e;
@@ -827,10 +964,9 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
                st, sp);
         return cudaGetLastError();
     }
-    if ((e = set_smem(k_ypass<R, true>, smyi))) return e;
-    launch(k_ypass<R, true>, gyi, FFT_THREADS<R>, smyi, s, W, p.nx, p.ny, p.My, Kz, p.ry, twy, tkyi, st, sp);
-    if ((e = set_smem(k_zinv<R>, smz))) return e;
-    launch(k_zinv<R>, dim3(gz.x, gz.y, nout), FFT_THREADS<R>, smz, s, W, phi, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st, sp);
+    if ((e = launch_ypass<R, true>(p.My, gyi, smyi, s, W, p.nx, p.ny, p.My, Kz, p.ry, twy, tkyi, st, sp))) return e;
+    if ((e = set_smem(k_zinv<R>, smzi))) return e;
+    launch(k_zinv<R>, dim3(gz.x, gz.y, nout), FFT_THREADS<R>, smzi, s, W, phi, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st, sp);
     return cudaGetLastError();
 }
 
@@ -838,17 +974,23 @@ template <typename R>
 static cudaError_t prepare_fft_t(const Plan& p) {
     cudaError_t e;
     const int NC = z_lines_per_block(p.Mz);
-    const size_t smz = sizeof(Cx<R>) * (size_t)(p.Mz + 2 * NC * fft_ls(p.Mz));
-    const int nbuf = (p.spectral && sizeof(R) == 4) ? 3 : 2;
+    const size_t smz = smem_zf<R>(p.Mz, NC), smzi = smem_zi<R>(p.Mz, NC);
+    const bool spec = p.spectral && sizeof(R) == 4;
+    const int nbuf = spec ? 3 : 2;
     const int tky = strided_cols<R>(p.My), tkx = strided_cols<R>(p.Mx, nbuf), tkyi = strided_cols<R>(p.My, nbuf);
-    const size_t smy = sizeof(Cx<R>) * (size_t)(p.My + 2 * tky * fft_ls(p.My));
-    const size_t smyi = sizeof(Cx<R>) * (size_t)(p.My + nbuf * tkyi * fft_ls(p.My));
-    const size_t smx = sizeof(Cx<R>) * (size_t)(p.Mx + nbuf * tkx * fft_ls(p.Mx));
-    if ((e = set_smem(k_zfwd<R>, smz))) return e;
-    if ((e = set_smem(k_ypass<R, false>, smy))) return e;
-    if ((e = set_smem(k_xconv<R>, smx))) return e;
-    if ((e = set_smem(k_ypass<R, true>, smyi))) return e;
-    if ((e = set_smem(k_zinv<R>, smz))) return e;
+    const size_t smy = smem_yf<R>(p.My, tky), smyi = smem_yi<R>(p.My, tkyi, spec), smx = smem_x<R>(p.Mx, tkx, spec);
+    if constexpr (sizeof(R) == 4) {
+        auto opt = [&](int M, auto&& f) { return streamed<R>(M) ? stream_host(M, f) : cudaSuccess; };
+        if ((e = opt(p.Mz, [&](auto L) { return set_smem(k_zfwd_s<decltype(L)::value>, smz); }))) return e;
+        if ((e = opt(p.My, [&](auto L) { return set_smem(k_ypass_s<false, decltype(L)::value>, smy); }))) return e;
+        if ((e = opt(p.My, [&](auto L) { return set_smem(k_ypass_s<true, decltype(L)::value>, smyi); }))) return e;
+        if ((e = opt(p.Mx, [&](auto L) { return set_smem(k_xconv_s<decltype(L)::value>, smx); }))) return e;
+    }
+    if (!streamed<R>(p.Mz) && (e = set_smem(k_zfwd<R>, smz))) return e;
+    if (!streamed<R>(p.My) && (e = set_smem(k_ypass<R, false>, smy))) return e;
+    if (!streamed<R>(p.My) && (e = set_smem(k_ypass<R, true>, smyi))) return e;
+    if (!streamed<R>(p.Mx) && (e = set_smem(k_xconv<R>, smx))) return e;
+    if ((e = set_smem(k_zinv<R>, smzi))) return e;
     if (plane_fits<R>(p, optin_smem())) {
         if ((e = set_smem(k_zy_fwd<R>, plane_smem<R>(p)))) return e;
         if ((e = set_smem(k_yz_inv<R>, plane_smem<R>(p)))) return e;
@@ -907,52 +1049,52 @@ cudaError_t launch_field_grids(const Plan& p, const Layout& L, char* ws, cudaStr
     const Plan& p = B.p;                                                        \
     const ScState* st = reinterpret_cast<const ScState*>(ws + L.state);
 
-__global__ void __launch_bounds__(FFT_THREADS<float>) kb_zfwd(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(FFT_THREADS<float>, FFT_MINB) kb_zfwd(const BatchBeam* __restrict__ beams,
                                                        const int* __restrict__ start, int nb) {
     pdl_wait();
     BATCH_BEAM(BS_FFT_Z)
-    zfwd_body<float>(reinterpret_cast<float*>(ws + L.qgrid), reinterpret_cast<const long long*>(ws + L.qfix),
+    zfwd_body<float, ST_ANY>(reinterpret_cast<float*>(ws + L.qgrid), reinterpret_cast<const long long*>(ws + L.qfix),
                      reinterpret_cast<Cx<float>*>(ws + L.W), p.ny, p.nz, p.My, p.Mz / 2 + 1, p.rz,
                      reinterpret_cast<const Cx<float>*>(ws + L.tw_z), B.fft_nc, st, vb);
 }
 
 // forward y pass
-__global__ void __launch_bounds__(FFT_THREADS<float>) kb_yfwd(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(FFT_THREADS<float>, FFT_MINB) kb_yfwd(const BatchBeam* __restrict__ beams,
                                                        const int* __restrict__ start, int nb) {
     pdl_wait();
     BATCH_BEAM(BS_FFT_Y)
-    ypass_body<float, false>(reinterpret_cast<Cx<float>*>(ws + L.W), p.nx, p.ny, p.My, p.Mz / 2 + 1, p.ry,
+    ypass_body<float, false, ST_ANY>(reinterpret_cast<Cx<float>*>(ws + L.W), p.nx, p.ny, p.My, p.Mz / 2 + 1, p.ry,
                              reinterpret_cast<const Cx<float>*>(ws + L.tw_y), B.fft_tky, st, vb);
 }
 
 // inverse y pass: block row 0 takes W (and, with spectral fields, W x D(ky)
 // into W3), row 1 the x-differenced W2 (as k_ypass's blockIdx.y)
-__global__ void __launch_bounds__(FFT_THREADS<float>) kb_yinv(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(FFT_THREADS<float>, FFT_MINB) kb_yinv(const BatchBeam* __restrict__ beams,
                                                        const int* __restrict__ start, int nb) {
     pdl_wait();
     BATCH_BEAM(BS_FFT_YI)
     const Spec<float> sp = spec_of<float>(p, L, ws, true);
     const Cx<float>* tw = reinterpret_cast<const Cx<float>*>(ws + L.tw_y);
     if (vb.y == 0)
-        ypass_body<float, true>(reinterpret_cast<Cx<float>*>(ws + L.W), p.nx, p.ny, p.My, p.Mz / 2 + 1, p.ry, tw,
+        ypass_body<float, true, ST_ANY>(reinterpret_cast<Cx<float>*>(ws + L.W), p.nx, p.ny, p.My, p.Mz / 2 + 1, p.ry, tw,
                                 B.fft_tky, st, vb, sp.W3, sp.dy);
     else
-        ypass_body<float, true>(sp.W2, p.nx, p.ny, p.My, p.Mz / 2 + 1, p.ry, tw, B.fft_tky, st, vb);
+        ypass_body<float, true, ST_ANY>(sp.W2, p.nx, p.ny, p.My, p.Mz / 2 + 1, p.ry, tw, B.fft_tky, st, vb);
 }
 
-__global__ void __launch_bounds__(FFT_THREADS<float>) kb_xconv(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(FFT_THREADS<float>, FFT_MINB) kb_xconv(const BatchBeam* __restrict__ beams,
                                                         const int* __restrict__ start, int nb) {
     pdl_wait();
     BATCH_BEAM(BS_FFT_X)
     const Spec<float> sp = spec_of<float>(p, L, ws, true);
-    xconv_body<float>(reinterpret_cast<Cx<float>*>(ws + L.W), reinterpret_cast<const float*>(ws + L.green), p.nx,
+    xconv_body<float, ST_ANY>(reinterpret_cast<Cx<float>*>(ws + L.W), reinterpret_cast<const float*>(ws + L.green), p.nx,
                       p.My, p.Mz / 2 + 1, p.My / 2 + 1, p.rx, reinterpret_cast<const Cx<float>*>(ws + L.tw_x),
                       B.fft_tkx, st, vb, sp.W2, sp.dx);
 }
 
 // inverse z pass: block group f writes output f (the potential; with spectral
 // fields also Ex, Ey, Ez), as k_zinv's blockIdx.z
-__global__ void __launch_bounds__(FFT_THREADS<float>) kb_zinv(const BatchBeam* __restrict__ beams,
+__global__ void __launch_bounds__(FFT_THREADS<float>, FFT_MINB) kb_zinv(const BatchBeam* __restrict__ beams,
                                                        const int* __restrict__ start, int nb) {
     pdl_wait();
     BATCH_BEAM(BS_FFT_ZI)
@@ -989,8 +1131,9 @@ __global__ void kb_field_octs(const BatchBeam* __restrict__ beams, const int* __
 // others: the batch caps each beam's strided-pass blocks at what lets four
 // blocks share an SM (228 KB per SM, 1 KB reserved per block).
 constexpr size_t BATCH_FFT_SMEM = 233472 / 4 - 1024;
-static int batch_cols(int tk, int M, int nbuf) {
-    while (tk > 2 && sizeof(Cx<float>) * (size_t)(M + nbuf * tk * fft_ls(M)) > BATCH_FFT_SMEM) tk /= 2;
+template <typename F>
+static int batch_cols(int tk, F&& smem) {
+    while (tk > 2 && smem(tk) > BATCH_FFT_SMEM) tk /= 2;
     return tk;
 }
 
@@ -999,8 +1142,13 @@ void batch_fft_tiling(BatchBeam& B, size_t smem[3]) {
     const int Kz = p.Mz / 2 + 1;
     const int nbuf = p.spectral ? 3 : 2;  // line buffers of the x pass and the y passes
     B.fft_nc = z_lines_per_block(p.Mz);
-    B.fft_tky = batch_cols(pass_cols<float>(p.fft_cols_y, p.My, nbuf), p.My, nbuf);
-    B.fft_tkx = batch_cols(pass_cols<float>(p.fft_cols_x, p.Mx, nbuf), p.Mx, nbuf);
+    auto smem_y = [&](int tk) {
+        const size_t f = smem_yf<float>(p.My, tk), i = smem_yi<float>(p.My, tk, p.spectral);
+        return f > i ? f : i;
+    };
+    auto smem_xx = [&](int tk) { return smem_x<float>(p.Mx, tk, p.spectral); };
+    B.fft_tky = batch_cols(pass_cols<float>(p.fft_cols_y, p.My, nbuf), smem_y);
+    B.fft_tkx = batch_cols(pass_cols<float>(p.fft_cols_x, p.Mx, nbuf), smem_xx);
     B.gx[BS_FFT_Z] = (p.ny + 2 * B.fft_nc - 1) / (2 * B.fft_nc);
     B.gy[BS_FFT_Z] = p.nx;
     B.gx[BS_FFT_Y] = (p.nx * Kz + B.fft_tky - 1) / B.fft_tky;  // columns (x, kz)
@@ -1013,9 +1161,10 @@ void batch_fft_tiling(BatchBeam& B, size_t smem[3]) {
     B.gy[BS_FFT_ZI] = p.nx * (p.spectral ? 3 : 1);  // spectral fields: Ex, Ey, Ez (no potential)
     B.gx[BS_FIELD] = p.ny;
     B.gy[BS_FIELD] = p.nx;
-    smem[0] = sizeof(Cx<float>) * (size_t)(p.Mz + 2 * B.fft_nc * fft_ls(p.Mz));
-    smem[1] = sizeof(Cx<float>) * (size_t)(p.My + nbuf * B.fft_tky * fft_ls(p.My));
-    smem[2] = sizeof(Cx<float>) * (size_t)(p.Mx + nbuf * B.fft_tkx * fft_ls(p.Mx));
+    smem[0] = smem_zi<float>(p.Mz, B.fft_nc);
+    if (smem_zf<float>(p.Mz, B.fft_nc) > smem[0]) smem[0] = smem_zf<float>(p.Mz, B.fft_nc);
+    smem[1] = smem_y(B.fft_tky);
+    smem[2] = smem_xx(B.fft_tkx);
 }
 
 cudaError_t prepare_batch_fft() {

@@ -1,5 +1,5 @@
 // Batched FFTs of lines held in shared memory: mixed-radix (3/2/4/8)
-// Stockham passes, and for the common FP32 lengths the two-step form below.
+// Stockham passes, and for the common lengths (64 to 256) the two-step form below.
 //
 // The lines of one thread block live in shared memory, line l at a + l*ls,
 // elements contiguous.  Each stage reads radix-r butterfly inputs with stride
@@ -183,7 +183,7 @@ __device__ __forceinline__ void stockham_stage_c(const Cx<R>* __restrict__ a, Cx
 }
 
 // ---------------------------------------------------------------------------
-// Two-step FFT (FP32 lines of length L = P * Q).  With n = Q n1 + n2 and
+// Two-step FFT (lines of length L = P * Q, P <= Q).  With n = Q n1 + n2 and
 // k = k1 + P k2,
 //   X[k1 + P k2] = sum_n2 w_Q^(n2 k2) w_L^(n2 k1) sum_n1 w_P^(n1 k1) x[Q n1 + n2].
 // Step 1, one work item per (line, n2): the P-point DFT over n1 in registers,
@@ -191,13 +191,21 @@ __device__ __forceinline__ void stockham_stage_c(const Cx<R>* __restrict__ a, Cx
 // Q + 1.  Step 2, one item per (line, k1): the Q-point DFT over n2 in
 // registers, stored in natural order.  Every butterfly stays in registers:
 // one shared-memory round trip and one barrier per step against one per
-// radix stage of the Stockham passes, and about half their instructions
-// (measured alone on this GPU: 1.8x the Stockham rate at L = 128, 2x at 256).
-// Work items run line-fastest (LF) when a power-of-two count of 16 or more
-// lines share the block: the lanes of a half-warp then hold 16 lines at the
-// same offset, which the odd line stride puts on distinct banks.  The
-// twiddles come as tw2[k1 * Q + n2] = w_L^(n2 k1) (load_twiddles lays the
-// table out so for these lengths).
+// radix stage of the Stockham passes, and about half their instructions.
+// Work items run line-fastest (LF) when a power-of-two count of 8 (FP64) or 16
+// lines or more shares the block: the lanes of a quarter- or half-warp then
+// hold as many lines at the same offset, which the odd line stride puts on
+// distinct banks.  The twiddles come as tw2[k1 * Q + n2] = w_L^(n2 k1)
+// (load_twiddles lays the table out so for these lengths).
+//
+// The register DFTs count instructions, FP64 ones above all (this GPU issues
+// them at about 1/64 of the FP32 rate): the factors of the odd half are folded
+// into the final additions as fused multiply-adds (a rotation by c - i s costs
+// c (1 - i s/c), two instructions, and the factor c rides on the four
+// additions; Linzer and Feig's form), and HALF leaves out what the caller's
+// zero padding makes trivial -- HALF_IN: the second half of the inputs is zero;
+// HALF_OUT: only the first half of the outputs is wanted.  Instructions of
+// dft8 / dft16: 52 / 148 in full, 36 / 104 with HALF_IN, 44 / 132 with HALF_OUT.
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ __forceinline__ R fmar(R a, R b, R c) {
@@ -209,87 +217,19 @@ __device__ __forceinline__ Cx<R> cmulc(Cx<R> v, R wr, R wi) {  // v * (wr + i wi
     return cx<R>(fmar<R>(v.x, wr, -(v.y * wi)), fmar<R>(v.x, wi, v.y * wr));
 }
 
-// 16-point DFT, natural order in and out: two 8-point DFTs of the even and
-// odd elements, the odd ones times w16^k
-template <typename R, bool INV>
-__device__ __forceinline__ void dft16(Cx<R>* v) {
-    Cx<R> e[8], o[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        e[i] = v[2 * i];
-        o[i] = v[2 * i + 1];
-    }
-    dft8<R, INV>(e);
-    dft8<R, INV>(o);
-    const R c1 = (R)0.92387953251128675613, s1 = (R)0.38268343236508977173, h = (R)0.70710678118654752440;
-    const R sg = INV ? (R)1 : (R)-1;  // w16^k = cos(2 pi k / 16) + i sg sin(2 pi k / 16)
-    o[1] = cmulc<R>(o[1], c1, sg * s1);
-    o[2] = cx<R>((o[2].x - sg * o[2].y) * h, (o[2].y + sg * o[2].x) * h);
-    o[3] = cmulc<R>(o[3], s1, sg * c1);
-    o[4] = INV ? cmul_pi(o[4]) : cmul_mi(o[4]);
-    o[5] = cmulc<R>(o[5], -s1, sg * c1);
-    o[6] = cx<R>((-o[6].x - sg * o[6].y) * h, (-o[6].y + sg * o[6].x) * h);
-    o[7] = cmulc<R>(o[7], -c1, sg * s1);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        v[k] = cadd(e[k], o[k]);
-        v[k + 8] = csub(e[k], o[k]);
-    }
-}
-
-// 12-point DFT, natural order: n = 4 n1 + n2, k = k1 + 3 k2; four 3-point
-// DFTs, the twiddles w12^(n2 k1), three 4-point DFTs
-template <typename R, bool INV>
-__device__ __forceinline__ void dft12(Cx<R>* v) {
-    Cx<R> y[4][3];
-#pragma unroll
-    for (int n2 = 0; n2 < 4; ++n2) {
-        Cx<R> a = v[n2], b = v[4 + n2], c = v[8 + n2];
-        dft3<R, INV>(a, b, c);
-        y[n2][0] = a;
-        y[n2][1] = b;
-        y[n2][2] = c;
-    }
-    const R r3 = (R)0.86602540378443864676, hf = (R)0.5;
-    const R sg = INV ? (R)1 : (R)-1;
-    y[1][1] = cmulc<R>(y[1][1], r3, sg * hf);             // w12^1
-    y[1][2] = cmulc<R>(y[1][2], hf, sg * r3);             // w12^2
-    y[2][1] = cmulc<R>(y[2][1], hf, sg * r3);             // w12^2
-    y[2][2] = cmulc<R>(y[2][2], -hf, sg * r3);            // w12^4
-    y[3][1] = INV ? cmul_pi(y[3][1]) : cmul_mi(y[3][1]);  // w12^3
-    y[3][2] = cx<R>(-y[3][2].x, -y[3][2].y);              // w12^6
-#pragma unroll
-    for (int k1 = 0; k1 < 3; ++k1) {
-        Cx<R> a0 = y[0][k1], a1 = y[1][k1], a2 = y[2][k1], a3 = y[3][k1];
-        dft4<Cx<R>, INV>(a0, a1, a2, a3);
-        v[k1] = a0;
-        v[k1 + 3] = a1;
-        v[k1 + 6] = a2;
-        v[k1 + 9] = a3;
-    }
-}
-
-// FP64 register DFTs.  The FP64 passes are bound by the FP64 pipe, so these
-// count instructions: the factors of the odd half are folded into the final
-// additions as fused multiply-adds (a rotation by c - i s costs c (1 - i s/c),
-// two instructions, and the factor c rides on the four additions; Linzer and
-// Feig's form), and HALF leaves out what the caller's zero padding makes
-// trivial -- HALF_IN: the second half of the inputs is zero; HALF_OUT: only the
-// first half of the outputs is wanted.  Instructions of dft8 / dft16: 52 / 148
-// in full, 36 / 104 with HALF_IN, 44 / 132 with HALF_OUT.
 enum DftPart { DFT_FULL = 0, HALF_IN = 1, HALF_OUT = 2 };
 
-template <bool INV, int PART>
-__device__ __forceinline__ void dft4d(double2& a0, double2& a1, double2& a2, double2& a3) {
+template <typename R, bool INV, int PART>
+__device__ __forceinline__ void dftp4(Cx<R>& a0, Cx<R>& a1, Cx<R>& a2, Cx<R>& a3) {
     if constexpr (PART == HALF_IN) {  // a2 = a3 = 0
-        const double2 t = INV ? cmul_pi(a1) : cmul_mi(a1);
-        const double2 x0 = a0;
+        const Cx<R> t = INV ? cmul_pi(a1) : cmul_mi(a1);
+        const Cx<R> x0 = a0;
         a2 = csub(x0, a1);
         a0 = cadd(x0, a1);
         a1 = cadd(x0, t);
         a3 = csub(x0, t);
     } else {
-        double2 t0 = cadd(a0, a2), t1 = csub(a0, a2), t2 = cadd(a1, a3), t3 = csub(a1, a3);
+        Cx<R> t0 = cadd(a0, a2), t1 = csub(a0, a2), t2 = cadd(a1, a3), t3 = csub(a1, a3);
         t3 = INV ? cmul_pi(t3) : cmul_mi(t3);
         a0 = cadd(t0, t2);
         a1 = cadd(t1, t3);
@@ -300,95 +240,95 @@ __device__ __forceinline__ void dft4d(double2& a0, double2& a1, double2& a2, dou
     }
 }
 // e + f q (into x) and e - f q (into y, unless only the first half is wanted)
-template <int PART>
-__device__ __forceinline__ void pm_fma(double2& x, double2& y, double2 e, double2 q, double f) {
-    x.x = fma(f, q.x, e.x);
-    x.y = fma(f, q.y, e.y);
+template <typename R, int PART>
+__device__ __forceinline__ void pm_fma(Cx<R>& x, Cx<R>& y, Cx<R> e, Cx<R> q, R f) {
+    x.x = fmar<R>(f, q.x, e.x);
+    x.y = fmar<R>(f, q.y, e.y);
     if constexpr (PART != HALF_OUT) {
-        y.x = fma(-f, q.x, e.x);
-        y.y = fma(-f, q.y, e.y);
+        y.x = fmar<R>(-f, q.x, e.x);
+        y.y = fmar<R>(-f, q.y, e.y);
     }
 }
-template <int PART>
-__device__ __forceinline__ void pm(double2& x, double2& y, double2 e, double2 o) {
+template <typename R, int PART>
+__device__ __forceinline__ void pm(Cx<R>& x, Cx<R>& y, Cx<R> e, Cx<R> o) {
     x = cadd(e, o);
     if constexpr (PART != HALF_OUT) y = csub(e, o);
 }
-template <bool INV, int PART>
-__device__ __forceinline__ void dft8d(double2* v) {
-    double2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
+template <typename R, bool INV, int PART>
+__device__ __forceinline__ void dftp8(Cx<R>* v) {
+    Cx<R> e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6], o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
     constexpr int IN = PART == HALF_IN ? HALF_IN : DFT_FULL;
-    dft4d<INV, IN>(e0, e1, e2, e3);
-    dft4d<INV, IN>(o0, o1, o2, o3);
-    const double h = 0.70710678118654752440;
+    dftp4<R, INV, IN>(e0, e1, e2, e3);
+    dftp4<R, INV, IN>(o0, o1, o2, o3);
+    const R h = (R) 0.70710678118654752440;
     // w8 = h (1 -+ i), w8^3 = h (-1 -+ i)
-    const double2 q1 = INV ? cx<double>(o1.x - o1.y, o1.x + o1.y) : cx<double>(o1.x + o1.y, o1.y - o1.x);
-    const double2 q3 = INV ? cx<double>(o3.x + o3.y, o3.y - o3.x) : cx<double>(o3.x - o3.y, o3.x + o3.y);
-    pm<PART>(v[0], v[4], e0, o0);
-    pm_fma<PART>(v[1], v[5], e1, q1, h);
-    pm<PART>(v[2], v[6], e2, INV ? cmul_pi(o2) : cmul_mi(o2));
-    pm_fma<PART>(v[3], v[7], e3, q3, -h);
+    const Cx<R> q1 = INV ? cx<R>(o1.x - o1.y, o1.x + o1.y) : cx<R>(o1.x + o1.y, o1.y - o1.x);
+    const Cx<R> q3 = INV ? cx<R>(o3.x + o3.y, o3.y - o3.x) : cx<R>(o3.x - o3.y, o3.x + o3.y);
+    pm<R, PART>(v[0], v[4], e0, o0);
+    pm_fma<R, PART>(v[1], v[5], e1, q1, h);
+    pm<R, PART>(v[2], v[6], e2, INV ? cmul_pi(o2) : cmul_mi(o2));
+    pm_fma<R, PART>(v[3], v[7], e3, q3, -h);
 }
-template <bool INV, int PART>
-__device__ __forceinline__ void dft16d(double2* v) {
-    double2 e[8], o[8];
+template <typename R, bool INV, int PART>
+__device__ __forceinline__ void dftp16(Cx<R>* v) {
+    Cx<R> e[8], o[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
         e[i] = v[2 * i];
         o[i] = v[2 * i + 1];
     }
     constexpr int IN = PART == HALF_IN ? HALF_IN : DFT_FULL;
-    dft8d<INV, IN>(e);
-    dft8d<INV, IN>(o);
-    const double c = 0.92387953251128675613, t = 0.41421356237309504880, h = 0.70710678118654752440;
-    const double g = INV ? t : -t;       // w16 = c (1 + i g), w16^7 = -c (1 - i g)
+    dftp8<R, INV, IN>(e);
+    dftp8<R, INV, IN>(o);
+    const R c = (R)0.92387953251128675613, t = (R)0.41421356237309504880, h = (R)0.70710678118654752440;
+    const R g = INV ? t : -t;       // w16 = c (1 + i g), w16^7 = -c (1 - i g)
     // w16^3 = c (t + i sg), w16^5 = c (-t + i sg), sg = +-1
-    const double2 q1 = cx<double>(fma(-g, o[1].y, o[1].x), fma(g, o[1].x, o[1].y));
-    const double2 q2 = INV ? cx<double>(o[2].x - o[2].y, o[2].x + o[2].y) : cx<double>(o[2].x + o[2].y, o[2].y - o[2].x);
-    const double2 q3 = INV ? cx<double>(fma(t, o[3].x, -o[3].y), fma(t, o[3].y, o[3].x))
-                           : cx<double>(fma(t, o[3].x, o[3].y), fma(t, o[3].y, -o[3].x));
-    const double2 q5 = INV ? cx<double>(fma(-t, o[5].x, -o[5].y), fma(-t, o[5].y, o[5].x))
-                           : cx<double>(fma(-t, o[5].x, o[5].y), fma(-t, o[5].y, -o[5].x));
-    const double2 q6 = INV ? cx<double>(o[6].x + o[6].y, o[6].y - o[6].x) : cx<double>(o[6].x - o[6].y, o[6].x + o[6].y);
-    const double2 q7 = cx<double>(fma(g, o[7].y, o[7].x), fma(-g, o[7].x, o[7].y));
-    pm<PART>(v[0], v[8], e[0], o[0]);
-    pm_fma<PART>(v[1], v[9], e[1], q1, c);
-    pm_fma<PART>(v[2], v[10], e[2], q2, h);
-    pm_fma<PART>(v[3], v[11], e[3], q3, c);
-    pm<PART>(v[4], v[12], e[4], INV ? cmul_pi(o[4]) : cmul_mi(o[4]));
-    pm_fma<PART>(v[5], v[13], e[5], q5, c);
-    pm_fma<PART>(v[6], v[14], e[6], q6, -h);
-    pm_fma<PART>(v[7], v[15], e[7], q7, -c);
+    const Cx<R> q1 = cx<R>(fmar<R>(-g, o[1].y, o[1].x), fmar<R>(g, o[1].x, o[1].y));
+    const Cx<R> q2 = INV ? cx<R>(o[2].x - o[2].y, o[2].x + o[2].y) : cx<R>(o[2].x + o[2].y, o[2].y - o[2].x);
+    const Cx<R> q3 = INV ? cx<R>(fmar<R>(t, o[3].x, -o[3].y), fmar<R>(t, o[3].y, o[3].x))
+                           : cx<R>(fmar<R>(t, o[3].x, o[3].y), fmar<R>(t, o[3].y, -o[3].x));
+    const Cx<R> q5 = INV ? cx<R>(fmar<R>(-t, o[5].x, -o[5].y), fmar<R>(-t, o[5].y, o[5].x))
+                           : cx<R>(fmar<R>(-t, o[5].x, o[5].y), fmar<R>(-t, o[5].y, -o[5].x));
+    const Cx<R> q6 = INV ? cx<R>(o[6].x + o[6].y, o[6].y - o[6].x) : cx<R>(o[6].x - o[6].y, o[6].x + o[6].y);
+    const Cx<R> q7 = cx<R>(fmar<R>(g, o[7].y, o[7].x), fmar<R>(-g, o[7].x, o[7].y));
+    pm<R, PART>(v[0], v[8], e[0], o[0]);
+    pm_fma<R, PART>(v[1], v[9], e[1], q1, c);
+    pm_fma<R, PART>(v[2], v[10], e[2], q2, h);
+    pm_fma<R, PART>(v[3], v[11], e[3], q3, c);
+    pm<R, PART>(v[4], v[12], e[4], INV ? cmul_pi(o[4]) : cmul_mi(o[4]));
+    pm_fma<R, PART>(v[5], v[13], e[5], q5, c);
+    pm_fma<R, PART>(v[6], v[14], e[6], q6, -h);
+    pm_fma<R, PART>(v[7], v[15], e[7], q7, -c);
 }
 // 12 points, n = 4 n1 + n2, k = k1 + 3 k2 (dft12)
-template <bool INV, int PART>
-__device__ __forceinline__ void dft12d(double2* v) {
-    double2 y[4][3];
-    const double s3 = INV ? -0.86602540378443864676 : 0.86602540378443864676;
+template <typename R, bool INV, int PART>
+__device__ __forceinline__ void dftp12(Cx<R>* v) {
+    Cx<R> y[4][3];
+    const R s3 = INV ? (R)-0.86602540378443864676 : (R)0.86602540378443864676;
 #pragma unroll
     for (int n2 = 0; n2 < 4; ++n2) {
-        const double2 a = v[n2], b = v[4 + n2], c = v[8 + n2];
+        const Cx<R> a = v[n2], b = v[4 + n2], c = v[8 + n2];
         if (PART == HALF_IN && n2 >= 2) {  // b = c = 0
             y[n2][0] = y[n2][1] = y[n2][2] = a;
         } else {
-            const double2 t = PART == HALF_IN ? b : cadd(b, c), d = PART == HALF_IN ? b : csub(b, c);
-            const double2 m = cx<double>(fma(-0.5, t.x, a.x), fma(-0.5, t.y, a.y));
+            const Cx<R> t = PART == HALF_IN ? b : cadd(b, c), d = PART == HALF_IN ? b : csub(b, c);
+            const Cx<R> m = cx<R>(fmar<R>((R)-0.5, t.x, a.x), fmar<R>((R)-0.5, t.y, a.y));
             y[n2][0] = cadd(a, t);
-            y[n2][1] = cx<double>(fma(s3, d.y, m.x), fma(-s3, d.x, m.y));
-            y[n2][2] = cx<double>(fma(-s3, d.y, m.x), fma(s3, d.x, m.y));
+            y[n2][1] = cx<R>(fmar<R>(s3, d.y, m.x), fmar<R>(-s3, d.x, m.y));
+            y[n2][2] = cx<R>(fmar<R>(-s3, d.y, m.x), fmar<R>(s3, d.x, m.y));
         }
     }
-    const double r3 = 0.86602540378443864676, hf = 0.5, sg = INV ? 1.0 : -1.0;
-    y[1][1] = cmulc<double>(y[1][1], r3, sg * hf);
-    y[1][2] = cmulc<double>(y[1][2], hf, sg * r3);
-    y[2][1] = cmulc<double>(y[2][1], hf, sg * r3);
-    y[2][2] = cmulc<double>(y[2][2], -hf, sg * r3);
+    const R r3 = (R)0.86602540378443864676, hf = (R)0.5, sg = INV ? (R)1 : (R)-1;
+    y[1][1] = cmulc<R>(y[1][1], r3, sg * hf);
+    y[1][2] = cmulc<R>(y[1][2], hf, sg * r3);
+    y[2][1] = cmulc<R>(y[2][1], hf, sg * r3);
+    y[2][2] = cmulc<R>(y[2][2], -hf, sg * r3);
     y[3][1] = INV ? cmul_pi(y[3][1]) : cmul_mi(y[3][1]);
-    y[3][2] = cx<double>(-y[3][2].x, -y[3][2].y);
+    y[3][2] = cx<R>(-y[3][2].x, -y[3][2].y);
 #pragma unroll
     for (int k1 = 0; k1 < 3; ++k1) {
-        double2 a0 = y[0][k1], a1 = y[1][k1], a2 = y[2][k1], a3 = y[3][k1];
-        dft4d<INV, PART == HALF_OUT ? HALF_OUT : DFT_FULL>(a0, a1, a2, a3);
+        Cx<R> a0 = y[0][k1], a1 = y[1][k1], a2 = y[2][k1], a3 = y[3][k1];
+        dftp4<R, INV, PART == HALF_OUT ? HALF_OUT : DFT_FULL>(a0, a1, a2, a3);
         v[k1] = a0;
         v[k1 + 3] = a1;
         if (PART != HALF_OUT) {
@@ -397,19 +337,11 @@ __device__ __forceinline__ void dft12d(double2* v) {
         }
     }
 }
-template <bool INV, int P, int PART>
-__device__ __forceinline__ void dft_reg64(double2* v) {
-    if constexpr (P == 8) dft8d<INV, PART>(v);
-    else if constexpr (P == 12) dft12d<INV, PART>(v);
-    else dft16d<INV, PART>(v);
-}
-
-template <typename R, bool INV, int P>
+template <typename R, bool INV, int P, int PART>
 __device__ __forceinline__ void dft_reg(Cx<R>* v) {
-    if constexpr (P == 8) dft8<R, INV>(v);
-    else if constexpr (P == 12) dft12<R, INV>(v);
-    else if constexpr (P == 16) dft16<R, INV>(v);
-    else static_assert(P == 8 || P == 12 || P == 16, "register DFT sizes 8, 12, 16");
+    if constexpr (P == 8) dftp8<R, INV, PART>(v);
+    else if constexpr (P == 12) dftp12<R, INV, PART>(v);
+    else dftp16<R, INV, PART>(v);
 }
 
 // v * w (forward) or v * conj(w) (inverse), with fused multiply-adds
@@ -419,79 +351,18 @@ __device__ __forceinline__ Cx<R> twmul(Cx<R> v, Cx<R> w) {
     return cx<R>(fmar<R>(v.x, w.x, -(v.y * w.y)), fmar<R>(v.x, w.y, v.y * w.x));
 }
 
-// Q of the factorisation L = P * Q of the two-step lengths (FP32); 0: the
-// Stockham passes.  Measured in whole kicks on this GPU: the two-step passes
-// are faster where the passes are bound by the SMs' issue rate (meshes of
-// 96 to 128 cells per axis padded to 192 and 256, and batches), the Stockham
-// passes where one wave of blocks makes them latency-bound (64-cell axes
-// padded to 128: 0.228 against 0.221 ms per 2M / 64^3 kick).
+// Q of the factorisation L = P * Q of the two-step lengths; 0: the Stockham
+// passes
 __host__ __device__ constexpr int two_step_q(int L) {
-    return L == 96 ? 12 : (L == 192 ? 16 : (L == 256 ? 16 : 0));
-}
-// the same for FP64, whose passes count FP64 instructions (below)
-__host__ __device__ constexpr int two_step_q64(int L) {
     return L == 64 ? 8 : (L == 96 ? 12 : (L == 128 || L == 192 || L == 256 ? 16 : 0));
 }
 
-// ls >= fft_ls(L) >= P (Q + 1); a holds the input, b is scratch; the result
-// is returned in a.  LF: nl is a power of two, lg its log2.  Called by every
-// thread of the block; ends with a barrier.
-template <typename R, bool INV, int L, bool LF>
-__device__ __forceinline__ Cx<R>* fft_two_step(Cx<R>* a, Cx<R>* b, int ls, int nl, int lg, const Cx<R>* tw2) {
-    constexpr int Q = two_step_q(L), P = L / Q;
-    static_assert(Q > 0 && P * Q == L && P * (Q + 1) <= fft_ls(L), "two-step factorisation");
-    for (int idx = threadIdx.x; idx < nl * Q; idx += blockDim.x) {
-        int line, n2;
-        if (LF) {
-            n2 = idx >> lg;
-            line = idx & (nl - 1);
-        } else {
-            line = idx / Q;
-            n2 = idx - line * Q;
-        }
-        const Cx<R>* src = a + line * ls + n2;
-        Cx<R> v[P];
-#pragma unroll
-        for (int n1 = 0; n1 < P; ++n1) v[n1] = src[n1 * Q];
-        dft_reg<R, INV, P>(v);
-        Cx<R>* dst = b + line * ls + n2;
-        dst[0] = v[0];
-#pragma unroll
-        for (int k1 = 1; k1 < P; ++k1) dst[k1 * (Q + 1)] = twmul<R, INV>(v[k1], tw2[k1 * Q + n2]);
-    }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < nl * P; idx += blockDim.x) {
-        int line, k1;
-        if (LF) {
-            k1 = idx >> lg;
-            line = idx & (nl - 1);
-        } else {
-            line = idx / P;
-            k1 = idx - line * P;
-        }
-        const Cx<R>* src = b + line * ls + k1 * (Q + 1);
-        Cx<R> u[Q];
-#pragma unroll
-        for (int n2 = 0; n2 < Q; ++n2) u[n2] = src[n2];
-        dft_reg<R, INV, Q>(u);
-        Cx<R>* dst = a + line * ls + k1;
-#pragma unroll
-        for (int k2 = 0; k2 < Q; ++k2) dst[k2 * P] = u[k2];
-    }
-    __syncthreads();
-    return a;
-}
-
-template <typename R, bool INV, int L>
-__device__ __forceinline__ Cx<R>* fft_two_step_any(Cx<R>* a, Cx<R>* b, int ls, int nl, const Cx<R>* tw2) {
-    if (nl >= 16 && (nl & (nl - 1)) == 0) return fft_two_step<R, INV, L, true>(a, b, ls, nl, 31 - __clz(nl), tw2);
-    return fft_two_step<R, INV, L, false>(a, b, ls, nl, 0, tw2);
-}
-
-// FP64 lines in two register steps, L = P * Q, P <= Q.  HALF: the passes of the
+// ls >= fft_ls(L) >= P (Q + 1); a holds the input, b is scratch; the result is
+// returned in a.  LF: nl is a power of two, lg its log2.  Called by every thread
+// of the block; ends with a barrier.  HALF: the passes of the
 // zero-padded convolution, whose forward lines are zero past the mesh (at most
 // L / 2 points) and whose inverse lines are only read up to it.  Forward (and
-// without HALF): as fft_two_step, the P-point DFTs first, over inputs of which
+// without HALF): the P-point DFTs first, over inputs of which
 // the second half is zero.  Inverse with HALF: the transposed flow
 //   x[Q k1 + k2] = sum_n1 w_P^(n1 k1) w_L^(n1 k2) sum_n2 w_Q^(n2 k2) X[n1 + P n2],
 // the Q-point DFTs first, then P-point ones of which the first half of the
@@ -500,9 +371,9 @@ __device__ __forceinline__ Cx<R>* fft_two_step_any(Cx<R>* a, Cx<R>* b, int ls, i
 // Stockham passes 3104 each); one shared-memory round trip per step.
 // Measured, 63^3 (128-point lines): x pass 124 -> 92 us, y passes 33 -> 25, z
 // passes 20 and 24 -> 16 and 22 (256-thread blocks of 16 columns).
-template <bool INV, int L, bool LF, bool HALF>
-__device__ __forceinline__ double2* fft_two_step64(double2* a, double2* b, int ls, int nl, int lg, const double2* tw2) {
-    constexpr int Q = two_step_q64(L), P = L / Q;
+template <typename R, bool INV, int L, bool LF, bool HALF>
+__device__ __forceinline__ Cx<R>* fft_two_step(Cx<R>* a, Cx<R>* b, int ls, int nl, int lg, const Cx<R>* tw2) {
+    constexpr int Q = two_step_q(L), P = L / Q;
     static_assert(Q > 0 && P * Q == L && P <= Q && P * (Q + 1) <= fft_ls(L), "two-step factorisation");
     constexpr bool T = INV && HALF;             // the transposed flow
     constexpr int A = T ? P : Q, B = T ? Q : P;  // work items per line of the first and of the second step
@@ -518,26 +389,26 @@ __device__ __forceinline__ double2* fft_two_step64(double2* a, double2* b, int l
     for (int idx = threadIdx.x; idx < nl * A; idx += blockDim.x) {
         int line, m;
         split(idx, A, line, m);
-        const double2* src = a + line * ls + m;
+        const Cx<R>* src = a + line * ls + m;
         if constexpr (T) {
-            double2 v[Q];
+            Cx<R> v[Q];
 #pragma unroll
             for (int n2 = 0; n2 < Q; ++n2) v[n2] = src[n2 * P];
-            dft_reg64<INV, Q, DFT_FULL>(v);
-            double2* dst = b + line * ls + m * (Q + 1);
+            dft_reg<R, INV, Q, DFT_FULL>(v);
+            Cx<R>* dst = b + line * ls + m * (Q + 1);
             dst[0] = v[0];
 #pragma unroll
-            for (int k2 = 1; k2 < Q; ++k2) dst[k2] = twmul<double, INV>(v[k2], tw2[m * Q + k2]);
+            for (int k2 = 1; k2 < Q; ++k2) dst[k2] = twmul<R, INV>(v[k2], tw2[m * Q + k2]);
         } else {
-            double2 v[P];
+            Cx<R> v[P];
 #pragma unroll
             for (int n1 = 0; n1 < P; ++n1)
                 if (!HALF || n1 < P / 2) v[n1] = src[n1 * Q];
-            dft_reg64<INV, P, HALF ? HALF_IN : DFT_FULL>(v);
-            double2* dst = b + line * ls + m;
+            dft_reg<R, INV, P, HALF ? HALF_IN : DFT_FULL>(v);
+            Cx<R>* dst = b + line * ls + m;
             dst[0] = v[0];
 #pragma unroll
-            for (int k1 = 1; k1 < P; ++k1) dst[k1 * (Q + 1)] = twmul<double, INV>(v[k1], tw2[k1 * Q + m]);
+            for (int k1 = 1; k1 < P; ++k1) dst[k1 * (Q + 1)] = twmul<R, INV>(v[k1], tw2[k1 * Q + m]);
         }
     }
     __syncthreads();
@@ -545,21 +416,21 @@ __device__ __forceinline__ double2* fft_two_step64(double2* a, double2* b, int l
         int line, m;
         split(idx, B, line, m);
         if constexpr (T) {
-            const double2* src = b + line * ls + m;
-            double2 u[P];
+            const Cx<R>* src = b + line * ls + m;
+            Cx<R> u[P];
 #pragma unroll
             for (int n1 = 0; n1 < P; ++n1) u[n1] = src[n1 * (Q + 1)];
-            dft_reg64<INV, P, HALF_OUT>(u);
-            double2* dst = a + line * ls + m;
+            dft_reg<R, INV, P, HALF_OUT>(u);
+            Cx<R>* dst = a + line * ls + m;
 #pragma unroll
             for (int k1 = 0; k1 < P / 2; ++k1) dst[k1 * Q] = u[k1];
         } else {
-            const double2* src = b + line * ls + m * (Q + 1);
-            double2 u[Q];
+            const Cx<R>* src = b + line * ls + m * (Q + 1);
+            Cx<R> u[Q];
 #pragma unroll
             for (int n2 = 0; n2 < Q; ++n2) u[n2] = src[n2];
-            dft_reg64<INV, Q, DFT_FULL>(u);
-            double2* dst = a + line * ls + m;
+            dft_reg<R, INV, Q, DFT_FULL>(u);
+            Cx<R>* dst = a + line * ls + m;
 #pragma unroll
             for (int k2 = 0; k2 < Q; ++k2) dst[k2 * P] = u[k2];
         }
@@ -567,11 +438,11 @@ __device__ __forceinline__ double2* fft_two_step64(double2* a, double2* b, int l
     __syncthreads();
     return a;
 }
-template <bool INV, int L, bool HALF>
-__device__ __forceinline__ double2* fft_two_step64_any(double2* a, double2* b, int ls, int nl, const double2* tw2) {
-    if (nl >= 8 && (nl & (nl - 1)) == 0)
-        return fft_two_step64<INV, L, true, HALF>(a, b, ls, nl, 31 - __clz(nl), tw2);
-    return fft_two_step64<INV, L, false, HALF>(a, b, ls, nl, 0, tw2);
+template <typename R, bool INV, int L, bool HALF>
+__device__ __forceinline__ Cx<R>* fft_two_step_any(Cx<R>* a, Cx<R>* b, int ls, int nl, const Cx<R>* tw2) {
+    if (nl >= (sizeof(R) == 8 ? 8 : 16) && (nl & (nl - 1)) == 0)
+        return fft_two_step<R, INV, L, true, HALF>(a, b, ls, nl, 31 - __clz(nl), tw2);
+    return fft_two_step<R, INV, L, false, HALF>(a, b, ls, nl, 0, tw2);
 }
 
 // ls must be at least fft_ls(L)
@@ -587,12 +458,9 @@ __device__ __forceinline__ Cx<R>* fft_stages_c(Cx<R>* a, Cx<R>* b, int ls, int n
     }
 }
 
-// Whether a line length of this precision takes the two-step form (its
-// twiddle table then stays w_L^m in the workspace, the stage table otherwise).
-template <typename R>
-__host__ __device__ constexpr bool uses_two_step(int L) {
-    return (sizeof(R) == 4 ? two_step_q(L) : two_step_q64(L)) != 0;
-}
+// Whether a line length takes the two-step form (its twiddle table then stays
+// w_L^m in the workspace, the stage table otherwise).
+__host__ __device__ constexpr bool uses_two_step(int L) { return two_step_q(L) != 0; }
 
 // FFT of nl lines of length rp.L; a holds the input, b is scratch of the
 // same shape.  Returns the buffer that holds the result.  Must be called by
@@ -601,37 +469,19 @@ __host__ __device__ constexpr bool uses_two_step(int L) {
 // the first L / 2 results (inverse; the rest may not be written).
 template <typename R, bool INV, bool HALF = false>
 __device__ Cx<R>* fft_lines(Cx<R>* a, Cx<R>* b, int ls, int nl, const RadixPlan& rp, const Cx<R>* tw) {
-    if constexpr (sizeof(R) == 8) {
-        switch (rp.L) {
-            case 64: return fft_two_step64_any<INV, 64, HALF>(a, b, ls, nl, tw);
-            case 96: return fft_two_step64_any<INV, 96, HALF>(a, b, ls, nl, tw);
-            case 128: return fft_two_step64_any<INV, 128, HALF>(a, b, ls, nl, tw);
-            case 192: return fft_two_step64_any<INV, 192, HALF>(a, b, ls, nl, tw);
-            case 256: return fft_two_step64_any<INV, 256, HALF>(a, b, ls, nl, tw);
-            default: break;
-        }
-    }
-    if constexpr (sizeof(R) == 4) {  // FP32: two register steps (tw laid out by load_twiddles)
-        switch (rp.L) {
-            case 96: return fft_two_step_any<R, INV, 96>(a, b, ls, nl, tw);
-            case 192: return fft_two_step_any<R, INV, 192>(a, b, ls, nl, tw);
-            case 256: return fft_two_step_any<R, INV, 256>(a, b, ls, nl, tw);
-            default: break;
-        }
-    }
     switch (rp.L) {  // the padded lengths of meshes up to 256 per axis
+        case 64: return fft_two_step_any<R, INV, 64, HALF>(a, b, ls, nl, tw);
+        case 96: return fft_two_step_any<R, INV, 96, HALF>(a, b, ls, nl, tw);
+        case 128: return fft_two_step_any<R, INV, 128, HALF>(a, b, ls, nl, tw);
+        case 192: return fft_two_step_any<R, INV, 192, HALF>(a, b, ls, nl, tw);
+        case 256: return fft_two_step_any<R, INV, 256, HALF>(a, b, ls, nl, tw);
         case 8: return fft_stages_c<R, INV, 8, 0, 1>(a, b, ls, nl, tw);
         case 12: return fft_stages_c<R, INV, 12, 0, 1>(a, b, ls, nl, tw);
         case 16: return fft_stages_c<R, INV, 16, 0, 1>(a, b, ls, nl, tw);
         case 24: return fft_stages_c<R, INV, 24, 0, 1>(a, b, ls, nl, tw);
-        case 48: return fft_stages_c<R, INV, 48, 0, 1>(a, b, ls, nl, tw);
-        case 96: if constexpr (!uses_two_step<R>(96)) return fft_stages_c<R, INV, 96, 0, 1>(a, b, ls, nl, tw); break;
-        case 192: if constexpr (!uses_two_step<R>(192)) return fft_stages_c<R, INV, 192, 0, 1>(a, b, ls, nl, tw); break;
-        case 384: return fft_stages_c<R, INV, 384, 0, 1>(a, b, ls, nl, tw);
         case 32: return fft_stages_c<R, INV, 32, 0, 1>(a, b, ls, nl, tw);
-        case 64: if constexpr (!uses_two_step<R>(64)) return fft_stages_c<R, INV, 64, 0, 1>(a, b, ls, nl, tw); break;
-        case 128: if constexpr (!uses_two_step<R>(128)) return fft_stages_c<R, INV, 128, 0, 1>(a, b, ls, nl, tw); break;
-        case 256: if constexpr (!uses_two_step<R>(256)) return fft_stages_c<R, INV, 256, 0, 1>(a, b, ls, nl, tw); break;
+        case 48: return fft_stages_c<R, INV, 48, 0, 1>(a, b, ls, nl, tw);
+        case 384: return fft_stages_c<R, INV, 384, 0, 1>(a, b, ls, nl, tw);
         case 512: return fft_stages_c<R, INV, 512, 0, 1>(a, b, ls, nl, tw);
         default: break;
     }
@@ -685,7 +535,7 @@ __host__ __device__ inline int stage_tw_exponent(int L, int i) {
 // src already holds the stage table and is copied.
 template <typename R>
 __device__ __forceinline__ void load_twiddles(Cx<R>* dst, const Cx<R>* src, int L) {
-    const int Q = sizeof(R) == 4 ? two_step_q(L) : two_step_q64(L);
+    const int Q = two_step_q(L);
     if (Q) {
         for (int i = threadIdx.x; i < L; i += blockDim.x) {
             const int k1 = i / Q, n2 = i - k1 * Q;

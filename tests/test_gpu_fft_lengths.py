@@ -1,0 +1,34 @@
+"""Transforms at every line length of the two-step form (64, 96, 128, 192 and
+256 points) on meshes that fill half of the padded length, leave one cell or
+many unused, and mix lengths with the Stockham ones: the potential within 1e-12
+(FP64) and 1e-6 (FP32) relative in norm of the oracle's, whose FFTs are numpy's
+on 2N - 1 points."""
+import numpy as np
+import pytest
+
+from conftest import has_gpu
+from oracle import sc_oracle
+
+pytestmark = pytest.mark.gpu
+
+if not has_gpu():
+    pytest.skip("needs a CUDA GPU", allow_module_level=True)
+
+from ocelot_gb300 import SpaceCharge  # noqa: E402
+
+MESHES = [([32, 48, 64], (64, 96, 128)), ([64, 32, 48], (128, 64, 96)),
+                                         ([96, 128, 20], (192, 256, 48)), ([17, 96, 128], (48, 192, 256)),
+                                         ([33, 49, 65], (96, 128, 192)), ([30, 100, 97], (64, 256, 256)),
+                                         ([128, 9, 33], (256, 24, 96))]
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-12), ("fp32", 1e-6)])
+@pytest.mark.parametrize("mesh,padded", MESHES)
+def test_potential_at_two_step_lengths(mesh, padded, precision, tol):
+    sc = SpaceCharge(nmesh_xyz=mesh, precision=precision)
+    assert sc.engine().fft_shape() == padded
+    q = np.random.default_rng(sum(mesh)).random(mesh) * 1e-15
+    steps = (3e-6, 4e-6, 2e-5)
+    ref = sc_oracle.potential(q, steps)
+    phi = sc.potential(q, steps)
+    assert np.linalg.norm(phi - ref) / np.linalg.norm(ref) < tol
