@@ -174,12 +174,18 @@ __global__ void k_init_ws(ScState* st, Cx<R>* tx, int Mx, Cx<R>* ty, int My, Cx<
         st->ws_magic = WS_MAGIC;
     }
     // w_M^m, laid out as fft_lines reads it: entry i holds m = i for the
-    // two-step lengths, the stage table's m for the Stockham lengths (entries
-    // past its M - R0 hold w_M^i, unused)
+    // two-step lengths (FP64: as the fixed-point factor FxW of the same size),
+    // the stage table's m for the Stockham lengths (entries past its M - R0
+    // hold w_M^i, unused)
     double s, c;
     auto entry = [&](int M) {
         const int m = (uses_two_step(M) || i >= M - next_radix(M)) ? i : stage_tw_exponent(M, i);
         sincospi(2.0 * m / M, &s, &c);
+        if constexpr (sizeof(R) == 8)
+            if (uses_two_step(M)) {
+                const FxW w = {FxC(c), FxC(-s)};
+                return cx<R>(__hiloint2double(w.r.L, w.r.H), __hiloint2double(w.i.L, w.i.H));
+            }
         return cx<R>((R)c, (R)-s);
     };
     if (i < Mx) tx[i] = entry(Mx);

@@ -21,16 +21,16 @@
 #include "sc_common.cuh"
 #include "sc_fft_dev.cuh"
 #include "sc_fft_stream.cuh"
+#include "sc_fft_fx.cuh"
 
 namespace ocsc {
 
-// FP64: blocks of 128 threads over half the columns (strided_cols), four or
-// more per SM (128 registers): the x pass of a 63^3 mesh is 1040 blocks, 6.8 per
-// SM, instead of 520, 3.4 (two resident: the second round half empty), and one
-// block's loads overlap the others' arithmetic
+// threads of the staged passes (the lengths outside the two-step form)
 template <typename R>
 constexpr int FFT_THREADS = sizeof(R) == 8 ? 128 : 256;
 constexpr int FFT_MINB = 4;
+// the fixed-point passes: 128 registers
+constexpr int FX_MINB(int L) { return 512 / fx_threads(L); }
 
 // complex lines (two real lines each) per block of the z passes: up to 8,
 // so that a 64^3 mesh gives 256 blocks
@@ -42,7 +42,6 @@ static inline int z_lines_per_block(int Mz) {
 // of 16 columns would not fit in shared memory (FP64 at M = 512)
 template <typename R>
 static inline int strided_cols(int M, int nbuf = 2) {
-    // FP64: as many as give the block's 128 threads a work item each (Q per line, two_step_q)
     int tk = sizeof(R) == 8 && M > 64 ? 8 : 16;
     while (tk > 2 && sizeof(Cx<R>) * (size_t)(M + nbuf * tk * fft_ls(M)) > 200 * 1024) tk /= 2;
     return tk;
@@ -52,24 +51,29 @@ static inline int strided_cols(int M, int nbuf = 2) {
 // (sc_fft_stream.cuh), else twiddles and whole line buffers
 template <typename R>
 static inline size_t smem_zf(int M, int NC) {
+    if (sizeof(R) == 8 && uses_two_step(M)) return fx_smem_z(M, NC);
     return sizeof(Cx<R>) * (streamed<R>(M) ? M + NC * (size_t)(stream_la(M) + stream_lb<R>(M))
                                                 : M + 2 * NC * (size_t)fft_ls(M));
 }
 template <typename R>
 static inline size_t smem_zi(int M, int NC) {
+    if (sizeof(R) == 8 && uses_two_step(M)) return fx_smem_zi(M, NC);
     return sizeof(Cx<R>) * (M + 2 * NC * (size_t)fft_ls(M));
 }
 template <typename R>
 static inline size_t smem_yf(int M, int TK) {
+    if (sizeof(R) == 8 && uses_two_step(M)) return fx_smem_cols(M);
     return sizeof(Cx<R>) * (streamed<R>(M) ? M + TK * (size_t)stream_lb<R>(M) : M + 2 * TK * (size_t)fft_ls(M));
 }
 template <typename R>
 static inline size_t smem_yi(int M, int TK, bool w3) {
+    if (sizeof(R) == 8 && uses_two_step(M)) return fx_smem_cols(M);
     return sizeof(Cx<R>) * (streamed<R>(M) ? (w3 ? 2 : 1) * (M + TK * (size_t)stream_lb<R>(M))
                                                 : M + (w3 ? 3 : 2) * TK * (size_t)fft_ls(M));
 }
 template <typename R>
 static inline size_t smem_x(int M, int TK, bool w2) {
+    if (sizeof(R) == 8 && uses_two_step(M)) return fx_smem_cols(M);
     return sizeof(Cx<R>) * (streamed<R>(M)
                                 ? (w2 ? 2 : 1) * M + TK * (size_t)(stream_la(M) +
                                                                    (w2 && stream_dual_x(M) ? 2 : 1) * stream_lb<R>(M))
@@ -80,6 +84,7 @@ static inline size_t smem_x(int M, int TK, bool w2) {
 // changes no result.
 template <typename R>
 static inline int pass_cols(int want, int M, int nbuf = 2) {
+    if (sizeof(R) == 8 && uses_two_step(M)) return FX_COLS;
     const int fit = strided_cols<R>(M, nbuf);
     return (want > 0 && want < fit) ? want : fit;
 }
@@ -238,7 +243,7 @@ __device__ __forceinline__ void zfwd_body(R* __restrict__ q, const long long* __
         load_twiddles<R>(tw, twg, Mz);
         stage_charge_lines<R>(q, qfix, a, lz, x, y0, NC, ny, nz, Mz, st, (long long)vb.ny * ny * nz, 21);
         __syncthreads();
-        res = fft_lines<R, false, true>(a, b, lz, NC, rz, tw);
+        res = fft_lines<R, false, true, false>(a, b, lz, NC, rz, tw);
     }
     for (DivWalk w(threadIdx.x, blockDim.x, Kz); w.q < NC; w.next()) {
         const int c = w.q, k = w.r;
@@ -267,6 +272,33 @@ __global__ void __launch_bounds__(128, 8) k_zfwd_s(float* __restrict__ q, const 
                                                    const ScState* st) {
     pdl_wait();
     zfwd_body<float, L>(q, qfix, W, ny, nz, My, Kz, rz, twg, NC, st, hw_vblk());
+}
+
+template <int L>
+__global__ void __launch_bounds__(fx_threads(L), FX_MINB(L)) k_zfwd_fx(double* __restrict__ q, double2* __restrict__ W,
+                                                                    int ny, int nz, int My, int Kz,
+                                                                    const double2* __restrict__ twg, int NC,
+                                                                    const ScState* st) {
+    pdl_wait();
+    if (st->status) return;
+    zfwd_fx<L>(q, W, ny, nz, My, Kz, twg, NC, st, hw_vblk());
+}
+template <bool INV, int L>
+__global__ void __launch_bounds__(fx_threads(L), FX_MINB(L)) k_ypass_fx(double2* __restrict__ W, int nx, int ny, int Kz,
+                                                                     const double2* __restrict__ twg,
+                                                                     const ScState* st) {
+    pdl_wait();
+    if (st->status) return;
+    ypass_fx<INV, L>(W, nx, ny, Kz, twg, hw_vblk());
+}
+template <int L>
+__global__ void __launch_bounds__(fx_threads(L), FX_MINB(L)) k_xconv_fx(double2* __restrict__ W,
+                                                                     const double* __restrict__ G, int nx, int My,
+                                                                     int Kz, int Ky, const double2* __restrict__ twg,
+                                                                     const ScState* st) {
+    pdl_wait();
+    if (st->status) return;
+    xconv_fx<L>(W, G, nx, My, Kz, Ky, twg, st, hw_vblk());
 }
 
 // strided pass along y: forward (rows < ny in, all My out) or inverse (all in, rows < ny out),
@@ -317,13 +349,13 @@ __device__ __forceinline__ void ypass_body(Cx<R>* __restrict__ W, int nx, int ny
         }
     }
     __syncthreads();
-    Cx<R>* res = fft_lines<R, INV, true>(a, b, ls, TK, ry, tw);
+    Cx<R>* res = fft_lines<R, INV, true, false>(a, b, ls, TK, ry, tw);
     const int nout = INV ? ny : My;
     if (live)
         for (int y = cm.r0; y < nout; y += cm.rs) W[base + (size_t)y * Kz] = res[cm.kk * ls + y];
     if (W3) {
         __syncthreads();  // a and b are free
-        Cx<R>* res3 = fft_lines<R, INV, true>(c, a, ls, TK, ry, tw);
+        Cx<R>* res3 = fft_lines<R, INV, true, false>(c, a, ls, TK, ry, tw);
         if (live)
             for (int y = cm.r0; y < nout; y += cm.rs) W3[base + (size_t)y * Kz] = res3[cm.kk * ls + y];
     }
@@ -394,7 +426,7 @@ __device__ __forceinline__ void xconv_body(Cx<R>* __restrict__ W, const R* __res
             if (x0 + u * cm.rs < Mx) la[x0 + u * cm.rs] = v[u];
     }
     __syncthreads();
-    Cx<R>* res = fft_lines<R, false, true>(a, b, ls, TK, rx, tw);
+    Cx<R>* res = fft_lines<R, false, true, false>(a, b, ls, TK, rx, tw);
     Cx<R>* lr = res + cm.kk * ls;
     Cx<R>* lc = c + cm.kk * ls;
     for (int x0 = cm.r0; x0 < Mx; x0 += U * cm.rs) {
@@ -421,12 +453,12 @@ __device__ __forceinline__ void xconv_body(Cx<R>* __restrict__ W, const R* __res
         }
     }
     __syncthreads();
-    Cx<R>* res2 = fft_lines<R, true, true>(res, res == a ? b : a, ls, TK, rx, tw);
+    Cx<R>* res2 = fft_lines<R, true, true, false>(res, res == a ? b : a, ls, TK, rx, tw);
     if (live)
         for (int x = cm.r0; x < nx; x += cm.rs) W[(size_t)x * ncol + col] = res2[cm.kk * ls + x];
     if (W2) {
         __syncthreads();  // a and b are free
-        Cx<R>* res3 = fft_lines<R, true, true>(c, a, ls, TK, rx, tw);
+        Cx<R>* res3 = fft_lines<R, true, true, false>(c, a, ls, TK, rx, tw);
         if (live)
             for (int x = cm.r0; x < nx; x += cm.rs) W2[(size_t)x * ncol + col] = res3[cm.kk * ls + x];
     }
@@ -527,7 +559,7 @@ __device__ __forceinline__ void zinv_body(const Cx<R>* __restrict__ W, R* __rest
         }
     }
     __syncthreads();
-    Cx<R>* res = fft_lines<R, true, true>(a, b, lz, NC, rz, tw);
+    Cx<R>* res = fft_lines<R, true, true, sizeof(R) == 4>(a, b, lz, NC, rz, tw);
     for (DivWalk w(threadIdx.x, blockDim.x, nz); w.q < NC; w.next()) put(w.q, w.r, res[w.q * lz + w.r]);
 }
 
@@ -545,6 +577,16 @@ __global__ void __launch_bounds__(FFT_THREADS<R>, FFT_MINB) k_zinv(const Cx<R>* 
     R mul;
     inv_out<R>(sp, st, f, W, phi, src, out, dz, mul);
     zinv_body<R>(src, out, ny, nz, My, Kz, rz, twg, NC, st, hw_vblk(), dz, mul, f - 1, (int)gridDim.y);
+}
+
+template <int L>
+__global__ void __launch_bounds__(fx_threads(L), FX_MINB(L)) k_zinv_fx(const double2* __restrict__ W,
+                                                                    double* __restrict__ phi, int ny, int nz, int My,
+                                                                    int Kz, const double2* __restrict__ twg, int NC,
+                                                                    const ScState* st) {
+    pdl_wait();
+    if (st->status) return;
+    zinv_fx<L>(W, phi, ny, nz, My, Kz, twg, NC, out_scale64(st), hw_vblk());
 }
 
 // FP64 form: Ex,Ey,Ez = forward differences / h, zero on the last plane
@@ -669,7 +711,7 @@ __global__ void k_field_octs_spectral(const float* __restrict__ ex, const float*
 // lines use the second buffer (forward) or whichever buffer the y result
 // does not occupy (inverse).
 // ---------------------------------------------------------------------------
-// FP64: 512, for the 128 registers of the two-step transforms
+// FP64: 512, for the 128 registers of the fixed-point transforms
 template <typename R>
 constexpr int PLANE_THREADS = sizeof(R) == 8 ? 512 : 1024;
 
@@ -878,45 +920,62 @@ static cudaError_t stream_host(int L, F&& f) {
         default: return cudaErrorInvalidValue;
     }
 }
-// launches of the separate passes: the streamed kernel of the length, or the staged one
-template <typename R, typename... A>
-static cudaError_t launch_zfwd(int M, dim3 g, size_t sm, cudaStream_t s, A... a) {
+// Launches of the separate passes: the kernel of the line length (FP32
+// streamed, FP64 fixed point) for the two-step lengths, the staged one for others.
+template <typename R>
+static cudaError_t launch_zfwd(const Plan& p, dim3 g, size_t sm, cudaStream_t s, R* q, const long long* qfix, Cx<R>* W,
+                               int Kz, const Cx<R>* tw, int NC, const ScState* st) {
     cudaError_t e;
-    if constexpr (sizeof(R) == 4)
-        if (streamed<R>(M))
-            return stream_host(M, [&](auto L) -> cudaError_t {
-                auto* k = k_zfwd_s<decltype(L)::value>;
-                if ((e = set_smem(k, sm))) return e;
-                return launch(k, g, 128, sm, s, a...);
-            });
+    if (uses_two_step(p.Mz))
+        return stream_host(p.Mz, [&](auto L) -> cudaError_t {
+            constexpr int LL = decltype(L)::value;
+            if constexpr (sizeof(R) == 4) {
+                if ((e = set_smem(k_zfwd_s<LL>, sm))) return e;
+                return launch(k_zfwd_s<LL>, g, 128, sm, s, q, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, tw, NC, st);
+            } else {
+                if ((e = set_smem(k_zfwd_fx<LL>, sm))) return e;
+                return launch(k_zfwd_fx<LL>, g, NC * two_step_q(LL), sm, s, q, W, p.ny, p.nz, p.My, Kz, tw, NC, st);
+            }
+        });
     if ((e = set_smem(k_zfwd<R>, sm))) return e;
-    return launch(k_zfwd<R>, g, FFT_THREADS<R>, sm, s, a...);
+    return launch(k_zfwd<R>, g, FFT_THREADS<R>, sm, s, q, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, tw, NC, st);
 }
-template <typename R, bool INV, typename... A>
-static cudaError_t launch_ypass(int M, dim3 g, size_t sm, cudaStream_t s, A... a) {
+template <typename R, bool INV>
+static cudaError_t launch_ypass(const Plan& p, dim3 g, size_t sm, cudaStream_t s, Cx<R>* W, int Kz, const Cx<R>* tw,
+                                int TK, const ScState* st, const Spec<R>& sp) {
     cudaError_t e;
-    if constexpr (sizeof(R) == 4)
-        if (streamed<R>(M))
-            return stream_host(M, [&](auto L) -> cudaError_t {
-                constexpr int LL = decltype(L)::value;
+    if (uses_two_step(p.My))
+        return stream_host(p.My, [&](auto L) -> cudaError_t {
+            constexpr int LL = decltype(L)::value;
+            if constexpr (sizeof(R) == 4) {
                 if ((e = set_smem(k_ypass_s<INV, LL>, sm))) return e;
-                return launch(k_ypass_s<INV, LL>, g, stream_threads(LL), sm, s, a...);
-            });
+                return launch(k_ypass_s<INV, LL>, g, stream_threads(LL), sm, s, W, p.nx, p.ny, p.My, Kz, p.ry, tw, TK, st,
+                              sp);
+            } else {
+                if ((e = set_smem(k_ypass_fx<INV, LL>, sm))) return e;
+                return launch(k_ypass_fx<INV, LL>, g, fx_threads(LL), sm, s, W, p.nx, p.ny, Kz, tw, st);
+            }
+        });
     if ((e = set_smem(k_ypass<R, INV>, sm))) return e;
-    return launch(k_ypass<R, INV>, g, FFT_THREADS<R>, sm, s, a...);
+    return launch(k_ypass<R, INV>, g, FFT_THREADS<R>, sm, s, W, p.nx, p.ny, p.My, Kz, p.ry, tw, TK, st, sp);
 }
-template <typename R, typename... A>
-static cudaError_t launch_xconv(int M, dim3 g, size_t sm, cudaStream_t s, A... a) {
+template <typename R>
+static cudaError_t launch_xconv(const Plan& p, dim3 g, size_t sm, cudaStream_t s, Cx<R>* W, const R* G, int Kz, int Ky,
+                                const Cx<R>* tw, int TK, const ScState* st, const Spec<R>& sp) {
     cudaError_t e;
-    if constexpr (sizeof(R) == 4)
-        if (streamed<R>(M))
-            return stream_host(M, [&](auto L) -> cudaError_t {
-                constexpr int LL = decltype(L)::value;
+    if (uses_two_step(p.Mx))
+        return stream_host(p.Mx, [&](auto L) -> cudaError_t {
+            constexpr int LL = decltype(L)::value;
+            if constexpr (sizeof(R) == 4) {
                 if ((e = set_smem(k_xconv_s<LL>, sm))) return e;
-                return launch(k_xconv_s<LL>, g, stream_threads(LL), sm, s, a...);
-            });
+                return launch(k_xconv_s<LL>, g, stream_threads(LL), sm, s, W, G, p.nx, p.My, Kz, Ky, p.rx, tw, TK, st, sp);
+            } else {
+                if ((e = set_smem(k_xconv_fx<LL>, sm))) return e;
+                return launch(k_xconv_fx<LL>, g, fx_threads(LL), sm, s, W, G, p.nx, p.My, Kz, Ky, tw, st);
+            }
+        });
     if ((e = set_smem(k_xconv<R>, sm))) return e;
-    return launch(k_xconv<R>, g, FFT_THREADS<R>, sm, s, a...);
+    return launch(k_xconv<R>, g, FFT_THREADS<R>, sm, s, W, G, p.nx, p.My, Kz, Ky, p.rx, tw, TK, st, sp);
 }
 
 template <typename R>
@@ -949,14 +1008,13 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
         if ((e = set_smem(k_zy_fwd<R>, smp))) return e;
         launch(k_zy_fwd<R>, p.nx, PLANE_THREADS<R>, smp, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, p.ry, twz, twy, st);
     } else if (part != CONV_REST) {
-        if ((e = launch_zfwd<R>(p.Mz, gz, smz, s, qgrid, qfix, W, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st))) return e;
-        if ((e = launch_ypass<R, false>(p.My, gy, smy, s, W, p.nx, p.ny, p.My, Kz, p.ry, twy, tky, st, Spec<R>{})))
-            return e;
+        if ((e = launch_zfwd<R>(p, gz, smz, s, qgrid, qfix, W, Kz, twz, NC, st))) return e;
+        if ((e = launch_ypass<R, false>(p, gy, smy, s, W, Kz, twy, tky, st, Spec<R>{}))) return e;
     }
     if (part == CONV_FORWARD) return cudaGetLastError();
     const size_t smx = smem_x<R>(p.Mx, tkx, sp.W2 != nullptr);
     dim3 gx((p.My * Kz + tkx - 1) / tkx);  // the x pass's columns (ky, kz)
-    if ((e = launch_xconv<R>(p.Mx, gx, smx, s, W, G, p.nx, p.My, Kz, Ky, p.rx, twx, tkx, st, sp))) return e;
+    if ((e = launch_xconv<R>(p, gx, smx, s, W, G, Kz, Ky, twx, tkx, st, sp))) return e;
     const int nout = sp.W2 ? 4 - sp.f0 : 1;  // [the potential,] Ex, Ey, Ez
     if (plane_inv) {
         if ((e = set_smem(k_yz_inv<R>, smp))) return e;
@@ -964,7 +1022,15 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
                st, sp);
         return cudaGetLastError();
     }
-    if ((e = launch_ypass<R, true>(p.My, gyi, smyi, s, W, p.nx, p.ny, p.My, Kz, p.ry, twy, tkyi, st, sp))) return e;
+    if ((e = launch_ypass<R, true>(p, gyi, smyi, s, W, Kz, twy, tkyi, st, sp))) return e;
+    if (sizeof(R) == 8 && uses_two_step(p.Mz)) {
+        if constexpr (sizeof(R) == 8)
+            return stream_host(p.Mz, [&](auto LZ) -> cudaError_t {
+                constexpr int LL = decltype(LZ)::value;
+                if ((e = set_smem(k_zinv_fx<LL>, smzi))) return e;
+                return launch(k_zinv_fx<LL>, gz, NC * two_step_q(LL), smzi, s, W, phi, p.ny, p.nz, p.My, Kz, twz, NC, st);
+            });
+    }
     if ((e = set_smem(k_zinv<R>, smzi))) return e;
     launch(k_zinv<R>, dim3(gz.x, gz.y, nout), FFT_THREADS<R>, smzi, s, W, phi, p.ny, p.nz, p.My, Kz, p.rz, twz, NC, st, sp);
     return cudaGetLastError();
@@ -979,18 +1045,34 @@ static cudaError_t prepare_fft_t(const Plan& p) {
     const int nbuf = spec ? 3 : 2;
     const int tky = strided_cols<R>(p.My), tkx = strided_cols<R>(p.Mx, nbuf), tkyi = strided_cols<R>(p.My, nbuf);
     const size_t smy = smem_yf<R>(p.My, tky), smyi = smem_yi<R>(p.My, tkyi, spec), smx = smem_x<R>(p.Mx, tkx, spec);
-    if constexpr (sizeof(R) == 4) {
-        auto opt = [&](int M, auto&& f) { return streamed<R>(M) ? stream_host(M, f) : cudaSuccess; };
-        if ((e = opt(p.Mz, [&](auto L) { return set_smem(k_zfwd_s<decltype(L)::value>, smz); }))) return e;
-        if ((e = opt(p.My, [&](auto L) { return set_smem(k_ypass_s<false, decltype(L)::value>, smy); }))) return e;
-        if ((e = opt(p.My, [&](auto L) { return set_smem(k_ypass_s<true, decltype(L)::value>, smyi); }))) return e;
-        if ((e = opt(p.Mx, [&](auto L) { return set_smem(k_xconv_s<decltype(L)::value>, smx); }))) return e;
-    }
-    if (!streamed<R>(p.Mz) && (e = set_smem(k_zfwd<R>, smz))) return e;
-    if (!streamed<R>(p.My) && (e = set_smem(k_ypass<R, false>, smy))) return e;
-    if (!streamed<R>(p.My) && (e = set_smem(k_ypass<R, true>, smyi))) return e;
-    if (!streamed<R>(p.Mx) && (e = set_smem(k_xconv<R>, smx))) return e;
-    if ((e = set_smem(k_zinv<R>, smzi))) return e;
+    auto prep = [&](int M, auto&& two_step, auto* staged, size_t sm) -> cudaError_t {
+        return uses_two_step(M) ? stream_host(M, two_step) : set_smem(staged, sm);
+    };
+    if ((e = prep(p.Mz, [&](auto L) {
+             constexpr int LL = decltype(L)::value;
+             if constexpr (sizeof(R) == 4) return set_smem(k_zfwd_s<LL>, smz);
+             else return set_smem(k_zfwd_fx<LL>, smz);
+         }, k_zfwd<R>, smz))) return e;
+    if ((e = prep(p.My, [&](auto L) {
+             constexpr int LL = decltype(L)::value;
+             if constexpr (sizeof(R) == 4) return set_smem(k_ypass_s<false, LL>, smy);
+             else return set_smem(k_ypass_fx<false, LL>, smy);
+         }, k_ypass<R, false>, smy))) return e;
+    if ((e = prep(p.My, [&](auto L) {
+             constexpr int LL = decltype(L)::value;
+             if constexpr (sizeof(R) == 4) return set_smem(k_ypass_s<true, LL>, smyi);
+             else return set_smem(k_ypass_fx<true, LL>, smyi);
+         }, k_ypass<R, true>, smyi))) return e;
+    if ((e = prep(p.Mx, [&](auto L) {
+             constexpr int LL = decltype(L)::value;
+             if constexpr (sizeof(R) == 4) return set_smem(k_xconv_s<LL>, smx);
+             else return set_smem(k_xconv_fx<LL>, smx);
+         }, k_xconv<R>, smx))) return e;
+    if ((e = prep(p.Mz, [&](auto L) {
+             constexpr int LL = decltype(L)::value;
+             if constexpr (sizeof(R) == 4) return set_smem(k_zinv<R>, smzi);
+             else return set_smem(k_zinv_fx<LL>, smzi);
+         }, k_zinv<R>, smzi))) return e;
     if (plane_fits<R>(p, optin_smem())) {
         if ((e = set_smem(k_zy_fwd<R>, plane_smem<R>(p)))) return e;
         if ((e = set_smem(k_yz_inv<R>, plane_smem<R>(p)))) return e;

@@ -10,7 +10,7 @@
 // of entries per stage, read by consecutive lanes); the inverse uses their
 // conjugates and leaves the 1/L normalisation to the caller.
 #pragma once
-#include "sc_common.cuh"
+#include "sc_fx.cuh"
 
 namespace ocsc {
 
@@ -198,23 +198,30 @@ __device__ __forceinline__ void stockham_stage_c(const Cx<R>* __restrict__ a, Cx
 // distinct banks.  The twiddles come as tw2[k1 * Q + n2] = w_L^(n2 k1)
 // (load_twiddles lays the table out so for these lengths).
 //
-// The register DFTs count instructions, FP64 ones above all (this GPU issues
-// them at about 1/64 of the FP32 rate): the factors of the odd half are folded
+// The register DFTs count instructions: the factors of the odd half are folded
 // into the final additions as fused multiply-adds (a rotation by c - i s costs
 // c (1 - i s/c), two instructions, and the factor c rides on the four
 // additions; Linzer and Feig's form), and HALF leaves out what the caller's
 // zero padding makes trivial -- HALF_IN: the second half of the inputs is zero;
 // HALF_OUT: only the first half of the outputs is wanted.  Instructions of
 // dft8 / dft16: 52 / 148 in full, 36 / 104 with HALF_IN, 44 / 132 with HALF_OUT.
+// The FP64 form runs the same DFTs on 64-bit integers (R = Fx), where a factor
+// is applied once and the product added and subtracted.
 // ---------------------------------------------------------------------------
+// the constants of the register DFTs, and a constant times a value plus another
+template <typename R> struct KT { using T = R; };
+template <> struct KT<Fx> { using T = FxC; };
+template <typename R> using Kc = typename KT<R>::T;
 template <typename R>
-__device__ __forceinline__ R fmar(R a, R b, R c) {
-    if constexpr (sizeof(R) == 4) return fmaf(a, b, c);
-    else return fma(a, b, c);
+__device__ __forceinline__ R fmar(Kc<R> k, R b, R c) {
+    if constexpr (sizeof(R) == 4) return fmaf(k, b, c);
+    else return fx_mul(b, k) + c;
 }
-template <typename R>
-__device__ __forceinline__ Cx<R> cmulc(Cx<R> v, R wr, R wi) {  // v * (wr + i wi), constant factor
-    return cx<R>(fmar<R>(v.x, wr, -(v.y * wi)), fmar<R>(v.x, wi, v.y * wr));
+__device__ __forceinline__ Cx<float> cmulc(Cx<float> v, float wr, float wi) {  // v * (wr + i wi), constant factor
+    return cx<float>(fmaf(v.x, wr, -(v.y * wi)), fmaf(v.x, wi, v.y * wr));
+}
+__device__ __forceinline__ Cx<Fx> cmulc(Cx<Fx> v, FxC wr, FxC wi) {
+    return cx<Fx>(fx_mul2(v.x, wr, v.y, -wi), fx_mul2(v.x, wi, v.y, wr));
 }
 
 enum DftPart { DFT_FULL = 0, HALF_IN = 1, HALF_OUT = 2 };
@@ -241,7 +248,13 @@ __device__ __forceinline__ void dftp4(Cx<R>& a0, Cx<R>& a1, Cx<R>& a2, Cx<R>& a3
 }
 // e + f q (into x) and e - f q (into y, unless only the first half is wanted)
 template <typename R, int PART>
-__device__ __forceinline__ void pm_fma(Cx<R>& x, Cx<R>& y, Cx<R> e, Cx<R> q, R f) {
+__device__ __forceinline__ void pm_fma(Cx<R>& x, Cx<R>& y, Cx<R> e, Cx<R> q, Kc<R> f) {
+    if constexpr (sizeof(R) == 8) {  // one product for both signs
+        const Cx<R> p = cx<R>(fx_mul(q.x, f), fx_mul(q.y, f));
+        x = cadd(e, p);
+        if constexpr (PART != HALF_OUT) y = csub(e, p);
+        return;
+    }
     x.x = fmar<R>(f, q.x, e.x);
     x.y = fmar<R>(f, q.y, e.y);
     if constexpr (PART != HALF_OUT) {
@@ -260,7 +273,7 @@ __device__ __forceinline__ void dftp8(Cx<R>* v) {
     constexpr int IN = PART == HALF_IN ? HALF_IN : DFT_FULL;
     dftp4<R, INV, IN>(e0, e1, e2, e3);
     dftp4<R, INV, IN>(o0, o1, o2, o3);
-    const R h = (R) 0.70710678118654752440;
+    const Kc<R> h = Kc<R>(0.70710678118654752440);
     // w8 = h (1 -+ i), w8^3 = h (-1 -+ i)
     const Cx<R> q1 = INV ? cx<R>(o1.x - o1.y, o1.x + o1.y) : cx<R>(o1.x + o1.y, o1.y - o1.x);
     const Cx<R> q3 = INV ? cx<R>(o3.x + o3.y, o3.y - o3.x) : cx<R>(o3.x - o3.y, o3.x + o3.y);
@@ -280,8 +293,8 @@ __device__ __forceinline__ void dftp16(Cx<R>* v) {
     constexpr int IN = PART == HALF_IN ? HALF_IN : DFT_FULL;
     dftp8<R, INV, IN>(e);
     dftp8<R, INV, IN>(o);
-    const R c = (R)0.92387953251128675613, t = (R)0.41421356237309504880, h = (R)0.70710678118654752440;
-    const R g = INV ? t : -t;       // w16 = c (1 + i g), w16^7 = -c (1 - i g)
+    const Kc<R> c = Kc<R>(0.92387953251128675613), t = Kc<R>(0.41421356237309504880), h = Kc<R>(0.70710678118654752440);
+    const Kc<R> g = INV ? t : -t;       // w16 = c (1 + i g), w16^7 = -c (1 - i g)
     // w16^3 = c (t + i sg), w16^5 = c (-t + i sg), sg = +-1
     const Cx<R> q1 = cx<R>(fmar<R>(-g, o[1].y, o[1].x), fmar<R>(g, o[1].x, o[1].y));
     const Cx<R> q2 = INV ? cx<R>(o[2].x - o[2].y, o[2].x + o[2].y) : cx<R>(o[2].x + o[2].y, o[2].y - o[2].x);
@@ -304,7 +317,7 @@ __device__ __forceinline__ void dftp16(Cx<R>* v) {
 template <typename R, bool INV, int PART>
 __device__ __forceinline__ void dftp12(Cx<R>* v) {
     Cx<R> y[4][3];
-    const R s3 = INV ? (R)-0.86602540378443864676 : (R)0.86602540378443864676;
+    const Kc<R> s3 = INV ? Kc<R>(-0.86602540378443864676) : Kc<R>(0.86602540378443864676);
 #pragma unroll
     for (int n2 = 0; n2 < 4; ++n2) {
         const Cx<R> a = v[n2], b = v[4 + n2], c = v[8 + n2];
@@ -312,17 +325,18 @@ __device__ __forceinline__ void dftp12(Cx<R>* v) {
             y[n2][0] = y[n2][1] = y[n2][2] = a;
         } else {
             const Cx<R> t = PART == HALF_IN ? b : cadd(b, c), d = PART == HALF_IN ? b : csub(b, c);
-            const Cx<R> m = cx<R>(fmar<R>((R)-0.5, t.x, a.x), fmar<R>((R)-0.5, t.y, a.y));
+            const Cx<R> m = cx<R>(fmar<R>(Kc<R>(-0.5), t.x, a.x), fmar<R>(Kc<R>(-0.5), t.y, a.y));
             y[n2][0] = cadd(a, t);
             y[n2][1] = cx<R>(fmar<R>(s3, d.y, m.x), fmar<R>(-s3, d.x, m.y));
             y[n2][2] = cx<R>(fmar<R>(-s3, d.y, m.x), fmar<R>(s3, d.x, m.y));
         }
     }
-    const R r3 = (R)0.86602540378443864676, hf = (R)0.5, sg = INV ? (R)1 : (R)-1;
-    y[1][1] = cmulc<R>(y[1][1], r3, sg * hf);
-    y[1][2] = cmulc<R>(y[1][2], hf, sg * r3);
-    y[2][1] = cmulc<R>(y[2][1], hf, sg * r3);
-    y[2][2] = cmulc<R>(y[2][2], -hf, sg * r3);
+    const Kc<R> r3 = Kc<R>(0.86602540378443864676), hf = Kc<R>(0.5);
+    const Kc<R> sr3 = INV ? r3 : -r3, shf = INV ? hf : -hf;
+    y[1][1] = cmulc(y[1][1], r3, shf);
+    y[1][2] = cmulc(y[1][2], hf, sr3);
+    y[2][1] = cmulc(y[2][1], hf, sr3);
+    y[2][2] = cmulc(y[2][2], -hf, sr3);
     y[3][1] = INV ? cmul_pi(y[3][1]) : cmul_mi(y[3][1]);
     y[3][2] = cx<R>(-y[3][2].x, -y[3][2].y);
 #pragma unroll
@@ -350,6 +364,11 @@ __device__ __forceinline__ Cx<R> twmul(Cx<R> v, Cx<R> w) {
     if (INV) return cx<R>(fmar<R>(v.x, w.x, v.y * w.y), fmar<R>(v.y, w.x, -(v.x * w.y)));
     return cx<R>(fmar<R>(v.x, w.x, -(v.y * w.y)), fmar<R>(v.x, w.y, v.y * w.x));
 }
+template <bool INV>
+__device__ __forceinline__ Cx<Fx> twmul(Cx<Fx> v, FxW w) {
+    if (INV) return cx<Fx>(fx_mul2(v.x, w.r, v.y, w.i), fx_mul2(v.y, w.r, -v.x, w.i));
+    return cx<Fx>(fx_mul2(v.x, w.r, -v.y, w.i), fx_mul2(v.x, w.i, v.y, w.r));
+}
 
 // Q of the factorisation L = P * Q of the two-step lengths; 0: the Stockham
 // passes
@@ -367,10 +386,7 @@ __host__ __device__ constexpr int two_step_q(int L) {
 //   x[Q k1 + k2] = sum_n1 w_P^(n1 k1) w_L^(n1 k2) sum_n2 w_Q^(n2 k2) X[n1 + P n2],
 // the Q-point DFTs first, then P-point ones of which the first half of the
 // outputs is kept; the twiddles are the same table w_L^(n1 k2) at n1 * Q + k2.
-// FP64 instructions per 128-point line: 2180 forward, 2308 inverse (the
-// Stockham passes 3104 each); one shared-memory round trip per step.
-// Measured, 63^3 (128-point lines): x pass 124 -> 92 us, y passes 33 -> 25, z
-// passes 20 and 24 -> 16 and 22 (256-thread blocks of 16 columns).
+// One shared-memory round trip per step.  FP32 lines; double ones go through fft_fx.
 template <typename R, bool INV, int L, bool LF, bool HALF>
 __device__ __forceinline__ Cx<R>* fft_two_step(Cx<R>* a, Cx<R>* b, int ls, int nl, int lg, const Cx<R>* tw2) {
     constexpr int Q = two_step_q(L), P = L / Q;
@@ -438,11 +454,138 @@ __device__ __forceinline__ Cx<R>* fft_two_step(Cx<R>* a, Cx<R>* b, int ls, int n
     __syncthreads();
     return a;
 }
+
+// The steps of the two-step form in block fixed point (sc_fx.cuh), one work
+// item each; tab: the line's table, tw: the twiddles as tw2.  The first steps
+// return the magnitude of what they stored: the line's largest decides how far
+// the second steps shift the table down to make room for their growth (no bits
+// are given up where the line leaves room, and a line's spike costs only
+// what it needs).
+template <int L>
+struct FxSteps {
+    static constexpr int Q = two_step_q(L), P = L / Q, ROW = Q + 1;
+    static constexpr int B_HALF = fx_bit(P / 2), B_FULL = fx_bit(P), B_INV = fx_bit(Q);  // input bits
+    template <bool INV>
+    static __device__ __forceinline__ unsigned tw_put(Fx2 v, FxW w, bool one, Fx2* dst) {
+        const Fx2 t = one ? v : twmul<INV>(v, w);
+        *dst = t;
+        return max(fx_mag(t.x), fx_mag(t.y));
+    }
+    // P-point DFTs first: v[n1] = x[Q n1 + m]
+    template <bool INV, int PART>
+    static __device__ __forceinline__ unsigned first(Fx2 (&v)[P], int m, const FxW* tw, Fx2* tab) {
+        dft_reg<Fx, INV, P, PART>(v);
+        unsigned mag = 0;
+#pragma unroll
+        for (int k1 = 0; k1 < P; ++k1)
+            mag = max(mag, tw_put<INV>(v[k1], tw[k1 * Q + m], k1 == 0, tab + k1 * ROW + m));
+        return mag;
+    }
+    // then u[k2] = X[k1 + P k2]
+    template <bool INV>
+    static __device__ __forceinline__ void second(Fx2 (&u)[Q], int k1, const Fx2* tab, int sh) {
+#pragma unroll
+        for (int n2 = 0; n2 < Q; ++n2) u[n2] = fx_down(tab[k1 * ROW + n2], sh);
+        dft_reg<Fx, INV, Q, DFT_FULL>(u);
+    }
+    // the transposed flow: Q-point DFTs first, v[n2] = X[n1 + P n2]
+    static __device__ __forceinline__ unsigned t_first(Fx2 (&v)[Q], int n1, const FxW* tw, Fx2* tab) {
+        dft_reg<Fx, true, Q, DFT_FULL>(v);
+        unsigned mag = 0;
+#pragma unroll
+        for (int k2 = 0; k2 < Q; ++k2)
+            mag = max(mag, tw_put<true>(v[k2], tw[n1 * Q + k2], k2 == 0, tab + n1 * ROW + k2));
+        return mag;
+    }
+    // then u[k1] = x[Q k1 + k2], k1 < P / 2
+    static __device__ __forceinline__ void t_second(Fx2 (&u)[P], int k2, const Fx2* tab, int sh) {
+#pragma unroll
+        for (int n1 = 0; n1 < P; ++n1) u[n1] = fx_down(tab[n1 * ROW + k2], sh);
+        dft_reg<Fx, true, P, HALF_OUT>(u);
+    }
+};
+
+// fft_two_step for double lines (lg >= 0: line-fastest).  Each line's exponent and
+// table magnitude stand in the slot after its table.  The error against 80-bit
+// arithmetic, as a fraction of the double two-step form's (2-norm; random lines,
+// charge and spectrum shaped ones, spikes, 20 decades): 0.45 - 0.7 at 64 to 128
+// points, 0.47 - 0.9 at 192 and 256.
+template <bool INV, int L, bool HALF>
+__device__ __forceinline__ Cx<double>* fft_fx(Cx<double>* a, Cx<double>* b, int ls, int nl, int lg,
+                                              const Cx<double>* tw2) {
+    using S = FxSteps<L>;
+    constexpr int Q = S::Q, P = S::P, SLOT = P * S::ROW;
+    static_assert(Q > 0 && P * Q == L && P <= Q && SLOT < fft_ls(L), "two-step factorisation");
+    constexpr bool T = INV && HALF;             // the transposed flow
+    constexpr int A = T ? P : Q, B = T ? Q : P;  // work items per line of the first and of the second step
+    constexpr int NIN = T ? Q : (HALF ? P / 2 : P);  // inputs of an item of the first step
+    constexpr int BIT = T ? S::B_INV : (HALF ? S::B_HALF : S::B_FULL);
+    const FxW* tw = reinterpret_cast<const FxW*>(tw2);
+    Fx2* tb = reinterpret_cast<Fx2*>(b);
+    auto slot = [&](int line) { return reinterpret_cast<int*>(tb + line * ls + SLOT); };
+    auto split = [&](int idx, int per, int& line, int& m) {
+        if (lg >= 0) {
+            m = idx >> lg;
+            line = idx & (nl - 1);
+        } else {
+            line = idx / per;
+            m = idx - line * per;
+        }
+    };
+    for (int l = threadIdx.x; l < nl; l += blockDim.x) slot(l)[0] = slot(l)[1] = 0;
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < nl * A; idx += blockDim.x) {
+        int line, m, e = 0;
+        split(idx, A, line, m);
+#pragma unroll
+        for (int n = 0; n < NIN; ++n) {
+            const Cx<double> c = a[line * ls + m + n * A];
+            e = max(e, max(fx_exp(c.x), fx_exp(c.y)));
+        }
+        atomicMax(slot(line), e);
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < nl * A; idx += blockDim.x) {
+        int line, m;
+        split(idx, A, line, m);
+        const int E = slot(line)[0];
+        Fx2 v[T ? Q : P];
+#pragma unroll
+        for (int n = 0; n < NIN; ++n) {
+            const Cx<double> c = a[line * ls + m + n * A];
+            v[n] = cx<Fx>(fx_from<BIT>(c.x, E), fx_from<BIT>(c.y, E));
+        }
+        unsigned mag;
+        if constexpr (T) mag = S::t_first(v, m, tw, tb + line * ls);
+        else mag = S::template first<INV, HALF ? HALF_IN : DFT_FULL>(v, m, tw, tb + line * ls);
+        atomicMax(slot(line) + 1, (int)mag);
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < nl * B; idx += blockDim.x) {
+        int line, m;
+        split(idx, B, line, m);
+        const int* sl = slot(line);
+        const int sh = fx_room<T ? P : Q>((unsigned)sl[1]);
+        const FxOut o(sl[0], BIT - sh);
+        Fx2 u[T ? P : Q];
+        if constexpr (T) S::t_second(u, m, tb + line * ls, sh);
+        else S::template second<INV>(u, m, tb + line * ls, sh);
+        Cx<double>* dst = a + line * ls + m;
+#pragma unroll
+        for (int k = 0; k < (T ? P / 2 : Q); ++k) dst[k * B] = cx<double>(fx_to(u[k].x, o), fx_to(u[k].y, o));
+    }
+    __syncthreads();
+    return a;
+}
 template <typename R, bool INV, int L, bool HALF>
 __device__ __forceinline__ Cx<R>* fft_two_step_any(Cx<R>* a, Cx<R>* b, int ls, int nl, const Cx<R>* tw2) {
-    if (nl >= (sizeof(R) == 8 ? 8 : 16) && (nl & (nl - 1)) == 0)
-        return fft_two_step<R, INV, L, true, HALF>(a, b, ls, nl, 31 - __clz(nl), tw2);
-    return fft_two_step<R, INV, L, false, HALF>(a, b, ls, nl, 0, tw2);
+    if constexpr (sizeof(R) == 8) {
+        return fft_fx<INV, L, HALF>(a, b, ls, nl, nl >= 8 && (nl & (nl - 1)) == 0 ? 31 - __clz(nl) : -1, tw2);
+    } else {
+        if (nl >= 16 && (nl & (nl - 1)) == 0)
+            return fft_two_step<R, INV, L, true, HALF>(a, b, ls, nl, 31 - __clz(nl), tw2);
+        return fft_two_step<R, INV, L, false, HALF>(a, b, ls, nl, 0, tw2);
+    }
 }
 
 // ls must be at least fft_ls(L)
@@ -467,14 +610,20 @@ __host__ __device__ constexpr bool uses_two_step(int L) { return two_step_q(L) !
 // every thread of the block; ends with a barrier.  HALF (the convolution's
 // passes): the caller's input is zero from L / 2 on (forward) or it reads only
 // the first L / 2 results (inverse; the rest may not be written).
-template <typename R, bool INV, bool HALF = false>
+// TWO: false where the caller has other code for the two-step lengths.
+template <typename R, bool INV, bool HALF = false, bool TWO = true>
 __device__ Cx<R>* fft_lines(Cx<R>* a, Cx<R>* b, int ls, int nl, const RadixPlan& rp, const Cx<R>* tw) {
+    if constexpr (TWO) {
+        switch (rp.L) {
+            case 64: return fft_two_step_any<R, INV, 64, HALF>(a, b, ls, nl, tw);
+            case 96: return fft_two_step_any<R, INV, 96, HALF>(a, b, ls, nl, tw);
+            case 128: return fft_two_step_any<R, INV, 128, HALF>(a, b, ls, nl, tw);
+            case 192: return fft_two_step_any<R, INV, 192, HALF>(a, b, ls, nl, tw);
+            case 256: return fft_two_step_any<R, INV, 256, HALF>(a, b, ls, nl, tw);
+            default: break;
+        }
+    }
     switch (rp.L) {  // the padded lengths of meshes up to 256 per axis
-        case 64: return fft_two_step_any<R, INV, 64, HALF>(a, b, ls, nl, tw);
-        case 96: return fft_two_step_any<R, INV, 96, HALF>(a, b, ls, nl, tw);
-        case 128: return fft_two_step_any<R, INV, 128, HALF>(a, b, ls, nl, tw);
-        case 192: return fft_two_step_any<R, INV, 192, HALF>(a, b, ls, nl, tw);
-        case 256: return fft_two_step_any<R, INV, 256, HALF>(a, b, ls, nl, tw);
         case 8: return fft_stages_c<R, INV, 8, 0, 1>(a, b, ls, nl, tw);
         case 12: return fft_stages_c<R, INV, 12, 0, 1>(a, b, ls, nl, tw);
         case 16: return fft_stages_c<R, INV, 16, 0, 1>(a, b, ls, nl, tw);

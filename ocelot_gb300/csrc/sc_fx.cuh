@@ -1,0 +1,160 @@
+// Block fixed point for the FP64 form's transforms: the values of one line as
+// 64-bit integers under one exponent.
+//
+// Why: this GPU issues an FP64 instruction of a warp in 18 to 20 cycles of an SM
+// (two lanes a cycle), while a 64-bit integer addition is two instructions at 64
+// lanes a cycle or more, and a product's upper half three wide multiplications and a
+// few additions.  A 128-point line costs 50e3 SM cycles per 32 lines on the
+// FP64 pipe (2200 instructions) and about 6e3 in integers, with the conversions
+// to and from double another 5e3.
+//
+// Precision: a line is scaled so that its largest component takes bits 52 to 55
+// (the rest up to bit 62 is room for the transform's growth), so every input is rounded
+// at 2^-53 .. 2^-55 of the line's largest value, and every product at 2^-62 of the line's bound;
+// additions are exact.  Against a double transform, whose every operation
+// rounds at 2^-53 of its own result, the error in the 2-norm is the smaller one
+// (measured beside fft_fx).  As with any FFT the error is
+// one of the line's norm, not of each value.
+//
+// A line with a NaN or an infinity comes out as NaNs (a double transform spreads
+// them over the line too); one of denormals only comes out as zeros.
+#pragma once
+#include "sc_common.cuh"
+
+namespace ocsc {
+
+struct Fx {
+    long long v;
+};
+__host__ __device__ __forceinline__ Fx operator+(Fx a, Fx b) { return Fx{a.v + b.v}; }
+__host__ __device__ __forceinline__ Fx operator-(Fx a, Fx b) { return Fx{a.v - b.v}; }
+__host__ __device__ __forceinline__ Fx operator-(Fx a) { return Fx{-a.v}; }
+__host__ __device__ __forceinline__ Fx& operator+=(Fx& a, Fx b) { a.v += b.v; return a; }
+__host__ __device__ __forceinline__ Fx& operator-=(Fx& a, Fx b) { a.v -= b.v; return a; }
+struct __align__(16) Fx2 {
+    Fx x, y;
+};
+template <> struct CT<Fx> { using T = Fx2; };
+
+// a factor |w| <= 1 as H / 2^31 + L / 2^62, 0 <= L < 2^31 (1 itself as 1 - 2^-62)
+struct FxC {
+    int H, L;
+    __host__ __device__ constexpr FxC(int h, int l) : H(h), L(l) {}
+    __host__ __device__ constexpr explicit FxC(double w) : H(0), L(0) {
+        const double q = w * 4611686018427387904.0;
+        const long long i = q >= 4611686018427387904.0 ? 4611686018427387903ll : (long long)q;
+        H = (int)(i >> 31);
+        L = (int)(i & 0x7fffffff);
+    }
+    __host__ __device__ constexpr FxC operator-() const { return FxC(-H, -L); }
+};
+// the table entry of a twiddle wr + i wi
+struct __align__(16) FxW {
+    FxC r, i;
+};
+
+__host__ __device__ __forceinline__ int fx_hi(Fx a) { return (int)(a.v >> 32); }
+__host__ __device__ __forceinline__ int fx_lo(Fx a) { return (int)((unsigned)a.v >> 1); }
+
+// a w, |a| < 2^62: the 64-bit operand as its high word and 31 bits of its low one
+__host__ __device__ __forceinline__ Fx fx_mul(Fx a, FxC w) {
+    const int ah = fx_hi(a), al = fx_lo(a);
+    long long m = (1ll << 29) + (long long)ah * w.L;
+    m += (long long)al * w.H;
+    const long long h = (long long)ah * w.H;
+    return Fx{h + h + (m >> 30)};
+}
+// a u + b w for |a|, |b| < 2^61 and u^2 + w^2 <= 1: the middle sum stays below 1.92 * 2^62
+__host__ __device__ __forceinline__ Fx fx_mul2(Fx a, FxC u, Fx b, FxC w) {
+    const int ah = fx_hi(a), al = fx_lo(a), bh = fx_hi(b), bl = fx_lo(b);
+    long long m = (1ll << 29) + (long long)ah * u.L;
+    m += (long long)al * u.H;
+    m += (long long)bh * w.L;
+    m += (long long)bl * w.H;
+    long long h = (long long)ah * u.H;
+    h += (long long)bh * w.H;
+    return Fx{h + h + (m >> 30)};
+}
+
+// the bit of the largest input's leading one, so that a DFT over n inputs
+// stays below 2^61.5: each output is at most n sqrt(2) 2^(bit + 1)
+__host__ __device__ constexpr int fx_bit(int n) {
+    int lg = 0;
+    while ((1 << lg) < n) ++lg;
+    return 60 - lg;
+}
+// magnitude of a value for a maximum: its high word's (+ 1 for negative ones)
+__host__ __device__ __forceinline__ unsigned fx_mag(Fx a) {
+    const int h = fx_hi(a);
+    return (unsigned)(h < 0 ? ~h : h);
+}
+// bits to shift out before an n-point DFT of values of magnitudes up to mag
+template <int N>
+__device__ __forceinline__ int fx_room(unsigned mag) {
+    const int bits = 64 - __clz((int)mag);  // |value| < 2^bits
+    const int s = bits - (fx_bit(N) + 1);
+    return s > 0 ? s : 0;
+}
+// a / 2^s rounded, 0 <= s < 32
+__host__ __device__ __forceinline__ Fx fx_down(Fx a, int s) {
+    return Fx{(a.v + ((1ll << s) >> 1)) >> s};
+}
+__host__ __device__ __forceinline__ Fx2 fx_down(Fx2 a, int s) { return Fx2{fx_down(a.x, s), fx_down(a.y, s)}; }
+
+constexpr int FX_BAD = 0x7ff;  // the line exponent of a NaN or an infinity
+
+// biased exponent bits of a double (0 for zeros and denormals)
+__device__ __forceinline__ int fx_exp(double d) { return (__double2hiint(d) >> 20) & 0x7ff; }
+
+// logical right shift; 0 for 64 and more
+__device__ __forceinline__ unsigned long long fx_shr(unsigned long long m, int s) {
+#ifdef __CUDA_ARCH__
+    unsigned long long r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(m), "r"(s));
+    return r;
+#else
+    return s > 63 ? 0 : m >> s;
+#endif
+}
+
+// d as an integer of a line of exponent E >= fx_exp(d): a value with exponent E has
+// bit B as its leading one
+template <int B>
+__device__ __forceinline__ Fx fx_from(double d, int E) {
+    const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+    const int e = (hi >> 20) & 0x7ff;
+    const unsigned long long m = ((unsigned long long)(hi << 11 | lo >> 21 | 0x80000000u) << 32) | (lo << 11);
+    const int s = E - e + (62 - B) + (e == 0 ? 64 : 0);
+    const long long r = (long long)((fx_shr(m, s) + 1) >> 1);
+    const long long sg = (int)hi >> 31;
+    return Fx{(r ^ sg) - sg};
+}
+
+// what fx_to needs of a line of exponent E with bit B for 2^E
+struct FxOut {
+    int ebase, ezero, ovf;
+    __device__ __forceinline__ FxOut(int E, int B) {
+        const bool bad = E == FX_BAD;
+        ebase = bad ? 1 << 20 : E - B + 63;
+        ezero = bad ? 1 << 20 : 0;
+        ovf = bad ? 0x7ff80000 : 0x7ff00000;
+    }
+};
+// the nearest double
+__device__ __forceinline__ double fx_to(Fx a, FxOut o) {
+    const long long sg = a.v >> 63;
+    const unsigned long long u = (unsigned long long)((a.v ^ sg) - sg);
+    const int n = __clzll((long long)u);
+    const unsigned long long w = u << (n & 63);
+    const unsigned long long m = ((w >> 10) + 1) >> 1;
+    const int e = u ? o.ebase - n : o.ezero;
+    unsigned hi = (unsigned)(m >> 32) + ((unsigned)(e - 1) << 20), lo = (unsigned)m;
+    if (e < 1) hi = lo = 0;
+    if (e > 2046) {
+        hi = (unsigned)o.ovf;
+        lo = 0;
+    }
+    return __hiloint2double((int)(hi | ((unsigned)sg & 0x80000000u)), (int)lo);
+}
+
+}  // namespace ocsc

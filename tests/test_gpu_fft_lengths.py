@@ -32,3 +32,23 @@ def test_potential_at_two_step_lengths(mesh, padded, precision, tol):
     ref = sc_oracle.potential(q, steps)
     phi = sc.potential(q, steps)
     assert np.linalg.norm(phi - ref) / np.linalg.norm(ref) < tol
+
+
+@pytest.mark.parametrize("mesh,padded", MESHES)
+def test_fp64_potential_scales_by_powers_of_two(mesh, padded):
+    """A line's exponent is the only place where its magnitude enters the FP64
+    transforms, so scaling the charge by a power of two scales every bit of the
+    potential; charges over many decades, an empty grid and one bad value."""
+    sc = SpaceCharge(nmesh_xyz=mesh, precision="fp64")
+    g = np.random.default_rng(sum(mesh) + 1)
+    q = g.random(mesh) * 10.0 ** (-20 * g.random(mesh)) * 1e-12
+    q[g.random(mesh) < 0.5] = 0
+    steps = (1e-5, 2e-5, 4e-5)
+    p = np.asarray(sc.potential(q, steps))
+    assert np.isfinite(p).all() and p.any()
+    for k in (-500, 600):
+        assert np.array_equal(np.asarray(sc.potential(np.ldexp(q, k), steps)), np.ldexp(p, k))
+    assert not np.asarray(sc.potential(np.zeros(mesh), steps)).any()
+    for bad in (np.nan, np.inf):
+        q[1, 2, 3] = bad
+        assert not np.isfinite(np.asarray(sc.potential(q, steps))).any()
