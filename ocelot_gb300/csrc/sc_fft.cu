@@ -908,18 +908,6 @@ __host__ __device__ __forceinline__ Spec<R> spec_of(const Plan& p, const Layout&
     return sp;
 }
 
-// f(IntC<L>) on the host for a streamed length (with_stream's list)
-template <typename F>
-static cudaError_t stream_host(int L, F&& f) {
-    switch (L) {
-        case 64: return f(IntC<64>{});
-        case 96: return f(IntC<96>{});
-        case 128: return f(IntC<128>{});
-        case 192: return f(IntC<192>{});
-        case 256: return f(IntC<256>{});
-        default: return cudaErrorInvalidValue;
-    }
-}
 // Launches of the separate passes: the kernel of the line length (FP32
 // streamed, FP64 fixed point) for the two-step lengths, the staged one for others.
 template <typename R>
@@ -927,7 +915,7 @@ static cudaError_t launch_zfwd(const Plan& p, dim3 g, size_t sm, cudaStream_t s,
                                int Kz, const Cx<R>* tw, int NC, const ScState* st) {
     cudaError_t e;
     if (uses_two_step(p.Mz))
-        return stream_host(p.Mz, [&](auto L) -> cudaError_t {
+        return two_step_host(p.Mz, [&](auto L) -> cudaError_t {
             constexpr int LL = decltype(L)::value;
             if constexpr (sizeof(R) == 4) {
                 if ((e = set_smem(k_zfwd_s<LL>, sm))) return e;
@@ -945,7 +933,7 @@ static cudaError_t launch_ypass(const Plan& p, dim3 g, size_t sm, cudaStream_t s
                                 int TK, const ScState* st, const Spec<R>& sp) {
     cudaError_t e;
     if (uses_two_step(p.My))
-        return stream_host(p.My, [&](auto L) -> cudaError_t {
+        return two_step_host(p.My, [&](auto L) -> cudaError_t {
             constexpr int LL = decltype(L)::value;
             if constexpr (sizeof(R) == 4) {
                 if ((e = set_smem(k_ypass_s<INV, LL>, sm))) return e;
@@ -964,7 +952,7 @@ static cudaError_t launch_xconv(const Plan& p, dim3 g, size_t sm, cudaStream_t s
                                 const Cx<R>* tw, int TK, const ScState* st, const Spec<R>& sp) {
     cudaError_t e;
     if (uses_two_step(p.Mx))
-        return stream_host(p.Mx, [&](auto L) -> cudaError_t {
+        return two_step_host(p.Mx, [&](auto L) -> cudaError_t {
             constexpr int LL = decltype(L)::value;
             if constexpr (sizeof(R) == 4) {
                 if ((e = set_smem(k_xconv_s<LL>, sm))) return e;
@@ -1025,7 +1013,7 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
     if ((e = launch_ypass<R, true>(p, gyi, smyi, s, W, Kz, twy, tkyi, st, sp))) return e;
     if (sizeof(R) == 8 && uses_two_step(p.Mz)) {
         if constexpr (sizeof(R) == 8)
-            return stream_host(p.Mz, [&](auto LZ) -> cudaError_t {
+            return two_step_host(p.Mz, [&](auto LZ) -> cudaError_t {
                 constexpr int LL = decltype(LZ)::value;
                 if ((e = set_smem(k_zinv_fx<LL>, smzi))) return e;
                 return launch(k_zinv_fx<LL>, gz, NC * two_step_q(LL), smzi, s, W, phi, p.ny, p.nz, p.My, Kz, twz, NC, st);
@@ -1046,7 +1034,7 @@ static cudaError_t prepare_fft_t(const Plan& p) {
     const int tky = strided_cols<R>(p.My), tkx = strided_cols<R>(p.Mx, nbuf), tkyi = strided_cols<R>(p.My, nbuf);
     const size_t smy = smem_yf<R>(p.My, tky), smyi = smem_yi<R>(p.My, tkyi, spec), smx = smem_x<R>(p.Mx, tkx, spec);
     auto prep = [&](int M, auto&& two_step, auto* staged, size_t sm) -> cudaError_t {
-        return uses_two_step(M) ? stream_host(M, two_step) : set_smem(staged, sm);
+        return uses_two_step(M) ? two_step_host(M, two_step) : set_smem(staged, sm);
     };
     if ((e = prep(p.Mz, [&](auto L) {
              constexpr int LL = decltype(L)::value;
@@ -1069,9 +1057,8 @@ static cudaError_t prepare_fft_t(const Plan& p) {
              else return set_smem(k_xconv_fx<LL>, smx);
          }, k_xconv<R>, smx))) return e;
     if ((e = prep(p.Mz, [&](auto L) {
-             constexpr int LL = decltype(L)::value;
              if constexpr (sizeof(R) == 4) return set_smem(k_zinv<R>, smzi);
-             else return set_smem(k_zinv_fx<LL>, smzi);
+             else return set_smem(k_zinv_fx<decltype(L)::value>, smzi);
          }, k_zinv<R>, smzi))) return e;
     if (plane_fits<R>(p, optin_smem())) {
         if ((e = set_smem(k_zy_fwd<R>, plane_smem<R>(p)))) return e;

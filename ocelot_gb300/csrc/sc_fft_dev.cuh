@@ -605,6 +605,27 @@ __device__ __forceinline__ Cx<R>* fft_stages_c(Cx<R>* a, Cx<R>* b, int ls, int n
 // w_L^m in the workspace, the stage table otherwise).
 __host__ __device__ constexpr bool uses_two_step(int L) { return two_step_q(L) != 0; }
 
+template <int V>
+struct IntC {
+    static constexpr int value = V;
+};
+// f(IntC<L>) on the host for a two-step length L
+template <typename F>
+static cudaError_t two_step_host(int L, F&& f) {
+    switch (L) {
+        case 64: return f(IntC<64>{});
+        case 96: return f(IntC<96>{});
+        case 128: return f(IntC<128>{});
+        case 192: return f(IntC<192>{});
+        case 256: return f(IntC<256>{});
+        default: return cudaErrorInvalidValue;
+    }
+}
+static_assert(uses_two_step(64) && uses_two_step(96) && uses_two_step(128) && uses_two_step(192) &&
+                  uses_two_step(256) && !uses_two_step(32) && !uses_two_step(48) && !uses_two_step(384) &&
+                  !uses_two_step(512),
+              "two_step_host lists the two-step lengths");
+
 // FFT of nl lines of length rp.L; a holds the input, b is scratch of the
 // same shape.  Returns the buffer that holds the result.  Must be called by
 // every thread of the block; ends with a barrier.  HALF (the convolution's

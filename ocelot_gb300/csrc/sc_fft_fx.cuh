@@ -213,6 +213,7 @@ __device__ __forceinline__ void zfwd_fx(const double* __restrict__ q, double2* _
     Fx2* tabs = reinterpret_cast<Fx2*>(spec + NC * fx_line(L));
     const int x = vb.y, y0 = vb.x * 2 * NC;
     const long long ncell = (long long)vb.ny * ny * nz;
+    (void)ncell;  // read by the index checks of checked builds
     const int c = threadIdx.x / Q, m = threadIdx.x - c * Q;  // blockDim = NC Q
     const int ra = y0 + 2 * c, rb = ra + 1;
     double2 d[P / 2];
@@ -314,6 +315,45 @@ __device__ __forceinline__ void zinv_fx(const double2* __restrict__ W, double* _
         double* p = phi + ((size_t)x * ny + ra) * nz + z;
         if (z < nz && ra < ny) p[0] = out(fx_to(u[k1].x, o));
         if (z < nz && rb < ny) p[nz] = out(fx_to(u[k1].y, o));
+    }
+}
+
+// Forward transform of one even line pair per line (the Green passes): item m of
+// line c reads ld(n), n = Q n1 + m, and the outputs k <= L / 2 go to st(k, value)
+template <int L, typename Load, typename Store>
+__device__ __forceinline__ void even_fx(int c, int m, const double2* __restrict__ twg, Load&& ld, Store&& put) {
+    using S = FxSteps<L>;
+    constexpr int Q = S::Q, P = S::P;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    __shared__ FxLines ln;
+    FxW* tw = reinterpret_cast<FxW*>(smraw);
+    Fx2* tab = reinterpret_cast<Fx2*>(tw + L) + c * fx_tab(L);
+    double2 d[P];
+#pragma unroll
+    for (int n1 = 0; n1 < P; ++n1) d[n1] = ld(n1 * Q + m);
+    fx_clear(ln);
+    load_twiddles<double>(reinterpret_cast<double2*>(tw), twg, L);
+    __syncthreads();
+    atomicMax(&ln.e[c], fx_exp_of(d));
+    __syncthreads();
+    const int E = ln.e[c];
+    {
+        Fx2 v[P];
+#pragma unroll
+        for (int n1 = 0; n1 < P; ++n1) v[n1] = cx<Fx>(fx_from<S::B_FULL>(d[n1].x, E), fx_from<S::B_FULL>(d[n1].y, E));
+        atomicMax(&ln.m[0][c], (int)S::template first<false, DFT_FULL>(v, m, tw, tab));
+    }
+    __syncthreads();
+    if (m < P) {
+        const int sh = fx_room<Q>((unsigned)ln.m[0][c]);
+        const FxOut o(E, S::B_FULL - sh);
+        Fx2 u[Q];
+        S::template second<false>(u, m, tab, sh);
+#pragma unroll
+        for (int k2 = 0; k2 <= Q / 2; ++k2) {
+            const int k = m + P * k2;
+            if (k <= L / 2) put(k, make_double2(fx_to(u[k2].x, o), fx_to(u[k2].y, o)));
+        }
     }
 }
 

@@ -25,10 +25,6 @@ namespace ocsc {
 template <typename R>
 __host__ __device__ constexpr bool streamed(int L) { return sizeof(R) == 4 && uses_two_step(L); }
 
-template <int V>
-struct IntC {
-    static constexpr int value = V;
-};
 // f(IntC<L>) for a streamed length L; false (and nothing done) for any other
 template <typename R, typename F>
 __device__ __forceinline__ bool with_stream(int L, F&& f) {

@@ -23,7 +23,7 @@
 #include <mutex>
 
 #include "sc_common.cuh"
-#include "sc_fft_dev.cuh"
+#include "sc_fft_fx.cuh"
 #include "sc_igf_fn.cuh"
 
 namespace ocsc {
@@ -405,7 +405,7 @@ __device__ __forceinline__ void green_z_body(const R* __restrict__ k1, R* __rest
             if (cs[u] < NC) A[cs[u] * lz + zz[u]] = cx<R>(re[u], im[u]);
     }
     __syncthreads();
-    Cx<R>* res = fft_lines<R, false>(A, B, lz, NC, rz, tw);
+    Cx<R>* res = fft_lines<R, false, false, sizeof(R) == 4>(A, B, lz, NC, rz, tw);
     for (DivWalk w(threadIdx.x, blockDim.x, Kz); w.q < NC; w.next()) {
         const int c = w.q, k = w.r;
         const int ya = y0 + 2 * c, yb = ya + 1;
@@ -466,7 +466,7 @@ __device__ __forceinline__ void green_strided_body(const R* __restrict__ in, R* 
             if (l0 + u * cm.rs < M) la[l0 + u * cm.rs] = cx<R>(re[u], im[u]);
     }
     __syncthreads();
-    Cx<R>* res = fft_lines<R, false>(A, B, ls, GTK, rp, tw);
+    Cx<R>* res = fft_lines<R, false, false, sizeof(R) == 4>(A, B, ls, GTK, rp, tw);
     if (live)
         for (int l = cm.r0; l < nout; l += cm.rs) {
             const Cx<R> v = res[cm.kk * ls + l];
@@ -484,6 +484,66 @@ __global__ void __launch_bounds__(GT) k_green_strided(const R* __restrict__ in, 
     pdl_wait();
     green_strided_body<R>(in, out, n, nin_stride, nout, Kz, outer_in_stride, outer_out_stride, nouter, rp, twg, GTK,
                           a, st, hw_vblk());
+}
+
+// The same passes of the FP64 form for the two-step lengths, streamed in block
+// fixed point (sc_fft_fx.cuh): FX_COLS complex lines per block, half the outputs
+// converted and stored.  63^3, staged fixed point -> streamed: z 13.4 -> 6.4 us, y
+// 13.3 -> 6.6, x 8.9 -> 6.5 (double two-step passes 17, 33 and 23); what bounds
+// them is the integer pipes and one wave of blocks with three barriers
+template <int L>
+__global__ void __launch_bounds__(fx_threads(L), 512 / fx_threads(L))
+    k_green_z_fx(const double* __restrict__ k1, double* __restrict__ s1, int ny, int nz, int Kz,
+                 const double2* __restrict__ twg, IgfArgs a, const ScState* st) {
+    pdl_wait();
+    if (igf_skip(st, a)) return;
+    constexpr int Q = two_step_q(L);
+    const int c = threadIdx.x / Q, m = threadIdx.x - c * Q;
+    const int x = blockIdx.y, ya = blockIdx.x * 2 * FX_COLS + 2 * c, yb = ya + 1;
+    const double* ra = k1 + ((size_t)x * ny + ya) * nz;
+    double* oa = s1 + ((size_t)x * ny + ya) * Kz;
+    even_fx<L>(
+        c, m, twg,
+        [&](int n) {
+            const int zs = even_src(n, nz, L);
+            const bool ok = zs >= 0 && SC_IDX_OK(st, 33, ((long long)x * ny + (ya < ny ? ya : 0)) * nz + zs,
+                                                 (long long)gridDim.y * ny * nz);
+            return make_double2(ok && ya < ny ? ra[zs] : 0.0, ok && yb < ny ? ra[nz + zs] : 0.0);
+        },
+        [&](int k, double2 v) {
+            if (!SC_IDX_OK(st, 35, ((long long)x * ny + (yb < ny ? yb : ya)) * Kz + k, (long long)gridDim.y * ny * Kz))
+                return;
+            if (ya < ny) oa[k] = v.x;
+            if (yb < ny) oa[Kz + k] = v.y;
+        });
+}
+template <int L>
+__global__ void __launch_bounds__(fx_threads(L), 512 / fx_threads(L))
+    k_green_strided_fx(const double* __restrict__ in, double* __restrict__ out, int n, int nin_stride, int Kz,
+                       int outer_in_stride, int outer_out_stride, int nouter, const double2* __restrict__ twg,
+                       IgfArgs a, const ScState* st) {
+    pdl_wait();
+    if (igf_skip(st, a)) return;
+    const int c = threadIdx.x & (FX_COLS - 1), m = threadIdx.x / FX_COLS;
+    const int P = (Kz + 1) / 2;
+    const int f = blockIdx.x * FX_COLS + c;
+    const bool live = f < nouter * P;
+    const int o = f / P, ka = 2 * (f - o * P), kb = ka + 1;
+    const double* src = in + (size_t)o * outer_in_stride + ka;
+    double* dst = out + (size_t)o * outer_out_stride + ka;
+    even_fx<L>(
+        c, m, twg,
+        [&](int l) {
+            const int ls = live ? even_src(l, n, L) : -1;
+            const double* p = src + (size_t)(ls < 0 ? 0 : ls) * nin_stride;
+            return make_double2(ls >= 0 ? p[0] : 0.0, ls >= 0 && kb < Kz ? p[1] : 0.0);
+        },
+        [&](int k, double2 v) {
+            if (!live) return;
+            double* p = dst + (size_t)k * nin_stride;
+            p[0] = v.x;
+            if (kb < Kz) p[1] = v.y;
+        });
 }
 
 
@@ -544,6 +604,49 @@ cudaError_t launch_igf(const Plan& p, const Layout& L, char* ws, cudaStream_t s)
     return cudaGetLastError();
 }
 
+// Launch of a pass (only: set its kernel's shared memory, no launch): the
+// fixed-point kernel of the length for FP64 lines of the two-step form, the staged one for others
+template <typename R>
+static cudaError_t green_z(const Plan& p, bool only, cudaStream_t s, const R* k1, R* s1, const Cx<R>* tw,
+                           const IgfArgs& a, const ScState* st) {
+    cudaError_t e;
+    const int Kz = p.Mz / 2 + 1;
+    if constexpr (sizeof(R) == 8)
+        if (uses_two_step(p.Mz))
+            return two_step_host(p.Mz, [&](auto L) -> cudaError_t {
+                constexpr int LL = decltype(L)::value;
+                if ((e = set_smem(k_green_z_fx<LL>, fx_smem_zi(LL, FX_COLS))) || only) return e;
+                return launch(k_green_z_fx<LL>, dim3((p.ny + 2 * FX_COLS - 1) / (2 * FX_COLS), p.nx), fx_threads(LL),
+                              fx_smem_zi(LL, FX_COLS), s, k1, s1, p.ny, p.nz, Kz, tw, a, st);
+            });
+    int NC = 2048 / p.Mz;
+    NC = NC < 1 ? 1 : (NC > 16 ? 16 : NC);
+    const size_t sm = sizeof(Cx<R>) * (size_t)(p.Mz + 2 * NC * fft_ls(p.Mz));
+    if ((e = set_smem(k_green_z<R>, sm)) || only) return e;
+    return launch(k_green_z<R>, dim3((p.ny + 2 * NC - 1) / (2 * NC), p.nx), GT, sm, s, k1, s1, p.ny, p.nz, Kz, p.rz, tw, NC,
+                  a, st);
+}
+// pairs: column pairs per outer index
+template <typename R>
+static cudaError_t green_strided(int M, const RadixPlan& rp, int pairs, bool only, cudaStream_t s, const R* in, R* out,
+                                 int n, int nin_stride, int nout, int Kz, int outer_in, int outer_out, int nouter,
+                                 const Cx<R>* tw, const IgfArgs& a, const ScState* st) {
+    cudaError_t e;
+    if constexpr (sizeof(R) == 8)
+        if (uses_two_step(M))
+            return two_step_host(M, [&](auto L) -> cudaError_t {
+                constexpr int LL = decltype(L)::value;
+                if ((e = set_smem(k_green_strided_fx<LL>, fx_smem_cols(LL))) || only) return e;
+                return launch(k_green_strided_fx<LL>, dim3((nouter * pairs + FX_COLS - 1) / FX_COLS), fx_threads(LL),
+                              fx_smem_cols(LL), s, in, out, n, nin_stride, Kz, outer_in, outer_out, nouter, tw, a, st);
+            });
+    const int tk = green_cols<R>(M);
+    const size_t sm = sizeof(Cx<R>) * (size_t)(M + 2 * tk * fft_ls(M));
+    if ((e = set_smem(k_green_strided<R>, sm)) || only) return e;
+    return launch(k_green_strided<R>, dim3((nouter * pairs + tk - 1) / tk), GT, sm, s, in, out, n, nin_stride, nout, Kz,
+                  outer_in, outer_out, nouter, rp, tw, tk, a, st);
+}
+
 template <typename R>
 static cudaError_t spectrum_t(const Plan& p, const Layout& L, char* ws, cudaStream_t s) {
     const ScState* st = reinterpret_cast<const ScState*>(ws + L.state);
@@ -561,40 +664,26 @@ static cudaError_t spectrum_t(const Plan& p, const Layout& L, char* ws, cudaStre
     const Cx<R>* twy = reinterpret_cast<const Cx<R>*>(ws + L.tw_y);
     const Cx<R>* twz = reinterpret_cast<const Cx<R>*>(ws + L.tw_z);
     cudaError_t e;
-    int NC = 2048 / p.Mz;
-    NC = NC < 1 ? 1 : (NC > 16 ? 16 : NC);
-    const size_t smz = sizeof(Cx<R>) * (size_t)(p.Mz + 2 * NC * fft_ls(p.Mz));
-    if ((e = set_smem(k_green_z<R>, smz))) return e;
-    dim3 gz((p.ny + 2 * NC - 1) / (2 * NC), p.nx);
-    launch(k_green_z<R>, gz, GT, smz, s, k1, s1, p.ny, p.nz, Kz, p.rz, twz, NC, a, st);
-    // S2 along y: for each x, rows y < ny of S1[x] -> rows ky < Ky of S2[x]
-    const int tky = green_cols<R>(p.My), tkx = green_cols<R>(p.Mx);
-    const size_t smy = sizeof(Cx<R>) * (size_t)(p.My + 2 * tky * fft_ls(p.My));
-    const size_t smx = sizeof(Cx<R>) * (size_t)(p.Mx + 2 * tkx * fft_ls(p.Mx));
-    if ((e = set_smem(k_green_strided<R>, smx > smy ? smx : smy))) return e;
     const int P = (Kz + 1) / 2;  // column pairs per outer index
-    dim3 gy((p.nx * P + tky - 1) / tky);
-    launch(k_green_strided<R>, gy, GT, smy, s, s1, s2, p.ny, Kz, Ky, Kz, p.ny * Kz, Ky * Kz, p.nx, p.ry, twy, tky, a,
-           st);
+    if ((e = green_z<R>(p, false, s, k1, s1, twz, a, st))) return e;
+    // S2 along y: for each x, rows y < ny of S1[x] -> rows ky < Ky of S2[x]
+    if ((e = green_strided<R>(p.My, p.ry, P, false, s, s1, s2, p.ny, Kz, Ky, Kz, p.ny * Kz, Ky * Kz, p.nx, twy, a, st)))
+        return e;
     // S3 along x: for each ky, rows x < nx of S2[.][ky] -> rows kx < Kx of G[.][ky]
-    dim3 gx((Ky * P + tkx - 1) / tkx);
-    launch(k_green_strided<R>, gx, GT, smx, s, s2, g, p.nx, Ky * Kz, Kx, Kz, Kz, Kz, Ky, p.rx, twx, tkx, a, st);
+    if ((e = green_strided<R>(p.Mx, p.rx, P, false, s, s2, g, p.nx, Ky * Kz, Kx, Kz, Kz, Kz, Ky, twx, a, st))) return e;
     return cudaGetLastError();
 }
 
 template <typename R>
 static cudaError_t prepare_green_t(const Plan& p) {
     cudaError_t e;
-    int NC = 2048 / p.Mz;
-    NC = NC < 1 ? 1 : (NC > 16 ? 16 : NC);
-    const size_t smz = sizeof(Cx<R>) * (size_t)(p.Mz + 2 * NC * fft_ls(p.Mz));
-    const int tky = green_cols<R>(p.My), tkx = green_cols<R>(p.Mx);
-    const size_t smy = sizeof(Cx<R>) * (size_t)(p.My + 2 * tky * fft_ls(p.My));
-    const size_t smx = sizeof(Cx<R>) * (size_t)(p.Mx + 2 * tkx * fft_ls(p.Mx));
     if ((e = prefer_shared(k_igf_corners<R>))) return e;
     if ((e = prefer_shared(k_igf_diff<R>))) return e;
-    if ((e = set_smem(k_green_z<R>, smz))) return e;
-    return set_smem(k_green_strided<R>, smx > smy ? smx : smy);
+    const IgfArgs a = {};
+    if ((e = green_z<R>(p, true, nullptr, nullptr, nullptr, nullptr, a, nullptr))) return e;
+    if ((e = green_strided<R>(p.My, p.ry, 1, true, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, 0, 1, nullptr, a, nullptr)))
+        return e;
+    return green_strided<R>(p.Mx, p.rx, 1, true, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, 0, 1, nullptr, a, nullptr);
 }
 
 cudaError_t prepare_green_kernels(const Plan& p) {
