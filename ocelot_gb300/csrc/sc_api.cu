@@ -666,7 +666,7 @@ int sc_kick(sc_plan* plan, void* ws_v, size_t ws_bytes, double* rp, int64_t ld, 
     SC_CUDA(launch_convolve(p, L, ws, ws + L.qgrid, ws + L.phi, s, qfix, CONV_REST, true, p.record_field != 0),
             "convolve");
     mark(plan, 7, s);
-    SC_CUDA(launch_field_grids(p, L, ws, s), "field grids");
+    SC_CUDA(launch_field_grids(p, L, ws, s, true), "field grids");
     mark(plan, 8, s);
     SC_CUDA(launch_gather_kick(p, L, ws, kp, rp, s), "gather/kick");
     mark(plan, 9, s);
@@ -704,7 +704,7 @@ int sc_el_field(sc_plan* plan, void* ws_v, size_t ws_bytes, double* X, const dou
     SC_CUDA(launch_convolve(p, L, ws, ws + L.qgrid, ws + L.phi, s,
                             p.sorted_deposit ? nullptr : reinterpret_cast<const long long*>(ws + L.qfix), CONV_ALL, true),
             "convolve");
-    SC_CUDA(launch_field_grids(p, L, ws, s), "field grids");
+    SC_CUDA(launch_field_grids(p, L, ws, s, false), "field grids");
     SC_CUDA(launch_gather_xyz(p, L, ws, kp, exyz, s), "gather");
     return SC_OK;
 }

@@ -79,6 +79,8 @@ struct ScState {
     unsigned int done_extent;
     unsigned int kick_next;      // tiles claimed by the gather + kick (reset by the frame finalize)
     unsigned int igf_next;       // corners of the exact IGF table claimed (reset with the mesh)
+    int phi_exp;                 // FP64: largest biased exponent of the potential (reset with the mesh)
+    double escale[3];            // FP64 kick: the field per unit of the fixed-point differences
     int frame_timeout;           // a frame block's bulk-copy wait gave up (the finalize reports it)
     int check_code;              // checked builds: first failed index check (kernel code)
     int first_error;             // first non-OK status of any kick since sc_workspace_init
@@ -262,7 +264,11 @@ enum ConvPart { CONV_ALL = 0, CONV_FORWARD = 1, CONV_REST = 2 };
 cudaError_t launch_convolve(const Plan& p, const Layout& L, char* ws, const void* qgrid_in,
                             void* phi_out, cudaStream_t s, const long long* qfix = nullptr, int part = CONV_ALL,
                             bool fields = false, bool want_phi = true);
-cudaError_t launch_field_grids(const Plan& p, const Layout& L, char* ws, cudaStream_t s);
+// the FP64 kick's fixed-point field grids: in the work grid, which is free once
+// the potential is made (nx My Kz complex entries hold three integers per cell)
+inline long long* field_fx(const Layout& L, char* ws) { return reinterpret_cast<long long*>(ws + L.W); }
+// kick: for the kick (the FP64 form then writes the fixed-point differences too)
+cudaError_t launch_field_grids(const Plan& p, const Layout& L, char* ws, cudaStream_t s, bool kick);
 // kernels launch_convolve(CONV_ALL) launches for this plan
 int convolve_launches(const Plan& p);
 

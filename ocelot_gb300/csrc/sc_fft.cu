@@ -38,6 +38,12 @@ static inline int z_lines_per_block(int Mz) {
     int nc = 1024 / Mz;
     return nc < 1 ? 1 : (nc > 8 ? 8 : nc);
 }
+// the fixed-point z passes: a whole number of warps of two_step_q(Mz) threads a line
+template <typename R>
+static inline int z_lines(int Mz) {
+    const int nc = z_lines_per_block(Mz);
+    return sizeof(R) == 8 && uses_two_step(Mz) ? nc & ~3 : nc;
+}
 // columns per block in the strided passes: 16, fewer when two line buffers
 // of 16 columns would not fit in shared memory (FP64 at M = 512)
 template <typename R>
@@ -511,12 +517,14 @@ __device__ __forceinline__ void zinv_body(const Cx<R>* __restrict__ W, R* __rest
     OutScale64 out64 = {};
     if constexpr (sizeof(R) == 8) out64 = out_scale64(st);
     const R fscale = (R)st->phi_scalef * mul;  // (float)(norm / denom), computed once by the mesh finalize
+    int pe = 0;  // FP64: the largest exponent stored
     auto put = [&](int c, int z, Cx<R> v) {
         if (z >= nz) return;
         const int ya = y0 + 2 * c, yb = ya + 1;
         if constexpr (sizeof(R) == 8) {
-            if (ya < ny) phi[((size_t)x * ny + ya) * nz + z] = out64(v.x);
-            if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = out64(v.y);
+            double* p = phi + ((size_t)x * ny + ya) * nz + z;
+            if (ya < ny) pe = max(pe, fx_exp(p[0] = out64(v.x)));
+            if (yb < ny) pe = max(pe, fx_exp(p[nz] = out64(v.y)));
         } else {
             const bool zx = zero_axis == 0 && x == nx - 1, zz = zero_axis == 2 && z == nz - 1;
             const bool za = zx || zz || (zero_axis == 1 && ya == ny - 1);
@@ -561,6 +569,7 @@ __device__ __forceinline__ void zinv_body(const Cx<R>* __restrict__ W, R* __rest
     __syncthreads();
     Cx<R>* res = fft_lines<R, true, true, sizeof(R) == 4>(a, b, lz, NC, rz, tw);
     for (DivWalk w(threadIdx.x, blockDim.x, nz); w.q < NC; w.next()) put(w.q, w.r, res[w.q * lz + w.r]);
+    if constexpr (sizeof(R) == 8) phi_raise(st, pe);
 }
 
 // blockIdx.z: the output (0 the potential; with spectral fields 1 Ex, 2 Ey, 3 Ez)
@@ -586,30 +595,48 @@ __global__ void __launch_bounds__(fx_threads(L), FX_MINB(L)) k_zinv_fx(const dou
                                                                     const ScState* st) {
     pdl_wait();
     if (st->status) return;
-    zinv_fx<L>(W, phi, ny, nz, My, Kz, twg, NC, out_scale64(st), hw_vblk());
+    zinv_fx<L>(W, phi, ny, nz, My, Kz, twg, NC, out_scale64(st), st, hw_vblk());
 }
 
 // FP64 form: Ex,Ey,Ez = forward differences / h, zero on the last plane
 // (sc.py:195-200); the quotient from the reciprocal 1/h with one correction
 // (the IEEE division's result up to its last bit).  One block per (x, y) line
 // of cells, one thread per z: no index division.
+//
+// fe != nullptr (the kick): the differences also as integers under the
+// potential's largest exponent, [3][nx][ny][nz]; differences of integers are
+// exact, and an integer's unit is 2^-59 of the largest potential, a 64th of
+// what the double potential itself is rounded at.  escale turns them into fields.
 __global__ void k_field_grids(const double* __restrict__ phi, double* __restrict__ ex, double* __restrict__ ey,
-                              double* __restrict__ ez, int nx, int ny, int nz, const ScState* st) {
+                              double* __restrict__ ez, long long* __restrict__ fe, int nx, int ny, int nz,
+                              ScState* st) {
     pdl_wait();
     if (st->status) return;
     const int j = blockIdx.x, i = blockIdx.y;
     const double hx = st->steps[0], hy = st->steps[1], hz = st->steps[2];
     const double rx = st->isteps[0], ry = st->isteps[1], rz = st->isteps[2];
+    const int E = st->phi_exp;
+    const size_t ncell = (size_t)nx * ny * nz;
+    if (fe && i == 0 && j == 0 && threadIdx.x < 3)
+        st->escale[threadIdx.x] = E == FX_BAD ? NAN : ldexp(st->isteps[threadIdx.x], E - 1023 - FX_PHI);
     auto over = [](double a, double h, double r) {
         const double q = a * r;
         return fma(fma(-q, h, a), r, q);
     };
     for (int k = threadIdx.x; k < nz; k += blockDim.x) {
         const int c = (i * ny + j) * nz + k;
+        const bool inx = i < nx - 1, iny = j < ny - 1, inz = k < nz - 1;
         const double p = phi[c];
-        ex[c] = i < nx - 1 ? over(p - phi[c + ny * nz], hx, rx) : 0.0;
-        ey[c] = j < ny - 1 ? over(p - phi[c + nz], hy, ry) : 0.0;
-        ez[c] = k < nz - 1 ? over(p - phi[c + 1], hz, rz) : 0.0;
+        const double px = inx ? phi[c + ny * nz] : p, py = iny ? phi[c + nz] : p, pz = inz ? phi[c + 1] : p;
+        ex[c] = inx ? over(p - px, hx, rx) : 0.0;
+        ey[c] = iny ? over(p - py, hy, ry) : 0.0;
+        ez[c] = inz ? over(p - pz, hz, rz) : 0.0;
+        if (fe) {
+            const Fx f = fx_from<FX_PHI>(p, E);
+            fe[c] = (f - fx_from<FX_PHI>(px, E)).v;
+            fe[ncell + c] = (f - fx_from<FX_PHI>(py, E)).v;
+            fe[2 * ncell + c] = (f - fx_from<FX_PHI>(pz, E)).v;
+        }
     }
 }
 
@@ -834,13 +861,15 @@ __device__ __forceinline__ void yz_inv_body(const Cx<R>* __restrict__ W, R* __re
     OutScale64 out64 = {};
     if constexpr (sizeof(R) == 8) out64 = out_scale64(st);
     const R fscale = (R)st->phi_scalef * mul;  // (float)(norm / denom), computed once by the mesh finalize
+    int pe = 0;  // FP64: the largest exponent stored
     for (DivWalk w(threadIdx.x, blockDim.x, nz); w.q < ncz; w.next()) {
         const int c = w.q, z = w.r;
         const int ya = 2 * c, yb = ya + 1;
         const Cx<R> v = res[c * lz + z];
         if constexpr (sizeof(R) == 8) {
-            phi[((size_t)x * ny + ya) * nz + z] = out64(v.x);
-            if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = out64(v.y);
+            double* p = phi + ((size_t)x * ny + ya) * nz + z;
+            pe = max(pe, fx_exp(p[0] = out64(v.x)));
+            if (yb < ny) pe = max(pe, fx_exp(p[nz] = out64(v.y)));
         } else {
             const bool zx = zero_axis == 0 && x == nx - 1, zz = zero_axis == 2 && z == nz - 1;
             const bool za = zx || zz || (zero_axis == 1 && ya == ny - 1);
@@ -849,6 +878,7 @@ __device__ __forceinline__ void yz_inv_body(const Cx<R>* __restrict__ W, R* __re
             if (yb < ny) phi[((size_t)x * ny + yb) * nz + z] = zb ? (R)0 : v.y * fscale;
         }
     }
+    if constexpr (sizeof(R) == 8) phi_raise(st, pe);
 }
 
 // blockIdx.y: the output (0 the potential; with spectral fields 1 Ex, 2 Ey, 3 Ez)
@@ -979,7 +1009,7 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
     const Cx<R>* twy = reinterpret_cast<const Cx<R>*>(ws + L.tw_y);
     const Cx<R>* twz = reinterpret_cast<const Cx<R>*>(ws + L.tw_z);
     cudaError_t e;
-    const int NC = z_lines_per_block(p.Mz);
+    const int NC = z_lines<R>(p.Mz);
     const size_t smz = smem_zf<R>(p.Mz, NC), smzi = smem_zi<R>(p.Mz, NC);
     dim3 gz((p.ny + 2 * NC - 1) / (2 * NC), p.nx);
     const int tky = pass_cols<R>(p.fft_cols_y, p.My), tkx = pass_cols<R>(p.fft_cols_x, p.Mx, nbuf);
@@ -1027,7 +1057,7 @@ static cudaError_t convolve_t(const Plan& p, const Layout& L, char* ws, R* qgrid
 template <typename R>
 static cudaError_t prepare_fft_t(const Plan& p) {
     cudaError_t e;
-    const int NC = z_lines_per_block(p.Mz);
+    const int NC = z_lines<R>(p.Mz);
     const size_t smz = smem_zf<R>(p.Mz, NC), smzi = smem_zi<R>(p.Mz, NC);
     const bool spec = p.spectral && sizeof(R) == 4;
     const int nbuf = spec ? 3 : 2;
@@ -1081,7 +1111,7 @@ cudaError_t launch_convolve(const Plan& p, const Layout& L, char* ws, const void
 }
 
 template <typename R>
-static cudaError_t field_t(const Plan& p, const Layout& L, char* ws, cudaStream_t s) {
+static cudaError_t field_t(const Plan& p, const Layout& L, char* ws, cudaStream_t s, bool kick) {
     const ScState* st = reinterpret_cast<const ScState*>(ws + L.state);
     const int bt = p.nz < 256 ? ((p.nz + 31) / 32) * 32 : 256;
     const dim3 grid(p.ny, p.nx);
@@ -1097,12 +1127,13 @@ static cudaError_t field_t(const Plan& p, const Layout& L, char* ws, cudaStream_
     else
         launch(k_field_grids, grid, bt, 0, s, reinterpret_cast<const double*>(ws + L.phi),
                reinterpret_cast<double*>(ws + L.ex), reinterpret_cast<double*>(ws + L.ey),
-               reinterpret_cast<double*>(ws + L.ez), p.nx, p.ny, p.nz, st);
+               reinterpret_cast<double*>(ws + L.ez), kick ? field_fx(L, ws) : nullptr, p.nx, p.ny, p.nz,
+               reinterpret_cast<ScState*>(ws + L.state));
     return cudaGetLastError();
 }
 
-cudaError_t launch_field_grids(const Plan& p, const Layout& L, char* ws, cudaStream_t s) {
-    return p.prec == SC_FP64 ? field_t<double>(p, L, ws, s) : field_t<float>(p, L, ws, s);
+cudaError_t launch_field_grids(const Plan& p, const Layout& L, char* ws, cudaStream_t s, bool kick) {
+    return p.prec == SC_FP64 ? field_t<double>(p, L, ws, s, kick) : field_t<float>(p, L, ws, s, kick);
 }
 
 // ---------------------------------------------------------------------------

@@ -262,7 +262,8 @@ __device__ __forceinline__ void zfwd_fx(const double* __restrict__ q, double2* _
 // above L / 2 (that sum in double, as there), out(v) scales a value of the potential
 template <int L, typename Out>
 __device__ __forceinline__ void zinv_fx(const double2* __restrict__ W, double* __restrict__ phi, int ny, int nz, int My,
-                                        int Kz, const double2* __restrict__ twg, int NC, Out out, VBlk vb) {
+                                        int Kz, const double2* __restrict__ twg, int NC, Out out, const ScState* st,
+                                        VBlk vb) {
     using S = FxSteps<L>;
     constexpr int Q = S::Q, P = S::P;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -309,13 +310,19 @@ __device__ __forceinline__ void zinv_fx(const double2* __restrict__ W, double* _
     const FxOut o(E, S::B_INV - sh);
     Fx2 u[P];
     S::t_second(u, m, tab, sh);
+    int e = 0;
 #pragma unroll
     for (int k1 = 0; k1 < P / 2; ++k1) {
         const int z = k1 * Q + m;
         double* p = phi + ((size_t)x * ny + ra) * nz + z;
-        if (z < nz && ra < ny) p[0] = out(fx_to(u[k1].x, o));
-        if (z < nz && rb < ny) p[nz] = out(fx_to(u[k1].y, o));
+        auto put = [&](double* dst, double v) {
+            *dst = v;
+            e = max(e, fx_exp(v));
+        };
+        if (z < nz && ra < ny) put(p, out(fx_to(u[k1].x, o)));
+        if (z < nz && rb < ny) put(p + nz, out(fx_to(u[k1].y, o)));
     }
+    phi_raise(st, e);
 }
 
 // Forward transform of one even line pair per line (the Green passes): item m of

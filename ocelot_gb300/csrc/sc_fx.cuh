@@ -157,4 +157,23 @@ __device__ __forceinline__ double fx_to(Fx a, FxOut o) {
     return __hiloint2double((int)(hi | ((unsigned)sg & 0x80000000u)), (int)lo);
 }
 
+// the nearest double of the integer itself
+__device__ __forceinline__ double fx_double(Fx a) {
+    const long long sg = a.v >> 63;
+    const unsigned long long u = (unsigned long long)((a.v ^ sg) - sg);
+    const int n = __clzll((long long)u);
+    const unsigned long long m = (((u << (n & 63)) >> 10) + 1) >> 1;
+    const unsigned hi = (unsigned)(m >> 32) + ((unsigned)(1085 - n) << 20) | ((unsigned)sg & 0x80000000u);
+    return u ? __hiloint2double((int)hi, (int)(unsigned)m) : 0.0;
+}
+
+// Field grids of the FP64 kick: differences of the potential as integers whose
+// bit FX_PHI stands for 2^(the largest exponent of the potential)
+constexpr int FX_PHI = 58;
+// the potential's largest exponent over a grid: every thread of the warp calls it
+__device__ __forceinline__ void phi_raise(const ScState* st, int e) {
+    e = __reduce_max_sync(~0u, e);
+    if ((threadIdx.x & 31) == 0) atomicMax(&const_cast<ScState*>(st)->phi_exp, e);
+}
+
 }  // namespace ocsc

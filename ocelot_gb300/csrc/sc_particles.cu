@@ -27,6 +27,7 @@
 // Reductions are deterministic: a fixed grid, shuffle trees within blocks,
 // per-block partials in HBM and a one-block finalize in a fixed order.
 #include "sc_common.cuh"
+#include "sc_fx.cuh"
 
 namespace ocsc {
 
@@ -735,6 +736,7 @@ __device__ __forceinline__ void mesh_finish(const double* mn, const double* mx, 
         st->phi_scalef = (float)scale;
         st->igf_rebuild = same ? 0 : 1;
         st->igf_next = 0;
+        st->phi_exp = 0;
     }
 }
 
@@ -1782,8 +1784,8 @@ __device__ __forceinline__ double sample64(const double* __restrict__ F, int i, 
     const double v = lerp64(y0, y1, tx);
     return ok ? v : 0.0;
 }
-// the three staggered components at grid coordinates X: 48 FP64 instructions
-// (the eight-corner sums with their weights were 96)
+// the three staggered components at grid coordinates X (el_field): 48 FP64
+// instructions (the eight-corner sums with their weights were 96)
 __device__ __forceinline__ void gather64(const double* __restrict__ ex, const double* __restrict__ ey,
                                          const double* __restrict__ ez, int nx, int ny, int nz, const double (&X)[3],
                                          double (&e)[3]) {
@@ -1836,15 +1838,67 @@ __device__ __forceinline__ bool near_edge64(double X, int n) {
     return fabsf(x) < 1e-6f || fabsf(x + 0.5f) < 1e-6f || fabsf(x - top) < 1e-4f || fabsf(x - (top - 0.5f)) < 1e-4f;
 }
 
-// Gather + kick of the FP64 form.  Bound by the FP64 pipe: 118 instructions per
-// particle, from rparticles alone, in units of the reference momentum (mad64):
+// The gather of the FP64 kick in integers (k_field_grids' fe; a 64-bit sum or
+// product on the integer pipes costs a tenth of an FP64 instruction here):
+// coordinates in units of 2^-54 of a cell, weights with 62 bits, the same
+// trilinear form as gather64.  The coordinate's bits below 2^-54 are floored away, so
+// every range test decides as on the double.
+struct AxisFx {
+    int ia, ib;
+    FxC ta, tb;
+    bool oka, okb;
+};
+__device__ __forceinline__ AxisFx axis_fx(double X, int n) {
+    const int hi = __double2hiint(X), e = (hi >> 20) & 0x7ff;
+    const unsigned lo = (unsigned)__double2loint(X);
+    const unsigned long long m =
+        ((unsigned long long)((unsigned)hi << 11 | lo >> 21 | 0x80000000u) << 32) | (lo << 11);
+    const bool far = e >= 1023 + 9;  // |X| >= 512, infinities and NaN: outside every mesh
+    const int s = 1023 + 9 - e;      // m 2^-s: |X| in units of 2^-54
+    long long v = (long long)fx_shr(m, s);
+    if (hi < 0 && !zero64(X)) v = ~(long long)fx_shr(m - 1, s);
+    if (far) v = -1ll << 60;
+    const long long top = (long long)(n - 1) << 54;
+    auto at = [&](long long w, int& i, FxC& t, bool& ok) {
+        ok = w >= 0 && w <= top;
+        i = (int)(w >> 54);
+        t = FxC((int)((unsigned)(w >> 23) & 0x7fffffffu), (int)(((unsigned)w << 8) & 0x7fffffffu));
+        if (i >= n - 1) i = n - 2, t = FxC(0x7fffffff, 0x7fffffff);
+        i = i < 0 ? 0 : i;
+    };
+    AxisFx A{0, 0, FxC(0, 0), FxC(0, 0), false, false};
+    at(v, A.ia, A.ta, A.oka);
+    at(v + (1ll << 53), A.ib, A.tb, A.okb);
+    return A;
+}
+__device__ __forceinline__ Fx lerp_fx(long long a, long long b, FxC t) { return Fx{a} + fx_mul(Fx{b - a}, t); }
+__device__ __forceinline__ double sample_fx(const long long* __restrict__ F, int i, int j, int k, FxC tx, FxC ty,
+                                            FxC tz, int ny, int nz, bool ok, double scale) {
+    const long long* b = F + ((size_t)i * ny + j) * nz + k;
+    const size_t sx = (size_t)ny * nz;
+    const Fx y0 = lerp_fx(lerp_fx(b[0], b[1], tz).v, lerp_fx(b[nz], b[nz + 1], tz).v, ty);
+    const Fx y1 = lerp_fx(lerp_fx(b[sx], b[sx + 1], tz).v, lerp_fx(b[sx + nz], b[sx + nz + 1], tz).v, ty);
+    return ok ? fx_double(lerp_fx(y0.v, y1.v, tx)) * scale : 0.0;
+}
+__device__ __forceinline__ void gather_fx(const long long* __restrict__ fe, int nx, int ny, int nz,
+                                          const double (&X)[3], const ScState* st, double (&e)[3]) {
+    const AxisFx x = axis_fx(X[0], nx), y = axis_fx(X[1], ny), z = axis_fx(X[2], nz);
+    const size_t nc = (size_t)nx * ny * nz;
+    e[0] = sample_fx(fe, x.ia, y.ib, z.ib, x.ta, y.tb, z.tb, ny, nz, x.oka && y.okb && z.okb, st->escale[0]);
+    e[1] = sample_fx(fe + nc, x.ib, y.ia, z.ib, x.tb, y.ta, z.tb, ny, nz, x.okb && y.oka && z.okb, st->escale[1]);
+    e[2] = sample_fx(fe + 2 * nc, x.ib, y.ib, z.ia, x.tb, y.tb, z.ta, ny, nz, x.okb && y.okb && z.oka, st->escale[2]);
+}
+
+// Gather + kick of the FP64 form.  Bound by the FP64 pipe: 73 instructions per
+// particle (the gather's 48 run as integers beside them, gather_fx: 2M / 64^3
+// 460 -> 287 us, 200k / 63^3 51 -> 37), from rparticles alone, in units of the reference momentum (mad64):
 //   p' = p + Tk e   (Tk: the frame's rotation with the kick's factors, so the
 //                    rotation into the frame and back is done once, on e)
 //   e' = sqrt(|p'|^2 + (m c / pref)^2),  w = -z_lab / pz'
 //   tau' = w e',  x = x_lab + x' w,  delta' = delta + (|p'|^2 - |p|^2) / (e + e')
 // -- sc.py:218-250 and xp_2_xxstg_mad (coord_transform.py:16-54) with the
 // normalisations cancelled; the reference's operations took 226 and read 84
-// bytes a particle of stored coordinates (2M / 64^3: 885 -> 469 us).  (delta as
+// bytes a particle of stored coordinates.  (delta as
 // an increment: e' - 1/beta_ref, ten instructions less, carries the rounding
 // of e' ~ 1 into delta ~ 1e-3.)  The grid
 // coordinates are lab position x Tg - X_off (Tg: rotation, gamma0 and steps in
@@ -1852,8 +1906,8 @@ __device__ __forceinline__ bool near_edge64(double X, int n) {
 // rec != nullptr (the record-field mode): the field samples before the gamma0
 // factor go to rec[i], rec[nX + i], rec[2 nX + i]
 constexpr int KICK64_THREADS = 128;
-__global__ void __launch_bounds__(KICK64_THREADS, 4) k_kick64(double* __restrict__ rp, const double* __restrict__ ex,
-                                               const double* __restrict__ ey, const double* __restrict__ ez,
+__global__ void __launch_bounds__(KICK64_THREADS, 4) k_kick64(double* __restrict__ rp,
+                                               const long long* __restrict__ fe,
                                                const __grid_constant__ KickParams kp, const ScState* st,
                                                double* __restrict__ rec) {
     pdl_wait();
@@ -1879,7 +1933,7 @@ __global__ void __launch_bounds__(KICK64_THREADS, 4) k_kick64(double* __restrict
             for (int j = 0; j < 3; ++j) X[j] = Xe[j];
         }
         double e[3];
-        gather64(ex, ey, ez, kp.nx, kp.ny, kp.nz, X, e);
+        gather_fx(fe, kp.nx, kp.ny, kp.nz, X, st, e);
         if (rec) {
             rec[i] = e[0];
             rec[kp.nX + i] = e[1];
@@ -2660,9 +2714,7 @@ cudaError_t launch_gather_kick(const Plan& p, const Layout& L, char* ws, const K
     const ScState* st = reinterpret_cast<const ScState*>(ws + L.state);
     const int nb = particle_blocks(p, kp.n);
     if (p.prec == SC_FP64)
-        launch(k_kick64, (int)((kp.n + KICK64_THREADS - 1) / KICK64_THREADS), KICK64_THREADS, 0, s, rp,
-               reinterpret_cast<const double*>(ws + L.ex),
-               reinterpret_cast<const double*>(ws + L.ey), reinterpret_cast<const double*>(ws + L.ez), kp, st,
+        launch(k_kick64, (int)((kp.n + KICK64_THREADS - 1) / KICK64_THREADS), KICK64_THREADS, 0, s, rp, field_fx(L, ws), kp, st,
                p.record_field ? reinterpret_cast<double*>(ws + L.X) : nullptr);
     else
     {
