@@ -136,6 +136,7 @@ Layout make_layout(const Plan& p, int64_t n) {
     L.W2 = take(p.spectral ? cs * (size_t)p.nx * p.My * Kz : 0);
     L.W3 = take(p.spectral ? cs * (size_t)p.nx * p.My * Kz : 0);
     L.X = take(rs * 3 * (size_t)((n + 3) / 4 * 4));
+    L.lab = take(p.prec == SC_FP64 ? 8 * 4 * (size_t)((n + 3) / 4 * 4) : 0);
     L.keys = take(4 * (size_t)n);
     // the radix sort's buffers: only the sorted deposit uses them
     const size_t ns = p.sorted_deposit ? (size_t)n : 0;

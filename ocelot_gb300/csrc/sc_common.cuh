@@ -168,6 +168,7 @@ struct Layout {
     size_t state, tw_x, tw_y, tw_z;              // twiddles (Cx<R>[M])
     size_t part_frame, part_ext;                 // per-block partial sums (double)
     size_t X;                                    // 3 x n: lab positions (FP32) of a kick, grid coordinates (R) of el_field
+    size_t lab;                                  // FP64: 4 x n: lab position and longitudinal momentum of a kick
     size_t keys, sort_keys, sort_perm, sort_q, sort_tmp_k, sort_tmp_v, sort_hist, sort_tot;
     size_t qgrid, phi, ex, ey, ez;               // [nx][ny][nz] (R)
     size_t exq, eyq, ezq;                        // FP32 form: [nx][ny][nz] gather octs (8 floats, 32-byte aligned)

@@ -827,10 +827,12 @@ __device__ __forceinline__ Mad64 mad64(double x, double xq, double y, double yq,
 }
 
 // bound by the FP64 pipe, 28 instructions per particle (it read the rows and
-// stored six FP64 lab coordinates with 98 before: 2M particles 344 -> 114 us)
+// stored six FP64 lab coordinates with 98 before: 2M particles 344 -> 114 us; the
+// position and longitudinal momentum that the kick takes from here add 64 MB of writes
+// and no time)
 __global__ void __launch_bounds__(PT) k_frame64(const double* __restrict__ rp, const double* __restrict__ q,
-                                                KickParams kp, float* __restrict__ X, double* __restrict__ part,
-                                                ScState* st) {
+                                                KickParams kp, float* __restrict__ X, double* __restrict__ lab,
+                                                double* __restrict__ part, ScState* st) {
     pdl_wait();
     __shared__ double sm[8][PT];
     double a[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -844,7 +846,9 @@ __global__ void __launch_bounds__(PT) k_frame64(const double* __restrict__ rp, c
         for (int j = 0; j < 3; ++j) {
             a[3 + j] = fma(qi, m.l[j], a[3 + j]);
             X[j * nX + i] = d2f(m.l[j]);
+            lab[j * nX + i] = m.l[j];
         }
+        lab[3 * nX + i] = m.pz;
         a[6] += qi;
         a[7] += fabs(qi);
     }
@@ -1889,25 +1893,26 @@ __device__ __forceinline__ void gather_fx(const long long* __restrict__ fe, int 
     e[2] = sample_fx(fe + 2 * nc, x.ib, y.ib, z.ia, x.tb, y.tb, z.ta, ny, nz, x.okb && y.okb && z.oka, st->escale[2]);
 }
 
-// Gather + kick of the FP64 form.  Bound by the FP64 pipe: 73 instructions per
+// Gather + kick of the FP64 form.  Bound by the FP64 pipe, 51 instructions per
 // particle (the gather's 48 run as integers beside them, gather_fx: 2M / 64^3
-// 460 -> 287 us, 200k / 63^3 51 -> 37), from rparticles alone, in units of the reference momentum (mad64):
+// 460 -> 287 us, 200k / 63^3 51 -> 37; the lab position and momentum come from
+// the frame pass, 32 bytes a particle instead of 22 instructions: 287 -> 234 and
+// 37 -> 30), in units of the reference momentum (mad64):
 //   p' = p + Tk e   (Tk: the frame's rotation with the kick's factors, so the
 //                    rotation into the frame and back is done once, on e)
 //   e' = sqrt(|p'|^2 + (m c / pref)^2),  w = -z_lab / pz'
 //   tau' = w e',  x = x_lab + x' w,  delta' = delta + (|p'|^2 - |p|^2) / (e + e')
 // -- sc.py:218-250 and xp_2_xxstg_mad (coord_transform.py:16-54) with the
-// normalisations cancelled; the reference's operations took 226 and read 84
-// bytes a particle of stored coordinates.  (delta as
-// an increment: e' - 1/beta_ref, ten instructions less, carries the rounding
-// of e' ~ 1 into delta ~ 1e-3.)  The grid
-// coordinates are lab position x Tg - X_off (Tg: rotation, gamma0 and steps in
+// normalisations cancelled.  (delta as an increment: e' - 1/beta_ref, ten
+// instructions less, carries the rounding of e' ~ 1 into delta ~ 1e-3.)  The
+// grid coordinates are lab position x Tg - X_off (Tg: rotation, gamma0 and steps in
 // one matrix).
 // rec != nullptr (the record-field mode): the field samples before the gamma0
 // factor go to rec[i], rec[nX + i], rec[2 nX + i]
 constexpr int KICK64_THREADS = 128;
 __global__ void __launch_bounds__(KICK64_THREADS, 4) k_kick64(double* __restrict__ rp,
                                                const long long* __restrict__ fe,
+                                               const double* __restrict__ lab,
                                                const __grid_constant__ KickParams kp, const ScState* st,
                                                double* __restrict__ rec) {
     pdl_wait();
@@ -1922,11 +1927,11 @@ __global__ void __launch_bounds__(KICK64_THREADS, 4) k_kick64(double* __restrict
     const double o0 = st->xoff[0], o1 = st->xoff[1], o2 = st->xoff[2];
     const double mu2 = kp.r_grbr * kp.r_grbr;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double xq = rp[ld + i], yq = rp[3 * ld + i];
-        const Mad64 m = mad64(rp[i], xq, rp[2 * ld + i], yq, rp[4 * ld + i], rp[5 * ld + i], kp);
-        double X[3] = {fma(m.l[2], Tg[2][0], fma(m.l[1], Tg[1][0], fma(m.l[0], Tg[0][0], -o0))),
-                       fma(m.l[2], Tg[2][1], fma(m.l[1], Tg[1][1], fma(m.l[0], Tg[0][1], -o1))),
-                       fma(m.l[2], Tg[2][2], fma(m.l[1], Tg[1][2], fma(m.l[0], Tg[0][2], -o2)))};
+        const double xq = rp[ld + i], yq = rp[3 * ld + i], d = rp[5 * ld + i];
+        const double l0 = lab[i], l1 = lab[kp.nX + i], l2 = lab[2 * kp.nX + i], p3 = lab[3 * kp.nX + i];
+        double X[3] = {fma(l2, Tg[2][0], fma(l1, Tg[1][0], fma(l0, Tg[0][0], -o0))),
+                       fma(l2, Tg[2][1], fma(l1, Tg[1][1], fma(l0, Tg[0][1], -o1))),
+                       fma(l2, Tg[2][2], fma(l1, Tg[1][2], fma(l0, Tg[0][2], -o2)))};
         if (near_edge64(X[0], kp.nx) || near_edge64(X[1], kp.ny) || near_edge64(X[2], kp.nz)) {
             double Xe[3];
             grid64_exact(rp, ld, i, &kp, st, Xe);
@@ -1942,17 +1947,16 @@ __global__ void __launch_bounds__(KICK64_THREADS, 4) k_kick64(double* __restrict
         const double dx = fma(Tk[0][2], e[2], fma(Tk[0][1], e[1], Tk[0][0] * e[0]));
         const double dy = fma(Tk[1][2], e[2], fma(Tk[1][1], e[1], Tk[1][0] * e[0]));
         const double dz = fma(Tk[2][2], e[2], fma(Tk[2][1], e[1], Tk[2][0] * e[0]));
-        const double px = xq + dx, py = yq + dy, pz = m.pz + dz;
+        const double px = xq + dx, py = yq + dy, pz = p3 + dz;
         const double en = sqrt64(fma(px, px, fma(py, py, fma(pz, pz, mu2))));
-        const double dp2 = fma(dx, xq + px, fma(dy, yq + py, dz * (m.pz + pz)));  // |p'|^2 - |p|^2
-        const double w = -m.l[2] * rcp64(pz);
-        const double d = rp[5 * ld + i];
-        rp[i] = fma(px, w, m.l[0]);
+        const double dp2 = fma(dx, xq + px, fma(dy, yq + py, dz * (p3 + pz)));  // |p'|^2 - |p|^2
+        const double w = -l2 * rcp64(pz);
+        rp[i] = fma(px, w, l0);
         rp[ld + i] = px;
-        rp[2 * ld + i] = fma(py, w, m.l[1]);
+        rp[2 * ld + i] = fma(py, w, l1);
         rp[3 * ld + i] = py;
         rp[4 * ld + i] = w * en;
-        rp[5 * ld + i] = fma(dp2, rcp64_once(m.e + en), d);
+        rp[5 * ld + i] = fma(dp2, rcp64_once(kp.r_betaref + d + en), d);
     }
 }
 
@@ -2641,7 +2645,8 @@ cudaError_t launch_frame(const Plan& p, const Layout& L, char* ws, const KickPar
     double* part = reinterpret_cast<double*>(ws + L.part_frame);
     const int nb = particle_blocks(p, kp.n);
     if (p.prec == SC_FP64)
-        launch(k_frame64, nb, PT, 0, s, rp, q, kp, reinterpret_cast<float*>(ws + L.X), part, st);
+        launch(k_frame64, nb, PT, 0, s, rp, q, kp, reinterpret_cast<float*>(ws + L.X),
+               reinterpret_cast<double*>(ws + L.lab), part, st);
     else {
         // the exact deposit's fixed-point grid is zeroed here, so the keys
         // kernel follows the extent kernel without a memset between them
@@ -2714,7 +2719,8 @@ cudaError_t launch_gather_kick(const Plan& p, const Layout& L, char* ws, const K
     const ScState* st = reinterpret_cast<const ScState*>(ws + L.state);
     const int nb = particle_blocks(p, kp.n);
     if (p.prec == SC_FP64)
-        launch(k_kick64, (int)((kp.n + KICK64_THREADS - 1) / KICK64_THREADS), KICK64_THREADS, 0, s, rp, field_fx(L, ws), kp, st,
+        launch(k_kick64, (int)((kp.n + KICK64_THREADS - 1) / KICK64_THREADS), KICK64_THREADS, 0, s, rp, field_fx(L, ws),
+               reinterpret_cast<const double*>(ws + L.lab), kp, st,
                p.record_field ? reinterpret_cast<double*>(ws + L.X) : nullptr);
     else
     {
