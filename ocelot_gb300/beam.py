@@ -75,11 +75,19 @@ class DeviceParticleArray:
         return cls(rp.to(dev, non_blocking=True), q.to(dev, non_blocking=True), p_array.E, getattr(p_array, "s", 0.0))
 
     def to_host(self, p_array=None):
-        host = self.rparticles.cpu().numpy()
-        if p_array is None:
-            p_array = ParticleArray(host.shape[1])
-            p_array.q_array = self.q_array.cpu().numpy()
-        p_array.rparticles[...] = host
+        import torch
+        out = None if p_array is None else p_array.rparticles
+        if (isinstance(out, np.ndarray) and out.dtype == np.float64 and out.dtype.isnative and
+                out.shape == tuple(self.rparticles.shape) and out.flags.c_contiguous and out.flags.writeable):
+            # straight into the caller's array: no second array whose pages are touched for
+            # the first time
+            torch.from_numpy(out).copy_(self.rparticles)
+        else:
+            host = self.rparticles.cpu().numpy()
+            if p_array is None:
+                p_array = ParticleArray(host.shape[1])
+                p_array.q_array = self.q_array.cpu().numpy()
+            p_array.rparticles[...] = host
         p_array.E = self.E
         p_array.s = self.s
         return p_array

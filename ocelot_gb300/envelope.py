@@ -55,22 +55,51 @@ class Twiss:
                 f"beta_y={self.beta_y}, alpha_x={self.alpha_x}, alpha_y={self.alpha_y})")
 
 
+def _sigma(tws) -> np.ndarray:
+    return np.array([[tws.xx, tws.xy, tws.xpx, tws.xpy],
+                     [tws.xy, tws.yy, tws.ypx, tws.ypy],
+                     [tws.xpx, tws.ypx, tws.pxpx, tws.pxpy],
+                     [tws.xpy, tws.ypy, tws.pxpy, tws.pypy]])
+
+
+def _set_eigen_emittances(twiss) -> None:
+    """The eigen-emittances of several Twiss, their eigenvalues taken in one call."""
+    sigma = [(t, _sigma(t)) for t in twiss]
+    good = [(t, m @ _S4) for t, m in sigma if np.isfinite(m).all()]
+    for t, _ in sigma:
+        t.eigemit_1 = t.eigemit_2 = float("nan")
+    if not good:
+        return
+    w = np.sort(np.abs(np.linalg.eigvals(np.stack([m for _, m in good])).imag), axis=1)
+    for (t, _), v in zip(good, w):  # v = [e2, e2, e1, e1]
+        t.eigemit_1, t.eigemit_2 = float(0.5 * (v[2] + v[3])), float(0.5 * (v[0] + v[1]))
+
+
 def eigen_emittances(tws) -> tuple[float, float]:
-    sigma = np.array([[tws.xx, tws.xy, tws.xpx, tws.xpy],
-                      [tws.xy, tws.yy, tws.ypx, tws.ypy],
-                      [tws.xpx, tws.ypx, tws.pxpx, tws.pxpy],
-                      [tws.xpy, tws.ypy, tws.pxpy, tws.pypy]])
-    if not np.all(np.isfinite(sigma)):
-        return float("nan"), float("nan")
-    w = np.sort(np.abs(np.linalg.eigvals(sigma @ _S4).imag))
-    # w = [e2, e2, e1, e1]
-    return float(0.5 * (w[2] + w[3])), float(0.5 * (w[0] + w[1]))
+    t = Twiss()
+    t.__dict__.update(tws.__dict__)
+    _set_eigen_emittances([t])
+    return t.eigemit_1, t.eigemit_2
+
+
+def twiss_table(moments, energies, charge: float, at) -> list:
+    """Twiss of every slot of the sc_moments table at energies[k] and s = at[k]."""
+    out = [_twiss(m, E, charge, s) for m, E, s in zip(moments, energies, at)]
+    _set_eigen_emittances([t for m, t in zip(moments, out) if m[0] >= 3])
+    return out
 
 
 def twiss_from_moments(m, energy: float, charge: float, s: float = 0.0) -> Twiss:
     """A Twiss from one slot of the sc_moments table (get_envelope's steps
     after the moments, analysis.py:83-226)."""
     m = np.asarray(m, dtype=np.float64)
+    tws = _twiss(m, energy, charge, s)
+    if m[0] >= 3:
+        _set_eigen_emittances([tws])
+    return tws
+
+
+def _twiss(m, energy: float, charge: float, s: float) -> Twiss:
     tws = Twiss()
     tws.E = energy
     tws.q = charge
@@ -88,7 +117,6 @@ def twiss_from_moments(m, energy: float, charge: float, s: float = 0.0) -> Twiss
     relbeta = np.sqrt(1 - relgamma ** -2) if relgamma != 0 else 1.
     tws.emit_xn = float(tws.emit_x * relgamma * relbeta)
     tws.emit_yn = float(tws.emit_y * relgamma * relbeta)
-    tws.eigemit_1, tws.eigemit_2 = eigen_emittances(tws)
     with np.errstate(divide="ignore", invalid="ignore"):
         tws.beta_x = float(np.float64(tws.xx) / tws.emit_x)
         tws.beta_y = float(np.float64(tws.yy) / tws.emit_y)

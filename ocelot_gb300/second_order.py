@@ -198,6 +198,9 @@ def element_map2(e, length: float, energy: float):
     return R1, T0, B
 
 
+_PJ, _PK = np.triu_indices(6)  # the pairs j <= k in lexicographic order
+
+
 def pack_map(R, T, B) -> np.ndarray:
     """One map in the device layout: R (row-major), B, then Tc[6][21], the
     coefficient of x_j x_k (j <= k, lexicographic pairs) in output i:
@@ -205,11 +208,8 @@ def pack_map(R, T, B) -> np.ndarray:
     out = np.zeros(MAP2_DOUBLES)
     out[:36] = np.asarray(R, dtype=np.float64).reshape(-1)
     out[36:42] = np.asarray(B, dtype=np.float64).reshape(-1)
-    q = 0
-    for j in range(6):
-        for k in range(j, 6):
-            out[42 + np.arange(6) * 21 + q] = T[:, j, k] + (T[:, k, j] if k != j else 0.0)
-            q += 1
+    both = T[:, _PJ, _PK] + np.where(_PJ != _PK, T[:, _PK, _PJ], 0.0)
+    out[42:] = both.reshape(-1)
     return out
 
 

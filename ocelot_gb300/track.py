@@ -30,6 +30,7 @@ the device after every step, ``envelope.py``).
 from __future__ import annotations
 
 import ctypes as C
+import gc
 import math
 from typing import NamedTuple
 
@@ -145,12 +146,17 @@ def element_map(e, length: float, energy: float):
 # ---------------------------------------------------------------------------
 # The Navigator's kick schedule
 # ---------------------------------------------------------------------------
+def _isclose(a: float, b: float) -> bool:
+    # np.isclose of two floats with its default tolerances, without its 15 us
+    return a == b or (math.isfinite(b) and abs(a - b) <= 1e-8 + 1e-5 * abs(b))
+
+
 def _section_length(total: float, start: float, want: float) -> float:
     # the length OpticElement.get_section_tms builds a slice map for
     # (elements/optic_element.py:376-403)
-    if start < 1e-10 and np.isclose(want, total):
+    if start < 1e-10 and _isclose(want, total):
         return total
-    if start + want > total or np.isclose(start + want, total):
+    if start + want > total or _isclose(start + want, total):
         return total - start
     return want
 
@@ -213,13 +219,22 @@ def kick_schedule(lengths, unit_step: float, step: int = 1):
 def step_maps(elements, energy: float, unit_step: float, step: int = 1):
     """Composed map (R, B) and kick (zstep, z0) of every step."""
     lengths = [_element_params(e)[0] for e in elements]
-    steps = []
-    for slices, zstep, z0 in kick_schedule(lengths, unit_step, step):
+    return _composed_maps(elements, energy, kick_schedule(lengths, unit_step, step))
+
+
+def _composed_maps(elements, energy: float, schedule):
+    # equal slices (a periodic line has few different ones) share a map
+    params = [_element_params(e) for e in elements]
+    made, steps = {}, []
+    for slices, zstep, z0 in schedule:
         R, B = np.eye(6), np.zeros(6)
         for i, dl in slices:
             if dl == 0.0:
                 continue
-            Ri, Bi = element_map(elements[i], dl, energy)
+            key = (params[i], dl)
+            if key not in made:
+                made[key] = element_map(elements[i], dl, energy)
+            Ri, Bi = made[key]
             R, B = Ri @ R, Ri @ B + Bi
         steps.append((R, B, zstep, z0))
     return steps
@@ -354,6 +369,7 @@ def step_slices(elements, energy: float, steps, order: int = 2, s: float = 0.0):
     from .second_order import element_map2, pack_map
     zero_t = np.zeros((6, 6, 6))
     E = energy
+    made = {}  # equal slices (a periodic line has few different ones) share a record
     out = []
     for sections, kicks, z0, dz in steps:
         recs, kinds = [], []
@@ -370,12 +386,16 @@ def step_slices(elements, energy: float, steps, order: int = 2, s: float = 0.0):
             s += length
             if length == 0.0:
                 continue
-            if order == 2:
-                recs.append(pack_map(*element_map2(e, length, E)))
-            else:
-                R, B = element_map(e, length, E)
-                recs.append(pack_map(R, zero_t, B))
-            kinds.append(CV.map_kind(recs[-1]))
+            key = (_element_params(e), length, E)
+            if key not in made:
+                if order == 2:
+                    rec = pack_map(*element_map2(e, length, E))
+                else:
+                    R, B = element_map(e, length, E)
+                    rec = pack_map(R, zero_t, B)
+                made[key] = (rec, CV.map_kind(rec))
+            recs.append(made[key][0])
+            kinds.append(made[key][1])
         table = np.array(recs).reshape(-1, CV.MAP2_DOUBLES)
         out.append(StepSlices(table, np.array(kinds, dtype=np.int32), [(j, E, zstep) for j, zstep in kicks], z0, E,
                               dz))
@@ -474,7 +494,8 @@ class DeviceTrack:
             eng.ensure(self.n)
         if self.composed:
             self.steps = []
-            maps = step_maps(seq, self.E, unit_step, int(processes[0][0].step))
+            schedule = kick_schedule(lengths, unit_step, int(processes[0][0].step))
+            maps = _composed_maps(seq, self.E, schedule)
             table = np.zeros((len(maps), 42))
             for k, (R, B, zstep, z0) in enumerate(maps):
                 table[k, :36] = R.reshape(-1)
@@ -482,7 +503,7 @@ class DeviceTrack:
                 self.steps.append((((0, self.E, zstep) + self._draws(processes[0][0], zstep),), z0))
             self.E_end = self.E
             self.s_end = float(self.beam.s)
-            for slices, _, _ in kick_schedule(lengths, unit_step, int(processes[0][0].step)):
+            for slices, _, _ in schedule:
                 for _, dl in slices:
                     self.s_end += dl
             self._step_E = [self.E] * len(self.steps)
@@ -583,19 +604,18 @@ class DeviceTrack:
         """Twiss of the beam before the first step and after every step, as
         the reference's track() returns them (s = the sum of the step lengths
         so far, E = the beam energy after the step).  Waits for the job."""
-        from .envelope import twiss_from_moments
+        from .envelope import twiss_table
         if not self.twiss:
             raise RuntimeError("the job was created with twiss=False")
         if not self.finished:
             raise RuntimeError("the job has steps left to run")
         self.synchronize()
         m = self.moments.cpu().numpy()
-        out = [twiss_from_moments(m[0], self.E, self.q_total, 0.0)]
-        L = 0.
+        at, L = [0.0], 0.
         for k in range(len(self.steps)):
             L += self._step_dz[k]
-            out.append(twiss_from_moments(m[k + 1], self._step_E[k], self.q_total, 0.0 + L))
-        return out
+            at.append(0.0 + L)
+        return twiss_table(m, [self.E] + list(self._step_E), self.q_total, at)
 
     def _graph(self, kicks):
         import torch
@@ -604,9 +624,23 @@ class DeviceTrack:
             g = torch.cuda.CUDAGraph()
             with torch.cuda.device(self.dev):
                 self.stream.synchronize()
-                # recording does not execute: counter and particles are untouched
-                with torch.cuda.graph(g, stream=self.stream):
-                    self._launch(kicks)
+                # Recording does not execute: counter and particles are untouched.  The
+                # launches allocate nothing, so the recording needs none of torch.cuda.graph's
+                # collection of garbage and emptying of the allocator's cache, which the
+                # next job's workspace is then allocated from again; no collection
+                # may run meanwhile (what it frees could query events).
+                collecting = gc.isenabled()
+                gc.disable()
+                try:
+                    with torch.cuda.stream(self.stream):
+                        g.capture_begin()
+                        try:
+                            self._launch(kicks)
+                        finally:
+                            g.capture_end()
+                finally:
+                    if collecting:
+                        gc.enable()
             self._graphs[kicks] = g
         return g
 
