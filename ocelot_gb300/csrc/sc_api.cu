@@ -375,7 +375,14 @@ int sc_plan_create(sc_plan** out, int nx, int ny, int nz, int mode) {
     p.part_blocks = p.sm_count * 4;
     for (int k = 0; k < 3; ++k) p.wait_limit[k] = MBAR_WAIT_LIMIT;
     p.kick_variant = default_kick_variant();
-    p.fft_plane_fwd = p.fft_plane_inv = 1;
+    // FP64: separate passes -- a plane's block converts and transforms its lines in
+    // fixed point alone on its SM, with a wave of nx blocks (kick of 10k
+    // particles, plane -> separate: 31^3 106 -> 91 us, 48^3 155 -> 129, 24^3 122 -> 113,
+    // 12^3 equal).  FP32: the plane passes save a launch each (32^3 59.1 -> 57.6 us)
+    // while the inverse's blocks, one per x plane and output, fill one wave; beyond
+    // that the separate ones win (64 x 32 x 32 64.5 -> 61.8, 100 x 32 x 24 68.7 -> 66.9)
+    p.fft_plane_fwd = p.prec == SC_FP64 ? 0 : 1;
+    p.fft_plane_inv = p.prec == SC_FP64 ? 0 : nx * (p.spectral ? 3 : 1) <= p.sm_count;
     p.fft_cols_x = p.fft_cols_y = 0;
     // everything that is not a stream operation happens here, so that kicks
     // can be recorded in a CUDA graph
