@@ -1,13 +1,15 @@
 // FP64 square root, quotient, logarithm and arctangent for the exact integrated
 // Green's function (igf_point in sc_green.cu).  That table is bound by the FP64
-// pipe (about 1/64 of the FP32 rate on this GPU), so these spend FP64
-// instructions only where 53 bits are needed: table-driven reductions in the
-// manner of P. T. P. Tang (ACM TOMS 16, 1990), the leading terms of the
-// remaining series in FP64, the higher ones -- below 2^-32 of the result -- and
-// every exponent and table-index step on the FP32 and integer pipes.  Results
-// are within 0.51 (sqrt, quotient) and 0.53 (log, atan) ulp of the exact value
+// pipe (about 1/64 of the FP32 rate on this GPU), so the square root, the
+// quotients and the reference's own products and sums are FP64 and everything else
+// runs on the integer pipes beside them: table-driven reductions in the manner
+// of P. T. P. Tang (ACM TOMS 16, 1990), the remaining series in 64-bit integers,
+// its terms below 2^-26 (log) and 2^-34 (atan) in FP32.  Results are
+// within 0.50 (sqrt, quotient), 0.51 (log) and 0.64 (atan) ulp of the exact value
 // over the arguments tried (10 million each against extended precision).
-// Instructions: sqrt 7, quotient 5, log 10, atan 15.
+// FP64 instructions: sqrt 7, quotient 5, log none, atan 7 (10 and 15 in a form
+// with its series in FP64: 63^3 beside the other stream 75 -> 53 us at 10k
+// particles, 84 -> 56 at 200k).
 //
 // Arguments must be positive and well inside the exponent range (igf_point
 // checks the mesh steps once and falls back to the CUDA functions).
@@ -24,6 +26,9 @@
 
 namespace ocsc {
 namespace igf {
+
+constexpr long long LN2_HI = 49946518145322873ll;  // ln 2 in units of 2^-56
+constexpr long long LN2_LO = 2882134964ll;  // and the rest of it in units of 2^-88
 
 SC_HD double bits_d(unsigned hi, unsigned lo) {
 #ifdef __CUDA_ARCH__
@@ -113,49 +118,99 @@ SC_HD double div_(double n, double d) {
     return fma(fma(-q, d, n), y, q);
 }
 
+// upper half of a product
+SC_HD long long mulhi(long long a, long long b) {
+#ifdef __CUDA_ARCH__
+    return __mul64hi(a, b);
+#else
+    return (long long)(((__int128)a * b) >> 64);
+#endif
+}
+SC_HD int clz64(unsigned long long v) {
+#ifdef __CUDA_ARCH__
+    return __clzll((long long)v);
+#else
+    return v ? __builtin_clzll(v) : 64;
+#endif
+}
+SC_HD unsigned long long shr64(unsigned long long v, int n) {  // 0 for n > 63
+#ifdef __CUDA_ARCH__
+    unsigned long long r;
+    asm("shr.u64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(n));
+    return r;
+#else
+    return n > 63 ? 0 : v >> n;
+#endif
+}
+// the nearest double of v 2^-s
+SC_HD double to_double(long long v, int s) {
+    const long long sg = v >> 63;
+    const unsigned long long u = (unsigned long long)((v ^ sg) - sg);
+    const int n = clz64(u);
+    const unsigned long long m = (((u << (n & 63)) >> 10) + 1) >> 1;
+    const unsigned hi = ((unsigned)(m >> 32) + ((unsigned)(1085 - n - s) << 20)) | ((unsigned)sg & 0x80000000u);
+    return u ? bits_d(hi, (unsigned)m) : 0.0;
+}
+
 // log(x) for normal x > 0: x = 2^k m, m in [1, 2); with the table's short 1/c
-// near 1/m, r = m (1/c) - 1 (exact up to 2^-62), |r| < 2^-7.9, and
-// log x = (k ln2_hi + hi) + r - r^2/2 + r^3/3 + [r^4 (..) + k ln2_lo + lo in FP32]
+// near 1/m, r = m (1/c) - 1, exact in units of 2^-66, |r| < 2^-7.9, and
+// log x = k ln2 - log(1/c) + r - r^2 (1/2 - r/3 + r^2/4 - [r^3/5 - r^4/6 in FP32]),
+// in integers; the sum in units of 2^-56 or 2^-58
 SC_HD double log_(double x, const LogEntry* __restrict__ tab) {
     const unsigned hx = hi_d(x);
-    const float k = (float)((int)(hx >> 20) - 1023);
+    const int k = (int)(hx >> 20) - 1023;
     const LogEntry t = tab[(hx >> 13) & 127u];
-    const double m = bits_d((hx & 0xfffffu) | 0x3ff00000u, lo_d(x));
-    const double r = fma(m, widen(t.invc), -1.0);
-    const double hi = fma(widen(k), 0x1.62e42fefa3800p-1, t.hi);  // exact: both multiples of 2^-42
-    const double w = hi + r, e = (hi - w) + r;
-    const float rf = narrow(r), r2f = rf * rf;
-    const float s = fmaf(rf, fmaf(rf, fmaf(rf, 0.142857143f, -0.166666667f), 0.2f), -0.25f);
-    const float tail = fmaf(r2f * r2f, s, fmaf(k, 0x1.ef357ap-45f, t.lo));
-    const double q = fma(r, 0x1.5555555555555p-2, -0.5);
-    return w + (fma(r * r, q, widen(tail)) + e);
+    const unsigned long long m = ((unsigned long long)((hx & 0xfffffu) | 0x100000u) << 32) | lo_d(x);
+    const long long r = (long long)(m * (unsigned long long)(unsigned)t.ic);  // 2^-66; the 1 is 2^66, gone
+    const long long r4 = (long long)((unsigned long long)r << 4);
+    const long long r2 = mulhi(r4, r4);                                       // 2^-76
+    const float rf = (float)(int)(r >> 32) * 0x1p-34f;
+    const float f = (rf * rf) * rf * fmaf(rf, -0.166666667f, 0.2f);
+    const long long u = (1ll << 61) - (mulhi(r, 0x5555555555555555ll) >> 4) + (r2 >> 16) -
+                        (long long)((unsigned long long)(long long)(int)(f * 0x1p50f) << 12);  // 2^-62
+    const long long q = r - (mulhi(r2, u) >> 8);                              // 2^-66
+    const long long low = (((long long)k * LN2_LO) >> 26) + t.t + (q >> 4);   // 2^-62
+    const int sh = (unsigned)(k + 40) <= 80u ? 2 : 0;  // |log x| < 2^5: two bits more
+    const long long v = (long long)((unsigned long long)((long long)k * LN2_HI) << sh) + ((low + (32 >> sh)) >> (6 - sh));
+    return to_double(v, 56 + sh);
 }
 
 // atan(w), any sign of a finite w: |w| <= 1 about c = j/128 as atan c + atan((w - c) / (1 + c w)),
-// |w| > 1 about 1/c as pi/2 - atan c + atan((c w - 1) / (w + c)); the quotient t, |t| <= 2^-8, and
-// t - t^3/3 in FP64, the rest of the series in FP32
+// |w| > 1 about 1/c as pi/2 - atan c + atan((c w - 1) / (w + c)), |w| < 3.5/128 as itself; the
+// quotient t, |t| <= 2^-8, in FP64, t - t (t^2/3 - t^4/5 + [t^6/7 - t^8/9 + t^10/11 in FP32]) and the
+// sum in integers, in units that leave the result 59 bits or more
 SC_HD double atan_(double w, const AtanEntry* __restrict__ tab) {
     const unsigned sign = hi_d(w) & 0x80000000u;
     const double a = bits_d(hi_d(w) & 0x7fffffffu, lo_d(w));
     const bool big = hi_d(a) >= 0x3ff00000u;  // |w| >= 1
     const float af = narrow(a);
     const float u = big ? 1.0f / af : af;
-    const int j = (int)(u * 128.0f + 0.5f);  // 0 .. 128
+    int j = (int)(u * 128.0f + 0.5f);  // 0 .. 128
+    const bool tiny = !big && j < 4;   // the quotient's rounding would be the result's
+    if (tiny) j = 0;
     const float cf = (float)j * 0.0078125f;
     const double c = widen(cf), mc = widen(-cf);
     // N = w - c, D = 1 + c w, or N = c w - 1, D = w + c
     const double N = fma(big ? c : 1.0, a, big ? -1.0 : mc);
     const double D = fma(big ? 1.0 : c, a, big ? c : 1.0);
     const double t = div_(N, D);
-    const double hi = big ? tab[j].hi2 : tab[j].hi;
-    const float lo = big ? tab[j].lo2 : tab[j].lo;
-    const float tf = narrow(t), t2f = tf * tf;
-    const float tail = fmaf(tf * (t2f * t2f), fmaf(t2f, -0.142857143f, 0.2f), lo);
-    const double t3 = (t * t) * t;
-    const double corr = fma(t3, -0x1.5555555555555p-2, widen(tail));
-    const double s = hi + t, e = (hi - s) + t;
-    const double v = s + (e + corr);
-    return bits_d(hi_d(v) ^ sign, lo_d(v));
+    const AtanEntry E = tab[j];
+    const unsigned ht = hi_d(t);
+    const int e = (int)((ht >> 20) & 0x7ffu) - 1023;
+    const unsigned long long m = (((unsigned long long)((ht & 0xfffffu) | 0x100000u) << 32) | lo_d(t)) << 9;  // |t| 2^(61 - e)
+    const long long tq = (long long)shr64(m, -5 - e);  // 2^-66
+    const long long t2 = mulhi(tq, tq);                // 2^-68
+    const long long t4 = mulhi(t2 << 5, t2 << 5);      // 2^-82
+    const float t2f = (float)(int)(t2 >> 32) * 0x1p-36f;
+    const float f = (t2f * t2f) * t2f * fmaf(t2f, fmaf(t2f, 0.0909090909f, -0.111111111f), 0.142857143f);
+    const long long corr = mulhi(t2, 0x5555555555555555ll) - (mulhi(t4, 0x3333333333333333ll) >> 14) +
+                           ((long long)(int)(f * 0x1p64f) << 4);  // 2^-68
+    const int s = tiny ? 61 - e : (big ? 61 : E.s);
+    const long long T = (long long)shr64(m, 61 - e - s);
+    const long long p = T - (mulhi(T, corr << 6) >> 10);
+    const long long v = tiny ? p : (big ? E.hi2 : E.hi) + ((int)ht < 0 ? -p : p);
+    const double res = tiny && e < -1000 ? a : to_double(v, s);
+    return bits_d(hi_d(res) ^ sign, lo_d(res));
 }
 
 // IG of sc.py:109-133 at one corner: the reference's operations, the four
