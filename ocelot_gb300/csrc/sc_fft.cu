@@ -31,6 +31,7 @@ constexpr int FFT_THREADS = sizeof(R) == 8 ? 128 : 256;
 constexpr int FFT_MINB = 4;
 // the fixed-point passes: 128 registers
 constexpr int FX_MINB(int L) { return 512 / fx_threads(L); }
+constexpr int FX_MINB_XY(int L) { return 512 / fx_threads_xy(L); }
 
 // complex lines (two real lines each) per block of the z passes: up to 8,
 // so that a 64^3 mesh gives 256 blocks
@@ -38,11 +39,11 @@ static inline int z_lines_per_block(int Mz) {
     int nc = 1024 / Mz;
     return nc < 1 ? 1 : (nc > 8 ? 8 : nc);
 }
-// the fixed-point z passes: a whole number of warps of two_step_q(Mz) threads a line
+// the fixed-point z passes: whole warps of two_step_q(Mz) threads a line
 template <typename R>
 static inline int z_lines(int Mz) {
     const int nc = z_lines_per_block(Mz);
-    return sizeof(R) == 8 && uses_two_step(Mz) ? nc & ~3 : nc;
+    return sizeof(R) == 8 && uses_two_step(Mz) ? (Mz > 192 ? 4 : 8) : nc;
 }
 // columns per block in the strided passes: 16, fewer when two line buffers
 // of 16 columns would not fit in shared memory (FP64 at M = 512)
@@ -290,7 +291,7 @@ __global__ void __launch_bounds__(fx_threads(L), FX_MINB(L)) k_zfwd_fx(double* _
     zfwd_fx<L>(q, W, ny, nz, My, Kz, twg, NC, st, hw_vblk());
 }
 template <bool INV, int L>
-__global__ void __launch_bounds__(fx_threads(L), FX_MINB(L)) k_ypass_fx(double2* __restrict__ W, int nx, int ny, int Kz,
+__global__ void __launch_bounds__(fx_threads_xy(L), FX_MINB_XY(L)) k_ypass_fx(double2* __restrict__ W, int nx, int ny, int Kz,
                                                                      const double2* __restrict__ twg,
                                                                      const ScState* st) {
     pdl_wait();
@@ -298,7 +299,7 @@ __global__ void __launch_bounds__(fx_threads(L), FX_MINB(L)) k_ypass_fx(double2*
     ypass_fx<INV, L>(W, nx, ny, Kz, twg, hw_vblk());
 }
 template <int L>
-__global__ void __launch_bounds__(fx_threads(L), FX_MINB(L)) k_xconv_fx(double2* __restrict__ W,
+__global__ void __launch_bounds__(fx_threads_xy(L), FX_MINB_XY(L)) k_xconv_fx(double2* __restrict__ W,
                                                                      const double* __restrict__ G, int nx, int My,
                                                                      int Kz, int Ky, const double2* __restrict__ twg,
                                                                      const ScState* st) {
@@ -971,7 +972,7 @@ static cudaError_t launch_ypass(const Plan& p, dim3 g, size_t sm, cudaStream_t s
                               sp);
             } else {
                 if ((e = set_smem(k_ypass_fx<INV, LL>, sm))) return e;
-                return launch(k_ypass_fx<INV, LL>, g, fx_threads(LL), sm, s, W, p.nx, p.ny, Kz, tw, st);
+                return launch(k_ypass_fx<INV, LL>, g, fx_threads_xy(LL), sm, s, W, p.nx, p.ny, Kz, tw, st);
             }
         });
     if ((e = set_smem(k_ypass<R, INV>, sm))) return e;
@@ -989,7 +990,7 @@ static cudaError_t launch_xconv(const Plan& p, dim3 g, size_t sm, cudaStream_t s
                 return launch(k_xconv_s<LL>, g, stream_threads(LL), sm, s, W, G, p.nx, p.My, Kz, Ky, p.rx, tw, TK, st, sp);
             } else {
                 if ((e = set_smem(k_xconv_fx<LL>, sm))) return e;
-                return launch(k_xconv_fx<LL>, g, fx_threads(LL), sm, s, W, G, p.nx, p.My, Kz, Ky, tw, st);
+                return launch(k_xconv_fx<LL>, g, fx_threads_xy(LL), sm, s, W, G, p.nx, p.My, Kz, Ky, tw, st);
             }
         });
     if ((e = set_smem(k_xconv<R>, sm))) return e;

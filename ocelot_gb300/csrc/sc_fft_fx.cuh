@@ -3,8 +3,7 @@
 // inputs go from global memory into registers, the line's exponent is agreed on
 // through shared memory, and the transform, the Green product and the inverse
 // run in integers until the results are converted and stored.  Eight columns
-// (z: NC lines) per block, one work item of the wider step per thread, four
-// blocks' worth of 128 registers per SM so that one block's loads and
+// (z: NC lines) per block, 128 registers a thread and 512 threads' worth of blocks per SM so that one block's loads and
 // barriers overlap the others' arithmetic.
 //
 // What bounds them: issue slots of the integer pipes (about half of them the
@@ -18,7 +17,13 @@
 namespace ocsc {
 
 constexpr int FX_COLS = 8;
+// Threads of a block of lines: of the wider step's items (Q per line) where there are
+// few lines (z and Green passes, 2000 at 63^3: a round more would be exposed), of
+// the narrower one's (P) in the x and y passes, where enough blocks stand beside
+// each other and no warp should idle in the narrower step (x pass 31 -> 27 us, y
+// 12 -> 9.6 and 10 -> 8.9, but Green passes 6.5 -> 9)
 constexpr int fx_threads(int L) { return FX_COLS * two_step_q(L); }
+constexpr int fx_threads_xy(int L) { return two_step_q(L) ? FX_COLS * (L / two_step_q(L)) : 0; }
 // table of a line (odd stride), and dynamic shared memory of a pass over n lines
 __host__ __device__ constexpr int fx_tab(int L) { return two_step_q(L) ? ((L / two_step_q(L)) * (two_step_q(L) + 1)) | 1 : 0; }
 __host__ __device__ constexpr int fx_line(int L) { return L | 1; }
@@ -60,41 +65,53 @@ __device__ __forceinline__ void ypass_fx(double2* __restrict__ W, int nx, int ny
     constexpr int Q = S::Q, P = S::P;
     constexpr int A = INV ? P : Q, NIN = INV ? Q : P / 2;   // first step: items, inputs of one
     constexpr int B = INV ? Q : P, NOUT = INV ? P / 2 : Q;  // second step: items, outputs of one
+    constexpr int RA = (A + P - 1) / P, RB = (B + P - 1) / P;  // rounds
     constexpr int BIT = INV ? S::B_INV : S::B_HALF;
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ FxLines ln;
     FxW* tw = reinterpret_cast<FxW*>(smraw);
-    const int kk = threadIdx.x & (FX_COLS - 1), m = threadIdx.x / FX_COLS;
+    const int kk = threadIdx.x & (FX_COLS - 1), m0 = threadIdx.x / FX_COLS;
     Fx2* tab = reinterpret_cast<Fx2*>(tw + L) + kk * fx_tab(L);
     const int col = vb.x * FX_COLS + kk;
     const bool live = col < nx * Kz;
     const int x = col / Kz, k = col - x * Kz;
     double2* line = W + (size_t)x * L * Kz + k;  // element y of the column at line[y * Kz]
-    double2 d[NIN];
+    double2 d[RA][NIN];
+    int e = 0;
 #pragma unroll
-    for (int n = 0; n < NIN; ++n) {
-        const int y = n * A + m;
-        d[n] = (m < A && live && (INV || y < ny)) ? line[(size_t)y * Kz] : make_double2(0, 0);
-    }
+    for (int r = 0; r < RA; ++r)
+#pragma unroll
+        for (int n = 0; n < NIN; ++n) {
+            const int m = m0 + r * P, y = n * A + m;
+            d[r][n] = (m < A && live && (INV || y < ny)) ? line[(size_t)y * Kz] : make_double2(0, 0);
+        }
     fx_clear(ln);
     load_twiddles<double>(reinterpret_cast<double2*>(tw), twg, L);
+#pragma unroll
+    for (int r = 0; r < RA; ++r) e = max(e, fx_exp_of(d[r]));
     __syncthreads();
-    fx_raise(&ln.e[kk], fx_exp_of(d));
+    fx_raise(&ln.e[kk], e);
     __syncthreads();
     const int E = ln.e[kk];
     unsigned mag = 0;
-    if (m < A) {
+#pragma unroll
+    for (int r = 0; r < RA; ++r) {
+        const int m = m0 + r * P;
+        if (m >= A) break;
         Fx2 v[INV ? Q : P];
 #pragma unroll
-        for (int n = 0; n < NIN; ++n) v[n] = cx<Fx>(fx_from<BIT>(d[n].x, E), fx_from<BIT>(d[n].y, E));
-        if constexpr (INV) mag = S::t_first(v, m, tw, tab);
-        else mag = S::template first<false, HALF_IN>(v, m, tw, tab);
+        for (int n = 0; n < NIN; ++n) v[n] = cx<Fx>(fx_from<BIT>(d[r][n].x, E), fx_from<BIT>(d[r][n].y, E));
+        if constexpr (INV) mag = max(mag, S::t_first(v, m, tw, tab));
+        else mag = max(mag, S::template first<false, HALF_IN>(v, m, tw, tab));
     }
     fx_raise(&ln.m[0][kk], (int)mag);
     __syncthreads();
-    if (m < B) {
-        const int sh = fx_room<INV ? P : Q>((unsigned)ln.m[0][kk]);
-        const FxOut o(E, BIT - sh);
+    const int sh = fx_room<INV ? P : Q>((unsigned)ln.m[0][kk]);
+    const FxOut o(E, BIT - sh);
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+        const int m = m0 + r * P;
+        if (m >= B) break;
         Fx2 u[INV ? P : Q];
         if constexpr (INV) S::t_second(u, m, tab, sh);
         else S::template second<false>(u, m, tab, sh);
@@ -118,6 +135,7 @@ __device__ __forceinline__ void xconv_fx(double2* __restrict__ W, const double* 
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ FxLines ln;
     FxW* tw = reinterpret_cast<FxW*>(smraw);
+    constexpr int RQ = (Q + P - 1) / P;  // rounds of the Q-item steps
     const int kk = threadIdx.x & (FX_COLS - 1), m = threadIdx.x / FX_COLS;
     Fx2* tab = reinterpret_cast<Fx2*>(tw + L) + kk * fx_tab(L);
     const int col = vb.x * FX_COLS + kk;
@@ -130,23 +148,32 @@ __device__ __forceinline__ void xconv_fx(double2* __restrict__ W, const double* 
     int E;
     unsigned mag = 0;
     {
-        double2 d[P / 2];
+        double2 d[RQ][P / 2];
 #pragma unroll
-        for (int n1 = 0; n1 < P / 2; ++n1) {
-            const int x = n1 * Q + m;
-            d[n1] = (x < nx && live) ? W[(size_t)x * ncol + col] : make_double2(0, 0);
-        }
+        for (int r = 0; r < RQ; ++r)
+#pragma unroll
+            for (int n1 = 0; n1 < P / 2; ++n1) {
+                const int x = n1 * Q + m + r * P;
+                d[r][n1] = (m + r * P < Q && x < nx && live) ? W[(size_t)x * ncol + col] : make_double2(0, 0);
+            }
         fx_clear(ln);
         load_twiddles<double>(reinterpret_cast<double2*>(tw), twg, L);
+        int e = 0;
+#pragma unroll
+        for (int r = 0; r < RQ; ++r) e = max(e, fx_exp_of(d[r]));
         __syncthreads();
-        fx_raise(&ln.e[kk], fx_exp_of(d));
+        fx_raise(&ln.e[kk], e);
         __syncthreads();
         E = ln.e[kk];
-        Fx2 v[P];
 #pragma unroll
-        for (int n1 = 0; n1 < P / 2; ++n1)
-            v[n1] = cx<Fx>(fx_from<S::B_HALF>(d[n1].x, E), fx_from<S::B_HALF>(d[n1].y, E));
-        mag = S::template first<false, HALF_IN>(v, m, tw, tab);
+        for (int r = 0; r < RQ; ++r) {
+            if (m + r * P >= Q) break;
+            Fx2 v[P];
+#pragma unroll
+            for (int n1 = 0; n1 < P / 2; ++n1)
+                v[n1] = cx<Fx>(fx_from<S::B_HALF>(d[r][n1].x, E), fx_from<S::B_HALF>(d[r][n1].y, E));
+            mag = max(mag, S::template first<false, HALF_IN>(v, m + r * P, tw, tab));
+        }
     }
     double g[Q];
     int eg = 0;
@@ -154,7 +181,7 @@ __device__ __forceinline__ void xconv_fx(double2* __restrict__ W, const double* 
     for (int k2 = 0; k2 < Q; ++k2) {
         const int kx = m + P * k2, gx = kx <= L - kx ? kx : L - kx;
         const long long gi = (long long)gx * KyKz + gk;
-        g[k2] = (m < P && live && SC_IDX_OK(st, 23, gi, (long long)(L / 2 + 1) * KyKz)) ? G[gi] : 0.0;
+        g[k2] = (live && SC_IDX_OK(st, 23, gi, (long long)(L / 2 + 1) * KyKz)) ? G[gi] : 0.0;
         eg = max(eg, fx_exp(g[k2]));
     }
     fx_raise(&ln.m[0][kk], (int)mag);
@@ -165,37 +192,37 @@ __device__ __forceinline__ void xconv_fx(double2* __restrict__ W, const double* 
     int sh = fx_room<Q>((unsigned)ln.m[0][kk]);
     int bit = S::B_HALF - sh;  // the bit of 2^E in what is held
     mag = 0;
-    if (m < P) {
-        S::template second<false>(u, m, tab, sh);
+    S::template second<false>(u, m, tab, sh);
 #pragma unroll
-        for (int k2 = 0; k2 < Q; ++k2) {
-            const long long gf = fx_from<61>(g[k2], EG).v;  // G / 2^(EG - 1023) in bits 61 and below
-            const FxC c((int)(gf >> 31), (int)(gf & 0x7fffffff));
-            u[k2] = cx<Fx>(fx_mul(u[k2].x, c), fx_mul(u[k2].y, c));
-            mag = max(mag, max(fx_mag(u[k2].x), fx_mag(u[k2].y)));
-        }
+    for (int k2 = 0; k2 < Q; ++k2) {
+        const long long gf = fx_from<61>(g[k2], EG).v;  // G / 2^(EG - 1023) in bits 61 and below
+        const FxC c((int)(gf >> 31), (int)(gf & 0x7fffffff));
+        u[k2] = cx<Fx>(fx_mul(u[k2].x, c), fx_mul(u[k2].y, c));
+        mag = max(mag, max(fx_mag(u[k2].x), fx_mag(u[k2].y)));
     }
     // value = held * 2^(E - 1023 - bit) * 2^(EG - 1023 + 1)
     fx_raise(&ln.m[1][kk], (int)mag);
     __syncthreads();
     sh = fx_room<Q>((unsigned)ln.m[1][kk]);
     bit -= sh;
-    mag = 0;
-    if (m < P) {
 #pragma unroll
-        for (int k2 = 0; k2 < Q; ++k2) u[k2] = fx_down(u[k2], sh);
-        mag = S::t_first(u, m, tw, tab);  // over the row of the table that this thread has read
-    }
+    for (int k2 = 0; k2 < Q; ++k2) u[k2] = fx_down(u[k2], sh);
+    mag = S::t_first(u, m, tw, tab);  // over the row of the table that this thread has read
     fx_raise(&ln.m[2][kk], (int)mag);
     __syncthreads();
     sh = fx_room<P>((unsigned)ln.m[2][kk]);
     const FxOut o(E == FX_BAD || EG == FX_BAD ? FX_BAD : E, bit - sh - (EG - 1022));
-    Fx2 w[P];
-    S::t_second(w, m, tab, sh);
 #pragma unroll
-    for (int k1 = 0; k1 < P / 2; ++k1) {
-        const int x = k1 * Q + m;
-        if (live && x < nx) W[(size_t)x * ncol + col] = make_double2(fx_to(w[k1].x, o), fx_to(w[k1].y, o));
+    for (int r = 0; r < RQ; ++r) {
+        const int k2 = m + r * P;
+        if (k2 >= Q) break;
+        Fx2 w[P];
+        S::t_second(w, k2, tab, sh);
+#pragma unroll
+        for (int k1 = 0; k1 < P / 2; ++k1) {
+            const int x = k1 * Q + k2;
+            if (live && x < nx) W[(size_t)x * ncol + col] = make_double2(fx_to(w[k1].x, o), fx_to(w[k1].y, o));
+        }
     }
 }
 
