@@ -15,10 +15,10 @@
 // Each radix pass is three launches with no inter-block waiting:
 //   hist     per-block digit histogram of a tile of 256, 1024 or 4096 keys -> hist[digit][block]
 //   rowscan  one warp per digit: exclusive scan along the blocks, digit totals
-//   scatter  per block: digit bases from the totals, then 1, 4 or 16 rounds of 256 keys,
-//            ranking equal digits within a warp by __match_any_sync and across
-//            warps by a per-digit prefix in shared memory (stable order:
-//            round, warp, lane = particle order)
+//   scatter  per block: digit bases from the totals; each warp ranks the equal
+//            digits of its 1, 4 or 16 rounds of 32 keys by __match_any_sync and
+//            a count row, the warps are joined by a per-digit prefix in shared
+//            memory (stable order: warp, round, lane = particle order)
 #include "sc_common.cuh"
 
 namespace ocsc {
@@ -69,82 +69,103 @@ __global__ void k_rrowscan(uint32_t* __restrict__ hist, int nblk, int bins, uint
     if (lane == 0) tot[warp] = carry;
 }
 
+// Stable scatter of a block's RT * ITEMS keys, warp w the ITEMS rounds of 32 keys
+// from w * 32 * ITEMS on.  A warp ranks its keys alone, round after round, in
+// its own row of digit counts (the lanes of one digit found by a match, one of
+// them adds for all); then one scan over the warps' rows, and every key
+// knows its place.  Bound by latency: three barriers a block and the loads at
+// its start, all issued before the first of them.  (Rounds of RT keys with a
+// clear and a scan of the 512-digit table behind four barriers each, and the digit
+// bases scanned by one warp in 16 dependent steps, took 45 and 71 us for the two
+// passes of 2M keys, 13 a pass of 200k and 6.3 of 10k; this 42 and 60, 8 and 4.)
+template <int ITEMS>
 __global__ void __launch_bounds__(RT) k_rscatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                  int64_t n, int shift, int bins, const uint32_t* __restrict__ hist,
                                                  const uint32_t* __restrict__ tot, uint32_t* __restrict__ kout,
                                                  uint32_t* __restrict__ vout, const double* __restrict__ qsrc,
-                                                 void* __restrict__ qout, int qfloat, int items) {
+                                                 void* __restrict__ qout, int qfloat) {
     pdl_wait();
+    static_assert(RBINS == 2 * RT, "two digits per thread");
     __shared__ uint32_t base[RBINS];
     __shared__ uint32_t wc[RWARPS][RBINS];
+    __shared__ uint32_t wtot[RWARPS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // exclusive scan of the digit totals (at most 512, by warp 0) plus this
-    // block's offset within each digit -> where the block's keys of a digit go
-    if (warp == 0) {
-        uint32_t carry = 0;
-        for (int d0 = 0; d0 < bins; d0 += 32) {
-            const int d = d0 + lane;
-            const uint32_t v = d < bins ? tot[d] : 0u;
-            uint32_t inc = v;
+    const int64_t i0 = (int64_t)blockIdx.x * RT * ITEMS + warp * 32 * ITEMS + lane;
+    const uint32_t mask = (uint32_t)bins - 1;
+    uint32_t key[ITEMS], val[ITEMS], rk[ITEMS];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(FULLM, inc, o);
-                if (lane >= o) inc += t;
-            }
-            if (d < bins) base[d] = carry + inc - v + hist[(size_t)d * gridDim.x + blockIdx.x];
-            carry += __shfl_sync(FULLM, inc, 31);
+    for (int r = 0; r < ITEMS; ++r) {
+        const int64_t i = i0 + 32 * r;
+        key[r] = i < n ? kin[i] : 0u;
+        val[r] = i < n ? (vin ? vin[i] : (uint32_t)i) : 0u;
+    }
+    // exclusive scan of the digit totals plus this block's offset within each
+    // digit -> where the block's keys of a digit go
+    const int d0 = 2 * tid;
+    const uint32_t t0 = d0 < bins ? tot[d0] : 0u, t1 = d0 + 1 < bins ? tot[d0 + 1] : 0u;
+    const uint32_t h0 = d0 < bins ? hist[(size_t)d0 * gridDim.x + blockIdx.x] : 0u;
+    const uint32_t h1 = d0 + 1 < bins ? hist[(size_t)(d0 + 1) * gridDim.x + blockIdx.x] : 0u;
+#pragma unroll
+    for (int w = 0; w < RWARPS; ++w) wc[w][tid] = wc[w][tid + RT] = 0u;
+    uint32_t inc = t0 + t1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(FULLM, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) wtot[warp] = inc;
+    __syncthreads();
+    uint32_t before = inc - t0 - t1;
+    for (int w = 0; w < warp; ++w) before += wtot[w];
+    base[d0] = before + h0;
+    base[d0 + 1] = before + t0 + h1;
+    const uint32_t lt = (1u << lane) - 1u;
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const bool valid = i0 + 32 * r < n;
+        const uint32_t d = valid ? ((key[r] >> shift) & mask) : (uint32_t)RBINS;
+        const uint32_t peers = __match_any_sync(FULLM, d);
+        const uint32_t rank = __popc(peers & lt);
+        uint32_t old = 0u;
+        if (valid && rank == 0) {
+            old = wc[warp][d];
+            wc[warp][d] = old + __popc(peers);
+        }
+        rk[r] = rank + __shfl_sync(FULLM, old, __ffs(peers) - 1);
+        __syncwarp();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        const int dd = tid + j * RT;
+        uint32_t run = base[dd];
+#pragma unroll
+        for (int w = 0; w < RWARPS; ++w) {
+            const uint32_t c = wc[w][dd];
+            wc[w][dd] = run;
+            run += c;
         }
     }
     __syncthreads();
-    const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t mask = (uint32_t)bins - 1;
-    const int64_t tile = (int64_t)blockIdx.x * RT * items;
-    for (int r = 0; r < items; ++r) {
-        const int64_t i = tile + (int64_t)r * RT + tid;
-        const bool valid = i < n;
-        const uint32_t key = valid ? kin[i] : 0u;
-        const uint32_t val = valid ? (vin ? vin[i] : (uint32_t)i) : 0u;
-        const uint32_t d = valid ? ((key >> shift) & mask) : (uint32_t)RBINS;
-        for (int dd = tid; dd < bins; dd += RT)
 #pragma unroll
-            for (int w = 0; w < RWARPS; ++w) wc[w][dd] = 0u;
-        __syncthreads();
-        const uint32_t peers = __match_any_sync(FULLM, d);
-        const uint32_t rank = __popc(peers & lt);
-        if (valid && rank == 0) wc[warp][d] = __popc(peers);
-        __syncthreads();
-        for (int dd = tid; dd < bins; dd += RT) {
-            uint32_t run = base[dd];
-#pragma unroll
-            for (int w = 0; w < RWARPS; ++w) {
-                const uint32_t c = wc[w][dd];
-                wc[w][dd] = run;
-                run += c;
-            }
-            base[dd] = run;
+    for (int r = 0; r < ITEMS; ++r) {
+        if (i0 + 32 * r >= n) continue;
+        const uint32_t pos = wc[warp][(key[r] >> shift) & mask] + rk[r];
+        kout[pos] = key[r];
+        if (qsrc) {  // last pass of the deposit: carry the charge itself
+            const double qv = qsrc[val[r]];
+            if (qfloat) static_cast<float*>(qout)[pos] = (float)qv;
+            else static_cast<double*>(qout)[pos] = qv;
+        } else {
+            vout[pos] = val[r];
         }
-        __syncthreads();
-        if (valid) {
-            const uint32_t pos = wc[warp][d] + rank;
-            kout[pos] = key;
-            if (qsrc) {  // last pass of the deposit: carry the charge itself
-                const double qv = qsrc[val];
-                if (qfloat) static_cast<float*>(qout)[pos] = (float)qv;
-                else static_cast<double*>(qout)[pos] = qv;
-            } else {
-                vout[pos] = val;
-            }
-        }
-        __syncthreads();
     }
 }
 
-// Rounds of RT keys per block: every round pays a clear and a scan of the
-// digit table behind four barriers whatever its size, so small sorts take
-// one or four rounds per block (more blocks in parallel) and large ones 16
-// (fewer digit-table rows for the scans).  The stable order, and so the
-// result, does not depend on the tiling.
-static int sort_items(int64_t n) { return n <= (1 << 18) ? 1 : (n <= (1 << 20) ? 4 : RITEMS); }
+// Rounds of RT keys per block: small sorts take one or four (more blocks in
+// parallel), large ones 16 (fewer digit-table rows for the scans).  The stable
+// order, and so the result, does not depend on the tiling.
+static int sort_items(int64_t n) { return n <= (1 << 16) ? 1 : (n <= (1 << 19) ? 4 : RITEMS); }
 int sort_blocks(int64_t n) {
     const int64_t t = (int64_t)RT * sort_items(n);
     return (int)((n + t - 1) / t);
@@ -154,7 +175,9 @@ cudaError_t prepare_sort_kernels() {
     cudaError_t e;
     if ((e = prefer_shared(k_rhist))) return e;
     if ((e = prefer_shared(k_rrowscan))) return e;
-    return prefer_shared(k_rscatter);
+    if ((e = prefer_shared(k_rscatter<1>))) return e;
+    if ((e = prefer_shared(k_rscatter<4>))) return e;
+    return prefer_shared(k_rscatter<RITEMS>);
 }
 
 int sort_passes(int key_bits) { return key_bits <= 0 ? 1 : (key_bits + RMAXBITS - 1) / RMAXBITS; }
@@ -185,8 +208,9 @@ cudaError_t launch_sort(const uint32_t* keys_in, int64_t n, int key_bits, uint32
         launch(k_rhist, nb, RT, 0, s, sk, n, shift, bins, hist, items);
         launch(k_rrowscan, (bins * 32 + 255) / 256, 256, 0, s, hist, nb, bins, tot);
         const bool last = p == passes - 1;
-        launch(k_rscatter, nb, RT, 0, s, sk, sv, n, shift, bins, hist, tot, dk, dv, last ? q_src : nullptr,
-                                     last ? q_out : nullptr, q_float ? 1 : 0, items);
+        auto* scatter = items == 1 ? k_rscatter<1> : (items == 4 ? k_rscatter<4> : k_rscatter<RITEMS>);
+        launch(scatter, nb, RT, 0, s, sk, sv, n, shift, bins, hist, tot, dk, dv, last ? q_src : nullptr,
+               last ? q_out : nullptr, q_float ? 1 : 0);
         sk = dk;
         sv = dv;
         to_out = !to_out;
