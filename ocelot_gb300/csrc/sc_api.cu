@@ -141,10 +141,9 @@ Layout make_layout(const Plan& p, int64_t n) {
     // the radix sort's buffers: only the sorted deposit uses them
     const size_t ns = p.sorted_deposit ? (size_t)n : 0;
     L.sort_keys = take(4 * ns);
-    L.sort_perm = take(4 * ns);
     L.sort_q = take(rs * ns);
     L.sort_tmp_k = take(4 * ns);
-    L.sort_tmp_v = take(4 * ns);
+    L.sort_tmp_q = take(rs * ns);
     const size_t sb = ns ? (size_t)sort_blocks((int64_t)ns) : 1;
     L.sort_hist = take(p.sorted_deposit ? 4 * 512 * sb : 0);
     L.sort_tot = take(p.sorted_deposit ? 4 * 512 : 0);
@@ -651,11 +650,7 @@ int sc_kick(sc_plan* plan, void* ws_v, size_t ws_bytes, double* rp, int64_t ld, 
     SC_CUDA(launch_keys(p, L, ws, kp, rp, p.sorted_deposit ? nullptr : q, s, p.prec == SC_FP32), "keys");
     mark(plan, 3, s);
     if (p.sorted_deposit) {
-        SC_CUDA(launch_sort(reinterpret_cast<uint32_t*>(ws + L.keys), n, p.key_bits, reinterpret_cast<uint32_t*>(ws + L.sort_keys),
-                            reinterpret_cast<uint32_t*>(ws + L.sort_perm), reinterpret_cast<uint32_t*>(ws + L.sort_tmp_k),
-                            reinterpret_cast<uint32_t*>(ws + L.sort_tmp_v), reinterpret_cast<uint32_t*>(ws + L.sort_hist),
-                            reinterpret_cast<uint32_t*>(ws + L.sort_tot), s, q, ws + L.sort_q, p.prec == SC_FP32),
-                "sort");
+        SC_CUDA(launch_charge_sort(p, L, ws, q, n, s), "sort");
         mark(plan, 4, s);
         SC_CUDA(launch_deposit(p, L, ws, q, n, s), "deposit");
     } else {
@@ -700,11 +695,7 @@ int sc_el_field(sc_plan* plan, void* ws_v, size_t ws_bytes, double* X, const dou
     SC_CUDA(launch_extent_xyz(p, L, ws, kp, X, q, gamma, s), "extent");
     SC_CUDA(launch_keys(p, L, ws, kp, nullptr, p.sorted_deposit ? nullptr : q, s), "keys");
     if (p.sorted_deposit) {
-        SC_CUDA(launch_sort(reinterpret_cast<uint32_t*>(ws + L.keys), n, p.key_bits, reinterpret_cast<uint32_t*>(ws + L.sort_keys),
-                            reinterpret_cast<uint32_t*>(ws + L.sort_perm), reinterpret_cast<uint32_t*>(ws + L.sort_tmp_k),
-                            reinterpret_cast<uint32_t*>(ws + L.sort_tmp_v), reinterpret_cast<uint32_t*>(ws + L.sort_hist),
-                            reinterpret_cast<uint32_t*>(ws + L.sort_tot), s, q, ws + L.sort_q, p.prec == SC_FP32),
-                "sort");
+        SC_CUDA(launch_charge_sort(p, L, ws, q, n, s), "sort");
         SC_CUDA(launch_deposit(p, L, ws, q, n, s), "deposit");
     }
     SC_CUDA(launch_igf(p, L, ws, s), "igf");

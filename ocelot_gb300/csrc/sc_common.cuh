@@ -169,7 +169,7 @@ struct Layout {
     size_t part_frame, part_ext;                 // per-block partial sums (double)
     size_t X;                                    // 3 x n: lab positions (FP32) of a kick, grid coordinates (R) of el_field
     size_t lab;                                  // FP64: 4 x n: lab position and longitudinal momentum of a kick
-    size_t keys, sort_keys, sort_perm, sort_q, sort_tmp_k, sort_tmp_v, sort_hist, sort_tot;
+    size_t keys, sort_keys, sort_q, sort_tmp_k, sort_tmp_q, sort_hist, sort_tot;
     size_t qgrid, phi, ex, ey, ez;               // [nx][ny][nz] (R)
     size_t exq, eyq, ezq;                        // FP32 form: [nx][ny][nz] gather octs (8 floats, 32-byte aligned)
     size_t cell_start, cell_end;                 // [nx*ny*nz] uint32 run bounds (adjacent)
@@ -241,10 +241,10 @@ int sort_blocks(int64_t n);  // blocks of a sort of n keys (rows of its digit hi
 int sort_passes(int key_bits);
 // With q_src set, the last pass writes q_src[index] (as double or float) into
 // q_out instead of the permutation.
-cudaError_t launch_sort(const uint32_t* keys_in, int64_t n, int key_bits, uint32_t* keys_out,
-                        uint32_t* perm_out, uint32_t* tmp_k, uint32_t* tmp_v, uint32_t* hist,
-                        uint32_t* tot, cudaStream_t s, const double* q_src = nullptr, void* q_out = nullptr,
-                        bool q_float = false);
+cudaError_t launch_sort(const uint32_t* keys_in, int64_t n, int key_bits, uint32_t* keys_out, uint32_t* perm_out,
+                        uint32_t* tmp_k, uint32_t* tmp_v, uint32_t* hist, uint32_t* tot, cudaStream_t s);
+// the kick's keys, the charges (as R) travelling with them
+cudaError_t launch_charge_sort(const Plan& p, const Layout& L, char* ws, const double* q, int64_t n, cudaStream_t s);
 cudaError_t launch_deposit(const Plan& p, const Layout& L, char* ws, const double* q, int64_t n,
                            cudaStream_t s);
 

@@ -19,6 +19,8 @@
 //            digits of its 1, 4 or 16 rounds of 32 keys by __match_any_sync and
 //            a count row, the warps are joined by a per-digit prefix in shared
 //            memory (stable order: warp, round, lane = particle order)
+#include <type_traits>
+
 #include "sc_common.cuh"
 
 namespace ocsc {
@@ -77,27 +79,42 @@ __global__ void k_rrowscan(uint32_t* __restrict__ hist, int nblk, int bins, uint
 // its start, all issued before the first of them.  (Rounds of RT keys with a
 // clear and a scan of the 512-digit table behind four barriers each, and the digit
 // bases scanned by one warp in 16 dependent steps, took 45 and 71 us for the two
-// passes of 2M keys, 13 a pass of 200k and 6.3 of 10k; this 42 and 60, 8 and 4.)
-template <int ITEMS>
-__global__ void __launch_bounds__(RT) k_rscatter(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                                                 int64_t n, int shift, int bins, const uint32_t* __restrict__ hist,
-                                                 const uint32_t* __restrict__ tot, uint32_t* __restrict__ kout,
-                                                 uint32_t* __restrict__ vout, const double* __restrict__ qsrc,
-                                                 void* __restrict__ qout, int qfloat) {
+// passes of 2M keys, 13 a pass of 200k and 6.3 of 10k; this 42 and 60, 8 and 4;
+// with the charges travelling and STAGE 38 and 30, 7.3 and 3.2.)
+//
+// V: what travels with the keys -- the particle index (a sort's permutation) or, for
+// the deposit, the charge itself from the first pass on, read and written in
+// order (the last pass used to gather it by index: 2M random 8-byte reads).
+// vin == nullptr (the first pass): the index, or the charge qsrc[i].
+// STAGE: the keys and values are put in digit order in shared memory first and
+// leave in runs, eight of a digit in a tile of 4096; written where each thread
+// has them, every 4 bytes are a sector of their own.
+template <int ITEMS, typename V>
+__global__ void __launch_bounds__(RT) k_rscatter(const uint32_t* __restrict__ kin, const V* __restrict__ vin,
+                                                 const double* __restrict__ qsrc, int64_t n, int shift, int bins,
+                                                 const uint32_t* __restrict__ hist, const uint32_t* __restrict__ tot,
+                                                 uint32_t* __restrict__ kout, V* __restrict__ vout) {
     pdl_wait();
     static_assert(RBINS == 2 * RT, "two digits per thread");
+    constexpr bool STAGE = ITEMS >= 16;
+    constexpr size_t WC = sizeof(uint32_t) * RWARPS * RBINS, ST = STAGE ? RT * ITEMS * sizeof(V) : 0;
     __shared__ uint32_t base[RBINS];
-    __shared__ uint32_t wc[RWARPS][RBINS];
+    __shared__ __align__(16) unsigned char raw[WC > ST ? WC : ST];
     __shared__ uint32_t wtot[RWARPS];
+    uint32_t(*wc)[RBINS] = reinterpret_cast<uint32_t(*)[RBINS]>(raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t i0 = (int64_t)blockIdx.x * RT * ITEMS + warp * 32 * ITEMS + lane;
     const uint32_t mask = (uint32_t)bins - 1;
-    uint32_t key[ITEMS], val[ITEMS], rk[ITEMS];
+    uint32_t key[ITEMS], rk[ITEMS];
+    V val[ITEMS];
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
         const int64_t i = i0 + 32 * r;
         key[r] = i < n ? kin[i] : 0u;
-        val[r] = i < n ? (vin ? vin[i] : (uint32_t)i) : 0u;
+        if (i >= n) val[r] = V(0);
+        else if (vin) val[r] = vin[i];
+        else if constexpr (std::is_same<V, uint32_t>::value) val[r] = (V)i;
+        else val[r] = (V)qsrc[i];
     }
     // exclusive scan of the digit totals plus this block's offset within each
     // digit -> where the block's keys of a digit go
@@ -135,28 +152,73 @@ __global__ void __launch_bounds__(RT) k_rscatter(const uint32_t* __restrict__ ki
         __syncwarp();
     }
     __syncthreads();
+    uint32_t cnt[2];  // the block's keys of this thread's two digits
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-        const int dd = tid + j * RT;
-        uint32_t run = base[dd];
+        uint32_t run = STAGE ? 0u : base[d0 + j];
 #pragma unroll
         for (int w = 0; w < RWARPS; ++w) {
-            const uint32_t c = wc[w][dd];
-            wc[w][dd] = run;
+            const uint32_t c = wc[w][d0 + j];
+            wc[w][d0 + j] = run;
             run += c;
         }
+        cnt[j] = run;
+    }
+    if constexpr (STAGE) {  // digit starts within the tile
+        uint32_t in = cnt[0] + cnt[1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(FULLM, in, o);
+            if (lane >= o) in += t;
+        }
+        if (lane == 31) wtot[warp] = in;
+        __syncthreads();
+        uint32_t start = in - cnt[0] - cnt[1];
+        for (int w = 0; w < warp; ++w) start += wtot[w];
+#pragma unroll
+        for (int w = 0; w < RWARPS; ++w) {
+            wc[w][d0] += start;
+            wc[w][d0 + 1] += start + cnt[0];
+        }
+        base[d0] -= start;  // + the place in the tile: the place in the output (mod 2^32)
+        base[d0 + 1] -= start + cnt[0];
     }
     __syncthreads();
+    if constexpr (STAGE) {
+        const int64_t left = n - (int64_t)blockIdx.x * RT * ITEMS;
+        const int m = left < RT * ITEMS ? (int)left : RT * ITEMS;
 #pragma unroll
-    for (int r = 0; r < ITEMS; ++r) {
-        if (i0 + 32 * r >= n) continue;
-        const uint32_t pos = wc[warp][(key[r] >> shift) & mask] + rk[r];
-        kout[pos] = key[r];
-        if (qsrc) {  // last pass of the deposit: carry the charge itself
-            const double qv = qsrc[val[r]];
-            if (qfloat) static_cast<float*>(qout)[pos] = (float)qv;
-            else static_cast<double*>(qout)[pos] = qv;
-        } else {
+        for (int r = 0; r < ITEMS; ++r) rk[r] += wc[warp][(key[r] >> shift) & mask];
+        __syncthreads();  // the counts are done with
+        uint32_t* sk = reinterpret_cast<uint32_t*>(raw);
+        V* sv = reinterpret_cast<V*>(raw);
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+            if (i0 + 32 * r < n) sk[rk[r]] = key[r];
+        __syncthreads();
+        uint32_t pos[ITEMS];
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            const int j = r * RT + tid;
+            if (j >= m) continue;
+            const uint32_t kk = sk[j];
+            pos[r] = base[(kk >> shift) & mask] + (uint32_t)j;
+            kout[pos[r]] = kk;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+            if (i0 + 32 * r < n) sv[rk[r]] = val[r];
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+            if (r * RT + tid < m) vout[pos[r]] = sv[r * RT + tid];
+    } else {
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r) {
+            if (i0 + 32 * r >= n) continue;
+            const uint32_t pos = wc[warp][(key[r] >> shift) & mask] + rk[r];
+            kout[pos] = key[r];
             vout[pos] = val[r];
         }
     }
@@ -175,9 +237,15 @@ cudaError_t prepare_sort_kernels() {
     cudaError_t e;
     if ((e = prefer_shared(k_rhist))) return e;
     if ((e = prefer_shared(k_rrowscan))) return e;
-    if ((e = prefer_shared(k_rscatter<1>))) return e;
-    if ((e = prefer_shared(k_rscatter<4>))) return e;
-    return prefer_shared(k_rscatter<RITEMS>);
+    auto all = [&](auto v) -> cudaError_t {
+        using V = decltype(v);
+        if ((e = prefer_shared(k_rscatter<1, V>))) return e;
+        if ((e = prefer_shared(k_rscatter<4, V>))) return e;
+        return prefer_shared(k_rscatter<RITEMS, V>);
+    };
+    if ((e = all(0.0))) return e;
+    if ((e = all(0.0f))) return e;
+    return all(0u);
 }
 
 int sort_passes(int key_bits) { return key_bits <= 0 ? 1 : (key_bits + RMAXBITS - 1) / RMAXBITS; }
@@ -188,15 +256,15 @@ size_t sort_scratch_bytes(int64_t n, int key_bits) {
     return align_up(4 * (size_t)n) * 2 + align_up((size_t)RBINS * nb * 4) + align_up((size_t)RBINS * 4);
 }
 
-cudaError_t launch_sort(const uint32_t* keys_in, int64_t n, int key_bits, uint32_t* keys_out, uint32_t* perm_out,
-                        uint32_t* tmp_k, uint32_t* tmp_v, uint32_t* hist, uint32_t* tot, cudaStream_t s,
-                        const double* q_src, void* q_out, bool q_float) {
+template <typename V>
+static cudaError_t sort_t(const uint32_t* keys_in, int64_t n, int key_bits, uint32_t* keys_out, V* vals_out,
+                          uint32_t* tmp_k, V* tmp_v, uint32_t* hist, uint32_t* tot, cudaStream_t s, const double* q_src) {
     if (n <= 0) return cudaSuccess;
     const int nb = sort_blocks(n), items = sort_items(n);
     const int passes = sort_passes(key_bits);
     const int width = key_bits <= 0 ? 1 : (key_bits + passes - 1) / passes;  // <= RMAXBITS
     const uint32_t* sk = keys_in;
-    const uint32_t* sv = nullptr;
+    const V* sv = nullptr;
     bool to_out = (passes % 2) == 1;
     for (int p = 0; p < passes; ++p) {
         const int shift = width * p;
@@ -204,18 +272,31 @@ cudaError_t launch_sort(const uint32_t* keys_in, int64_t n, int key_bits, uint32
         dbits = dbits > width ? width : (dbits < 1 ? 1 : dbits);
         const int bins = 1 << dbits;
         uint32_t* dk = to_out ? keys_out : tmp_k;
-        uint32_t* dv = to_out ? perm_out : tmp_v;
+        V* dv = to_out ? vals_out : tmp_v;
         launch(k_rhist, nb, RT, 0, s, sk, n, shift, bins, hist, items);
         launch(k_rrowscan, (bins * 32 + 255) / 256, 256, 0, s, hist, nb, bins, tot);
-        const bool last = p == passes - 1;
-        auto* scatter = items == 1 ? k_rscatter<1> : (items == 4 ? k_rscatter<4> : k_rscatter<RITEMS>);
-        launch(scatter, nb, RT, 0, s, sk, sv, n, shift, bins, hist, tot, dk, dv, last ? q_src : nullptr,
-               last ? q_out : nullptr, q_float ? 1 : 0);
+        auto* scatter = items == 1 ? k_rscatter<1, V> : (items == 4 ? k_rscatter<4, V> : k_rscatter<RITEMS, V>);
+        launch(scatter, nb, RT, 0, s, sk, sv, q_src, n, shift, bins, hist, tot, dk, dv);
         sk = dk;
         sv = dv;
         to_out = !to_out;
     }
     return cudaGetLastError();
+}
+
+cudaError_t launch_sort(const uint32_t* keys_in, int64_t n, int key_bits, uint32_t* keys_out, uint32_t* perm_out,
+                        uint32_t* tmp_k, uint32_t* tmp_v, uint32_t* hist, uint32_t* tot, cudaStream_t s) {
+    return sort_t<uint32_t>(keys_in, n, key_bits, keys_out, perm_out, tmp_k, tmp_v, hist, tot, s, nullptr);
+}
+
+cudaError_t launch_charge_sort(const Plan& p, const Layout& L, char* ws, const double* q, int64_t n, cudaStream_t s) {
+    auto u32 = [&](size_t o) { return reinterpret_cast<uint32_t*>(ws + o); };
+    auto run = [&](auto v) {
+        using V = decltype(v);
+        return sort_t<V>(u32(L.keys), n, p.key_bits, u32(L.sort_keys), reinterpret_cast<V*>(ws + L.sort_q),
+                         u32(L.sort_tmp_k), reinterpret_cast<V*>(ws + L.sort_tmp_q), u32(L.sort_hist), u32(L.sort_tot), s, q);
+    };
+    return p.prec == SC_FP64 ? run(0.0) : run(0.0f);
 }
 
 // Cell bounds of the sorted runs: start[key] and end[key] (both 0 for an
