@@ -317,7 +317,10 @@ __global__ void k_cell_bounds(const uint32_t* __restrict__ sk, int64_t n, uint32
 // strictly sequential left fold in particle order from 0 -- np.bincount's
 // summation (sc.py:193), bit for bit.  (One warp per cell with every lane
 // folding the same shuffled values spent 32 lanes of this GPU's narrow FP64
-// pipe per addition: 370 us per 2M particles.)  FP32: one warp per cell,
+// pipe per addition: 370 us per 2M particles.)  Bound by the fullest cells, some 500
+// dependent additions and their loads: 16 loads at a time instead of 4 take 56 -> 44 us
+// at 2M / 64^3; loads kept ahead of the additions with predicated tails cost the
+// many short cells more than that.  FP32: one warp per cell,
 // lane-strided Kahan sums combined by a fixed shuffle tree with error-free
 // (two-sum) additions.  Empty cells get 0, so no memset of the grid.
 __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
@@ -338,7 +341,14 @@ __global__ void __launch_bounds__(256) k_deposit_cells(const R* __restrict__ sq,
             const uint32_t b = start[c], e = end[c];
             double sum = 0.0;
             uint32_t k = b;
-            for (; k + 4 <= e; k += 4) {  // four loads in flight, the additions in order
+            for (; k + 16 <= e; k += 16) {  // 16 loads in flight, the additions in order
+                double v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) v[u] = sq[k + u];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) sum = __dadd_rn(sum, v[u]);
+            }
+            for (; k + 4 <= e; k += 4) {
                 const double v0 = sq[k], v1 = sq[k + 1], v2 = sq[k + 2], v3 = sq[k + 3];
                 sum = __dadd_rn(__dadd_rn(__dadd_rn(__dadd_rn(sum, v0), v1), v2), v3);
             }
