@@ -81,6 +81,7 @@ struct ScState {
     unsigned int igf_next;       // corners of the exact IGF table claimed (reset with the mesh)
     int phi_exp;                 // FP64: largest biased exponent of the potential (reset with the mesh)
     double escale[3];            // FP64 kick: the field per unit of the fixed-point differences
+    double Tke[3][3];            // Tk for fields in those units
     int frame_timeout;           // a frame block's bulk-copy wait gave up (the finalize reports it)
     int check_code;              // checked builds: first failed index check (kernel code)
     int first_error;             // first non-OK status of any kick since sc_workspace_init

@@ -618,8 +618,13 @@ __global__ void k_field_grids(const double* __restrict__ phi, double* __restrict
     const double rx = st->isteps[0], ry = st->isteps[1], rz = st->isteps[2];
     const int E = st->phi_exp;
     const size_t ncell = (size_t)nx * ny * nz;
-    if (fe && i == 0 && j == 0 && threadIdx.x < 3)
-        st->escale[threadIdx.x] = E == FX_BAD ? NAN : ldexp(st->isteps[threadIdx.x], E - 1023 - FX_PHI);
+    if (fe && i == 0 && j == 0 && threadIdx.x < 3) {
+        const int a = threadIdx.x;
+        const double sc = E == FX_BAD ? NAN : ldexp(st->isteps[a], E - 1023 - FX_PHI);
+        st->escale[a] = sc;
+        for (int b = 0; b < 3; ++b)
+            st->Tke[b][a] = E == FX_BAD ? NAN : ldexp(st->Tk[b][a] * st->isteps[a], E - 1023 - FX_PHI);
+    }
     auto over = [](double a, double h, double r) {
         const double q = a * r;
         return fma(fma(-q, h, a), r, q);

@@ -1877,28 +1877,28 @@ __device__ __forceinline__ AxisFx axis_fx(double X, int n) {
 }
 __device__ __forceinline__ Fx lerp_fx(long long a, long long b, FxC t) { return Fx{a} + fx_mul(Fx{b - a}, t); }
 __device__ __forceinline__ double sample_fx(const long long* __restrict__ F, int i, int j, int k, FxC tx, FxC ty,
-                                            FxC tz, int ny, int nz, bool ok, double scale) {
+                                            FxC tz, int ny, int nz, bool ok) {
     const long long* b = F + ((size_t)i * ny + j) * nz + k;
     const size_t sx = (size_t)ny * nz;
     const Fx y0 = lerp_fx(lerp_fx(b[0], b[1], tz).v, lerp_fx(b[nz], b[nz + 1], tz).v, ty);
     const Fx y1 = lerp_fx(lerp_fx(b[sx], b[sx + 1], tz).v, lerp_fx(b[sx + nz], b[sx + nz + 1], tz).v, ty);
-    return ok ? fx_double(lerp_fx(y0.v, y1.v, tx)) * scale : 0.0;
+    return ok ? fx_double(lerp_fx(y0.v, y1.v, tx)) : 0.0;
 }
 __device__ __forceinline__ void gather_fx(const long long* __restrict__ fe, int nx, int ny, int nz,
-                                          const double (&X)[3], const ScState* st, double (&e)[3]) {
+                                          const double (&X)[3], double (&e)[3]) {
     const AxisFx x = axis_fx(X[0], nx), y = axis_fx(X[1], ny), z = axis_fx(X[2], nz);
     const size_t nc = (size_t)nx * ny * nz;
-    e[0] = sample_fx(fe, x.ia, y.ib, z.ib, x.ta, y.tb, z.tb, ny, nz, x.oka && y.okb && z.okb, st->escale[0]);
-    e[1] = sample_fx(fe + nc, x.ib, y.ia, z.ib, x.tb, y.ta, z.tb, ny, nz, x.okb && y.oka && z.okb, st->escale[1]);
-    e[2] = sample_fx(fe + 2 * nc, x.ib, y.ib, z.ia, x.tb, y.tb, z.ta, ny, nz, x.okb && y.okb && z.oka, st->escale[2]);
+    e[0] = sample_fx(fe, x.ia, y.ib, z.ib, x.ta, y.tb, z.tb, ny, nz, x.oka && y.okb && z.okb);
+    e[1] = sample_fx(fe + nc, x.ib, y.ia, z.ib, x.tb, y.ta, z.tb, ny, nz, x.okb && y.oka && z.okb);
+    e[2] = sample_fx(fe + 2 * nc, x.ib, y.ib, z.ia, x.tb, y.tb, z.ta, ny, nz, x.okb && y.okb && z.oka);
 }
 
-// Gather + kick of the FP64 form.  Bound by the FP64 pipe, 51 instructions per
+// Gather + kick of the FP64 form.  Bound by the FP64 pipe, 48 instructions per
 // particle (the gather's 48 run as integers beside them, gather_fx: 2M / 64^3
 // 460 -> 287 us, 200k / 63^3 51 -> 37; the lab position and momentum come from
 // the frame pass, 32 bytes a particle instead of 22 instructions: 287 -> 234 and
-// 37 -> 30), in units of the reference momentum (mad64):
-//   p' = p + Tk e   (Tk: the frame's rotation with the kick's factors, so the
+// 37 -> 30; Tke takes the integers as they are), in units of the reference momentum (mad64):
+//   p' = p + Tke e  (Tke: the frame's rotation with the kick's factors, so the
 //                    rotation into the frame and back is done once, on e)
 //   e' = sqrt(|p'|^2 + (m c / pref)^2),  w = -z_lab / pz'
 //   tau' = w e',  x = x_lab + x' w,  delta' = delta + (|p'|^2 - |p|^2) / (e + e')
@@ -1922,7 +1922,7 @@ __global__ void __launch_bounds__(KICK64_THREADS, 4) k_kick64(double* __restrict
     for (int i = 0; i < 3; ++i)
         for (int j = 0; j < 3; ++j) {
             Tg[i][j] = st->Tg[i][j];
-            Tk[i][j] = st->Tk[i][j];
+            Tk[i][j] = st->Tke[i][j];
         }
     const double o0 = st->xoff[0], o1 = st->xoff[1], o2 = st->xoff[2];
     const double mu2 = kp.r_grbr * kp.r_grbr;
@@ -1938,11 +1938,9 @@ __global__ void __launch_bounds__(KICK64_THREADS, 4) k_kick64(double* __restrict
             for (int j = 0; j < 3; ++j) X[j] = Xe[j];
         }
         double e[3];
-        gather_fx(fe, kp.nx, kp.ny, kp.nz, X, st, e);
+        gather_fx(fe, kp.nx, kp.ny, kp.nz, X, e);
         if (rec) {
-            rec[i] = e[0];
-            rec[kp.nX + i] = e[1];
-            rec[2 * kp.nX + i] = e[2];
+            for (int j = 0; j < 3; ++j) rec[j * kp.nX + i] = e[j] * st->escale[j];
         }
         const double dx = fma(Tk[0][2], e[2], fma(Tk[0][1], e[1], Tk[0][0] * e[0]));
         const double dy = fma(Tk[1][2], e[2], fma(Tk[1][1], e[1], Tk[1][0] * e[0]));
