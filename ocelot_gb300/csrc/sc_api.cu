@@ -388,7 +388,7 @@ int sc_plan_create(sc_plan** out, int nx, int ny, int nz, int mode) {
     SC_CUDA(prepare_fft_kernels(p), "kernel attributes");
     SC_CUDA(prepare_green_kernels(p), "kernel attributes");
     SC_CUDA(prepare_particle_kernels(), "kernel attributes");
-    SC_CUDA(prepare_sort_kernels(), "kernel attributes");
+    SC_CUDA(prepare_sort_kernels(p), "kernel attributes");
     sc_plan* h = new (std::nothrow) sc_plan;
     if (!h) return fail(SC_ERR_OOM, "out of host memory");
     h->p = p;

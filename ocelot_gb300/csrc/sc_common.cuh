@@ -423,7 +423,7 @@ inline cudaError_t prefer_shared(K kernel) {
 cudaError_t prepare_fft_kernels(const Plan& p);
 cudaError_t prepare_green_kernels(const Plan& p);
 cudaError_t prepare_particle_kernels();
-cudaError_t prepare_sort_kernels();
+cudaError_t prepare_sort_kernels(const Plan& p);
 
 // ---------------------------------------------------------------------------
 // bulk (TMA) copies between global and shared memory.  Loads complete on an

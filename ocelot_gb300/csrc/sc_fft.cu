@@ -17,7 +17,10 @@
 //          1/(Mx*My*Mz) and 1/(4*pi*eps0*hx*hy*hz)
 //
 // The complex work grid W[x][y][kz] (x < nx, y < My, kz <= Mz/2) stays in
-// HBM/L2 between passes; each pass stages whole lines in shared memory.
+// HBM/L2 between passes.  Lines of 64 to 256 points take two register steps,
+// streamed from and to global memory (sc_fft_stream.cuh in FP32, in 64-bit block
+// fixed point for FP64, sc_fft_fx.cuh); other lengths stage whole lines in
+// shared memory (sc_fft_dev.cuh).
 #include "sc_common.cuh"
 #include "sc_fft_dev.cuh"
 #include "sc_fft_stream.cuh"

@@ -15,7 +15,8 @@
 // floating-point operations in the reference's order (explicit _rn intrinsics,
 // so nothing is contracted into FMAs except where numpy's BLAS itself uses
 // FMAs: the 3x3 rotations), and computes the rest in FP64 with fewer
-// operations (kick64_one), because this GPU issues an FP64 instruction about
+// operations (k_kick64), the transforms and the gather in 64-bit integers, because
+// this GPU issues an FP64 instruction about
 // 1/64 as often as an FP32 one.  FP32
 // computes every per-particle quantity in FP32 and writes the kick as small
 // increments, each derived in closed form so that it carries no cancellation,
@@ -720,7 +721,7 @@ __device__ __forceinline__ void mesh_finish(const double* mn, const double* mx, 
         st->qfix_scale = ldexp(1.0, S);
         st->qfix_inv = (float)ldexp(1.0, -S);
     }
-    if (kick64) {  // kick64_one's two matrices, entry (lane / 3, lane % 3) in lane 0..8
+    if (kick64) {  // k_kick64's two matrices, entry (lane / 3, lane % 3) in lane 0..8
         const int i = lane / 3 % 3;
         const double t = i == 0 ? pre.T[0] : i == 1 ? pre.T[1] : pre.T[2];
         const double ist = __shfl_sync(FULL, r1, 6 + a);

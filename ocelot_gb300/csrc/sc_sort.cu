@@ -6,8 +6,8 @@
 // the keys are sorted by a stable least-significant-digit radix sort
 // (ceil(key_bits/9) passes of at most 9-bit digits: two passes for a 64^3
 // mesh), which puts the particles of each cell
-// in a contiguous run in particle order, the last pass carrying the charges
-// themselves; each cell's run is then summed by one warp.  In FP64 the sum is
+// in a contiguous run in particle order, the charges travelling with the keys;
+// each cell's run is then summed by one thread (FP64) or warp (FP32).  In FP64 the sum is
 // a sequential fold and reproduces bincount's sums bit for bit; in FP32 it is
 // Kahan-compensated.  The result does not
 // depend on scheduling, so it is the same alone and in a batch.
@@ -233,7 +233,9 @@ int sort_blocks(int64_t n) {
     return (int)((n + t - 1) / t);
 }
 
-cudaError_t prepare_sort_kernels() {
+// the kernels of a plan's deposit (none without the sorted one)
+cudaError_t prepare_sort_kernels(const Plan& p) {
+    if (!p.sorted_deposit) return cudaSuccess;
     cudaError_t e;
     if ((e = prefer_shared(k_rhist))) return e;
     if ((e = prefer_shared(k_rrowscan))) return e;
@@ -243,9 +245,7 @@ cudaError_t prepare_sort_kernels() {
         if ((e = prefer_shared(k_rscatter<4, V>))) return e;
         return prefer_shared(k_rscatter<RITEMS, V>);
     };
-    if ((e = all(0.0))) return e;
-    if ((e = all(0.0f))) return e;
-    return all(0u);
+    return p.prec == SC_FP64 ? all(0.0) : all(0.0f);
 }
 
 int sort_passes(int key_bits) { return key_bits <= 0 ? 1 : (key_bits + RMAXBITS - 1) / RMAXBITS; }
