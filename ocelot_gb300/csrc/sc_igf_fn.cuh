@@ -5,11 +5,12 @@
 // runs on the integer pipes beside them: table-driven reductions in the manner
 // of P. T. P. Tang (ACM TOMS 16, 1990), the remaining series in 64-bit integers,
 // its terms below 2^-26 (log) and 2^-34 (atan) in FP32.  Results are
-// within 0.50 (sqrt, quotient), 0.51 (log) and 0.64 (atan) ulp of the exact value
+// within 0.50 (sqrt), 0.51 (log) and 1.05 (atan of a quotient, whose own rounding and
+// the function's were 1.14 together) ulp of the exact value
 // over the arguments tried (10 million each against extended precision).
-// FP64 instructions: sqrt 7, quotient 5, log none, atan 7 (10 and 15 in a form
-// with its series in FP64: 63^3 beside the other stream 75 -> 53 us at 10k
-// particles, 84 -> 56 at 200k).
+// FP64 instructions: sqrt 7, log none, atan of a quotient 7 (10 and 20 in a form
+// with its series in FP64: 63^3 beside the other stream 75 -> 46 us at 10k
+// particles, 84 -> 54 at 200k).
 //
 // Arguments must be positive and well inside the exponent range (igf_point
 // checks the mesh steps once and falls back to the CUDA functions).
@@ -68,14 +69,8 @@ SC_HD float f_bits(unsigned u) {
     memcpy(&f, &u, 4);
     return f;
 }
-// FP64 <-> FP32 on the integer pipes (the conversions issue on the FP64 pipe):
-// rounded half up to FP32, below FP32's normal range 0; widened exactly, subnormals 0
-SC_HD float narrow(double d) {
-    const unsigned hi = hi_d(d), mag = hi & 0x7fffffffu;
-    if (mag < (897u << 20)) return 0.0f;
-    if (mag >= (1150u << 20)) return f_bits((hi & 0x80000000u) | 0x7f7fffffu);
-    return f_bits((hi & 0x80000000u) | (((mag << 3) | (lo_d(d) >> 29)) - (896u << 23) + ((lo_d(d) >> 28) & 1u)));
-}
+// FP32 -> FP64 on the integer pipes (the conversions issue on the FP64 pipe):
+// exact, subnormals 0
 SC_HD double widen(float f) {
     const unsigned u = bits_f(f), m = u & 0x7fffffffu;
     if (m < 0x00800000u) return bits_d(u & 0x80000000u, 0u);
@@ -175,25 +170,33 @@ SC_HD double log_(double x, const LogEntry* __restrict__ tab) {
     return to_double(v, 56 + sh);
 }
 
-// atan(w), any sign of a finite w: |w| <= 1 about c = j/128 as atan c + atan((w - c) / (1 + c w)),
-// |w| > 1 about 1/c as pi/2 - atan c + atan((c w - 1) / (w + c)), |w| < 3.5/128 as itself; the
-// quotient t, |t| <= 2^-8, in FP64, t - t (t^2/3 - t^4/5 + [t^6/7 - t^8/9 + t^10/11 in FP32]) and the
-// sum in integers, in units that leave the result 59 bits or more
-SC_HD double atan_(double w, const AtanEntry* __restrict__ tab) {
-    const unsigned sign = hi_d(w) & 0x80000000u;
-    const double a = bits_d(hi_d(w) & 0x7fffffffu, lo_d(w));
-    const bool big = hi_d(a) >= 0x3ff00000u;  // |w| >= 1
-    const float af = narrow(a);
+// w = |n| / |d| to FP32 accuracy, 2^-30 .. 2^30 (n, d normal)
+SC_HD float ratio(double n, double d) {
+    const unsigned hn = hi_d(n), hd = hi_d(d);
+    const float fn = f_bits(((hn & 0xfffffu) << 3) | (lo_d(n) >> 29) | 0x3f800000u);
+    const float fd = f_bits(((hd & 0xfffffu) << 3) | (lo_d(d) >> 29) | 0x3f800000u);
+    int e = (int)((hn >> 20) & 0x7ffu) - (int)((hd >> 20) & 0x7ffu);
+    e = e < -30 ? -30 : (e > 30 ? 30 : e);
+    return fn / fd * f_bits((unsigned)(127 + e) << 23);
+}
+// atan(n / d), any signs: with w = |n / d|, w <= 1 about c = j/128 as atan c + atan((n - c d) / (d + c n)),
+// w > 1 about 1/c as pi/2 - atan c + atan((c n - d) / (n + c d)), w < 3.5/128 as itself: one quotient t,
+// |t| <= 2^-8, and w itself never rounded; t in FP64, t - t (t^2/3 - t^4/5 + [t^6/7 - t^8/9 + t^10/11 in FP32]) and
+// the sum in integers, in units that leave the result 59 bits or more
+SC_HD double atan_(double n, double d, const AtanEntry* __restrict__ tab) {
+    const unsigned sign = (hi_d(n) ^ hi_d(d)) & 0x80000000u;
+    const double an = bits_d(hi_d(n) & 0x7fffffffu, lo_d(n)), ad = bits_d(hi_d(d) & 0x7fffffffu, lo_d(d));
+    const float af = ratio(an, ad);
+    const bool big = af > 1.0f;
     const float u = big ? 1.0f / af : af;
     int j = (int)(u * 128.0f + 0.5f);  // 0 .. 128
     const bool tiny = !big && j < 4;   // the quotient's rounding would be the result's
     if (tiny) j = 0;
     const float cf = (float)j * 0.0078125f;
-    const double c = widen(cf), mc = widen(-cf);
-    // N = w - c, D = 1 + c w, or N = c w - 1, D = w + c
-    const double N = fma(big ? c : 1.0, a, big ? -1.0 : mc);
-    const double D = fma(big ? 1.0 : c, a, big ? c : 1.0);
-    const double t = div_(N, D);
+    const double c = widen(cf);
+    const double p = big ? ad : an, q = big ? an : ad;  // p <= q
+    const double N = fma(-c, q, p), D = fma(c, p, q);
+    const double t = div_(big ? bits_d(hi_d(N) ^ 0x80000000u, lo_d(N)) : N, D);
     const AtanEntry E = tab[j];
     const unsigned ht = hi_d(t);
     const int e = (int)((ht >> 20) & 0x7ffu) - 1023;
@@ -207,9 +210,9 @@ SC_HD double atan_(double w, const AtanEntry* __restrict__ tab) {
                            ((long long)(int)(f * 0x1p64f) << 4);  // 2^-68
     const int s = tiny ? 61 - e : (big ? 61 : E.s);
     const long long T = (long long)shr64(m, 61 - e - s);
-    const long long p = T - (mulhi(T, corr << 6) >> 10);
-    const long long v = tiny ? p : (big ? E.hi2 : E.hi) + ((int)ht < 0 ? -p : p);
-    const double res = tiny && e < -1000 ? a : to_double(v, s);
+    const long long ti = T - (mulhi(T, corr << 6) >> 10);
+    const long long v = tiny ? ti : (big ? E.hi2 : E.hi) + ((int)ht < 0 ? -ti : ti);
+    const double res = tiny && e < -1000 ? t : to_double(v, s);
     return bits_d(hi_d(res) ^ sign, lo_d(res));
 }
 
@@ -219,11 +222,11 @@ SC_HD double point_(double x, double y, double z, const LogEntry* __restrict__ l
     const double x2 = x * x, y2 = y * y, z2 = z * z;
     const double r = sqrt_((x2 + y2) + z2);
     const double yz = y * z, zx = z * x, xy = x * y;
-    const double t1 = (-0.5 * x2) * atan_(div_(yz, x * r), at);
+    const double t1 = (-0.5 * x2) * atan_(yz, x * r, at);
     const double t2 = yz * log_(x + r, lt);
-    const double t3 = (0.5 * y2) * atan_(div_(zx, y * r), at);
+    const double t3 = (0.5 * y2) * atan_(zx, y * r, at);
     const double t4 = zx * log_(y + r, lt);
-    const double t5 = (0.5 * z2) * atan_(div_(xy, z * r), at);
+    const double t5 = (0.5 * z2) * atan_(xy, z * r, at);
     const double t6 = xy * log_(z + r, lt);
     return ((((t1 + t2) - t3) + t4) - t5) + t6;
 }
