@@ -14,8 +14,8 @@
 // -> streamed: 32^3 x pass 6.6 -> 3.9 us; 64^3 x pass 14.9 -> 8.1, y inverse 9.9 ->
 // 5.9, z forward 6.3 -> 6.0; 128 x 128 x 256 x pass 148 -> 97, y 33/106 -> 20/88; 16 uneven beams
 // x 125 -> 76, y 31/87 -> 23/60.  Not streamed, because measured slower so: the z
-// inverse (its step reads strided entries of two rows; 8.8 -> 9.6 us at 64^3)
-// and the FP64 passes (bound by the FP64 pipe; y inverse 25.8 -> 27.2 at 63^3).
+// inverse (its step reads strided entries of two rows; 8.8 -> 9.6 us at 64^3).
+// The FP64 form's passes are in sc_fft_fx.cuh.
 #pragma once
 #include "sc_fft_dev.cuh"
 
