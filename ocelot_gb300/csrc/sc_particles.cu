@@ -1100,7 +1100,9 @@ __device__ __forceinline__ void xyz_fine(const double* __restrict__ rp, int64_t 
 // transform's registers would slow every particle.
 // err (optional): a bound on |v - xyz_fine| per axis -- 2^-18 of each FP32
 // correction (a few roundings of ~2^-24 each, the approximate reciprocals'
-// ~2^-22, and margin) carried through the rotation.
+// ~2^-22, and margin) carried through the rotation, and 2^-46 of the lab
+// position for the FP64 roundings of the two evaluations (some 40 of 2^-53
+// together; those of 1 - 1/gamma^2 grow as 1/beta^2 = 1 + 1/(gamma beta)^2).
 __device__ __forceinline__ void xyz_fine32(const double* __restrict__ rp, int64_t ld, int64_t i,
                                            const KickParams& kp, const double (&T)[3][3], double g0, double v[3],
                                            double* err = nullptr) {
@@ -1118,9 +1120,11 @@ __device__ __forceinline__ void xyz_fine32(const double* __restrict__ rp, int64_
     v[2] *= g0;
     if (err) {
         const double e0 = fabs((double)c0), e1 = fabs((double)c1), e2 = fabs((double)c2);
+        const float size = (fabsf(d2f(x)) + fabsf(d2f(y)) + fabsf(tf) + fabsf(c0) + fabsf(c1) + fabsf(c2)) *
+                           (1.0f + kp.igrbr2_f);
         for (int j = 0; j < 3; ++j)
-            err[j] = ldexp(fma(e2, fabs(T[2][j]), fma(e1, fabs(T[1][j]), e0 * fabs(T[0][j]))), -18) *
-                     (j == 2 ? g0 : 1.0);
+            err[j] = (ldexp(fma(e2, fabs(T[2][j]), fma(e1, fabs(T[1][j]), e0 * fabs(T[0][j]))), -18) +
+                      f2d(size * 0x1p-46f)) * (j == 2 ? g0 : 1.0);
     }
 }
 
@@ -1537,8 +1541,10 @@ __device__ __forceinline__ long long to_fixed(double q, int S) {
 
 // NGP key of a near-face particle, equal to the FP64 form's: the grid
 // coordinate from the cheap estimate when every axis is farther from a face
-// than the estimate's error bound (plus 1e-12 cells for the FP64 roundings),
-// else from the FP64 form's operations.  Returns false outside the mesh.
+// than the estimate's error bound (plus 2^-46 of the offset and the mesh for
+// the FP64 roundings of the quotient and the difference, which are those of
+// a coordinate as large as the beam is far off the axis), else from the FP64
+// form's operations.  Returns false outside the mesh.
 __device__ __forceinline__ bool key_fine(const double* __restrict__ rp, int64_t ld, int64_t i, const KickParams& kp,
                                          const ScState* st, uint32_t& key, float (&gf)[3]) {
     double T[3][3];
@@ -1550,7 +1556,8 @@ __device__ __forceinline__ bool key_fine(const double* __restrict__ rp, int64_t 
     for (int j = 0; j < 3; ++j) {  // the FP64 form's grid coordinate (k_keys64)
         g[j] = __dsub_rn(div_checked(xv[j], st->steps[j], st->isteps[j]), st->xoff[j]);
         const double d = fabs(g[j] - rint(g[j]));
-        sure &= d > fma(err[j], st->isteps[j], 1e-12);
+        const float size = fabsf(st->xofff[j]) + (float)(j == 0 ? kp.nx : j == 1 ? kp.ny : kp.nz);
+        sure &= d > fma(err[j], st->isteps[j], f2d(size * 0x1p-46f));
     }
     if (!sure) {
         xyz_fine(rp, ld, i, kp, T, st->gamma0, xv);

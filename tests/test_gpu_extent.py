@@ -88,3 +88,41 @@ def test_fp64_gather_over_mesh_shapes(mesh, shift):
     for r in (1, 3, 5):
         k = ref[r] - rp[r]
         assert np.linalg.norm(out[r] - rp[r] - k) < 5e-9 * np.linalg.norm(k), r
+
+
+def _off_axis_beam(n=20_000, x0=0.1875, h=2.0 ** -23, cells=32, energy=0.130):
+    """A beam ``x0 / h`` = 1.6 million cells off the axis whose x lie on cell faces
+    or one last place (2^-55) below, and move by half that place on the way to
+    the lab: the last bit of the reference's operations decides their cells."""
+    rng = np.random.default_rng(11)
+    half = n // 2
+    gam = energy / sc_oracle.m_e_GeV
+    beta = np.sqrt(1 - gam ** -2)
+    rp = np.zeros((6, n))
+    k = rng.integers(1, cells, half)
+    k[0] = 0
+    tau = 1e-5 * (1 + rng.random(half))
+    drift = 2.0 ** -56 / (beta * tau) * (1 + 8e-7 * (rng.random(half) - 0.5))
+    drift[rng.random(half) < 0.8] = 0.0  # few enough that the mean stays on a whole cell
+    drift[k == 0] = 0.0
+    for s, sl in ((1, slice(0, half)), (-1, slice(half, n))):  # mirrored about the middle
+        rp[0, sl] = x0 + s * (k - cells // 2) * h
+        rp[1, sl] = s * drift
+        rp[4, sl] = tau
+    rp[0, half:][drift != 0] -= 2.0 ** -55
+    rp[2] = 1e-4 * rng.standard_normal(n)
+    return rp, np.full(n, 2.0 ** -52), (cells + 3, 20, 24), energy
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_cells_of_an_off_axis_beam_on_faces(precision):
+    """Far off the axis the last place of a coordinate is many 1e-12 of a cell."""
+    rp, q, mesh, energy = _off_axis_beam()
+    rec = {}
+    sc_oracle.sc_apply(rp.copy(), q, energy, 1e-6, mesh, record=rec)
+    d = torch.from_numpy(rp).to(DEV)
+    sc = SpaceCharge(nmesh_xyz=mesh, precision=precision, device=DEV)
+    sc.apply_device(d, torch.from_numpy(q).to(DEV), energy, 1e-6)
+    sc.check()
+    keys = sc.engine().region("keys")[:rp.shape[1]].cpu().numpy().astype(np.int64)
+    assert np.array_equal(keys, rec["keys"])
