@@ -779,8 +779,8 @@ __device__ void mesh_finalize(const double* part, int nblk, const KickParams& kp
 // ---------------------------------------------------------------------------
 // FP64 1/x and sqrt(x) for positive x well inside the exponent range: the
 // hardware's approximation and two Newton-Raphson steps (the square root by
-// Goldschmidt's iteration with a final residual correction).  Within an ulp or
-// so of the exact value, not always correctly rounded; five and eight FP64
+// Goldschmidt's iteration with a final residual correction).  Within half an ulp
+// of the exact value in 3e9 tries each; five and eight FP64
 // instructions instead of the dozen of the IEEE forms with their range checks.
 __device__ __forceinline__ double rcp64(double x) {
     double y;
@@ -788,11 +788,14 @@ __device__ __forceinline__ double rcp64(double x) {
     y = fma(y, fma(-x, y, 1.0), y);
     return fma(y, fma(-x, y, 1.0), y);
 }
-// one Newton-Raphson step: ~2^-44 relative, for a factor of a small increment
-__device__ __forceinline__ double rcp64_once(double x) {
+// the same from one cubic step, y (1 + e + e^2) with e = 1 - x y: 2^-52.99 of the
+// value in 3e9 tries (the two steps above 2^-53.00, one of them alone 2^-39.9: the
+// approximation has 2^-19.9), in four FP64 instructions
+__device__ __forceinline__ double rcp64_cubic(double x) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    return fma(y, fma(-x, y, 1.0), y);
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
 }
 __device__ __forceinline__ double sqrt64(double x) {
     double y;
@@ -1901,7 +1904,7 @@ __device__ __forceinline__ void gather_fx(const long long* __restrict__ fe, int 
     e[2] = sample_fx(fe + 2 * nc, x.ib, y.ib, z.ia, x.tb, y.tb, z.ta, ny, nz, x.okb && y.okb && z.oka);
 }
 
-// Gather + kick of the FP64 form.  Bound by the FP64 pipe, 48 instructions per
+// Gather + kick of the FP64 form.  Bound by the FP64 pipe, 49 instructions per
 // particle (the gather's 48 run as integers beside them, gather_fx: 2M / 64^3
 // 460 -> 287 us, 200k / 63^3 51 -> 37; the lab position and momentum come from
 // the frame pass, 32 bytes a particle instead of 22 instructions: 287 -> 234 and
@@ -1962,7 +1965,7 @@ __global__ void __launch_bounds__(KICK64_THREADS, 4) k_kick64(double* __restrict
         rp[2 * ld + i] = fma(py, w, l1);
         rp[3 * ld + i] = py;
         rp[4 * ld + i] = w * en;
-        rp[5 * ld + i] = fma(dp2, rcp64_once(kp.r_betaref + d + en), d);
+        rp[5 * ld + i] = fma(dp2, rcp64_cubic(kp.r_betaref + d + en), d);
     }
 }
 
