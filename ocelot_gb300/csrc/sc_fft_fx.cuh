@@ -35,9 +35,9 @@ __host__ __device__ constexpr size_t fx_smem_zi(int L, int NC) { return sizeof(F
 
 // per-line words of a block: exponents and magnitudes
 struct FxLines {
-    int e[FX_COLS], g[FX_COLS], m[3][FX_COLS];
+    int e[FX_COLS], m[3][FX_COLS];
 };
-static_assert(sizeof(FxLines) == 5 * FX_COLS * sizeof(int), "cleared word by word");
+static_assert(sizeof(FxLines) == 4 * FX_COLS * sizeof(int), "cleared word by word");
 __device__ __forceinline__ void fx_clear(FxLines& s) {
     int* w = reinterpret_cast<int*>(&s);
     for (int i = threadIdx.x; i < (int)(sizeof(FxLines) / sizeof(int)); i += blockDim.x) w[i] = 0;
@@ -47,6 +47,11 @@ __device__ __forceinline__ void fx_raise(int* word, int v) {
     v = max(v, __shfl_xor_sync(~0u, v, 8));
     v = max(v, __shfl_xor_sync(~0u, v, 16));
     if ((threadIdx.x & 31) < FX_COLS) atomicMax(word, v);
+}
+// the potential's largest exponent over a grid: every thread of the warp calls it
+__device__ __forceinline__ void phi_raise(const ScState* st, int e) {
+    e = __reduce_max_sync(~0u, e);
+    if ((threadIdx.x & 31) == 0) atomicMax(&const_cast<ScState*>(st)->phi_exp, e);
 }
 template <int N>
 __device__ __forceinline__ int fx_exp_of(const double2 (&d)[N]) {
@@ -176,42 +181,42 @@ __device__ __forceinline__ void xconv_fx(double2* __restrict__ W, const double* 
         }
     }
     double g[Q];
-    int eg = 0;
 #pragma unroll
     for (int k2 = 0; k2 < Q; ++k2) {
         const int kx = m + P * k2, gx = kx <= L - kx ? kx : L - kx;
         const long long gi = (long long)gx * KyKz + gk;
         g[k2] = (live && SC_IDX_OK(st, 23, gi, (long long)(L / 2 + 1) * KyKz)) ? G[gi] : 0.0;
-        eg = max(eg, fx_exp(g[k2]));
     }
     fx_raise(&ln.m[0][kk], (int)mag);
-    fx_raise(&ln.g[kk], eg);
     __syncthreads();
-    const int EG = ln.g[kk];
     Fx2 u[Q];
+    int top = 0;
     int sh = fx_room<Q>((unsigned)ln.m[0][kk]);
     int bit = S::B_HALF - sh;  // the bit of 2^E in what is held
-    mag = 0;
     S::template second<false>(u, m, tab, sh);
+    // the row of the table that this thread has just read holds its exponents
+    // until its products' shifts are known (16 registers less, 26 spilled)
+    Fx2* row = tab + m * S::ROW;
 #pragma unroll
     for (int k2 = 0; k2 < Q; ++k2) {
-        const long long gf = fx_from<61>(g[k2], EG).v;  // G / 2^(EG - 1023) in bits 61 and below
-        const FxC c((int)(gf >> 31), (int)(gf & 0x7fffffff));
+        int e;
+        const FxC c = fx_fraction(g[k2], e);
         u[k2] = cx<Fx>(fx_mul(u[k2].x, c), fx_mul(u[k2].y, c));
-        mag = max(mag, max(fx_mag(u[k2].x), fx_mag(u[k2].y)));
+        top = max(top, fx_top(u[k2], e));
+        row[k2].x.v = e;
     }
-    // value = held * 2^(E - 1023 - bit) * 2^(EG - 1023 + 1)
-    fx_raise(&ln.m[1][kk], (int)mag);
+    // value = held * 2^(E - 1023 - bit) * 2^(eg - 1022)
+    fx_raise(&ln.m[1][kk], top);
     __syncthreads();
-    sh = fx_room<Q>((unsigned)ln.m[1][kk]);
-    bit -= sh;
+    const int EG = ln.m[1][kk] - (fx_bit(Q) + 1);  // the exponent that leaves the largest its room
+    bit -= EG - 1022;
 #pragma unroll
-    for (int k2 = 0; k2 < Q; ++k2) u[k2] = fx_down(u[k2], sh);
+    for (int k2 = 0; k2 < Q; ++k2) u[k2] = fx_scale(u[k2], EG - (int)row[k2].x.v);
     mag = S::t_first(u, m, tw, tab);  // over the row of the table that this thread has read
     fx_raise(&ln.m[2][kk], (int)mag);
     __syncthreads();
     sh = fx_room<P>((unsigned)ln.m[2][kk]);
-    const FxOut o(E == FX_BAD || EG == FX_BAD ? FX_BAD : E, bit - sh - (EG - 1022));
+    const FxOut o(EG > 2 * FX_BAD ? FX_BAD : E, bit - sh);
 #pragma unroll
     for (int r = 0; r < RQ; ++r) {
         const int k2 = m + r * P;

@@ -19,7 +19,7 @@
 // A line with a NaN or an infinity comes out as NaNs (a double transform spreads
 // them over the line too); one of denormals only comes out as zeros.
 #pragma once
-#include "sc_common.cuh"
+#include "sc_cx.cuh"
 
 namespace ocsc {
 
@@ -57,12 +57,21 @@ __host__ __device__ __forceinline__ int fx_hi(Fx a) { return (int)(a.v >> 32); }
 __host__ __device__ __forceinline__ int fx_lo(Fx a) { return (int)((unsigned)a.v >> 1); }
 
 // a w, |a| < 2^62: the 64-bit operand as its high word and 31 bits of its low one
-__host__ __device__ __forceinline__ Fx fx_mul(Fx a, FxC w) {
+// (the product of the low parts, up to two units, and the low bit are left out)
+__host__ __device__ __forceinline__ Fx fx_mul(Fx a, FxC w, long long half = 1ll << 29) {
     const int ah = fx_hi(a), al = fx_lo(a);
-    long long m = (1ll << 29) + (long long)ah * w.L;
+    long long m = half + (long long)ah * w.L;
     m += (long long)al * w.H;
     const long long h = (long long)ah * w.H;
     return Fx{h + h + (m >> 30)};
+}
+// the same for a compile-time constant, with the mean of what is left out in the
+// rounding, as far as 0 still gives 0: a DFT sums the products of one constant, and
+// their common bias with them (256-point pass over one spike: 1.14 -> 0.99 of a
+// double pass's error)
+__host__ __device__ __forceinline__ Fx fx_mul_const(Fx a, FxC w) {
+    const long long half = (1ll << 29) + w.L / 2 + w.H / 4;
+    return fx_mul(a, w, half < 0 ? 0 : half > (1ll << 30) - 1 ? (1ll << 30) - 1 : half);
 }
 // a u + b w for |a|, |b| < 2^61 and u^2 + w^2 <= 1: the middle sum stays below 1.92 * 2^62
 __host__ __device__ __forceinline__ Fx fx_mul2(Fx a, FxC u, Fx b, FxC w) {
@@ -106,7 +115,7 @@ constexpr int FX_BAD = 0x7ff;  // the line exponent of a NaN or an infinity
 // biased exponent bits of a double (0 for zeros and denormals)
 __device__ __forceinline__ int fx_exp(double d) { return (__double2hiint(d) >> 20) & 0x7ff; }
 
-// logical right shift; 0 for 64 and more
+// shifts by 0 and more that give 0 (arithmetic: the sign) for 64 and more
 __device__ __forceinline__ unsigned long long fx_shr(unsigned long long m, int s) {
 #ifdef __CUDA_ARCH__
     unsigned long long r;
@@ -115,6 +124,46 @@ __device__ __forceinline__ unsigned long long fx_shr(unsigned long long m, int s
 #else
     return s > 63 ? 0 : m >> s;
 #endif
+}
+__device__ __forceinline__ long long fx_sar(long long v, int s) {
+#ifdef __CUDA_ARCH__
+    long long r;
+    asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
+    return r;
+#else
+    return v >> (s > 63 ? 63 : s);
+#endif
+}
+__device__ __forceinline__ long long fx_shl(long long v, int s) {
+#ifdef __CUDA_ARCH__
+    long long r;
+    asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(v), "r"(s));
+    return r;
+#else
+    return s > 63 ? 0 : (long long)((unsigned long long)v << s);
+#endif
+}
+// a / 2^s rounded, or a 2^-s for a negative s; |a| < 2^62, and the result's as well
+__device__ __forceinline__ Fx fx_scale(Fx a, int s) {
+    const int right = max(s, 0);
+    return Fx{fx_shl(fx_sar(a.v + (fx_shl(1ll, right) >> 1), right), max(-s, 0))};
+}
+__device__ __forceinline__ Fx2 fx_scale(Fx2 a, int s) { return Fx2{fx_scale(a.x, s), fx_scale(a.y, s)}; }
+
+// a double factor as w 2^(e - 1022), 1/2 <= |w| < 1 with all its bits
+__device__ __forceinline__ FxC fx_fraction(double g, int& e) {
+    const int hi = __double2hiint(g), sg = hi >> 31;
+    const unsigned lo = (unsigned)__double2loint(g);
+    e = fx_exp(g);
+    const int H = (int)(((unsigned)hi & 0xfffffu) << 10 | lo >> 22) | (e ? 0x40000000 : 0);
+    const int L = (int)((lo & 0x3fffffu) << 9);
+    e = max(e, 1);
+    return FxC((H ^ sg) - sg, (L ^ sg) - sg);
+}
+// a bound on the leading bit of a value under that exponent; above any of a
+// finite one where the factor is a NaN or an infinity
+__device__ __forceinline__ int fx_top(Fx2 a, int e) {
+    return e == FX_BAD ? 1 << 20 : 64 - __clz((int)max(fx_mag(a.x), fx_mag(a.y))) + e;
 }
 
 // d as an integer of a line of exponent E >= fx_exp(d): a value with exponent E has
@@ -170,10 +219,5 @@ __device__ __forceinline__ double fx_double(Fx a) {
 // Field grids of the FP64 kick: differences of the potential as integers whose
 // bit FX_PHI stands for 2^(the largest exponent of the potential)
 constexpr int FX_PHI = 58;
-// the potential's largest exponent over a grid: every thread of the warp calls it
-__device__ __forceinline__ void phi_raise(const ScState* st, int e) {
-    e = __reduce_max_sync(~0u, e);
-    if ((threadIdx.x & 31) == 0) atomicMax(&const_cast<ScState*>(st)->phi_exp, e);
-}
 
 }  // namespace ocsc
