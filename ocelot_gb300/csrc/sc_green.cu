@@ -135,10 +135,11 @@ __device__ __forceinline__ void igf_corner_xyz(unsigned c, int cy1, int cz1, dou
 }
 
 // Whether the corners may take igf::point_: steps well inside the exponent range
-// and not so unequal that x + r of a corner just below the axis vanishes
+// (the arguments of log_ then lie in 2^-160 .. 2^145) and not so unequal that x + r
+// of a corner just below the axis vanishes
 __device__ __forceinline__ bool igf_regular(double hx, double hy, double hz) {
     const double lo = fmin(hx, fmin(hy, hz)), hi = fmax(hx, fmax(hy, hz));
-    return lo > 1e-50 && hi < 1e50 && hi < lo * 0x1p20;
+    return lo > 1e-40 && hi < 1e40 && hi < lo * 0x1p20;
 }
 
 constexpr int IGF_THREADS = 256;

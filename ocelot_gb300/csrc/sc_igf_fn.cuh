@@ -5,15 +5,16 @@
 // runs on the integer pipes beside them: table-driven reductions in the manner
 // of P. T. P. Tang (ACM TOMS 16, 1990), the remaining series in 64-bit integers,
 // its terms below 2^-26 (log) and 2^-34 (atan) in FP32.  Results are
-// within 0.50 (sqrt), 0.51 (log) and 1.05 (atan of a quotient, whose own rounding and
-// the function's were 1.14 together) ulp of the exact value
-// over the arguments tried (10 million each against extended precision).
+// within 0.50 (sqrt), 0.80 (log; 0.51 for |log x| > 1, the most just beyond |x - 1| = 2^-8)
+// and 1.09 (atan of a quotient; 1.45 where it lies just below a power of two and the
+// quotient above) ulp of the exact value over the arguments tried (millions each against
+// 113-bit arithmetic).
 // FP64 instructions: sqrt 7, log none, atan of a quotient 7 (10 and 20 in a form
 // with its series in FP64: 63^3 beside the other stream 75 -> 46 us at 10k
 // particles, 84 -> 54 at 200k).
 //
-// Arguments must be positive and well inside the exponent range (igf_point
-// checks the mesh steps once and falls back to the CUDA functions).
+// Arguments must be positive and inside 2^+-180 (igf_regular checks the mesh steps
+// once; others take the CUDA functions, igf_point).
 #pragma once
 #include <string.h>
 
@@ -149,23 +150,35 @@ SC_HD double to_double(long long v, int s) {
 
 // log(x) for normal x > 0: x = 2^k m, m in [1, 2); with the table's short 1/c
 // near 1/m, r = m (1/c) - 1, exact in units of 2^-66, |r| < 2^-7.9, and
-// log x = k ln2 - log(1/c) + r - r^2 (1/2 - r/3 + r^2/4 - [r^3/5 - r^4/6 in FP32]),
-// in integers; the sum in units of 2^-56 or 2^-58
+// log x = k ln2 - log(1/c) + r - r^2 (1/2 - r/3 + r^2/4 - [r^3/5 - r^4/6 + r^5/7 - r^6/8 in FP32]),
+// in integers; the sum in units of 2^-56, 2^-58 or 2^-62, the finer ones for the smaller
+// results.  |x - 1| < 2^-8, where the result may be of any size, takes 1/c = 1: log x = r (1 - r (1/2 - ...)), r with all its bits.
 SC_HD double log_(double x, const LogEntry* __restrict__ tab) {
     const unsigned hx = hi_d(x);
     const int k = (int)(hx >> 20) - 1023;
     const LogEntry t = tab[(hx >> 13) & 127u];
+    const bool above = (hx >> 12) == (1023u << 8), below = (hx >> 13) == (1023u << 7) - 1u;
+    const unsigned ic = above ? 1u << 14 : (below ? 1u << 13 : (unsigned)t.ic);
     const unsigned long long m = ((unsigned long long)((hx & 0xfffffu) | 0x100000u) << 32) | lo_d(x);
-    const long long r = (long long)(m * (unsigned long long)(unsigned)t.ic);  // 2^-66; the 1 is 2^66, gone
+    const long long r = (long long)(m * (unsigned long long)ic);  // 2^-66; the 1 is 2^66, gone
     const long long r4 = (long long)((unsigned long long)r << 4);
-    const long long r2 = mulhi(r4, r4);                                       // 2^-76
+    const long long r2 = mulhi(r4, r4);                           // 2^-76
     const float rf = (float)(int)(r >> 32) * 0x1p-34f;
-    const float f = (rf * rf) * rf * fmaf(rf, -0.166666667f, 0.2f);
+    const float f = (rf * rf) * rf * fmaf(rf, fmaf(rf, fmaf(rf, -0.125f, 0.142857143f), -0.166666667f), 0.2f);
     const long long u = (1ll << 61) - (mulhi(r, 0x5555555555555555ll) >> 4) + (r2 >> 16) -
                         (long long)((unsigned long long)(long long)(int)(f * 0x1p50f) << 12);  // 2^-62
-    const long long q = r - (mulhi(r2, u) >> 8);                              // 2^-66
-    const long long low = (((long long)k * LN2_LO) >> 26) + t.t + (q >> 4);   // 2^-62
-    const int sh = (unsigned)(k + 40) <= 80u ? 2 : 0;  // |log x| < 2^5: two bits more
+    if (above || below) {
+        const long long sg = r >> 63;
+        const unsigned long long ur = (unsigned long long)((r ^ sg) - sg);
+        const int n = clz64(ur);                                  // 5 and more
+        const long long rn = (long long)(ur << ((n - 1) & 63));   // |r| 2^(65 + n)
+        const long long v = mulhi(rn, (1ll << 62) - ((mulhi(r4, u) + 32) >> 6));
+        return ur ? to_double((v ^ sg) - sg, 63 + n) : 0.0;
+    }
+    const long long q = r - (mulhi(r2, u) >> 8);                                     // 2^-66
+    const long long low = (((long long)k * LN2_LO + (1 << 25)) >> 26) + t.t + ((q + 8) >> 4);  // 2^-62
+    // bits more than 2^-56: |log x| < 2 for k = -2 .. 1, < 2^5 for -40 .. 40
+    const int sh = (unsigned)(k + 2) <= 3u ? 6 : ((unsigned)(k + 40) <= 80u ? 2 : 0);
     const long long v = (long long)((unsigned long long)((long long)k * LN2_HI) << sh) + ((low + (32 >> sh)) >> (6 - sh));
     return to_double(v, 56 + sh);
 }

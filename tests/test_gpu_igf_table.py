@@ -22,6 +22,7 @@ if not has_gpu():
     pytest.skip("needs a CUDA GPU", allow_module_level=True)
 
 from ocelot_gb300 import SpaceCharge  # noqa: E402
+from oracle import sc_oracle  # noqa: E402
 
 CASES = [
     ((64, 64, 64), (8.7e-6, 8.7e-6, 4.5e-3)),  # the 2M / 64^3 130 MeV beam's rest-frame cells
@@ -44,3 +45,21 @@ def test_hybrid_table_against_extended_precision(shape, h):
     # 7e-8 rms) beyond, then rounded to FP32
     assert rel.max() <= 4e-7, (shape, h, float(rel.max()), np.unravel_index(int(rel.argmax()), shape))
     assert np.sqrt(np.mean(rel ** 2)) <= 1.5e-7, (shape, h, float(np.sqrt(np.mean(rel ** 2))))
+
+
+@pytest.mark.parametrize("h", [(1e-9, 1e-9, 1e-2), (1e-2, 1e-9, 2e-9), (1e-45, 2e-45, 1e-45), (1e45, 1e45, 2e45),
+                               (1e-5, 2e-5, 4e-5), (0.03, 0.03, 0.06)],
+                         ids=["needles", "sheets", "tiny", "huge", "usual", "metres"])
+def test_exact_table_against_extended_precision(h):
+    """sym_kernel's FP64 table for steps of any size and ratio: those outside the
+    range of the table-driven functions take CUDA's, and a mesh of metres has corners
+    whose logarithms pass through 0.  The 8-corner difference leaves noise of its
+    terms' roundings (1e-11 of the table's norm for cubic cells, 1e-4 for these needles),
+    the reference's numpy as much; four times as much here would be another formula's."""
+    shape = (16, 20, 40)
+    exact = igf_extended(shape, h)
+    scale = float(np.abs(exact).max())
+    ref = sc_oracle.igf_kernel(shape, h)
+    k = SpaceCharge(precision="fp64").sym_kernel(shape, h)
+    noise, err = (np.linalg.norm(((t - exact) / scale).astype(float)) for t in (ref, k))
+    assert err <= 4 * noise, (h, err, noise)
