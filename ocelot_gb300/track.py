@@ -30,7 +30,6 @@ the device after every step, ``envelope.py``).
 from __future__ import annotations
 
 import ctypes as C
-import gc
 import math
 from typing import NamedTuple
 
@@ -627,20 +626,15 @@ class DeviceTrack:
                 # Recording does not execute: counter and particles are untouched.  The
                 # launches allocate nothing, so the recording needs none of torch.cuda.graph's
                 # collection of garbage and emptying of the allocator's cache, which the
-                # next job's workspace is then allocated from again; no collection
-                # may run meanwhile (what it frees could query events).
-                collecting = gc.isenabled()
-                gc.disable()
-                try:
-                    with torch.cuda.stream(self.stream):
-                        g.capture_begin()
-                        try:
-                            self._launch(kicks)
-                        finally:
-                            g.capture_end()
-                finally:
-                    if collecting:
-                        gc.enable()
+                # next job's workspace is then allocated from again.  "relaxed": what a
+                # collection (or another thread) frees or allocates meanwhile neither fails
+                # nor ends the recording.
+                with torch.cuda.stream(self.stream):
+                    g.capture_begin(capture_error_mode="relaxed")
+                    try:
+                        self._launch(kicks)
+                    finally:
+                        g.capture_end()
             self._graphs[kicks] = g
         return g
 

@@ -177,3 +177,34 @@ def test_random_mesh_track_equals_plugin_step_by_step(precision):
     sc2.check()
     assert np.random.random() == after_job
     assert np.array_equal(out, rp.cpu().numpy())
+
+
+def test_recording_lives_with_the_garbage_collector():
+    """The collector stays on while a step is recorded, and what it frees then (a
+    plan with its stream, events and pinned memory) leaves the recording as it was."""
+    import gc
+    import weakref
+    from ocelot_gb300.sc import Engine
+    ref = _run(graph=False)[1]
+    sc = SpaceCharge(step=1, nmesh_xyz=[int(v) for v in FODO["nmesh"]], precision="fp64")
+    job = T.DeviceTrack(_fodo(int(FODO["cells"])), sc, 0.25, _pa(FODO["rp_in"], FODO["q"], float(FODO["E"])), graph=True)
+    launch, seen = job._launch, []
+
+    def recorded(kicks):
+        if torch.cuda.is_current_stream_capturing():
+            enabled, freed = gc.isenabled(), weakref.ref(cycle.pop())
+            gc.collect()
+            seen.append(enabled and freed() is None)
+        launch(kicks)
+
+    job._launch = recorded
+    cycle = []
+    for _ in range(8):
+        eng = Engine((16, 16, 16), "fp64")
+        eng.ensure(100)
+        eng.itself = eng
+        cycle.append(eng)
+    del eng
+    out = job.run().result().rparticles
+    assert seen and all(seen)
+    assert np.array_equal(out, ref)
