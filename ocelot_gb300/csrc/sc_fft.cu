@@ -619,14 +619,14 @@ __global__ void k_field_grids(const double* __restrict__ phi, double* __restrict
     const int j = blockIdx.x, i = blockIdx.y;
     const double hx = st->steps[0], hy = st->steps[1], hz = st->steps[2];
     const double rx = st->isteps[0], ry = st->isteps[1], rz = st->isteps[2];
-    const int E = st->phi_exp;
+    const int E = max(st->phi_exp, 1);  // denormals have exponent 1
     const size_t ncell = (size_t)nx * ny * nz;
     if (fe && i == 0 && j == 0 && threadIdx.x < 3) {
         const int a = threadIdx.x;
-        const double sc = E == FX_BAD ? NAN : ldexp(st->isteps[a], E - 1023 - FX_PHI);
+        const double sc = E == FX_BAD ? NAN : ldexp(st->isteps[a], E - 1023);
         st->escale[a] = sc;
         for (int b = 0; b < 3; ++b)
-            st->Tke[b][a] = E == FX_BAD ? NAN : ldexp(st->Tk[b][a] * st->isteps[a], E - 1023 - FX_PHI);
+            st->Tke[b][a] = E == FX_BAD ? NAN : ldexp(st->Tk[b][a] * st->isteps[a], E - 1023);
     }
     auto over = [](double a, double h, double r) {
         const double q = a * r;

@@ -292,7 +292,10 @@ __device__ __forceinline__ Cx<double>* fft_fx(Cx<double>* a, Cx<double>* b, int 
             m = idx - line * per;
         }
     };
-    for (int l = threadIdx.x; l < nl; l += blockDim.x) slot(l)[0] = slot(l)[1] = 0;
+    for (int l = threadIdx.x; l < nl; l += blockDim.x) {
+        slot(l)[0] = 1;  // the exponent of denormals
+        slot(l)[1] = 0;
+    }
     __syncthreads();
     for (int idx = threadIdx.x; idx < nl * A; idx += blockDim.x) {
         int line, m, e = 0;

@@ -40,7 +40,8 @@ struct FxLines {
 static_assert(sizeof(FxLines) == 4 * FX_COLS * sizeof(int), "cleared word by word");
 __device__ __forceinline__ void fx_clear(FxLines& s) {
     int* w = reinterpret_cast<int*>(&s);
-    for (int i = threadIdx.x; i < (int)(sizeof(FxLines) / sizeof(int)); i += blockDim.x) w[i] = 0;
+    for (int i = threadIdx.x; i < (int)(sizeof(FxLines) / sizeof(int)); i += blockDim.x)
+        w[i] = i < FX_COLS ? 1 : 0;  // e: 1, the exponent of denormals
 }
 // raise *word to v: the lanes of a warp that share a column (lane mod 8) first
 __device__ __forceinline__ void fx_raise(int* word, int v) {

@@ -17,7 +17,7 @@
 // one of the line's norm, not of each value.
 //
 // A line with a NaN or an infinity comes out as NaNs (a double transform spreads
-// them over the line too); one of denormals only comes out as zeros.
+// them over the line too).
 #pragma once
 #include "sc_cx.cuh"
 
@@ -166,14 +166,15 @@ __device__ __forceinline__ int fx_top(Fx2 a, int e) {
     return e == FX_BAD ? 1 << 20 : 64 - __clz((int)max(fx_mag(a.x), fx_mag(a.y))) + e;
 }
 
-// d as an integer of a line of exponent E >= fx_exp(d): a value with exponent E has
-// bit B as its leading one
+// d as an integer of a line of exponent E >= fx_exp(d), E >= 1: a value with exponent E
+// has bit B as its leading one
 template <int B>
 __device__ __forceinline__ Fx fx_from(double d, int E) {
     const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
     const int e = (hi >> 20) & 0x7ff;
-    const unsigned long long m = ((unsigned long long)(hi << 11 | lo >> 21 | 0x80000000u) << 32) | (lo << 11);
-    const int s = E - e + (62 - B) + (e == 0 ? 64 : 0);
+    const unsigned long long m =
+        ((unsigned long long)(hi << 11 | lo >> 21 | (e ? 0x80000000u : 0u)) << 32) | (lo << 11);
+    const int s = E - max(e, 1) + (62 - B);
     const long long r = (long long)((fx_shr(m, s) + 1) >> 1);
     const long long sg = (int)hi >> 31;
     return Fx{(r ^ sg) - sg};
@@ -189,16 +190,15 @@ struct FxOut {
         ovf = bad ? 0x7ff80000 : 0x7ff00000;
     }
 };
-// the nearest double
+// the nearest double (below the normal range the nearest denormal)
 __device__ __forceinline__ double fx_to(Fx a, FxOut o) {
     const long long sg = a.v >> 63;
     const unsigned long long u = (unsigned long long)((a.v ^ sg) - sg);
     const int n = __clzll((long long)u);
     const unsigned long long w = u << (n & 63);
-    const unsigned long long m = ((w >> 10) + 1) >> 1;
-    const int e = u ? o.ebase - n : o.ezero;
-    unsigned hi = (unsigned)(m >> 32) + ((unsigned)(e - 1) << 20), lo = (unsigned)m;
-    if (e < 1) hi = lo = 0;
+    const int e = u ? o.ebase - n : o.ezero, en = max(e, 1);
+    const unsigned long long m = (fx_shr(w, 10 + en - e) + 1) >> 1;
+    unsigned hi = (unsigned)(m >> 32) + ((unsigned)(en - 1) << 20), lo = (unsigned)m;
     if (e > 2046) {
         hi = (unsigned)o.ovf;
         lo = 0;
@@ -206,13 +206,14 @@ __device__ __forceinline__ double fx_to(Fx a, FxOut o) {
     return __hiloint2double((int)(hi | ((unsigned)sg & 0x80000000u)), (int)lo);
 }
 
-// the nearest double of the integer itself
+// the nearest double of a 2^-S
+template <int S = 0>
 __device__ __forceinline__ double fx_double(Fx a) {
     const long long sg = a.v >> 63;
     const unsigned long long u = (unsigned long long)((a.v ^ sg) - sg);
     const int n = __clzll((long long)u);
     const unsigned long long m = (((u << (n & 63)) >> 10) + 1) >> 1;
-    const unsigned hi = (unsigned)(m >> 32) + ((unsigned)(1085 - n) << 20) | ((unsigned)sg & 0x80000000u);
+    const unsigned hi = (unsigned)(m >> 32) + ((unsigned)(1085 - S - n) << 20) | ((unsigned)sg & 0x80000000u);
     return u ? __hiloint2double((int)hi, (int)(unsigned)m) : 0.0;
 }
 

@@ -1893,7 +1893,7 @@ __device__ __forceinline__ double sample_fx(const long long* __restrict__ F, int
     const size_t sx = (size_t)ny * nz;
     const Fx y0 = lerp_fx(lerp_fx(b[0], b[1], tz).v, lerp_fx(b[nz], b[nz + 1], tz).v, ty);
     const Fx y1 = lerp_fx(lerp_fx(b[sx], b[sx + 1], tz).v, lerp_fx(b[sx + nz], b[sx + nz + 1], tz).v, ty);
-    return ok ? fx_double(lerp_fx(y0.v, y1.v, tx)) : 0.0;
+    return ok ? fx_double<FX_PHI>(lerp_fx(y0.v, y1.v, tx)) : 0.0;
 }
 __device__ __forceinline__ void gather_fx(const long long* __restrict__ fe, int nx, int ny, int nz,
                                           const double (&X)[3], double (&e)[3]) {

@@ -105,7 +105,7 @@ struct Fixed {
             for (int j = 0; j < Q; ++j) tw[i * Q + j] = fxw(L, (long)i * j);
     }
     static int exponent(const Line& in) {
-        int E = 0;
+        int E = 1;
         for (const double2& c : in) E = max(E, max(fx_exp(c.x), fx_exp(c.y)));
         return E;
     }
@@ -249,16 +249,16 @@ int main() {
     lines<128>();
     lines<192>();
     lines<256>();
-    // conversions: any value, any line exponent above its own
+    // conversions: any value, any line exponent above its own, denormals among both
     std::mt19937_64 g(5);
     long bad = 0;
     for (int i = 0; i < 1000000; ++i) {
         const long long v = (long long)g() >> (2 + g() % 62);
-        const int E = 60 + (int)(g() % 1900);
+        const int E = 1 + (int)(g() % 2000);
         bad += !nearest(fx_to(Fx{v}, FxOut(E, 54)), ldexpl((LD)v, E - 1023 - 54));
         bad += !nearest(fx_double(Fx{v}), (LD)v);
-        const double x = ldexp((double)(long long)g(), (int)(g() % 80) - 100);
-        const int EE = fx_exp(x) + (int)(g() % 70);
+        const double x = ldexp((double)(long long)g(), (int)(g() % 80) - (g() & 1 ? 100 : 1160));
+        const int EE = max(fx_exp(x), 1) + (int)(g() % 70);
         const LD r = floorl(fabsl(ldexpl((LD)x, 1023 - EE + 54)) + 0.5L);
         bad += fx_from<54>(x, EE).v != (long long)(x < 0 ? -r : r);
     }

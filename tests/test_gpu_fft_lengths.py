@@ -52,3 +52,22 @@ def test_fp64_potential_scales_by_powers_of_two(mesh, padded):
     for bad in (np.nan, np.inf):
         q[1, 2, 3] = bad
         assert not np.isfinite(np.asarray(sc.potential(q, steps))).any()
+
+
+@pytest.mark.parametrize("mesh", [[32, 48, 64], [96, 128, 20], [24, 20, 12]])
+def test_fp64_potential_at_the_edge_of_the_exponent_range(mesh):
+    """Denormal charges, and denormal potentials, are rounded to whole units of 2^-1074
+    and not dropped.  Cells of metres keep the spectrum's values near the charges' own
+    2^-1040, which have 34 bits left, and the potentials' below 2^-1029 at 45: 2^-28 of the same
+    charges in range (numpy's transforms: 5e-13)."""
+    sc = SpaceCharge(nmesh_xyz=mesh, precision="fp64")
+
+    def change(q, steps):
+        p, ref = np.asarray(sc.potential(q, steps)), np.asarray(sc.potential(np.ldexp(q, 1000), steps))
+        return np.linalg.norm(np.ldexp(p, 1000) - ref) / np.linalg.norm(ref), np.abs(p).max()
+
+    off, _ = change(np.ldexp(np.random.default_rng(3).random(mesh), -1040), (1.0, 2.0, 4.0))
+    assert off < 2.0 ** -28
+    off, top = change(np.ldexp(np.random.default_rng(4).random(mesh), -1015), (2.0 ** 60, 2.0 ** 60, 2.0 ** 61))
+    assert 0 < top < 2.0 ** -1022
+    assert off < 2.0 ** -28
