@@ -519,6 +519,8 @@ __device__ __forceinline__ void frame_finish(const double* acc, const KickParams
             st->kick_next = 0;  // the tile counter of this kick's gather + kick
             // the previous kick's outcome, kept before this kick resets the status
             if (prev != SC_OK && first == SC_OK) st->first_error = prev;
+            // a kick that stopped after its mesh has left no Green's function for it
+            if (prev != SC_OK) st->igf_h[0] = NAN;
             if (timeout) st->frame_timeout = 0;
             s_timeout = timeout;
         }
@@ -694,7 +696,8 @@ __device__ __forceinline__ void mesh_finish(const double* mn, const double* mx, 
         if (lane == 0) st->status = SC_ERR_DEGENERATE;
         return;
     }
-    const bool same = __all_sync(FULL, lane >= 3 || stepk == pre.igf_h);  // lane k < 3: axis k
+    // lane k < 3: axis k; pre.status: of the call before (el_field) or this kick's own
+    const bool same = pre.status == SC_OK && __all_sync(FULL, lane >= 3 || stepk == pre.igf_h);
     // near box of the hybrid Green's function along axis k (igf_box_of)
     int bk = v >= (double)nmk ? nmk : (int)ceil(v) + 1;
     if (bk > nmk) bk = nmk;
@@ -1422,6 +1425,7 @@ __global__ void __launch_bounds__(PT) k_extent_xyz(double* __restrict__ Xin, con
 // potential entry: explicit spacing
 __global__ void k_set_mesh(ScState* st, double hx, double hy, double hz, KickParams kp) {
     pdl_wait();
+    const bool ok = st->status == SC_OK;  // else the call before may not have made its Green's function
     st->status = SC_OK;
     st->steps[0] = hx;
     st->steps[1] = hy;
@@ -1440,7 +1444,7 @@ __global__ void k_set_mesh(ScState* st, double hx, double hy, double hz, KickPar
     st->igf_line = igf_line_of(h);
     st->igf_tbox[0] = igf_tbox_of(h, 0, kp.nx);
     st->igf_tbox[1] = igf_tbox_of(h, 1, kp.ny);
-    const bool same = hx == st->igf_h[0] && hy == st->igf_h[1] && hz == st->igf_h[2];
+    const bool same = ok && hx == st->igf_h[0] && hy == st->igf_h[1] && hz == st->igf_h[2];
     st->igf_rebuild = same ? 0 : 1;
     st->igf_next = 0;
     st->igf_h[0] = hx;
