@@ -62,30 +62,28 @@ def _sigma(tws) -> np.ndarray:
                      [tws.xpy, tws.ypy, tws.pxpy, tws.pypy]])
 
 
-def _set_eigen_emittances(twiss) -> None:
-    """The eigen-emittances of several Twiss, their eigenvalues taken in one call."""
-    sigma = [(t, _sigma(t)) for t in twiss]
-    good = [(t, m @ _S4) for t, m in sigma if np.isfinite(m).all()]
-    for t, _ in sigma:
-        t.eigemit_1 = t.eigemit_2 = float("nan")
-    if not good:
-        return
-    w = np.sort(np.abs(np.linalg.eigvals(np.stack([m for _, m in good])).imag), axis=1)
-    for (t, _), v in zip(good, w):  # v = [e2, e2, e1, e1]
-        t.eigemit_1, t.eigemit_2 = float(0.5 * (v[2] + v[3])), float(0.5 * (v[0] + v[1]))
+def _eigen_emittances(twiss) -> list:
+    """(eigemit_1, eigemit_2) of several Twiss-like objects, their eigenvalues taken in one call."""
+    sigma = [_sigma(t) for t in twiss]
+    good = [k for k, m in enumerate(sigma) if np.isfinite(m).all()]
+    out = [(float("nan"), float("nan"))] * len(sigma)
+    if good:
+        w = np.sort(np.abs(np.linalg.eigvals(np.stack([sigma[k] @ _S4 for k in good])).imag), axis=1)
+        for k, v in zip(good, w):  # v = [e2, e2, e1, e1]
+            out[k] = float(0.5 * (v[2] + v[3])), float(0.5 * (v[0] + v[1]))
+    return out
 
 
 def eigen_emittances(tws) -> tuple[float, float]:
-    t = Twiss()
-    t.__dict__.update(tws.__dict__)
-    _set_eigen_emittances([t])
-    return t.eigemit_1, t.eigemit_2
+    return _eigen_emittances([tws])[0]
 
 
 def twiss_table(moments, energies, charge: float, at) -> list:
     """Twiss of every slot of the sc_moments table at energies[k] and s = at[k]."""
     out = [_twiss(m, E, charge, s) for m, E, s in zip(moments, energies, at)]
-    _set_eigen_emittances([t for m, t in zip(moments, out) if m[0] >= 3])
+    many = [t for m, t in zip(moments, out) if m[0] >= 3]
+    for t, e in zip(many, _eigen_emittances(many)):
+        t.eigemit_1, t.eigemit_2 = e
     return out
 
 
@@ -95,7 +93,7 @@ def twiss_from_moments(m, energy: float, charge: float, s: float = 0.0) -> Twiss
     m = np.asarray(m, dtype=np.float64)
     tws = _twiss(m, energy, charge, s)
     if m[0] >= 3:
-        _set_eigen_emittances([tws])
+        tws.eigemit_1, tws.eigemit_2 = eigen_emittances(tws)
     return tws
 
 
