@@ -126,3 +126,40 @@ def test_cells_of_an_off_axis_beam_on_faces(precision):
     sc.check()
     keys = sc.engine().region("keys")[:rp.shape[1]].cpu().numpy().astype(np.int64)
     assert np.array_equal(keys, rec["keys"])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_mirrored_beam_up_to_the_tie_of_its_mesh(precision, monkeypatch):
+    """A beam symmetric about the axis has a mean of ~0 and extremes at whole grid
+    coordinates: rounding decides on which of two cells the mesh starts, and on which
+    side of a face the extremes lie.  Against the oracle on the device's choice of
+    these, the cells have to be the oracle's (within 1e-11 of a face either side's)
+    and the FP64 kick as near as for any other beam."""
+    n = 20_000
+    rp, q = _beam("mirrored", n)
+    rec = {}
+    sc_oracle.sc_apply(rp.copy(), q, 0.130, 0.1, MESH, record=rec)
+    d = torch.from_numpy(rp).to(DEV)
+    sc = SpaceCharge(nmesh_xyz=MESH, precision=precision, device=DEV)
+    sc.apply_device(d, torch.from_numpy(q).to(DEV), 0.130, 0.1)
+    sc.check()
+    keys = sc.engine().region("keys")[:n].cpu().numpy().astype(np.int64)
+    cells = np.stack([keys // (MESH[1] * MESH[2]), keys // MESH[2] % MESH[1], keys % MESH[2]], axis=1)
+    start = np.rint(np.median(cells - np.floor(rec["X"]) - 1, axis=0))
+    assert np.abs(start).max() <= 1
+    X = rec["X"] + start
+    side = cells - np.floor(X) - 1
+    assert np.abs(side).max() <= 1
+    assert (np.abs(X - np.rint(X))[side != 0] < 1e-11).all()
+    assert (side == 0).all(axis=1).mean() > 0.99
+    if precision == "fp64":
+        geometry = sc_oracle.mesh_geometry
+        monkeypatch.setattr(sc_oracle, "mesh_geometry", lambda *a, **k: (geometry(*a, **k)[0] + start, rec["steps"]))
+        monkeypatch.setattr(sc_oracle, "ngp_keys", lambda *a: keys)
+        ref = rp.copy()
+        sc_oracle.sc_apply(ref, q, 0.130, 0.1, MESH)
+        out = d.cpu().numpy()
+        assert max(np.linalg.norm(out[r] - ref[r]) / np.linalg.norm(ref[r]) for r in range(6)) < 1e-10
+        for r in (1, 3, 5):
+            k = ref[r] - rp[r]
+            assert np.linalg.norm(out[r] - ref[r]) < 5e-9 * np.linalg.norm(k), r
