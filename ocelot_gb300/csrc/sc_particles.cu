@@ -873,20 +873,8 @@ __global__ void __launch_bounds__(PT) k_frame64(const double* __restrict__ rp, c
     if (arrive_last(&st->done_frame, gridDim.x)) frame_finalize64(part, gridDim.x, kp, st);
 }
 
-// Pair-wise particle loop of the FP32 kernels: with VEC each thread takes two
-// adjacent particles and moves every row with one 16-byte access (rows
-// 16-byte aligned, even row stride); an odd last particle is taken alone.
-// The loop strides over the blocks of the beam (vb), not of the launch.
-#define PAIR_LOOP_BEGIN(n)                                                                        \
-    const int64_t npair_ = VEC ? (n) / 2 : (n);                                                   \
-    const int64_t ntot_ = npair_ + ((VEC && ((n) & 1)) ? 1 : 0);                                  \
-    for (int64_t p_ = vb.x * (int64_t)blockDim.x + threadIdx.x; p_ < ntot_;                       \
-         p_ += (int64_t)vb.nx * blockDim.x) {                                                     \
-        const bool pair_ = VEC && p_ < npair_;                                                    \
-        const int64_t i0_ = pair_ ? 2 * p_ : (VEC ? (n) - 1 : p_);                                \
-        const int W_ = pair_ ? 2 : 1;
-#define PAIR_LOOP_END }
-
+// One or two adjacent particles of a row (pair: one 16-byte access, the row 16-byte
+// aligned and i even).
 __device__ __forceinline__ void ld_row(const double* __restrict__ row, int64_t i, bool pair, double& a, double& b) {
     if (pair) {
         const double2 v = __ldg(reinterpret_cast<const double2*>(row + i));
@@ -896,10 +884,6 @@ __device__ __forceinline__ void ld_row(const double* __restrict__ row, int64_t i
         a = row[i];
         b = 0.0;
     }
-}
-__device__ __forceinline__ void st_row(double* __restrict__ row, int64_t i, bool pair, double a, double b) {
-    if (pair) *reinterpret_cast<double2*>(row + i) = make_double2(a, b);
-    else row[i] = a;
 }
 __device__ __forceinline__ void ld_rowf(const float* __restrict__ row, int64_t i, bool pair, float& a, float& b) {
     if (pair) {
@@ -954,7 +938,6 @@ struct FrameSums32 {
 
 // qzero != nullptr: the beam's blocks also clear its fixed-point charge grid
 // of nzero cells for the deposit of this kick
-template <bool VEC>
 __device__ __forceinline__ void frame32_body(const double* __restrict__ rp, const double* __restrict__ q,
                                              const KickParams& kp, float* __restrict__ X, double* __restrict__ part,
                                              ScState* st, unsigned long long* __restrict__ qzero, int64_t nzero,
@@ -964,27 +947,22 @@ __device__ __forceinline__ void frame32_body(const double* __restrict__ rp, cons
             qzero[i] = 0ull;
     FrameSums32 S;
     const int64_t n = kp.n, ld = kp.ld, nX = kp.nX;
-    PAIR_LOOP_BEGIN(n)
-    float f[2][7], l[2][3];
-    for (int k = 0; k < 7; ++k) {
-        double a, b;
-        ld_row(k < 6 ? rp + k * ld : q, i0_, pair_, a, b);
-        f[0][k] = d2f(a);
-        f[1][k] = d2f(b);
+    for (int64_t i = vb.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)vb.nx * blockDim.x) {
+        float f[7], l[3];
+        for (int k = 0; k < 6; ++k) f[k] = d2f(rp[k * ld + i]);
+        f[6] = d2f(q[i]);
+        S.add(f, kp, l);
+        for (int j = 0; j < 3; ++j) X[j * nX + i] = l[j];
     }
-    for (int w = 0; w < W_; ++w) S.add(f[w], kp, l[w]);
-    for (int j = 0; j < 3; ++j) st_rowf(X + j * nX, i0_, pair_, l[0][j], l[1][j]);
-    PAIR_LOOP_END
     S.out(reinterpret_cast<FramePart32*>(part), kp, st, vb);
 }
 
-template <bool VEC>
 __global__ void __launch_bounds__(PT, 3) k_frame32(const double* __restrict__ rp, const double* __restrict__ q,
                                                    KickParams kp, float* __restrict__ X, double* __restrict__ part,
                                                    ScState* st, unsigned long long* __restrict__ qzero,
                                                    int64_t nzero) {
     pdl_wait();
-    frame32_body<VEC>(rp, q, kp, X, part, st, qzero, nzero, hw_vblk());
+    frame32_body(rp, q, kp, X, part, st, qzero, nzero, hw_vblk());
 }
 
 // frame32_body with the six rows and the charges streamed through shared
@@ -1615,9 +1593,10 @@ __device__ __forceinline__ void keys32_body(float* __restrict__ X, uint32_t* __r
     const float ig0 = st->ig0f, g0 = st->g0f;
     const int S = st->qfix_shift;
     bool bad = false;
-    // the pair loop of PAIR_LOOP_BEGIN, KG pairs per thread per round: the
-    // loads of all KG pairs are issued before the first is processed, so a
-    // thread keeps KG times the bytes in flight
+    // With VEC a thread takes two adjacent particles (an odd last one alone), KG
+    // pairs per round: the loads of all KG pairs are issued before the first is
+    // processed, so a thread keeps KG times the bytes in flight.  The loop strides
+    // over the blocks of the beam (vb), not of the launch.
     constexpr int KG = 2;
     const int64_t npair_ = VEC ? n / 2 : n;
     const int64_t ntot_ = npair_ + ((VEC && (n & 1)) ? 1 : 0);
@@ -2502,7 +2481,7 @@ __global__ void __launch_bounds__(PT, 3) kb_frame32(const BatchBeam* __restrict_
     unsigned long long* qz = reinterpret_cast<unsigned long long*>(B.ws + B.L.qfix);
     const int64_t nc = (int64_t)B.p.nx * B.p.ny * B.p.nz;
     if (B.vec_rpq) frame32_tma_body(B.rp, B.q, B.kp, X, part, st, qz, nc, vb);
-    else frame32_body<false>(B.rp, B.q, B.kp, X, part, st, qz, nc, vb);
+    else frame32_body(B.rp, B.q, B.kp, X, part, st, qz, nc, vb);
 }
 
 __global__ void __launch_bounds__(PT, 3) kb_extent32(const BatchBeam* __restrict__ beams,
@@ -2667,7 +2646,7 @@ cudaError_t launch_frame(const Plan& p, const Layout& L, char* ws, const KickPar
         const int64_t nz = qz ? (int64_t)p.nx * p.ny * p.nz : 0;
         float* X = reinterpret_cast<float*>(ws + L.X);
         vec_ok(rp, kp.ld, q) ? launch(k_frame32_tma, nb, PT, FR_SMEM, s, rp, q, kp, X, part, st, qz, nz)
-                             : launch(k_frame32<false>, nb, PT, 0, s, rp, q, kp, X, part, st, qz, nz);
+                             : launch(k_frame32, nb, PT, 0, s, rp, q, kp, X, part, st, qz, nz);
     }
     return cudaGetLastError();
 }
