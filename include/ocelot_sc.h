@@ -367,11 +367,12 @@ int sc_kick_launches(const sc_plan* plan);
  *     particle (SC_REGION_FIELD), for error measurements; the FP32 form then
  *     runs its direct-access kick loop (same arithmetic, same particles). */
 #define SC_PARAM_RECORD_FIELD 1
-/*   SC_PARAM_FFT_PLANE_FWD / SC_PARAM_FFT_PLANE_INV: 1 (default) runs the z
- *     and y transforms of one x plane in one block where the plane fits
- *     shared memory (one launch per direction, 64 blocks on a 64^3 mesh); 0
- *     runs them as separate passes of many smaller blocks.  The lines go
- *     through the same transform code either way: identical results. */
+/*   SC_PARAM_FFT_PLANE_FWD / SC_PARAM_FFT_PLANE_INV: 1 runs the z and y
+ *     transforms of one x plane in one block where the plane fits shared
+ *     memory (one launch per direction, nx blocks); 0 runs them as separate
+ *     passes of many smaller blocks.  Identical results.  Defaults: FP64 0;
+ *     FP32 forward 1, inverse 1 while its blocks (nx, three times as many
+ *     with spectral fields) are no more than the GPU's SMs. */
 #define SC_PARAM_FFT_PLANE_FWD 2
 #define SC_PARAM_FFT_PLANE_INV 3
 /*   SC_PARAM_FFT_COLS_X / SC_PARAM_FFT_COLS_Y: lines (columns of the work
@@ -379,7 +380,9 @@ int sc_kick_launches(const sc_plan* plan);
  *     16, or 0 (default) for as many as fit, up to 16.  Fewer columns per
  *     block take less shared memory, so more blocks share an SM.  The lines
  *     are independent: identical results.  A batched kick also caps them so
- *     that four blocks share an SM. */
+ *     that four blocks share an SM.  FP64 lines of 64 to 256 points always
+ *     take 8 (accepted there, without effect); FP32 blocks of such lines have
+ *     threads for 16. */
 #define SC_PARAM_FFT_COLS_X 4
 #define SC_PARAM_FFT_COLS_Y 5
 #define SC_KICK_NVARIANTS 21
@@ -389,9 +392,9 @@ int sc_plan_get_param(const sc_plan* plan, int param, int* value);
  * kick variant. */
 int sc_kick_variant(int variant, int* tile, int* stages, int* particles_per_thread, int* blocks_per_sm);
 
-/* Failure detection of the bulk-copy waits.  The frame, extent and kick
- * kernels of the FP32 form stream particle rows through shared memory with
- * bulk copies and wait for each on an mbarrier with an iteration limit
+/* Failure detection of the bulk-copy waits.  The frame and kick kernels of
+ * the FP32 form and the extent kernel of both stream particle rows through
+ * shared memory with bulk copies and wait for each on an mbarrier with an iteration limit
  * (2^20 tries of about 1 us); a wait that runs out latches SC_ERR_TIMEOUT in
  * the workspace state, waits once more (full limit) for its copies still in
  * flight and returns, so the context stays usable and sc_read_status reports

@@ -222,8 +222,6 @@ cudaError_t launch_gather_xyz(const Plan& p, const Layout& L, char* ws, const Ki
 size_t sort_scratch_bytes(int64_t n, int key_bits);
 int sort_blocks(int64_t n);  // blocks of a sort of n keys (rows of its digit histogram)
 int sort_passes(int key_bits);
-// With q_src set, the last pass writes q_src[index] (as double or float) into
-// q_out instead of the permutation.
 cudaError_t launch_sort(const uint32_t* keys_in, int64_t n, int key_bits, uint32_t* keys_out, uint32_t* perm_out,
                         uint32_t* tmp_k, uint32_t* tmp_v, uint32_t* hist, uint32_t* tot, cudaStream_t s);
 // the kick's keys, the charges (as R) travelling with them
@@ -394,8 +392,8 @@ inline cudaError_t set_smem(K kernel, size_t bytes) {
 // Asks for an SM's whole shared memory beside this kernel.  A kernel that uses
 // little of it otherwise runs on an SM split in favour of L1, and a kernel of
 // the other stream that needs more shared memory than that split leaves waits
-// until the SM has drained: the radix scatter (18 KB a block) beside the Green's
-// function corners, for as long as those run.
+// until the SM has drained: the radix scatter (18 KB a block, 34 KB of FP64 charges in
+// tiles of 4096) beside the Green's function corners, for as long as those run.
 template <typename K>
 inline cudaError_t prefer_shared(K kernel) {
     return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributePreferredSharedMemoryCarveout,

@@ -42,7 +42,9 @@ static inline int z_lines_per_block(int Mz) {
     int nc = 1024 / Mz;
     return nc < 1 ? 1 : (nc > 8 ? 8 : nc);
 }
-// the fixed-point z passes: whole warps of two_step_q(Mz) threads a line
+// the fixed-point z passes: whole warps of two_step_q(Mz) threads a line.  Eight lines
+// a block against four, forward + inverse (us): 48^3 16.8 / 17.5, 63^3 25.0 / 24.9, 96^3
+// 51.7 / 54.9; at 256 points the other way, 100 x 100 x 120 94 / 89
 template <typename R>
 static inline int z_lines(int Mz) {
     const int nc = z_lines_per_block(Mz);

@@ -266,10 +266,7 @@ __device__ __forceinline__ Cx<R>* fft_two_step(Cx<R>* a, Cx<R>* b, int ls, int n
 }
 
 // fft_two_step for double lines (lg >= 0: line-fastest).  Each line's exponent and
-// table magnitude stand in the slot after its table.  The error against 80-bit
-// arithmetic, as a fraction of the double two-step form's (2-norm; random lines,
-// charge and spectrum shaped ones, spikes, 20 decades): 0.45 - 0.7 at 64 to 128
-// points, 0.47 - 0.9 at 192 and 256.
+// table magnitude stand in the slot after its table.
 template <bool INV, int L, bool HALF>
 __device__ __forceinline__ Cx<double>* fft_fx(Cx<double>* a, Cx<double>* b, int ls, int nl, int lg,
                                               const Cx<double>* tw2) {

@@ -9,7 +9,7 @@
 // What bounds them: issue slots of the integer pipes (about half of them the
 // conversions from and to double) and, at 64^3, one to two waves of blocks with
 // five barriers.  Measured, double two-step -> these, 63^3 (128-point lines):
-// x pass 82 -> 30 us, y forward 25 -> 12, y inverse 26 -> 10, z forward 16 -> 8,
+// x pass 82 -> 29 us, y forward 25 -> 12, y inverse 26 -> 10, z forward 16 -> 8,
 // z inverse 20.6 -> 14.3; the kick of 200k particles 400 -> 316 us.
 #pragma once
 #include "sc_fft_dev.cuh"
@@ -20,8 +20,9 @@ constexpr int FX_COLS = 8;
 // Threads of a block of lines: of the wider step's items (Q per line) where there are
 // few lines (z and Green passes, 2000 at 63^3: a round more would be exposed), of
 // the narrower one's (P) in the x and y passes, where enough blocks stand beside
-// each other and no warp should idle in the narrower step (x pass 31 -> 27 us, y
-// 12 -> 9.6 and 10 -> 8.9, but Green passes 6.5 -> 9)
+// each other and no warp should idle in the narrower step (x pass 31 -> 27 us, 29
+// with its Green products under their own exponents, y 12 -> 9.6 and 10 -> 8.9, but Green
+// passes 6.5 -> 9)
 constexpr int fx_threads(int L) { return FX_COLS * two_step_q(L); }
 constexpr int fx_threads_xy(int L) { return two_step_q(L) ? FX_COLS * (L / two_step_q(L)) : 0; }
 // table of a line (odd stride), and dynamic shared memory of a pass over n lines

@@ -8,13 +8,15 @@
 // FP64 pipe (2200 instructions) and about 6e3 in integers, with the conversions
 // to and from double another 5e3.
 //
-// Precision: a line is scaled so that its largest component takes bits 52 to 55
-// (the rest up to bit 62 is room for the transform's growth), so every input is rounded
-// at 2^-53 .. 2^-55 of the line's largest value, and every product at 2^-62 of the line's bound;
-// additions are exact.  Against a double transform, whose every operation
-// rounds at 2^-53 of its own result, the error in the 2-norm is the smaller one
-// (measured beside fft_fx).  As with any FFT the error is
-// one of the line's norm, not of each value.
+// Precision: a line is scaled so that its largest component has its leading one in
+// bit 56, 57 or 58 (fx_bit; the rest up to bit 61 is room for the transform's growth),
+// so every input is rounded at half a unit, 2^-57 .. 2^-59 of that power of two, and a
+// product leaves out up to two units; additions are exact.  Against a double transform, whose
+// every operation rounds at 2^-53 of its own result, the error in the 2-norm is the
+// smaller one: 0.31 to 0.78 of it for one transform, up to 0.99 for the x pass with its
+// Green product (tests/test_fixed_point_host.py: lines of every length, random, bunch
+// shaped, alternating, spikes, 20 decades).  As with any FFT the error is one of the
+// line's norm: a value 2^5 and more below the largest is held with less than 53 bits.
 //
 // A line with a NaN or an infinity comes out as NaNs (a double transform spreads
 // them over the line too).

@@ -1425,6 +1425,7 @@ __global__ void k_set_mesh(ScState* st, double hx, double hy, double hz, KickPar
     const bool same = ok && hx == st->igf_h[0] && hy == st->igf_h[1] && hz == st->igf_h[2];
     st->igf_rebuild = same ? 0 : 1;
     st->igf_next = 0;
+    st->phi_exp = 0;
     st->igf_h[0] = hx;
     st->igf_h[1] = hy;
     st->igf_h[2] = hz;

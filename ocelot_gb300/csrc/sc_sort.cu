@@ -225,8 +225,11 @@ __global__ void __launch_bounds__(RT) k_rscatter(const uint32_t* __restrict__ ki
 }
 
 // Rounds of RT keys per block: small sorts take one or four (more blocks in
-// parallel), large ones 16 (fewer digit-table rows for the scans).  The stable
-// order, and so the result, does not depend on the tiling.
+// parallel), large ones 16 (fewer digit-table rows for the scans, and runs that leave
+// in order).  The stable order, and so the result, does not depend on the tiling.
+// Both passes of a deposit's sort on 63^3 (us) with 1 / 4 / 16 rounds: 32k keys
+// 17.6 / 19.8 / 34.6, 64k 21.3 / 22.1 / 36.4, 128k 27.6 / 24.1 / 38.0, 256k 41.8 /
+// 27.3 / 39.6, 512k 71.8 / 41.6 / 39.1, 1M 126 / 70 / 56, 2M 233 / 114 / 86.
 static int sort_items(int64_t n) { return n <= (1 << 16) ? 1 : (n <= (1 << 19) ? 4 : RITEMS); }
 int sort_blocks(int64_t n) {
     const int64_t t = (int64_t)RT * sort_items(n);

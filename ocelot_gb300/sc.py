@@ -220,9 +220,9 @@ class Engine:
         return v.value
 
     def set_wait_limit(self, kernel: int = -1, tries: int = -1):
-        """Iteration limit of the bulk-copy waits of one FP32 kernel
-        (N.SC_WAIT_FRAME, _EXTENT, _KICK) or of all three (-1) for later
-        kicks; tries < 0 restores the default.  A wait that runs out latches
+        """Iteration limit of the bulk-copy waits of one kernel
+        (N.SC_WAIT_FRAME, _KICK: FP32; _EXTENT: both forms) or of all
+        three (-1) for later kicks; tries < 0 restores the default.  A wait that runs out latches
         SC_ERR_TIMEOUT (raised by ``check_status``) instead of spinning on."""
         N.check(self.lib.sc_plan_set_wait_limit(self.plan, int(kernel), int(tries)))
 
