@@ -1082,14 +1082,17 @@ __device__ __forceinline__ void xyz_fine(const double* __restrict__ rp, int64_t 
 // in FP64.  Only for the near-face particles of a keys block beyond the
 // KEYS_FINE that its list takes, inside the particle loop, where the FP64
 // transform's registers would slow every particle.
-// err (optional): a bound on |v - xyz_fine| per axis -- 2^-18 of each FP32
-// correction (a few roundings of ~2^-24 each, the approximate reciprocals'
-// ~2^-22, and margin) carried through the rotation, and 2^-46 of the lab
-// position for the FP64 roundings of the two evaluations (some 40 of 2^-53
-// together; those of 1 - 1/gamma^2 grow as 1/beta^2 = 1 + 1/(gamma beta)^2).
+// bound (optional): of the difference between the grid coordinates v / steps - xoff
+// here and with xyz_fine's v, per axis, in FP32 -- 2^-18 of each FP32 correction (a
+// few roundings of ~2^-24 each, the approximate reciprocals' ~2^-22, and margin)
+// carried through the rotation, 2^-46 of the lab position for the FP64 roundings of
+// the two evaluations (some 40 of 2^-53 together; those of 1 - 1/gamma^2 grow as
+// 1/beta^2 = 1 + 1/(gamma beta)^2), and as much of the offset and the mesh for those
+// of the quotient and the difference: a coordinate's last place is as large as the
+// beam is far off the axis.
 __device__ __forceinline__ void xyz_fine32(const double* __restrict__ rp, int64_t ld, int64_t i,
                                            const KickParams& kp, const double (&T)[3][3], double g0, double v[3],
-                                           double* err = nullptr) {
+                                           const ScState* st = nullptr, float* bound = nullptr) {
     const double x = rp[i], y = rp[2 * ld + i], tau = rp[4 * ld + i];
     float px, py, pz, E;
     mom32(d2f(rp[ld + i]), d2f(rp[3 * ld + i]), d2f(rp[5 * ld + i]), kp, px, py, pz, E);
@@ -1102,13 +1105,15 @@ __device__ __forceinline__ void xyz_fine32(const double* __restrict__ rp, int64_
     const double l2 = -tau + f2d(c2);
     for (int j = 0; j < 3; ++j) v[j] = fma(l2, T[2][j], fma(l1, T[1][j], l0 * T[0][j]));
     v[2] *= g0;
-    if (err) {
-        const double e0 = fabs((double)c0), e1 = fabs((double)c1), e2 = fabs((double)c2);
-        const float size = (fabsf(d2f(x)) + fabsf(d2f(y)) + fabsf(tf) + fabsf(c0) + fabsf(c1) + fabsf(c2)) *
-                           (1.0f + kp.igrbr2_f);
-        for (int j = 0; j < 3; ++j)
-            err[j] = (ldexp(fma(e2, fabs(T[2][j]), fma(e1, fabs(T[1][j]), e0 * fabs(T[0][j]))), -18) +
-                      f2d(size * 0x1p-46f)) * (j == 2 ? g0 : 1.0);
+    if (bound) {
+        const float e0 = fabsf(c0), e1 = fabsf(c1), e2 = fabsf(c2);
+        const float size = (fabsf(d2f(x)) + fabsf(d2f(y)) + fabsf(tf) + e0 + e1 + e2) * (1.0f + kp.igrbr2_f);
+        for (int j = 0; j < 3; ++j) {
+            const float rot = fmaf(e2, fabsf(st->Tf[2][j]), fmaf(e1, fabsf(st->Tf[1][j]), e0 * fabsf(st->Tf[0][j])));
+            const float err = fmaf(rot, 0x1p-18f, size * 0x1p-46f) * (j == 2 ? st->g0f : 1.0f);
+            const float off = fabsf(st->xofff[j]) + (float)(j == 0 ? kp.nx : j == 1 ? kp.ny : kp.nz);
+            bound[j] = fmaf(err, st->istepsf[j], off * 0x1p-46f) * 1.001f;
+        }
     }
 }
 
@@ -1527,23 +1532,20 @@ __device__ __forceinline__ long long to_fixed(double q, int S) {
 
 // NGP key of a near-face particle, equal to the FP64 form's: the grid
 // coordinate from the cheap estimate when every axis is farther from a face
-// than the estimate's error bound (plus 2^-46 of the offset and the mesh for
-// the FP64 roundings of the quotient and the difference, which are those of
-// a coordinate as large as the beam is far off the axis), else from the FP64
-// form's operations.  Returns false outside the mesh.
+// than the estimate's error bound, else from the FP64 form's operations.
+// Returns false outside the mesh.
 __device__ __forceinline__ bool key_fine(const double* __restrict__ rp, int64_t ld, int64_t i, const KickParams& kp,
                                          const ScState* st, uint32_t& key, float (&gf)[3]) {
     double T[3][3];
     for (int a = 0; a < 3; ++a)
         for (int b = 0; b < 3; ++b) T[a][b] = st->T[a][b];
-    double xv[3], err[3], g[3];
-    xyz_fine32(rp, ld, i, kp, T, st->gamma0, xv, err);
+    double xv[3], g[3];
+    float bound[3];
+    xyz_fine32(rp, ld, i, kp, T, st->gamma0, xv, st, bound);
     bool sure = true;
     for (int j = 0; j < 3; ++j) {  // the FP64 form's grid coordinate (k_keys64)
         g[j] = __dsub_rn(div_checked(xv[j], st->steps[j], st->isteps[j]), st->xoff[j]);
-        const double d = fabs(g[j] - rint(g[j]));
-        const float size = fabsf(st->xofff[j]) + (float)(j == 0 ? kp.nx : j == 1 ? kp.ny : kp.nz);
-        sure &= d > fma(err[j], st->isteps[j], f2d(size * 0x1p-46f));
+        sure &= fabs(g[j] - rint(g[j])) > f2d(bound[j]);
     }
     if (!sure) {
         xyz_fine(rp, ld, i, kp, T, st->gamma0, xv);
