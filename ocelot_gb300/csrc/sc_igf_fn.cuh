@@ -152,13 +152,13 @@ SC_HD double to_double(long long v, int s) {
 // near 1/m, r = m (1/c) - 1, exact in units of 2^-66, |r| < 2^-7.9, and
 // log x = k ln2 - log(1/c) + r - r^2 (1/2 - r/3 + r^2/4 - [r^3/5 - r^4/6 + r^5/7 - r^6/8 in FP32]),
 // in integers; the sum in units of 2^-56, 2^-58 or 2^-62, the finer ones for the smaller
-// results.  |x - 1| < 2^-8, where the result may be of any size, takes 1/c = 1: log x = r (1 - r (1/2 - ...)), r with all its bits.
+// results.  1 - 2^-8 <= x < 1 + 2^-8, where the result may be of any size, takes 1/c = 1: log x = r (1 - r (1/2 - ...)), r with all its bits.
 SC_HD double log_(double x, const LogEntry* __restrict__ tab) {
     const unsigned hx = hi_d(x);
     const int k = (int)(hx >> 20) - 1023;
     const LogEntry t = tab[(hx >> 13) & 127u];
-    const bool above = (hx >> 12) == (1023u << 8), below = (hx >> 13) == (1023u << 7) - 1u;
-    const unsigned ic = above ? 1u << 14 : (below ? 1u << 13 : (unsigned)t.ic);
+    const bool near1 = hx - 0x3fefe000u < 0x3000u;  // 1 - 2^-8 <= x < 1 + 2^-8: k is -1 or 0
+    const unsigned ic = near1 ? (1u << 14) >> (k & 1) : (unsigned)t.ic;
     const unsigned long long m = ((unsigned long long)((hx & 0xfffffu) | 0x100000u) << 32) | lo_d(x);
     const long long r = (long long)(m * (unsigned long long)ic);  // 2^-66; the 1 is 2^66, gone
     const long long r4 = (long long)((unsigned long long)r << 4);
@@ -167,20 +167,21 @@ SC_HD double log_(double x, const LogEntry* __restrict__ tab) {
     const float f = (rf * rf) * rf * fmaf(rf, fmaf(rf, fmaf(rf, -0.125f, 0.142857143f), -0.166666667f), 0.2f);
     const long long u = (1ll << 61) - (mulhi(r, 0x5555555555555555ll) >> 4) + (r2 >> 16) -
                         (long long)((unsigned long long)(long long)(int)(f * 0x1p50f) << 12);  // 2^-62
-    if (above || below) {
-        const long long sg = r >> 63;
-        const unsigned long long ur = (unsigned long long)((r ^ sg) - sg);
-        const int n = clz64(ur);                                  // 5 and more
-        const long long rn = (long long)(ur << ((n - 1) & 63));   // |r| 2^(65 + n)
-        const long long v = mulhi(rn, (1ll << 62) - ((mulhi(r4, u) + 32) >> 6));
-        return ur ? to_double((v ^ sg) - sg, 63 + n) : 0.0;
-    }
     const long long q = r - (mulhi(r2, u) >> 8);                                     // 2^-66
     const long long low = (((long long)k * LN2_LO + (1 << 25)) >> 26) + t.t + ((q + 8) >> 4);  // 2^-62
     // bits more than 2^-56: |log x| < 2 for k = -2 .. 1, < 2^5 for -40 .. 40
     const int sh = (unsigned)(k + 2) <= 3u ? 6 : ((unsigned)(k + 40) <= 80u ? 2 : 0);
-    const long long v = (long long)((unsigned long long)((long long)k * LN2_HI) << sh) + ((low + (32 >> sh)) >> (6 - sh));
-    return to_double(v, 56 + sh);
+    long long v = (long long)((unsigned long long)((long long)k * LN2_HI) << sh) + ((low + (32 >> sh)) >> (6 - sh));
+    int s = 56 + sh;
+    if (near1) {
+        const long long sg = r >> 63;
+        const unsigned long long ur = (unsigned long long)((r ^ sg) - sg);
+        const int n = clz64(ur);                                 // 5 and more
+        const long long rn = (long long)(ur << ((n - 1) & 63));  // |r| 2^(65 + n)
+        v = (mulhi(rn, (1ll << 62) - ((mulhi(r4, u) + 32) >> 6)) ^ sg) - sg;
+        s = 63 + n;
+    }
+    return to_double(v, s);
 }
 
 // w = |n| / |d| to FP32 accuracy, 2^-30 .. 2^30 (n, d normal)
