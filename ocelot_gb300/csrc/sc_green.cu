@@ -149,7 +149,7 @@ constexpr int IGF_SPLIT = IGF_THREADS / 6;  // corners per block per round in th
 // stored with the box's corner strides.
 // The whole octant (the exact table): one thread per corner, bound by the
 // FP64 pipe -- igf::point_, about 61 FP64 instructions where igf_point with
-// CUDA's functions has 226 (63^3 beside the other stream: 173 -> 54 us); igf_point stays
+// CUDA's functions has 226 (63^3 beside the other stream: 173 -> 56 us); igf_point stays
 // for steps that point_ does not cover.  The near box of the hybrid table has a few hundred corners, so
 // the time is the latency of one igf_point -- on this GPU's narrow FP64 pipe
 // some 20 us of dependent arithmetic through three arctangents and three

@@ -11,7 +11,7 @@
 // 113-bit arithmetic).
 // FP64 instructions: sqrt 7, log none, atan of a quotient 7 (10 and 20 in a form
 // with its series in FP64: 63^3 beside the other stream 75 -> 46 us at 10k
-// particles, 84 -> 54 at 200k).
+// particles, 84 -> 54 at 200k; 48 and 56 since the logarithm keeps its accuracy near 1).
 //
 // Arguments must be positive and inside 2^+-180 (igf_regular checks the mesh steps
 // once; others take the CUDA functions, igf_point).
